@@ -7,8 +7,7 @@
 #include <cstring>
 #include <stdexcept>
 
-#include "plain.cuh"
-#include "plain_static.cuh"
+#include "team.cuh"
 
 namespace pb {
 
@@ -21,68 +20,89 @@ namespace {
 
 inline size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// Exact row-store / record sizes of a static-band job; worst case for adaptive.
-void job_capacity(const HostWindow& w, int qlen, bool adaptive, int f, int wband, int64_t& rs_cap,
-                  int64_t& tb_cap, int& max_bn) {
+// Row-store blocks of a job (exact for the static band, the worst case for the
+// adaptive band) and the columns of its widest row.
+void job_capacity(const HostWindow& w, int qlen, bool adaptive, int f, int wband, int64_t& blocks, int& cols) {
     const int m = qlen + 1;
-    rs_cap = 0;
-    tb_cap = 0;
-    max_bn = 0;
+    blocks = 0;
+    cols = 8;
+    if (adaptive) {
+        // a row starts near 2 * wband columns and widens with the band state, up to the
+        // whole query; rows beyond the team's columns take more laps
+        blocks = (int64_t)w.n * (m / BLK + 1);
+        cols = (int)std::min<int64_t>((int64_t)(m / BLK + 1) * BLK, 6 * (int64_t)wband + STRIP);
+        return;
+    }
     for (int i = 0; i < w.n; i++) {
         int Bs, Be;
-        if (adaptive) {
-            Bs = 0;
-            Be = m / BLK + 2;
-        } else {
-            band_static(f, w.hq[i], w.tq[i], m, wband, Bs, Be);
-        }
+        band_static(f, w.hq[i], w.tq[i], m, wband, Bs, Be);
         if (i == 0) Bs = 0;
-        int bn = std::max(0, Be - Bs - 1);
-        int d = i == 0 ? 0 : w.in_ptr[i + 1] - w.in_ptr[i];
-        int bpc = d >= 2 ? 4 : 1;
-        rs_cap += (int64_t)bn * 16;
-        tb_cap += (int64_t)up16((size_t)bn * BLK * bpc);
-        max_bn = std::max(max_bn, bn);
+        const int bn = std::max(0, Be - Bs - 1);
+        blocks += bn;
+        cols = std::max(cols, ((Be - 2) / SBLK - Bs / SBLK + 1) * STRIP);
     }
-    rs_cap += 16;
-    tb_cap += 16;
 }
 
-template <int NT>
-void launch_plain(int njobs, const DpArgs* d_jobs, cudaStream_t s) {
-    k_plain<NT><<<njobs, NT, 0, s>>>(d_jobs);
+// A row's predecessor records in the backtrack's priority order (in_weight
+// descending, in-list position ascending; src/align.cpp:1601, 1637, 1708 keep
+// the first maximum), see TeamJob::ed.
+void pack_edges(const HostWindow& w, int4* ed) {
+    for (int r = 0; r < w.n; r++) {
+        const int e0 = w.in_ptr[r], d = w.in_ptr[r + 1] - e0;
+        int order[8];
+        std::vector<int> big;
+        int* o = order;
+        if (d > 8) {
+            big.resize(d);
+            o = big.data();
+        }
+        for (int k = 0; k < d; k++) {
+            int at = k;
+            while (at > 0 && w.in_w[e0 + o[at - 1]] < w.in_w[e0 + k]) {
+                o[at] = o[at - 1];
+                at--;
+            }
+            o[at] = k;
+        }
+        const int least = w.ind[r] / 10;
+        for (int k = 0; k < d; k++) {
+            const int e = e0 + o[k];
+            ed[e0 + k] = make_int4((w.in_row[e] << 4) | (w.in_w[e] >= least ? 8 : 0) | w.in_base[e], 0, 0, 0);
+        }
+    }
 }
 
-// Shared memory for the static kernel's row ring (below the 227 KB a block
-// may use, leaving part of the unified L1 for the read-only window arrays).
-// The adaptive kernel keeps its rows in global memory: a shared-memory ring
-// of a few full-width rows measured slower there (less L1 for the rest).
-constexpr int kRingBytes = 160 * 1024;
-constexpr int kRingMaxRows = 32;
-
-template <int NT>
-void launch_static(int njobs, const DpArgs* d_jobs, size_t dyn, cudaStream_t s) {
-    if (dyn > 48 * 1024)
-        cuda_check(cudaFuncSetAttribute(k_plain_static<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn),
-                   "smem attr (k_plain_static)");
-    k_plain_static<NT><<<njobs, NT, dyn, s>>>(d_jobs);
+template <int W, bool ADAPT, bool WIDE>
+void launch_team(int njobs, const TeamJob* d_jobs, cudaStream_t s) {
+    typedef TeamSmem<W, ADAPT, WIDE> S;
+    cuda_check(cudaFuncSetAttribute(k_align<W, ADAPT, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES),
+               "smem attr (k_align)");
+    k_align<W, ADAPT, WIDE><<<njobs, S::THREADS, S::BYTES, s>>>(d_jobs);
 }
 
-void launch_static_by_width(int max_bn, int njobs, const DpArgs* d_jobs, size_t dyn, cudaStream_t s) {
-    if (max_bn <= 64) launch_static<64>(njobs, d_jobs, dyn, s);
-    else if (max_bn <= 128) launch_static<128>(njobs, d_jobs, dyn, s);
-    else if (max_bn <= 192) launch_static<192>(njobs, d_jobs, dyn, s);
-    else if (max_bn <= 256) launch_static<256>(njobs, d_jobs, dyn, s);
-    else if (max_bn <= 384) launch_static<384>(njobs, d_jobs, dyn, s);
-    else launch_static<512>(njobs, d_jobs, dyn, s);
-}
-
-void launch_by_width(int max_bn, int njobs, const DpArgs* d_jobs, cudaStream_t s) {
-    if (max_bn <= 32) launch_plain<32>(njobs, d_jobs, s);
-    else if (max_bn <= 64) launch_plain<64>(njobs, d_jobs, s);
-    else if (max_bn <= 128) launch_plain<128>(njobs, d_jobs, s);
-    else if (max_bn <= 256) launch_plain<256>(njobs, d_jobs, s);
-    else launch_plain<512>(njobs, d_jobs, s);
+// One warp per 128 columns of the widest row, up to 16 (rows beyond that take
+// laps).
+void launch_teams(bool adaptive, bool wide, int cols, int njobs, const TeamJob* d, cudaStream_t s) {
+    const int strips = (cols + STRIP - 1) / STRIP;
+    if (wide) {
+        if (adaptive) launch_team<8, true, true>(njobs, d, s);
+        else launch_team<8, false, true>(njobs, d, s);
+    } else if (adaptive) {
+        if (strips <= 2) launch_team<2, true, false>(njobs, d, s);
+        else if (strips <= 4) launch_team<4, true, false>(njobs, d, s);
+        else if (strips <= 8) launch_team<8, true, false>(njobs, d, s);
+        else if (strips <= 12) launch_team<12, true, false>(njobs, d, s);
+        else launch_team<16, true, false>(njobs, d, s);
+    } else {
+        if (strips <= 2) launch_team<2, false, false>(njobs, d, s);
+        else if (strips <= 3) launch_team<3, false, false>(njobs, d, s);
+        else if (strips <= 4) launch_team<4, false, false>(njobs, d, s);
+        else if (strips <= 6) launch_team<6, false, false>(njobs, d, s);
+        else if (strips <= 8) launch_team<8, false, false>(njobs, d, s);
+        else if (strips <= 10) launch_team<10, false, false>(njobs, d, s);
+        else if (strips <= 12) launch_team<12, false, false>(njobs, d, s);
+        else launch_team<16, false, false>(njobs, d, s);
+    }
 }
 
 }  // namespace
@@ -134,48 +154,54 @@ void GpuEngine::align_many(const std::vector<const HostWindow*>& wins, const std
     const int J = (int)wins.size();
     outs.assign(J, AlignOut());
     if (J == 0) return;
+    // one launch runs one kind of band
+    bool any_adaptive = false, any_static = false;
+    for (int t = 0; t < J; t++) (p.f > 0 && abs[t] ? any_adaptive : any_static) = true;
+    if (any_adaptive && any_static) {
+        for (int t = 0; t < J; t++) {
+            std::vector<AlignOut> one;
+            align_many({wins[t]}, {qs[t]}, {qlens[t]}, {abs[t]}, p, one);
+            outs[t] = one[0];
+        }
+        return;
+    }
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     cudaStream_t s = (cudaStream_t)stream_;
     const Scoring sc = scoring_of(p);
 
     struct Lay {
-        size_t in_ptr, in_row, in_w, in_base, base, ind, hq, hq_loc, tq, out_ptr, out_row, qs;
-        size_t meta, state, rs, tb, res;
-        int64_t rs_cap, tb_cap;
+        size_t in_ptr, ed, hq, tq, ra, out_row, qs;
+        size_t rowi, fr, fe, state, store, res;
+        int64_t blocks;
         int32_t moves_cap;
         int w;
     };
     std::vector<Lay> L(J);
-    size_t up = up16(sizeof(DpArgs) * J);
-    int max_bn_all = 1;
-    bool any_adaptive = false;
+    size_t up = up16(sizeof(TeamJob) * J);
+    int cols = 8;
+    bool wide = false;
     for (int t = 0; t < J; t++) {
         const HostWindow& w = *wins[t];
-        const int n = w.n, E = (int)w.in_row.size(), E2 = (int)w.out_row.size();
+        const size_t n = (size_t)w.n, E = w.in_row.size();
         Lay& l = L[t];
         const int m = qlens[t] + 1;
         l.w = p.b + (p.f ? m / p.f : 0);
-        l.in_ptr = up; up += up16(4 * (size_t)(n + 1));
-        l.in_row = up; up += up16(4 * (size_t)E);
-        l.in_w = up; up += up16(4 * (size_t)E);
-        l.in_base = up; up += up16((size_t)E);
-        l.base = up; up += up16((size_t)n);
-        l.ind = up; up += up16(4 * (size_t)n);
-        l.hq = up; up += up16(4 * (size_t)n);
-        l.hq_loc = up; up += up16(4 * (size_t)n);
-        l.tq = up; up += up16(4 * (size_t)n);
-        l.out_ptr = up; up += up16(4 * (size_t)(n + 1));
-        l.out_row = up; up += up16(4 * (size_t)E2);
+        l.in_ptr = up; up += up16(4 * (n + 1));
+        l.ed = up; up += up16(16 * E);
+        l.hq = l.tq = l.ra = l.out_row = up;
+        if (any_adaptive) {
+            l.ra = up; up += up16(32 * n);
+            l.out_row = up; up += up16(4 * E);
+        } else {
+            l.hq = up; up += up16(4 * n);
+            l.tq = up; up += up16(4 * n);
+        }
         l.qs = up; up += up16((size_t)qs_bytes(qlens[t]));
-        const bool adaptive = p.f > 0 && abs[t];
-        int max_bn;
-        job_capacity(w, qlens[t], adaptive, p.f, l.w, l.rs_cap, l.tb_cap, max_bn);
-        // the CTA covers the widest row in one chunk (up to 512 threads): an
-        // adaptive row can widen to the full query (max_bn = m/8 + 2), and
-        // idle threads cost less than extra chunks, each a serial scan step
-        max_bn_all = std::max(max_bn_all, max_bn);
-        any_adaptive = any_adaptive || adaptive;
-        l.moves_cap = n + m + 8;
+        int c;
+        job_capacity(w, qlens[t], any_adaptive, p.f, l.w, l.blocks, c);
+        cols = std::max(cols, c);
+        wide = wide || !cell_packable(sc, w.n, m);
+        l.moves_cap = w.n + m + 8;
     }
     size_t res_begin = up;
     size_t pos = up;
@@ -185,73 +211,57 @@ void GpuEngine::align_many(const std::vector<const HostWindow*>& wins, const std
     }
     size_t res_end = pos;
     for (int t = 0; t < J; t++) {
-        const int n = wins[t]->n;
-        L[t].meta = pos; pos += up16(sizeof(RowMeta) * (size_t)n);
-        L[t].state = pos; pos += up16(4 * (size_t)AB_NSTATE * n);
-        L[t].rs = pos; pos += up16(4 * (size_t)L[t].rs_cap);
-        L[t].tb = pos; pos += up16((size_t)L[t].tb_cap);
+        const size_t n = (size_t)wins[t]->n;
+        L[t].rowi = pos; pos += 16 * n;
+        L[t].fr = pos; pos += any_adaptive ? 0 : 16 * n;
+        L[t].fe = pos; pos += 16 * wins[t]->in_row.size();
+        L[t].state = pos; pos += any_adaptive ? 32 * n : 0;
+        L[t].store = pos; pos += up16((size_t)L[t].blocks * BLK * (wide ? 8 : 4));
     }
     reserve_device(pos);
     reserve_host(res_end);
 
-    // static bands only: k_plain_static with a shared-memory ring of recent rows
-    int ring_rows = 0;
-    if (!any_adaptive) {
-        ring_rows = std::min(kRingMaxRows, kRingBytes / (max_bn_all * 64));
-        if (ring_rows < 2) ring_rows = 0;
-    }
-    const int ring_blocks = max_bn_all;
-    const size_t ring_bytes = (size_t)ring_rows * ring_blocks * 64;
-
     char* h = hbuf_;
     char* d = dbuf_;
-    DpArgs* jobs = reinterpret_cast<DpArgs*>(h);
+    TeamJob* jobs = reinterpret_cast<TeamJob*>(h);
     for (int t = 0; t < J; t++) {
         const HostWindow& w = *wins[t];
         const Lay& l = L[t];
-        auto cp = [&](size_t off, const void* src, size_t bytes) {
-            if (bytes) std::memcpy(h + off, src, bytes);
-        };
-        cp(l.in_ptr, w.in_ptr.data(), 4 * (size_t)(w.n + 1));
-        cp(l.in_row, w.in_row.data(), 4 * w.in_row.size());
-        cp(l.in_w, w.in_w.data(), 4 * w.in_w.size());
-        cp(l.in_base, w.in_base.data(), w.in_base.size());
-        cp(l.base, w.base.data(), (size_t)w.n);
-        cp(l.ind, w.ind.data(), 4 * (size_t)w.n);
-        cp(l.hq, w.hq.data(), 4 * (size_t)w.n);
-        cp(l.hq_loc, w.hq_loc.data(), 4 * (size_t)w.n);
-        cp(l.tq, w.tq.data(), 4 * (size_t)w.n);
-        cp(l.out_ptr, w.out_ptr.data(), 4 * (size_t)(w.n + 1));
-        cp(l.out_row, w.out_row.data(), 4 * w.out_row.size());
+        std::memcpy(h + l.in_ptr, w.in_ptr.data(), 4 * (size_t)(w.n + 1));
+        pack_edges(w, reinterpret_cast<int4*>(h + l.ed));
+        if (any_adaptive) {
+            int4* ra = reinterpret_cast<int4*>(h + l.ra);
+            for (int r = 0; r < w.n; r++) {
+                ra[2 * r] = make_int4(w.in_ptr[r], w.out_ptr[r], w.hq[r], w.tq[r]);
+                ra[2 * r + 1] = make_int4(w.hq_loc[r], w.base[r], w.in_ptr[r + 1] - w.in_ptr[r],
+                                          w.out_ptr[r + 1] - w.out_ptr[r]);
+            }
+            std::memcpy(h + l.out_row, w.out_row.data(), 4 * w.out_row.size());
+        } else {
+            std::memcpy(h + l.hq, w.hq.data(), 4 * (size_t)w.n);
+            std::memcpy(h + l.tq, w.tq.data(), 4 * (size_t)w.n);
+        }
         make_qs(qs[t], qlens[t], reinterpret_cast<uint8_t*>(h + l.qs));
-        DpArgs a;
+        TeamJob a;
         std::memset(&a, 0, sizeof(a));
-        a.v.n = w.n;
-        a.v.in_ptr = reinterpret_cast<const int32_t*>(d + l.in_ptr);
-        a.v.in_row = reinterpret_cast<const int32_t*>(d + l.in_row);
-        a.v.in_w = reinterpret_cast<const int32_t*>(d + l.in_w);
-        a.v.in_base = reinterpret_cast<const uint8_t*>(d + l.in_base);
-        a.v.base = reinterpret_cast<const uint8_t*>(d + l.base);
-        a.v.ind = reinterpret_cast<const int32_t*>(d + l.ind);
-        a.v.hq = reinterpret_cast<const int32_t*>(d + l.hq);
-        a.v.hq_loc = reinterpret_cast<const int32_t*>(d + l.hq_loc);
-        a.v.tq = reinterpret_cast<const int32_t*>(d + l.tq);
-        a.v.out_ptr = reinterpret_cast<const int32_t*>(d + l.out_ptr);
-        a.v.out_row = reinterpret_cast<const int32_t*>(d + l.out_row);
-        a.qs = reinterpret_cast<const uint8_t*>(d + l.qs);
+        a.n = w.n;
         a.qlen = qlens[t];
-        a.ab_band = abs[t];
         a.f = p.f;
         a.w = l.w;
-        a.sc = sc;
-        a.meta = reinterpret_cast<RowMeta*>(d + l.meta);
+        a.k = cell_consts(sc);
+        a.in_ptr = reinterpret_cast<const int32_t*>(d + l.in_ptr);
+        a.ed = reinterpret_cast<int4*>(d + l.ed);
+        a.hq = reinterpret_cast<const int32_t*>(d + l.hq);
+        a.tq = reinterpret_cast<const int32_t*>(d + l.tq);
+        a.ra = reinterpret_cast<const int4*>(d + l.ra);
+        a.out_row = reinterpret_cast<const int32_t*>(d + l.out_row);
+        a.qs = reinterpret_cast<const uint8_t*>(d + l.qs);
+        a.rowi = reinterpret_cast<int4*>(d + l.rowi);
+        a.fr = reinterpret_cast<int4*>(d + l.fr);
+        a.fe = reinterpret_cast<int4*>(d + l.fe);
         a.state = reinterpret_cast<int32_t*>(d + l.state);
-        a.rs = reinterpret_cast<int32_t*>(d + l.rs);
-        a.rs_cap = l.rs_cap;
-        a.tb = reinterpret_cast<uint8_t*>(d + l.tb);
-        a.tb_cap = l.tb_cap;
-        a.ring_rows = ring_rows;
-        a.ring_blocks = ring_rows > 0 ? ring_blocks : 0;
+        a.store = d + l.store;
+        a.store_cap = l.blocks;
         a.out = reinterpret_cast<int32_t*>(d + l.res);
         a.moves = reinterpret_cast<int32_t*>(d + l.res + 16);
         a.moves_cap = l.moves_cap;
@@ -259,9 +269,8 @@ void GpuEngine::align_many(const std::vector<const HostWindow*>& wins, const std
     }
     cuda_check(cudaMemcpyAsync(d, h, res_begin, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync(H2D)");
     if (timing) cuda_check(cudaEventRecord((cudaEvent_t)ev0_, s), "cudaEventRecord");
-    if (any_adaptive) launch_by_width(max_bn_all, J, reinterpret_cast<const DpArgs*>(d), s);
-    else launch_static_by_width(max_bn_all, J, reinterpret_cast<const DpArgs*>(d), ring_bytes, s);
-    cuda_check(cudaGetLastError(), "k_plain launch");
+    launch_teams(any_adaptive, wide, cols, J, reinterpret_cast<const TeamJob*>(d), s);
+    cuda_check(cudaGetLastError(), "k_align launch");
     if (timing) cuda_check(cudaEventRecord((cudaEvent_t)ev1_, s), "cudaEventRecord");
     cuda_check(cudaMemcpyAsync(h + res_begin, d + res_begin, res_end - res_begin, cudaMemcpyDeviceToHost, s),
                "cudaMemcpyAsync(D2H)");

@@ -1,0 +1,1184 @@
+// team.cuh - one banded POA alignment (one poa() call, src/align.cpp:1353-1737)
+// by a team of warps: the DP fill, then the backtrack over the stored values.
+//
+// What bounds it: an alignment is a chain of dependent rows (one per graph
+// rank), each only 30-200 blocks wide, so the time of one row step is the cost.
+// Evaluating the backtrack's comparisons for every cell (the record fill of
+// plain.cuh) made a row ~1,300 instructions per warp and ~4,300 cycles. Here
+// the fill stores values instead and the backtrack compares only the cells it
+// visits, which leaves ~15 integer operations per cell.
+//
+// Cells. A cell is stored as one 32-bit word, M << 8 | q, with
+//   q = max(0, g - (M - D)),  g = max(e1 - o1, 1):
+// the vertical term a successor takes is max(M + o1, D + e1) = M + o1 + q, and
+// M == D iff q == g. A D so far below M that q is 0 can neither win a
+// successor's maximum over M + o1 nor be a D the backtrack compares (it enters
+// a D cell only through M == D, or by an extension that beat M + o1), so the
+// word is an exact state, not an approximation. It needs |scores| < 2^20
+// (cell_packable), with NEG in place of NEG_INF: unreachable cells lie in
+// [NEG, NEG + 2^20], apart from every reachable value, and keep the
+// reference's order and differences among themselves. Alignments beyond that
+// range run the same code on {M, D} pairs (WIDE).
+//
+// Team. Columns are cut into strips of 128; strip s belongs to warp s % W, one
+// thread per 4 cells (half a block). A thread meets the same columns in every
+// row, so predecessor cells come back from the thread's own words in a
+// shared-memory ring of the last TR rows (16 or 32; 16 bytes per thread, no bank
+// conflicts) or, for rows further back, from the row store, and only the cell
+// left of a strip crosses warps. Per row: predecessor pass, warp prefix
+// maximum of the horizontal-gap keys, ONE barrier to exchange the warps'
+// maxima, finalise, store. The left neighbour's last cell is derived from its
+// published summary, so the next row does not wait for it to be stored.
+// Rows wider than the team's 128 * W columns take several laps.
+//
+// Adaptive band: row i + 1's band depends on row i's first maximum. The first
+// maximum of M is the first maximum of H0 = max(diagonal, vertical) (a gap
+// never exceeds the cell it opens from), so it is published with the same
+// barrier; an extra warp, which owns no columns, then updates the band state
+// and prepares the next row's header while the others finalise the row.
+//
+// Measured on a B200, DP kernels of one run, record fill -> this one: 10 reads
+// of 16,569 bp, static band, 346 -> 151 ms (fill 1,550 cycles per row of ~1,050
+// cells, backtrack 325 cycles per move); 24 reads of 443 bp 31 -> 12 ms; 10
+// reads of 5 kb at 10 % error, adaptive band, 308 -> 118 ms (2,900 cycles per
+// row). What is left is latency: ~230 dependent instructions per warp and row,
+// two cycles of each waiting on the instruction before it.
+#pragma once
+#include "plain.cuh"
+
+namespace pb {
+
+struct CellK {
+    int32_t match, mismatch, o1, e1;
+    int32_t gq;      // max(e1 - o1, 1)
+    uint32_t qmask;  // 255, or 0 when e1 == o1 (no extension beats a new gap)
+};
+
+PB_HD CellK cell_consts(const Scoring& s) {
+    CellK k;
+    k.match = s.match; k.mismatch = s.mismatch; k.o1 = s.o1; k.e1 = s.e1;
+    const int32_t g = s.e1 - s.o1;
+    k.gq = g > 1 ? g : 1;
+    k.qmask = g > 0 ? 255u : 0u;
+    return k;
+}
+
+// The packed cell holds every alignment of up to n rows and m columns.
+PB_HD bool cell_packable(const Scoring& s, int64_t n, int64_t m) {
+    int64_t big = 1;
+    const int64_t v[4] = {s.match, s.mismatch, s.o1, s.e1};
+    for (int k = 0; k < 4; k++) {
+        const int64_t a = v[k] < 0 ? -v[k] : v[k];
+        if (a > big) big = a;
+    }
+    return big < (1 << 20) && (n + m + 2) * big < (1 << 20) && (int64_t)s.e1 - s.o1 <= 255;
+}
+
+constexpr int32_t PACK_NEG = -(1 << 22);
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ int4 lds128(unsigned a) {
+    int4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ int32_t lds32(unsigned a) {
+    int32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts128(unsigned a, int4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+template <bool WIDE> struct Cells;
+
+template <> struct Cells<false> {
+    static constexpr int32_t NEG = PACK_NEG;
+    static constexpr int BYTES = 4;
+    int32_t c[4];
+    __device__ __forceinline__ void none() { c[0] = c[1] = c[2] = c[3] = NEG * 256; }
+    __device__ __forceinline__ void load(const void* p) {
+        const int4 v = *reinterpret_cast<const int4*>(p);
+        c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+    }
+    __device__ __forceinline__ void store(void* p) const {
+        *reinterpret_cast<int4*>(p) = make_int4(c[0], c[1], c[2], c[3]);
+    }
+    __device__ __forceinline__ void lds(unsigned a) {
+        const int4 v = lds128(a);
+        c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+    }
+    __device__ __forceinline__ void sts(unsigned a) const { sts128(a, make_int4(c[0], c[1], c[2], c[3])); }
+    static __device__ __forceinline__ int32_t lds_m(unsigned a) { return lds32(a) >> 8; }
+    static __device__ __forceinline__ int32_t load_m(const void* p) { return *reinterpret_cast<const int32_t*>(p) >> 8; }
+    __device__ __forceinline__ int32_t m(int l) const { return c[l] >> 8; }
+    // the vertical term max(M + o1, D + e1)
+    __device__ __forceinline__ int32_t v(int l, const CellK& k) const {
+        return (c[l] >> 8) + (int32_t)((uint32_t)c[l] & k.qmask) + k.o1;
+    }
+    __device__ __forceinline__ void set(int l, int32_t M, int32_t D, const CellK& k) {
+        c[l] = (int32_t)((uint32_t)M << 8) + mx(D - M + k.gq, 0);
+    }
+    // one cell of the row store, for the backtrack
+    struct One {
+        int32_t w;
+        static __device__ __forceinline__ One lds(unsigned a) { return One{lds32(a)}; }
+        __device__ __forceinline__ int32_t m() const { return w >> 8; }
+        __device__ __forceinline__ bool eq_md(const CellK& k) const { return (w & 255) == k.gq; }
+        __device__ __forceinline__ bool d_opens(int32_t d, const CellK& k) const { return m() + k.o1 == d; }
+        __device__ __forceinline__ bool d_extends(int32_t d, const CellK& k) const {
+            const int32_t q = (int32_t)((uint32_t)w & k.qmask);
+            return q > 0 && m() + k.o1 + q == d;
+        }
+    };
+};
+
+template <> struct Cells<true> {
+    static constexpr int32_t NEG = NEG_INF;
+    static constexpr int BYTES = 8;
+    int32_t M_[4], D_[4];
+    __device__ __forceinline__ void none() {
+#pragma unroll
+        for (int l = 0; l < 4; l++) M_[l] = D_[l] = NEG;
+    }
+    __device__ __forceinline__ void load(const void* p) {
+        const int4 a = reinterpret_cast<const int4*>(p)[0], b = reinterpret_cast<const int4*>(p)[1];
+        M_[0] = a.x; D_[0] = a.y; M_[1] = a.z; D_[1] = a.w;
+        M_[2] = b.x; D_[2] = b.y; M_[3] = b.z; D_[3] = b.w;
+    }
+    __device__ __forceinline__ void store(void* p) const {
+        reinterpret_cast<int4*>(p)[0] = make_int4(M_[0], D_[0], M_[1], D_[1]);
+        reinterpret_cast<int4*>(p)[1] = make_int4(M_[2], D_[2], M_[3], D_[3]);
+    }
+    __device__ __forceinline__ void lds(unsigned a) {
+        const int4 u = lds128(a), v = lds128(a + 16);
+        M_[0] = u.x; D_[0] = u.y; M_[1] = u.z; D_[1] = u.w;
+        M_[2] = v.x; D_[2] = v.y; M_[3] = v.z; D_[3] = v.w;
+    }
+    __device__ __forceinline__ void sts(unsigned a) const {
+        sts128(a, make_int4(M_[0], D_[0], M_[1], D_[1]));
+        sts128(a + 16, make_int4(M_[2], D_[2], M_[3], D_[3]));
+    }
+    static __device__ __forceinline__ int32_t lds_m(unsigned a) { return lds32(a); }
+    static __device__ __forceinline__ int32_t load_m(const void* p) { return *reinterpret_cast<const int32_t*>(p); }
+    __device__ __forceinline__ int32_t m(int l) const { return M_[l]; }
+    __device__ __forceinline__ int32_t v(int l, const CellK& k) const {
+        return mx(add32(M_[l], k.o1), add32(D_[l], k.e1));
+    }
+    __device__ __forceinline__ void set(int l, int32_t M, int32_t D, const CellK&) { M_[l] = M; D_[l] = D; }
+    struct One {
+        int32_t M, D;
+        static __device__ __forceinline__ One lds(unsigned a) { return One{lds32(a), lds32(a + 4)}; }
+        __device__ __forceinline__ int32_t m() const { return M; }
+        __device__ __forceinline__ bool eq_md(const CellK&) const { return M == D; }
+        __device__ __forceinline__ bool d_opens(int32_t d, const CellK& k) const { return add32(M, k.o1) == d; }
+        __device__ __forceinline__ bool d_extends(int32_t d, const CellK& k) const { return add32(D, k.e1) == d; }
+    };
+};
+
+// One alignment's rows and buffers (device pointers).
+struct TeamJob {
+    int32_t n, qlen, f, w;   // rows, query length, band parameters (w = b + m / f)
+    CellK k;
+    const int32_t* in_ptr;   // [n + 1] predecessors of each row
+    // [edges] in the backtrack's priority order (in_weight descending, in-list
+    // position ascending): x = predecessor row << 4 | (in_weight >= ind / 10) << 3
+    // | its base as the DP sees it; y, z, w = its band and row-store block,
+    // filled in here
+    int4* ed;
+    int4* fe;                // [edges] the same for the fill: {ring offset or -1, base in every byte, Bs, last block - Bs}
+    const int32_t *hq, *tq;  // [n] static band
+    const int4* ra;          // [2 n] adaptive band: {first in-edge, first out-edge, hq, tq}, {hq_loc, base, d, successors}
+    const int32_t* out_row;  // adaptive band: successor rows in out-list order
+    const uint8_t* qs;       // shifted query (dp_job.h)
+    int4* rowi;              // [n] {Bs, Be, row-store block, -}
+    int4* fr;                // [n] static band, for the fill: {Bs, last block - Bs, row-store block, d | flags | first record in the stage}
+    int32_t* state;          // [8 n] adaptive band state of rows outside the shared-memory window
+    char* store;             // cells, 8 per block
+    int64_t store_cap;       // blocks
+    int32_t* moves;
+    int32_t moves_cap;
+    int32_t* out;            // [0] status, [1] score, [2] moves, [3] cells
+};
+
+constexpr int TC = 4;           // cells per thread
+constexpr int STRIP = 32 * TC;  // columns per warp
+constexpr int SBLK = STRIP / BLK;
+constexpr int STG = 32;         // rows staged at a time (static band)
+constexpr int STG_E = 128;      // their predecessor records
+constexpr int HDR_E = 32;       // predecessor records in an adaptive row's header
+constexpr int SWIN = 256;       // rows of the adaptive state window (a power of two), half of them ahead
+constexpr int SW_INTS = 12;     // {Pl, Pr, Ol, Or, Ow, Sl, Mp, -, Bs, Be, tb, -}
+enum { SW_PL = 0, SW_PR, SW_OL, SW_OR, SW_OW, SW_SL, SW_MP, SW_BS = 8, SW_BE, SW_TB };
+// flags in a row header's last word: d in the low 10 bits
+enum { FR_D = 1023, FR_GENERAL = 1 << 10, FR_UNSTAGED = 1 << 11, FR_EOFF = 16 };
+
+struct TeamStage {
+    int4 row[STG];
+    int4 ed[STG_E];
+};
+struct TeamHdr {
+    int4 h;        // as TeamJob::fr
+    int4 g;        // {first in-edge, status, -, -}
+    int4 ed[HDR_E];
+};
+
+// Backtrack tile: BT_ROWS rows around the walk, BT_BLK blocks of each, their
+// rows and predecessor records (team_backtrack).
+constexpr int BT_ROWS = 64, BT_BLK = 8, BT_E = 160;
+
+template <bool WIDE>
+struct BtSmem {
+    static constexpr int ROWB = BT_BLK * BLK * Cells<WIDE>::BYTES;
+    static constexpr int CELLS = 0;
+    static constexpr int ROW = CELLS + BT_ROWS * ROWB;      // int4 {Bs, Be, store block, first block of the tile row}
+    static constexpr int PTR = ROW + BT_ROWS * 16;          // int [BT_ROWS + 1], padded
+    static constexpr int ED = PTR + (BT_ROWS + 4) * 4;
+    static constexpr int JUMP = ED + BT_E * 16;             // uint8 [5][BT_ROWS]: the tile row 1, 2, 4, 8, 16 heaviest predecessors back
+    static constexpr int BYTES = JUMP + 5 * BT_ROWS;
+};
+
+template <int W, bool ADAPT, bool WIDE>
+struct TeamSmem {
+    static constexpr int TR = W <= 6 && !WIDE ? 32 : 16;           // rows of the ring (a power of two)
+    static constexpr int CELLB = TC * Cells<WIDE>::BYTES;          // bytes per thread and row
+    static constexpr int ROWB = 32 * W * CELLB;
+    static constexpr int RING = TR * ROWB;
+    static constexpr int PUB = RING;                               // int4 [2][W]
+    static constexpr int BEST = PUB + 2 * W * 16;                  // int4 [2][W]
+    static constexpr int REST = BEST + 2 * W * 16;
+    static constexpr int FILL =
+        REST + (ADAPT ? 2 * (int)sizeof(TeamHdr) + SWIN * SW_INTS * 4 : 2 * (int)sizeof(TeamStage));
+    static constexpr int BYTES = FILL > BtSmem<WIDE>::BYTES ? FILL : BtSmem<WIDE>::BYTES;
+    static constexpr int THREADS = 32 * (W + (ADAPT ? 1 : 0));
+};
+
+// Named barriers: 1 the whole team, 2 the compute warps' maxima (they arrive,
+// the control warp waits), 3 the compute warps.
+template <int ID, int NT>
+__device__ __forceinline__ void bar_sync() { asm volatile("barrier.sync %0, %1;" ::"n"(ID), "n"(NT) : "memory"); }
+template <int ID, int NT>
+__device__ __forceinline__ void bar_arrive() { asm volatile("barrier.arrive %0, %1;" ::"n"(ID), "n"(NT) : "memory"); }
+
+// inclusive prefix maximum over the warp (a lane without a source gets its own
+// value back, which a maximum does not mind)
+__device__ __forceinline__ int32_t scan_max(int32_t v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) v = mx(v, __shfl_up_sync(0xffffffffu, v, o));
+    return v;
+}
+
+__device__ __forceinline__ int strips_of(int Bs, int Be) { return ((Be - 2) >> 4) - (Bs >> 4) + 1; }
+
+// Static band: every row's band and place in the row store, its header for
+// the fill, and each predecessor record's copy of its row's. Returns a status
+// (uniform).
+template <class S, int W, int NT>
+__device__ int team_rows_static(const TeamJob& a, int64_t* s_part, unsigned long long* s_fail, int64_t& cells) {
+    const int tid = threadIdx.x, n = a.n, m = a.qlen + 1;
+    if (tid == 0) *s_fail = ~0ull;
+    __syncthreads();
+    int64_t run = 0;
+    for (int r0 = 0; r0 < n; r0 += NT) {
+        const int i = r0 + tid;
+        int Bs = 0, Be = 1, d = 0;
+        if (i < n) {
+            band_static(a.f, a.hq[i], a.tq[i], m, a.w, Bs, Be);
+            if (i == 0) Bs = 0;
+            d = i == 0 ? 0 : a.in_ptr[i + 1] - a.in_ptr[i];
+        }
+        const int bn = Be - Bs - 1;
+        int64_t v = i < n && bn > 0 ? bn : 0, total;
+        // CTA-wide exclusive prefix sum
+        const int lane = tid & 31, wid = tid >> 5;
+        int64_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_part[wid] = x;
+        __syncthreads();
+        int64_t before = 0;
+        total = 0;
+        for (int k = 0; k < NT / 32; k++) {
+            const int64_t p = s_part[k];
+            if (k < wid) before += p;
+            total += p;
+        }
+        __syncthreads();
+        const int64_t off = run + before + x - v;
+        run += total;
+        if (i < n) {
+            int st = ST_OK;
+            if (bn < 0) st = ST_DEGENERATE;
+            else if (d > MAX_MULTI_PRED) st = ST_INDEGREE;
+            else if (off + bn > a.store_cap || off + bn > INT_MAX) st = ST_OOM;
+            if (st != ST_OK) atomicMin(s_fail, ((unsigned long long)i << 8) | (unsigned long long)st);
+            a.rowi[i] = make_int4(Bs, Be, (int)off, 0);
+        }
+    }
+    __syncthreads();
+    cells = run * BLK;
+    if (*s_fail != ~0ull) return (int)(*s_fail & 255ull);
+    for (int i = tid; i < n; i += NT) {
+        const int4 ri = a.rowi[i];
+        const int e0 = a.in_ptr[i], d = i == 0 ? 0 : a.in_ptr[i + 1] - e0;
+        const int eoff = e0 - a.in_ptr[i & ~(STG - 1)];
+        int fl = d;
+        if (i == 0 || ri.y - ri.x - 1 <= 0 || strips_of(ri.x, ri.y) > W) fl |= FR_GENERAL;
+        if (eoff + d > STG_E) fl |= FR_UNSTAGED;
+        else fl |= eoff << FR_EOFF;
+        a.fr[i] = make_int4(ri.x, ri.y - 2 - ri.x, ri.z, fl);
+        for (int e = e0; e < e0 + d; e++) {
+            int4 v = a.ed[e];
+            const int p = v.x >> 4;
+            const int4 pr = a.rowi[p];
+            v.y = pr.x; v.z = pr.y; v.w = pr.z;
+            a.ed[e] = v;
+            const bool near = i - p < S::TR && strips_of(pr.x, pr.y) <= W;
+            a.fe[e] = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : -1, (v.x & 7) * 0x01010101, pr.x, pr.y - 2 - pr.x);
+        }
+    }
+    __syncthreads();
+    return ST_OK;
+}
+
+template <int W>
+__device__ __forceinline__ void team_stage(const TeamJob& a, TeamStage& st, int i0) {
+    // rows [i0, i0 + STG) and their predecessor records, by the whole CTA
+    const int tid = threadIdx.x, n = a.n;
+    const int cnt = min(STG, n - i0);
+    if (cnt <= 0) return;
+    const int e0 = a.in_ptr[i0], ne = min(a.in_ptr[i0 + cnt] - e0, STG_E);
+    for (int x = tid; x < cnt; x += 32 * W) cp_async16(&st.row[x], a.fr + i0 + x);
+    for (int x = tid; x < ne; x += 32 * W) cp_async16(&st.ed[x], a.fe + e0 + x);
+    cp_async_commit_all();
+}
+
+// The fill of one row by a column-owning thread; see the file comment.
+template <int W, bool ADAPT, bool WIDE>
+struct TeamRow {
+    typedef Cells<WIDE> C;
+    typedef TeamSmem<W, ADAPT, WIDE> S;
+    static constexpr int32_t NEG = C::NEG;
+    static constexpr int32_t LOW = WIDE ? INT_MIN : -(1 << 30);
+    const TeamJob& a;
+    const CellK k;
+    char* const store;
+    const unsigned sb, own, leftw;  // shared memory: base, this thread's cells, the word left of them (within a ring row)
+    const int lane, wid;
+    const int32_t K;                // the gap term's floor: NEG_INF extended from column 0
+    int s_cur = INT_MIN / 2;        // this warp's strip
+    int col0 = 0, B = 0, Bz = 0;    // its first column, block (and that block, or a large value for block 0: no diagonal mask there)
+    uint32_t qw = 0;                // query codes of the thread's columns
+    int qn = 4;                     // code of the column after them (adaptive band)
+    int32_t edge = NEG;             // static band: M left of this warp's strip in the previous row
+    unsigned xp = 0;                // byte offset of the published summaries' half in use
+
+    __device__ TeamRow(char* sm, const TeamJob& job)
+        : a(job), k(job.k), store(job.store), sb((unsigned)__cvta_generic_to_shared(sm)),
+          own(threadIdx.x * S::CELLB), leftw((threadIdx.x == 0 ? 32 * W : threadIdx.x) * S::CELLB - C::BYTES),
+          lane(threadIdx.x & 31), wid(threadIdx.x >> 5), K(add32(add32(C::NEG, job.k.e1), -job.k.o1)) {}
+
+    __device__ __forceinline__ void take_strip(int s) {
+        s_cur = s;
+        col0 = s * STRIP + lane * TC;
+        B = col0 >> 3;
+        Bz = B == 0 ? INT_MAX : B;
+        const bool in = col0 + 8 <= (int)qs_bytes(a.qlen);
+        qw = in ? *reinterpret_cast<const uint32_t*>(a.qs + col0) : 0x04040404u;
+        if (ADAPT) qn = in ? a.qs[col0 + 4] : 4;
+    }
+
+    // One predecessor's terms. in: the block is in its band; src: cells; left: M of the cell before them.
+    __device__ __forceinline__ void fold(const C& pc, int32_t left, bool diag, uint32_t x, int32_t* P, int32_t* V) const {
+        // packed cells: a term pushed far below NEG drops out of the maximum
+        const int32_t sm = diag || WIDE ? k.match : -(1 << 23), sx = diag || WIDE ? k.mismatch : -(1 << 23);
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            const int32_t src = l == 0 ? left : pc.m(l > 0 ? l - 1 : 0);
+            const int32_t cand = src + ((x & (255u << (8 * l))) == 0 ? sm : sx);
+            if (!WIDE || diag) P[l] = mx(P[l], cand);
+            V[l] = mx(V[l], pc.v(l, k));
+        }
+    }
+
+    // prefix maximum within the warp and its summary; base: -(column in the row's band) * e1
+    __device__ __forceinline__ void publish(bool act, const int32_t* H, int32_t base, int32_t* key, int32_t& ex) const {
+        key[0] = H[0];
+        key[1] = H[1] - k.e1;
+        key[2] = H[2] - 2 * k.e1;
+        key[3] = H[3] - 3 * k.e1;
+        const int32_t k02 = mx(mx(key[0], key[1]), key[2]);
+        const int32_t incl = scan_max(act ? mx(k02, key[3]) + base : LOW);
+        ex = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) ex = LOW;
+        if (lane == 31)
+            sts128(sb + S::PUB + xp + wid * 16, make_int4(incl, act ? mx(ex, k02 + base) : ex, H[3], s_cur));
+    }
+    __device__ __forceinline__ void publish_none() const {
+        if (lane == 31) sts128(sb + S::PUB + xp + wid * 16, make_int4(LOW, LOW, NEG, INT_MAX));
+    }
+    // the row's first maximum so far in this warp: value, column, and the query code after that column
+    __device__ __forceinline__ void maximum(bool act, const int32_t* H, int4& best) const {
+        const int32_t lm = act ? mx(mx(H[0], H[1]), mx(H[2], H[3])) : INT_MIN;
+        const int32_t wm = __reduce_max_sync(0xffffffffu, lm);
+        if (wm > best.x) {
+            const int first = __ffs(__ballot_sync(0xffffffffu, lm == wm)) - 1;
+            const int l = H[0] == wm ? 0 : H[1] == wm ? 1 : H[2] == wm ? 2 : 3;
+            const int code = l == 3 ? qn : (int)((qw >> (8 * (l + 1))) & 255u);
+            const int v = __shfl_sync(0xffffffffu, (col0 + l) * 8 + code, first);
+            best = make_int4(wm, v >> 3, v & 7, 0);
+        }
+    }
+    __device__ __forceinline__ void put_maximum(const int4& best) const {
+        if (lane == 0) sts128(sb + S::BEST + xp + wid * 16, best);
+        __syncwarp();
+        bar_arrive<2, S::THREADS>();
+    }
+    __device__ __forceinline__ void finish(C& o, int i, const int32_t* H, const int32_t* V, const int32_t* key, int32_t run) const {
+        if (i == 0) {
+#pragma unroll
+            for (int l = 0; l < 4; l++) o.set(l, H[l], V[l], k);
+            return;
+        }
+        const int32_t g = k.o1 - k.e1;
+        o.set(0, mx(H[0], run + g), V[0], k);
+        run = mx(run, key[0]);
+        o.set(1, mx(H[1], run + (g + k.e1)), V[1], k);
+        run = mx(run, key[1]);
+        o.set(2, mx(H[2], run + (g + 2 * k.e1)), V[2], k);
+        run = mx(run, key[2]);
+        o.set(3, mx(H[3], run + (g + 3 * k.e1)), V[3], k);
+    }
+    __device__ __forceinline__ void sync_row() const {
+        if (ADAPT) bar_sync<3, 32 * W>();
+        else bar_sync<1, S::THREADS>();
+    }
+
+    // A row that fits the team's columns (i > 0). ed_at(e): fill record; far(e): its TeamJob::ed record.
+    template <class EdAt, class Far, class After>
+    __device__ __forceinline__ void row(int i, int4 h, EdAt ed_at, Far far, After after_barrier) {
+        const int Bs = h.x, span = h.y, d = h.w & FR_D;
+        const int S0 = Bs >> 4, S1 = (Bs + span) >> 4;
+        if ((unsigned)(s_cur - S0) >= (unsigned)W) {
+            int r = (wid - S0) % W;
+            take_strip(S0 + (r < 0 ? r + W : r));
+        }
+        const bool on = s_cur <= S1;
+        const int rel = col0 - Bs * BLK;
+        const bool act = on && (unsigned)(B - Bs) <= (unsigned)span;
+        const bool first = B == Bs && !(lane & 1);  // column 0 of the row's first block reads NEG_INF
+        int32_t P[4], V[4], H[4], key[4], ex = LOW, base = 0;
+        __syncwarp();
+        if (on) {
+#pragma unroll
+            for (int l = 0; l < 4; l++) P[l] = V[l] = NEG;
+            for (int e = 0; e < d; e++) {
+                const int4 er = ed_at(e);
+                const bool in = (unsigned)(B - er.z) <= (unsigned)er.w;
+                const bool diag = in && Bz > er.z;  // the fill's block mask for the diagonal (src/align.cpp:1467)
+                C pc;
+                int32_t left;
+                if (er.x >= 0) {
+                    pc.lds(sb + er.x + own);
+                    left = C::lds_m(sb + er.x + leftw);
+                    if (!ADAPT && lane == 0 && er.x == (int)(((i - 1) & (S::TR - 1)) * S::ROWB)) left = edge;
+                    if (!in) pc.none();
+                } else {
+                    const int4 fe = far(e);
+                    const char* src = store + ((int64_t)fe.w * BLK + (col0 - fe.y * BLK)) * C::BYTES;
+                    pc.none();
+                    left = NEG;
+                    if (in && act) {
+                        pc.load(src);
+                        if (B > fe.y || (lane & 1)) left = C::load_m(src - C::BYTES);
+                    }
+                }
+                if (first) left = NEG;
+                fold(pc, left, diag, qw ^ (uint32_t)er.y, P, V);
+            }
+#pragma unroll
+            for (int l = 0; l < 4; l++) H[l] = mx(P[l], V[l]);
+            if (ADAPT) {
+                int4 best = make_int4(INT_MIN, 0, 0, 0);
+                maximum(act, H, best);
+                put_maximum(best);
+            }
+            base = -rel * k.e1;
+            publish(act, H, base, key, ex);
+        } else {
+            if (ADAPT) put_maximum(make_int4(INT_MIN, 0, 0, 0));
+            publish_none();
+        }
+        sync_row();
+        after_barrier();
+        if (on) {
+            const int4 pv = lane < W ? lds128(sb + S::PUB + xp + lane * 16) : make_int4(LOW, LOW, NEG, INT_MAX);
+            const int4 L = lds128(sb + S::PUB + xp + (wid == 0 ? W - 1 : wid - 1) * 16);
+            const int32_t Pl = mx(K, __reduce_max_sync(0xffffffffu, pv.w < s_cur - 1 ? pv.x : LOW));
+            const bool hasl = s_cur > S0;
+            const int32_t Pr = hasl ? mx(Pl, L.x) : Pl;
+            if (!ADAPT && lane == 0) {
+                // M of the cell left of the strip, for the next row
+                const int32_t I = add32(k.o1 + (rel - 2) * k.e1, mx(Pl, L.y));
+                edge = mx(L.z, I);
+            }
+            if (act) {
+                C o;
+                finish(o, i, H, V, key, mx(Pr, ex) - base);
+                o.sts(sb + (i & (S::TR - 1)) * S::ROWB + own);
+                o.store(store + ((int64_t)h.z * BLK + rel) * C::BYTES);
+            }
+        }
+        xp ^= W * 16;
+    }
+
+    // Row 0, and rows wider than the team's columns: laps of W strips, every
+    // predecessor cell from the row store, and a barrier at the end of the row.
+    __device__ __forceinline__ void general(int i, int4 h, const int4* ed) {
+        const int Bs = h.x, bn = h.y + 1, d = h.w & FR_D;
+        const int S0 = Bs >> 4, S1 = bn > 0 ? (Bs + h.y) >> 4 : S0 - 1;
+        const int laps = S1 - S0 + 1 > W ? (S1 - S0 + W) / W : 1;
+        int r = (wid - S0) % W;
+        if (r < 0) r += W;
+        int32_t carry = K;
+        int4 best = make_int4(INT_MIN, Bs * BLK, 4, 0);
+        for (int c = 0; c < laps; c++) {
+            const int s = S0 + c * W + r;
+            const bool on = s <= S1;
+            int32_t P[4], V[4], H[4], key[4], ex = LOW, base = 0;
+            bool act = false;
+            int rel = 0;
+            if (on) {
+                if (s != s_cur) take_strip(s);
+                act = B >= Bs && B <= Bs + h.y;
+                rel = col0 - Bs * BLK;
+#pragma unroll
+                for (int l = 0; l < 4; l++) P[l] = V[l] = NEG;
+                if (i == 0 && col0 == 0) P[0] = 0;
+                for (int e = 0; e < d; e++) {
+                    const int4 fe = ed[e];
+                    const bool in = act && B >= fe.y && B <= fe.z - 2;
+                    const bool diag = in && (B > fe.y || B == 0);
+                    C pc;
+                    pc.none();
+                    int32_t left = NEG;
+                    if (in) {
+                        const char* src = store + ((int64_t)fe.w * BLK + (col0 - fe.y * BLK)) * C::BYTES;
+                        pc.load(src);
+                        if ((B > fe.y || (lane & 1)) && !(B == Bs && !(lane & 1))) left = C::load_m(src - C::BYTES);
+                    }
+                    fold(pc, left, diag, qw ^ (uint32_t)((fe.x & 7) * 0x01010101), P, V);
+                }
+#pragma unroll
+                for (int l = 0; l < 4; l++) H[l] = mx(P[l], V[l]);
+                base = -rel * k.e1;
+                publish(act, H, base, key, ex);
+                if (ADAPT) maximum(act, H, best);
+            } else {
+                publish_none();
+            }
+            if (ADAPT && c == laps - 1) put_maximum(best);
+            sync_row();
+            const int4 pv = lane < W ? lds128(sb + S::PUB + xp + lane * 16) : make_int4(LOW, LOW, NEG, INT_MAX);
+            const int32_t P0 = mx(carry, __reduce_max_sync(0xffffffffu, pv.w < s ? pv.x : LOW));
+            carry = mx(carry, __reduce_max_sync(0xffffffffu, pv.x));
+            if (on) {
+                if (!ADAPT && S1 - S0 < W) {
+                    // M of the cell left of the strip, for the next row
+                    const int32_t Pl = mx(K, __reduce_max_sync(0xffffffffu, pv.w < s - 1 ? pv.x : LOW));
+                    const int4 L = lds128(sb + S::PUB + xp + (wid == 0 ? W - 1 : wid - 1) * 16);
+                    edge = i == 0 ? L.z : mx(L.z, add32(k.o1 + (rel - lane * TC - 2) * k.e1, mx(Pl, L.y)));
+                }
+                if (act) {
+                    C o;
+                    finish(o, i, H, V, key, mx(P0, ex) - base);
+                    if (S1 - S0 < W) o.sts(sb + (i & (S::TR - 1)) * S::ROWB + own);
+                    o.store(store + ((int64_t)h.z * BLK + rel) * C::BYTES);
+                }
+            }
+            xp ^= W * 16;
+        }
+        if (!ADAPT) sync_row();
+    }
+};
+
+template <int W, bool WIDE>
+__device__ void team_fill_static(const TeamJob& a, char* smem) {
+    typedef TeamSmem<W, false, WIDE> S;
+    TeamRow<W, false, WIDE> t(smem, a);
+    TeamStage* stage = reinterpret_cast<TeamStage*>(smem + S::REST);
+    const unsigned stg = (unsigned)__cvta_generic_to_shared(stage);
+    team_stage<W>(a, stage[0], 0);
+    cp_async_wait_all();
+    bar_sync<1, S::THREADS>();
+    const int n = a.n;
+    int4 h = lds128(stg);
+    for (int i = 0; i < n; i++) {
+        const int x = i & (STG - 1);
+        const unsigned cur = stg + ((i / STG) & 1) * (unsigned)sizeof(TeamStage);
+        if (x == 0) team_stage<W>(a, stage[((i / STG) & 1) ^ 1], i + STG);
+        if (x == STG - 1) cp_async_wait_all();  // the next stage, published by this row's barrier
+        const unsigned nxt = x == STG - 1 ? stg + (((i / STG) & 1) ^ 1) * (unsigned)sizeof(TeamStage) : cur + (x + 1) * 16;
+        if (h.w & FR_GENERAL) {
+            t.general(i, h, a.ed + a.in_ptr[i]);
+            h = lds128(nxt);
+        } else {
+            const int4 hc = h;
+            const unsigned ed = cur + STG * 16 + (hc.w >> FR_EOFF) * 16;
+            const int4* far = a.ed;
+            t.row(i, hc,
+                  [&](int e) { return hc.w & FR_UNSTAGED ? a.fe[a.in_ptr[i] + e] : lds128(ed + e * 16); },
+                  [&](int e) { return far[a.in_ptr[i] + e]; }, [&]() { h = lds128(nxt); });
+        }
+    }
+    __syncthreads();
+}
+
+// The adaptive band's serial part (src/align.cpp:1433-1444, 1516-1568) on the
+// control warp. Its state lives in a shared-memory window of SWIN rows around
+// the current one (successors up to SWIN / 2 - 2 rows ahead, predecessors up to
+// SWIN / 2 behind), in global memory beyond it. Everything that does not need
+// row i's maximum is fetched while the other warps fill the row.
+template <int W, bool WIDE>
+__device__ void team_control(const TeamJob& a, char* smem, int64_t& cells_out) {
+    typedef TeamSmem<W, true, WIDE> S;
+    TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
+    int32_t* win = reinterpret_cast<int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
+    const int4* bests = reinterpret_cast<const int4*>(smem + S::BEST);
+    const int lane = threadIdx.x & 31;
+    const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n];
+    constexpr int AHEAD = SWIN / 2 - 1;
+    auto slot = [&](int r) { return win + (r & (SWIN - 1)) * SW_INTS; };
+    int4 ra0 = a.ra[0], ra1 = a.ra[1];  // row i
+    int4 rb0 = make_int4(0, 0, 0, 0), rb1 = rb0;  // row i + 1
+    if (n > 1) { rb0 = a.ra[2]; rb1 = a.ra[3]; }
+    int Bs, Be;
+    band_adaptive(ra0.z, ra0.w, m, a.w, m, 0, 0, 0, 0, Bs, Be);
+    Bs = 0;
+    int64_t tb = 0, cells = 0;
+    auto put_header = [&](int i, int d, int e0) {
+        const int bn = Be - Bs - 1;
+        int st = ST_OK;
+        if (bn < 0) st = ST_DEGENERATE;
+        else if (d > MAX_MULTI_PRED) st = ST_INDEGREE;
+        else if (tb + bn > a.store_cap || tb + bn > INT_MAX) st = ST_OOM;
+        if (lane == 0) {
+            TeamHdr& h = hdr[i & 1];
+            const bool gen = i == 0 || bn <= 0 || strips_of(Bs, Be) > W;
+            h.h = make_int4(Bs, Be - 2 - Bs, (int)tb, (d & FR_D) | (gen ? FR_GENERAL : 0));
+            h.g = make_int4(e0, st, 0, 0);
+            if (st == ST_OK) a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
+            int32_t* w = slot(i);
+            w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
+        }
+        return st;
+    };
+    int st = put_header(0, 0, 0);
+    int edx = 0, edx_n = 0;     // row i's and row i + 1's predecessor records (x), one per lane
+    int succ = -1, succ_n = -1; // row i's and row i + 1's successors, one per lane
+    if (lane < ra1.w) succ = a.out_row[ra0.y + lane];
+    if (n > 1) {
+        if (lane < rb1.z) edx_n = a.ed[rb0.x + lane].x;
+        if (lane < rb1.w) succ_n = a.out_row[rb0.y + lane];
+    }
+    int32_t pend = 0;  // state entering the window, one int per lane (8)
+    __syncwarp();
+    bar_sync<1, S::THREADS>();  // header 0
+    int xp = 0;
+    for (int i = 0; i < n; i++) {
+        if (st != ST_OK) {
+            if (lane == 0) a.out[0] = st;
+            cells_out = cells;
+            return;
+        }
+        const int bn = Be - Bs - 1;
+        const int d = i == 0 ? 0 : ra1.z, ns = ra1.w;
+        // the state that entered the window after the previous row
+        if (i > 0 && i - 1 + AHEAD < n && lane < 8) slot(i - 1 + AHEAD)[lane] = pend;
+        // loads two rows ahead
+        int4 rc0 = rb0, rc1 = rb1;
+        int edx_2 = 0, succ_2 = -1;
+        if (i + 2 < n) {
+            rc0 = a.ra[2 * (i + 2)];
+            rc1 = a.ra[2 * (i + 2) + 1];
+            // (the in-window in-edges and out-edges are the same edges: E of each)
+            const int e2 = rb0.x + rb1.z, o2 = rb0.y + rb1.w;
+            if (e2 + lane < E) edx_2 = a.ed[e2 + lane].x;
+            if (o2 + lane < E) succ_2 = a.out_row[o2 + lane];
+        }
+        __syncwarp();
+        // row i + 1's predecessor records
+        const int dn = i + 1 < n ? rb1.z : 0;
+        if (i + 1 < n) {
+            TeamHdr& h = hdr[(i + 1) & 1];
+            for (int k0 = 0; k0 < dn; k0 += 32) {
+                const int kk = k0 + lane;
+                if (kk < dn) {
+                    int4 v;
+                    v.x = k0 == 0 ? edx_n : a.ed[rb0.x + kk].x;
+                    const int p = v.x >> 4;
+                    if (i - p < AHEAD) {
+                        const int32_t* w = slot(p);
+                        v.y = w[SW_BS]; v.z = w[SW_BE]; v.w = w[SW_TB];
+                    } else {
+                        const int4 q = a.rowi[p];
+                        v.y = q.x; v.z = q.y; v.w = q.z;
+                    }
+                    const bool near = i + 1 - p < S::TR && strips_of(v.y, v.z) <= W;
+                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : -1, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+                    if (kk < HDR_E) h.ed[kk] = f;
+                    else a.fe[rb0.x + kk] = f;
+                    a.ed[rb0.x + kk] = v;
+                }
+            }
+        }
+        // row i's predecessors' slopes and maxima (their rows are done), its own
+        // state and the next row's
+        int psl = 0, pmp = INT_MIN / 2;
+        if (i > 0 && lane < d && d <= 32) {
+            const int p = edx >> 4;
+            const int32_t* w = i - p < AHEAD ? slot(p) : a.state + 8 * (int64_t)p;
+            psl = w[SW_SL];
+            pmp = w[SW_MP];
+        }
+        const int max_psl = __reduce_max_sync(0xffffffffu, psl);
+        int32_t* own = slot(i);
+        int sl = own[SW_SL], ow = own[SW_OW], ol = own[SW_OL], orr = own[SW_OR];
+        const int32_t* nw = slot(i + 1);
+        int nPl = nw[SW_PL], nPr = nw[SW_PR], nOl = nw[SW_OL], nOr = nw[SW_OR], nOw = nw[SW_OW];
+        bool to_next = __any_sync(0xffffffffu, lane < ns && succ == i + 1);
+        for (int k0 = 32; k0 < ns; k0 += 32)
+            to_next |= __any_sync(0xffffffffu, k0 + lane < ns && a.out_row[ra0.y + k0 + lane] == i + 1);
+        // the row's maxima: published in the last lap's half of the summaries
+        const int nst = bn > 0 ? strips_of(Bs, Be) : 0;
+        const int laps = nst > W ? (nst + W - 1) / W : 1;
+        xp = (xp + laps - 1) & 1;
+        bar_sync<2, S::THREADS>();
+        if (i >= 1) {
+            const int4 bw = lane < W ? bests[xp * W + lane] : make_int4(INT_MIN, INT_MAX, 4, 0);
+            const int32_t best = __reduce_max_sync(0xffffffffu, bw.x);
+            const int key = __reduce_min_sync(0xffffffffu, lane < W && bw.x == best ? bw.y * 8 + bw.z : INT_MAX);
+            const int acj = bn > 0 ? key >> 3 : Bs * BLK;
+            const int code = bn > 0 ? key & 7 : (int)a.qs[acj + 1];
+            int sl_best = INT_MIN, max_slp = 0;
+            bool is_match = false;
+            if (ra1.y == code) {  // cur.base == seq[max_acj]
+                if (d <= 32) {
+                    max_slp = max_psl;
+                    sl_best = __reduce_max_sync(0xffffffffu, pmp + 1 == acj ? psl + 1 : INT_MIN);
+                } else {
+                    for (int kk = lane; kk < d; kk += 32) {
+                        const int p = a.ed[ra0.x + kk].x >> 4;
+                        const int32_t* w = i - p < AHEAD ? slot(p) : a.state + 8 * (int64_t)p;
+                        max_slp = max(max_slp, w[SW_SL]);
+                        if (w[SW_MP] + 1 == acj) sl_best = max(sl_best, w[SW_SL] + 1);
+                    }
+                    max_slp = __reduce_max_sync(0xffffffffu, max_slp);
+                    sl_best = __reduce_max_sync(0xffffffffu, sl_best);
+                }
+                is_match = sl_best != INT_MIN;
+            }
+            if (is_match) sl = mx(sl, sl_best);
+            if (!is_match && max_slp < 30) ow = mn(ow + max_slp + 1, 5 * a.w);
+            if (sl >= 30) {
+                ol = orr = acj - ra1.x;
+                ow = 0;
+            }
+            if (to_next) {
+                nOl = sl >= 30 ? ol : mn(nOl, ol);
+                nOr = sl >= 30 ? orr : mx(nOr, orr);
+                nPl = mn(nPl, acj);
+                nPr = mx(nPr, acj + 1);
+                nOw = ow ? mx(nOw, ow) : ow;
+            }
+            cells += (int64_t)bn * BLK;
+            tb += bn;
+            if (i + 1 < n) {
+                band_adaptive(rb0.z, rb0.w, m, a.w, nPl, nPr, nOl, nOr, nOw, Bs, Be);
+                st = put_header(i + 1, dn, rb0.x);
+            }
+            bar_sync<1, S::THREADS>();  // header i + 1; row i's cells
+            if (lane == 0) {
+                own[SW_SL] = sl; own[SW_MP] = acj;
+                int32_t* gs = a.state + 8 * (int64_t)i;
+                gs[SW_SL] = sl; gs[SW_MP] = acj;
+            }
+            for (int k0 = 0; k0 < ns; k0 += 32) {
+                const int kk = k0 + lane;
+                if (kk < ns) {
+                    const int sr = k0 == 0 ? succ : a.out_row[ra0.y + kk];
+                    int32_t* w = sr - i < AHEAD ? slot(sr) : a.state + 8 * (int64_t)sr;
+                    w[SW_OL] = sl >= 30 ? ol : mn(w[SW_OL], ol);
+                    w[SW_OR] = sl >= 30 ? orr : mx(w[SW_OR], orr);
+                    w[SW_PL] = mn(w[SW_PL], acj);
+                    w[SW_PR] = mx(w[SW_PR], acj + 1);
+                    w[SW_OW] = ow ? mx(w[SW_OW], ow) : ow;
+                }
+            }
+        } else {
+            cells += (int64_t)bn * BLK;
+            tb += bn;
+            if (n > 1) {
+                band_adaptive(rb0.z, rb0.w, m, a.w, nPl, nPr, nOl, nOr, nOw, Bs, Be);
+                st = put_header(1, dn, rb0.x);
+            }
+            bar_sync<1, S::THREADS>();
+        }
+        __syncwarp();
+        xp ^= 1;
+        if (i + AHEAD < n && lane < 8) pend = a.state[8 * (int64_t)(i + AHEAD) + lane];
+        ra0 = rb0; ra1 = rb1; rb0 = rc0; rb1 = rc1;
+        edx = edx_n; edx_n = edx_2;
+        succ = succ_n; succ_n = succ_2;
+    }
+    cells_out = cells;
+}
+
+template <int W, bool WIDE>
+__device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) {
+    typedef TeamSmem<W, true, WIDE> S;
+    const int tid = threadIdx.x, n = a.n, m = a.qlen + 1;
+    int32_t* win = reinterpret_cast<int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
+    TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
+    for (int64_t x = tid; x < 8 * (int64_t)n; x += S::THREADS) a.state[x] = (x & 7) == SW_PL ? m : 0;
+    for (int x = tid; x < SWIN * SW_INTS; x += S::THREADS) win[x] = x % SW_INTS == SW_PL ? m : 0;
+    if (tid == 0) a.out[0] = ST_OK;
+    bar_sync<1, S::THREADS>();
+    if (tid >= 32 * W) {
+        team_control<W, WIDE>(a, smem, cells);
+    } else {
+        TeamRow<W, true, WIDE> t(smem, a);
+        const unsigned hb = (unsigned)__cvta_generic_to_shared(hdr);
+        bar_sync<1, S::THREADS>();  // header 0
+        for (int i = 0; i < n; i++) {
+            const unsigned hc = hb + (i & 1) * (unsigned)sizeof(TeamHdr);
+            const int4 h = lds128(hc), g = lds128(hc + 16);
+            if (g.y != ST_OK) break;
+            if (h.w & FR_GENERAL)
+                t.general(i, h, a.ed + g.x);
+            else
+                t.row(i, h, [&](int e) { return e < HDR_E ? lds128(hc + 32 + e * 16) : a.fe[g.x + e]; },
+                      [&](int e) { return a.ed[g.x + e]; }, [] {});
+            bar_sync<1, S::THREADS>();  // row i's cells, header i + 1
+        }
+    }
+    __syncthreads();
+    return a.out[0];
+}
+
+// Backtrack by one warp over the stored values, src/align.cpp:1572-1736: the
+// same steps, tests and tie rules as backtrack_records (dp_rowops.h), each test
+// evaluated on the cells the walk reaches, one lane per predecessor (they are
+// in priority order, so "the first that passes" is a ballot).
+//
+// A step is a chain of dependent reads and ~100 dependent instructions (1,250
+// cycles measured), so
+//  * what it reads comes from a tile in shared memory: BT_ROWS rows up to the
+//    walk's, for each its predecessor records and BT_BLK blocks around the
+//    column the walk would reach if it kept its distance from the band's left
+//    end. Cells outside the tile are read from the row store; a walk that
+//    leaves its row's blocks, or the tile's first row, loads the next tile;
+//  * runs of matches along the heaviest in-edges are taken in one step: lane t
+//    stands t such predecessors back (pointer jumping over the tile's rows) and
+//    t columns to the left, and tests whether its cell's first choice, a match
+//    with its heaviest predecessor, holds. The leading lanes' moves are the
+//    walk's. The cell that ends the run takes the full step.
+//
+// M == I is decided only when it is asked for, by looking for the cell the
+// gap opened from: I[j] is the maximum over k < j of M[k] + o1 + (j - 1 - k) * e1
+// and never exceeds M[j]. Once in a gap the walk carries the gap's value.
+template <bool WIDE>
+static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* smem, int lane, int32_t& nmoves) {
+    typedef typename Cells<WIDE>::One One;
+    typedef BtSmem<WIDE> T;
+    constexpr int32_t NEG = Cells<WIDE>::NEG;
+    constexpr int CB = Cells<WIDE>::BYTES, RL = T::ROWB / 16;  // 16-byte pieces of a tile row
+    const CellK k = a.k;
+    const One* store = reinterpret_cast<const One*>(a.store);
+    const int4* rowi = a.rowi;
+    const int4* edg = a.ed;
+    const uint8_t* qs = a.qs;
+    int32_t* moves = a.moves;
+    const int cap = a.moves_cap;
+    const unsigned sb = (unsigned)__cvta_generic_to_shared(smem);
+    int i = a.n - 1, acj = a.qlen + 1, op = ALL_OP;
+    int32_t carry = 0;  // the value of the gap the walk is in (op == D_OP or I_OP)
+    int32_t nm = 0;
+    int lo = INT_MAX, e_lo = 0, ne = 0;
+    int32_t st = ST_OK;
+    while (i > 0 || acj > 0) {
+        int4 R = make_int4(0, 0, 0, 0);
+        if (i >= lo) R = lds128(sb + T::ROW + (i - lo) * 16);
+        if (i < lo || (unsigned)((acj >> 3) - R.w) >= BT_BLK) {
+            // the tile that ends with row i
+            lo = max(0, i - BT_ROWS + 1);
+            const int cnt = i - lo + 1;
+            const int dB = (acj >> 3) - rowi[i].x;
+            __syncwarp();
+            for (int r = lane; r < cnt; r += 32) {
+                int4 v = rowi[lo + r];
+                v.w = v.x + max(0, dB - (BT_BLK - 3));
+                *reinterpret_cast<int4*>(smem + T::ROW + r * 16) = v;
+            }
+            for (int r = lane; r <= cnt; r += 32) *reinterpret_cast<int32_t*>(smem + T::PTR + r * 4) = a.in_ptr[lo + r];
+            __syncwarp();
+            e_lo = lds32(sb + T::PTR);
+            ne = min(lds32(sb + T::PTR + cnt * 4) - e_lo, BT_E);
+            for (int e = lane; e < ne; e += 32) cp_async16(smem + T::ED + e * 16, edg + e_lo + e);
+            for (int x = lane; x < cnt * RL; x += 32) {
+                const int r = x / RL, pc = x % RL;
+                const int4 v = *reinterpret_cast<const int4*>(smem + T::ROW + r * 16);
+                const int blk = v.w + pc * 16 / (BLK * CB);
+                if (blk <= v.y - 2)
+                    cp_async16(smem + T::CELLS + r * T::ROWB + pc * 16,
+                               a.store + ((int64_t)v.z + (v.w - v.x)) * (BLK * CB) + pc * 16);
+            }
+            cp_async_commit_all();
+            cp_async_wait_all();
+            __syncwarp();
+            uint8_t* jump = reinterpret_cast<uint8_t*>(smem + T::JUMP);
+            for (int r = lane; r < BT_ROWS; r += 32) {
+                int to = 255;
+                if (r < cnt && lo + r > 0) {
+                    const int e = lds32(sb + T::PTR + r * 4) - e_lo, e1 = lds32(sb + T::PTR + r * 4 + 4) - e_lo;
+                    if (e < e1 && e < ne) {
+                        const int p = lds32(sb + T::ED + e * 16) >> 4;
+                        if (p >= lo) to = p - lo;
+                    }
+                }
+                jump[r] = (uint8_t)to;
+            }
+#pragma unroll
+            for (int q = 1; q < 5; q++) {
+                __syncwarp();
+                for (int r = lane; r < BT_ROWS; r += 32) {
+                    const int h = jump[(q - 1) * BT_ROWS + r];
+                    jump[q * BT_ROWS + r] = h == 255 ? 255 : jump[(q - 1) * BT_ROWS + h];
+                }
+            }
+            __syncwarp();
+            R = lds128(sb + T::ROW + (i - lo) * 16);
+        }
+        if (op & M_OP) {
+            // a run of matches with the heaviest predecessors
+            const uint8_t* jump = reinterpret_cast<const uint8_t*>(smem + T::JUMP);
+            int r = i - lo;
+#pragma unroll
+            for (int q = 0; q < 5; q++)
+                if ((lane >> q) & 1) r = r == 255 ? 255 : jump[q * BT_ROWS + r];
+            const int c = acj - lane;
+            bool ok = false;
+            int32_t mv = 0;
+            const int to = r == 255 ? 255 : jump[r];
+            if (to != 255 && c > 0) {
+                const int4 A = lds128(sb + T::ROW + r * 16), P = lds128(sb + T::ROW + to * 16);
+                const int4 er = lds128(sb + T::ED + (lds32(sb + T::PTR + r * 4) - e_lo) * 16);
+                const int qc = qs[c], bl = (c - 1) >> 3;
+                // both cells in their rows' bands and in the tile
+                if ((c >> 3) <= A.y - 2 && (unsigned)((c >> 3) - A.w) < BT_BLK && bl <= P.y - 2 && (unsigned)(bl - P.w) < BT_BLK &&
+                    (er.x & 15) == (qc | 8)) {
+                    const int32_t x = One::lds(sb + T::CELLS + r * T::ROWB + (c - A.w * BLK) * CB).m();
+                    const int32_t y = One::lds(sb + T::CELLS + to * T::ROWB + (c - 1 - P.w * BLK) * CB).m();
+                    ok = x == add32(y, k.match);
+                    mv = mv_pack(MV_MATCH, lo + to, qc);
+                }
+            }
+            const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
+            const int run = min(bad ? __ffs(bad) - 1 : 32, cap - nm);
+            if (run > 0) {
+                if (lane < run) moves[nm + lane] = mv;
+                nm += run;
+                acj -= run;
+                op = ALL_OP;
+                i = __shfl_sync(0xffffffffu, to, run - 1) + lo;
+                continue;
+            }
+        }
+        const int Bs = R.x, Be = R.y;
+        if (acj > (Be - 1) * BLK || acj < Bs * BLK) { st = ST_BAND_ESCAPE; break; }
+        const int j = acj - Bs * BLK;
+        if (j >= (Be - Bs - 1) * BLK) { st = ST_BT_FAIL; break; }
+        if (nm + 1 > cap) { st = ST_OOM; break; }
+        const int e0 = lds32(sb + T::PTR + (i - lo) * 4) - e_lo;
+        const int d = i == 0 ? 0 : lds32(sb + T::PTR + (i - lo) * 4 + 4) - e_lo - e0;
+        const One cell = One::lds(sb + T::CELLS + (i - lo) * T::ROWB + (acj - R.w * BLK) * CB);
+        const int qc = acj > 0 ? qs[acj] : 4;
+        const int32_t M = cell.m();
+        const bool eq_md = cell.eq_md(k);
+        const int32_t dv = op == D_OP ? carry : M;
+        int p1 = -1, p4 = -1, po = -1, pe = -1;  // rows of the choices; p1 -2: the heaviest match fails its weight test
+        bool m4_match = false;
+        for (int k0 = 0; k0 < d; k0 += 32) {
+            bool em = false, bm = false, eo = false, ex = false;
+            int4 er = make_int4(0, 0, 0, 0);
+            if (k0 + lane < d) {
+                const int e = e0 + k0 + lane;
+                if (e < ne) er = lds128(sb + T::ED + e * 16);
+                else er = edg[e_lo + e];
+                const int p = er.x >> 4;
+                const int bl = (acj - 1) >> 3, bc = acj >> 3;
+                const bool inl = acj > 0 && bl >= er.y && bl <= er.z - 2;
+                const bool inc = bc >= er.y && bc <= er.z - 2;
+                int w0 = INT_MIN / 2;
+                if (p >= lo) w0 = lds32(sb + T::ROW + (p - lo) * 16 + 12);
+                One vl, vc;
+                if (inl) {
+                    if ((unsigned)(bl - w0) < BT_BLK) vl = One::lds(sb + T::CELLS + (p - lo) * T::ROWB + (acj - 1 - w0 * BLK) * CB);
+                    else vl = store[(int64_t)er.w * BLK + (acj - 1 - er.y * BLK)];
+                }
+                if (inc) {
+                    if ((unsigned)(bc - w0) < BT_BLK) vc = One::lds(sb + T::CELLS + (p - lo) * T::ROWB + (acj - w0 * BLK) * CB);
+                    else vc = store[(int64_t)er.w * BLK + (acj - er.y * BLK)];
+                    eo = vc.d_opens(dv, k);
+                    ex = vc.d_extends(dv, k);
+                }
+                if (inl) {
+                    bm = (er.x & 7) == qc;
+                    em = M == add32(vl.m(), bm ? k.match : k.mismatch);
+                }
+            }
+            const unsigned b1 = __ballot_sync(0xffffffffu, em && bm);
+            if (b1 && p1 == -1) {
+                const int x = __shfl_sync(0xffffffffu, er.x, __ffs(b1) - 1);
+                p1 = (x & 8) ? x >> 4 : -2;
+                if (p1 >= 0 && (op & M_OP) && acj > 0 && k0 == 0) break;  // the walk's first choice
+            }
+            const unsigned b4 = __ballot_sync(0xffffffffu, em), bo = __ballot_sync(0xffffffffu, eo),
+                           be = __ballot_sync(0xffffffffu, ex);
+            if (b4 && p4 < 0) {
+                const int f = __ffs(b4) - 1;
+                p4 = __shfl_sync(0xffffffffu, er.x, f) >> 4;
+                m4_match = (b1 >> f) & 1;
+            }
+            if (bo && po < 0) po = __shfl_sync(0xffffffffu, er.x, __ffs(bo) - 1) >> 4;
+            if (be && pe < 0) pe = __shfl_sync(0xffffffffu, er.x, __ffs(be) - 1) >> 4;
+        }
+        if ((op & M_OP) && acj > 0 && p1 >= 0) {
+            if (lane == 0) moves[nm] = mv_pack(MV_MATCH, p1, qc);
+            nm++;
+            op = ALL_OP; i = p1; acj--;
+            continue;
+        }
+        if ((op & D_OP) && (op == D_OP || eq_md) && (po >= 0 || pe >= 0)) {
+            if (po >= 0) { i = po; op = M_OP | I_OP; }
+            else { i = pe; op = D_OP; carry = add32(dv, -k.e1); }
+            continue;
+        }
+        if ((op & I_OP) && acj > 0 && j >= 1) {
+            const One* row = store + (int64_t)R.z * BLK;
+            bool in_gap = op == I_OP;
+            int32_t v = carry;
+            if (!in_gap) {  // M == I ?
+                v = M;
+                if (i == 0) {
+                    in_gap = M == NEG;
+                } else {
+                    for (int x0 = j - 1; x0 >= 0 && !in_gap; x0 -= 128) {
+                        bool hit = false;
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const int x = x0 - 32 * u - lane;
+                            if (x >= 0) hit |= add32(row[x].m(), k.o1 + (j - 1 - x) * k.e1) == v;
+                        }
+                        in_gap = __any_sync(0xffffffffu, hit);
+                    }
+                    in_gap = in_gap || add32(NEG, j * k.e1) == v;
+                }
+            }
+            if (in_gap) {
+                const bool iopen = add32(row[j - 1].m(), k.o1) == v;
+                const bool iext = i > 0 || k.e1 == 0;  // I is one or the other; row 0 holds NEG throughout
+                if (iopen || iext) {
+                    if (lane == 0) moves[nm] = mv_pack(MV_INSERT, 0, qc);
+                    nm++;
+                    if (iopen) op = M_OP | D_OP;
+                    else { op = I_OP; carry = add32(v, -k.e1); }
+                    acj--;
+                    continue;
+                }
+            }
+        }
+        if ((op & M_OP) && acj > 0 && p4 >= 0) {
+            if (lane == 0) moves[nm] = mv_pack(m4_match ? MV_MATCH : MV_MISMATCH, p4, qc);
+            nm++;
+            op = ALL_OP; i = p4; acj--;
+            continue;
+        }
+        st = ST_BT_FAIL;
+        break;
+    }
+    nmoves = nm;
+    return st;
+}
+
+// Score, status and moves of a filled alignment (warp 0).
+template <bool WIDE>
+static __device__ void team_finish(const TeamJob& a, char* smem, int64_t cells, int lane) {
+    const int m = a.qlen + 1;
+    int32_t nm = 0;
+    const int32_t st = team_backtrack<WIDE>(a, smem, lane, nm);
+    if (lane == 0) {
+        const int4 last = a.rowi[a.n - 1];
+        const int jm = m - last.x * BLK;
+        // column m lies in the last row's band (tlen[end] - tlen[end] = 0); the
+        // guard only keeps a malformed window from reading outside its row
+        const bool inb = jm >= 0 && jm / BLK < last.y - last.x - 1;
+        int32_t score = NEG_INF;
+        if (inb) {
+            score = reinterpret_cast<const typename Cells<WIDE>::One*>(a.store)[(int64_t)last.z * BLK + jm].m();
+            if (!WIDE && score < -(1 << 21)) score += NEG_INF - PACK_NEG;  // an unreachable end cell
+        }
+        a.out[1] = score;
+        a.out[2] = nm;
+        a.out[3] = (int32_t)(cells > INT_MAX ? INT_MAX : cells);
+        a.out[0] = st;
+    }
+}
+
+// One CTA per alignment.
+template <int W, bool ADAPT, bool WIDE>
+__global__ void __launch_bounds__(TeamSmem<W, ADAPT, WIDE>::THREADS, 1) k_align(const TeamJob* __restrict__ jobs) {
+    typedef TeamSmem<W, ADAPT, WIDE> S;
+    extern __shared__ __align__(16) char tsm[];
+    __shared__ TeamJob sa;
+    __shared__ int64_t s_part[W + 1];
+    __shared__ unsigned long long s_fail;
+    __shared__ int64_t s_cells;
+    if (threadIdx.x == 0) sa = jobs[blockIdx.x];
+    __syncthreads();
+    const TeamJob& a = sa;
+    int64_t cells = 0;
+    if (a.n <= 0) {
+        if (threadIdx.x == 0) a.out[0] = ST_BAD_ARG;
+        return;
+    }
+    int st;
+    if constexpr (ADAPT) {
+        st = team_fill_adaptive<W, WIDE>(a, tsm, cells);
+        if (threadIdx.x == 32 * W) s_cells = cells;
+        __syncthreads();
+        cells = s_cells;
+    } else {
+        st = team_rows_static<S, W, 32 * W>(a, s_part, &s_fail, cells);
+        if (st == ST_OK) team_fill_static<W, WIDE>(a, tsm);
+    }
+    if (st != ST_OK) {
+        if (threadIdx.x == 0) {
+            a.out[0] = st;
+            a.out[1] = 0;
+            a.out[2] = 0;
+            a.out[3] = 0;
+        }
+        return;
+    }
+    if (threadIdx.x < 32) team_finish<WIDE>(a, tsm, cells, threadIdx.x);
+}
+
+}  // namespace pb
