@@ -24,7 +24,7 @@
 #include <stdexcept>
 
 #include "gpu_engine.h"
-#include "plain.cuh"
+#include "warp.cuh"
 
 namespace pb {
 
@@ -34,26 +34,22 @@ inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct SlotLayout {
     int32_t NC, EC, QC;         // node, edge and query capacities
-    int32_t ring_rows, ring_blocks;
-    int64_t rs_cap, tb_cap;     // int32 units / bytes
+    int64_t store_cap;          // row store, blocks
     // byte offsets inside a slot
     int64_t hdr, base, par, aligned, ind, rank, in_head, in_tail, out_head, out_tail, in_cnt, out_cnt;
     int64_t e_from, e_to, e_w, e_nin, e_nout;
     int64_t rank_to_id, hlen, tlen, deg, stk, pre, score, hin, hout, stamp;
-    int64_t v_in_ptr, v_in_row, v_in_w, v_in_base, v_out_ptr, v_out_row, v_base, v_ind, v_hq, v_hq_loc, v_tq;
-    int64_t v_pmeta, v_desc;
-    int64_t meta, state, qs, moves, path, rs, tb;
+    int64_t v_in_ptr, v_out_ptr, v_out_row, v_maxs, v_ed, v_fe, v_rowi, v_fr, v_ra;
+    int64_t state, qs, moves, path, store;
     int64_t bytes;
 };
 
-SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int32_t ring_rows, int32_t ring_blocks, int64_t spill,
-                       int64_t tb_cap, bool adaptive) {
+SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int64_t store_bytes, bool stat, bool adaptive, bool wide) {
     SlotLayout L;
     std::memset(&L, 0, sizeof L);
     L.NC = NC; L.EC = EC; L.QC = QC;
-    L.ring_rows = ring_rows; L.ring_blocks = ring_blocks;
-    L.rs_cap = (int64_t)ring_rows * ring_blocks * 16 + spill;
-    L.tb_cap = tb_cap;
+    const int bb = BLK * (wide ? Cells<true>::BYTES : Cells<false>::BYTES);
+    L.store_cap = store_bytes / bb;
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t r = o; o = up256(o + bytes); return (int64_t)r; };
     const size_t n4 = 4 * (size_t)NC, e4 = 4 * (size_t)EC;
@@ -65,18 +61,21 @@ SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int32_t ring_rows, in
     L.rank_to_id = take(n4); L.hlen = take(n4); L.tlen = take(n4); L.deg = take(n4); L.stk = take(n4);
     L.pre = take(n4); L.score = take(n4);
     L.hin = take(n4); L.hout = take(n4); L.stamp = take(n4);
-    L.v_in_ptr = take(n4 + 4); L.v_in_row = take(e4); L.v_in_w = take(e4); L.v_in_base = take(EC);
-    L.v_out_ptr = take(n4 + 4); L.v_out_row = take(e4); L.v_base = take(NC); L.v_ind = take(n4);
-    L.v_hq = take(n4); L.v_hq_loc = take(n4); L.v_tq = take(n4);
-    L.v_pmeta = take(16 * (size_t)EC);
-    L.v_desc = take(48 * (size_t)NC);
-    L.meta = take(sizeof(RowMeta) * (size_t)NC);
-    L.state = take(adaptive ? 4 * (size_t)AB_NSTATE * NC : 64);
+    L.v_in_ptr = take(n4 + 4);
+    L.v_out_ptr = take(n4 + 4); L.v_out_row = take(e4); L.v_maxs = take(n4);
+    L.v_ed = take(16 * (size_t)EC);
+    L.v_rowi = take(16 * (size_t)NC);
+    if (stat) {
+        L.v_fe = take(16 * (size_t)EC);
+        L.v_fr = take(16 * (size_t)NC);
+    } else {
+        L.v_ra = take(32 * (size_t)NC);
+    }
+    L.state = take(adaptive ? 32 * (size_t)NC : 64);
     L.qs = take((size_t)qs_bytes(QC) + 64);
     L.moves = take(4 * ((size_t)NC + QC + 16));
     L.path = take(4 * ((size_t)NC + QC + 16));
-    L.rs = take(4 * (size_t)L.rs_cap);
-    L.tb = take((size_t)tb_cap);
+    L.store = take((size_t)L.store_cap * bb);
     L.bytes = (int64_t)up256(o);
     return L;
 }
@@ -89,13 +88,15 @@ struct BatchArgs {
     const int32_t* order;
     int32_t* counter;
     int32_t n_windows;
-    Scoring sc;
+    CellK k;
     int32_t b, f, ab_band;
     char* slots;
     SlotLayout L;
     int32_t smem_per_warp;   // bytes of dynamic shared memory per warp
-    int32_t sring_rows;      // shared-memory ring rows of the static-band fill (0 = all rows in global)
+    int32_t sring_rows;      // shared-memory ring rows of the static-band fill (a power of two; 0 = none)
     int32_t sring_blocks;    // blocks per ring row
+    int32_t state_rows;      // adaptive state window of the dynamic-band fill (a power of two)
+    int32_t stat_rows, stat_blocks;  // read statistics: the ring that "spilled" rows are counted against
     char* cons;
     int32_t cons_stride;
     int32_t* cons_len;
@@ -624,1233 +625,182 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
     }
 }
 
-// Everything the static-band fill needs about one row, in one 48-byte record
-// (three 16-byte loads, issued one row ahead): the band, where the row's M/D
-// blocks and records go, its predecessor range, and the first predecessor's
-// band/location/base/weight so single-predecessor rows need nothing else.
-struct __align__(16) RowDesc {
-    int32_t bsbe, st, tb, e0;      // Bs | Be << 16, row store location, record offset, first in-edge
-    int32_t d, ind, w1ok, prow0;   // in-window predecessors, in-degree count, in_weight >= ind/10, first pred row
-    int32_t pbsbe, pst, pbase, pw; // first predecessor: band, location, base (as the DP sees it), in_weight
-};
-
-// Static-band view (f > 0, no adaptive band): besides the predecessor lists,
-// every row's band, row-store location and record offset are a pure function
-// of hlen/tlen, so the warp computes them all here, in parallel, and attaches
-// to each in-edge the predecessor's (Bs, Be, location). The fill then needs
-// one coalesced load per predecessor and no per-row bookkeeping.
-// Row store location: ring slot -(r % R) - 1 in shared memory, or an offset
-// in the slot's spill area for rows with a successor R or more rows ahead.
-__device__ int build_view_static(DevGraph& g, char* s, const SlotLayout& L, WinView& v, int m, int f, int wband,
-                                 int R, int RB, int lane, int& beg_out) {
+// The DP rows of window [rank(source), rank(sink)] for one alignment, with the
+// whole warp: in-edges in the backtrack's priority order (TeamJob::ed), and
+// for the static band, whose rows depend only on hlen / tlen, every row's
+// band, row-store place and fill header; for the dynamic bands the control
+// data of TeamJob::ra. One walk over the in-lists fills the out-edges too:
+// their order within a row does not matter to the band update (successors
+// are distinct rows).
+template <bool STATIC, bool WIDE>
+__device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, TeamJob& v, int m, int wband, int lane, int& n_out,
+                          int& beg_out) {
+    const SlotLayout& L = A.L;
     const int beg_i = g.rank[0], end_i = g.rank[1];
     const int n = end_i - beg_i + 1;
     beg_out = beg_i;
+    n_out = n;
+    const bool whole = beg_i == 0 && n == g.hdr[0];  // every node is in the window
     int32_t* in_ptr = (int32_t*)(s + L.v_in_ptr);
-    int32_t* in_row = (int32_t*)(s + L.v_in_row);
-    int32_t* in_w = (int32_t*)(s + L.v_in_w);
-    uint8_t* in_base = (uint8_t*)(s + L.v_in_base);
-    int32_t* vind = (int32_t*)(s + L.v_ind);
-    int4* erec = (int4*)(s + L.v_pmeta);
-    RowDesc* desc = (RowDesc*)(s + L.v_desc);
-    RowMeta* meta = (RowMeta*)(s + L.meta);
+    int32_t* out_ptr = (int32_t*)(s + L.v_out_ptr);
+    int32_t* out_row = (int32_t*)(s + L.v_out_row);
+    int32_t* maxs = (int32_t*)(s + L.v_maxs);
+    int32_t* cur = (int32_t*)(s + L.deg);  // topsort scratch, free until the next sort
+    int4* ed = (int4*)(s + L.v_ed);
+    int4* fe = (int4*)(s + L.v_fe);
+    int4* rowi = (int4*)(s + L.v_rowi);
+    int4* fr = (int4*)(s + L.v_fr);
+    int4* ra = (int4*)(s + L.v_ra);
     const int h0 = g.hlen[beg_i], t0 = g.tlen[end_i];
-    const int64_t spill_cap = L.rs_cap;
-    // pass 1: per-row counts, band, widths
-    for (int r = lane; r < n; r += 32) {
-        const int u = g.rank_to_id[beg_i + r];
-        int ci = 0, maxs = r;
-        for (int e = g.in_head[u]; e >= 0; e = g.e_nin[e]) ci += (g.rank[g.e_from[e]] - beg_i >= 0);
-        for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) {
-            const int sr = g.rank[g.e_to[e]] - beg_i;
-            if (sr < n && sr > maxs) maxs = sr;
-        }
-        int Bs, Be;
-        band_static(f, g.hlen[beg_i + r] - h0, g.tlen[beg_i + r] - t0, m, wband, Bs, Be);
-        if (r == 0) Bs = 0;
-        const int bn = Be - Bs - 1;
-        const int d = r == 0 ? 0 : ci;
-        const int bpc = d >= 2 ? 4 : 1;
-        const bool spill = R == 0 || (maxs - r >= R) || bn > RB;
-        in_ptr[r + 1] = ci;
-        vind[r] = g.ind[u];
-        RowMeta rm;
-        rm.Bs = Bs;
-        rm.Be = Be;
-        rm.tb = bn > 0 ? (((int64_t)bn * BLK * bpc + 15) & ~(int64_t)15) : 0;   // widths, scanned below
-        rm.st = spill ? (bn > 0 ? (int64_t)bn * 16 : 0) : -1;
-        if (bn < 0 || d > MAX_MULTI_PRED) rm.Be = INT32_MIN;                  // flagged
-        meta[r] = rm;
-    }
-    __syncwarp();
-    // scans: in_ptr, record offsets, spill offsets
-    int ci_c = 0;
-    int64_t tb_c = 0, sp_c = 0;
+    // counts, bands, widths
     bool bad = false;
+    int ci_c = 0, co_c = 0, bn_c = 0;
     if (lane == 0) in_ptr[0] = 0;
     for (int c0 = 0; c0 < n; c0 += 32) {
         const int r = c0 + lane;
-        RowMeta rm;
-        int ci = 0;
-        int64_t tbw = 0, spw = 0;
-        bool sp = false;
+        int ci = 0, co = 0, bn = 0, Bs = 0, Be = 1;
         if (r < n) {
-            rm = meta[r];
-            ci = in_ptr[r + 1];
-            tbw = rm.tb;
-            sp = rm.st >= 0;
-            spw = sp ? rm.st : 0;
-            bad |= rm.Be == INT32_MIN;
+            const int u = g.rank_to_id[beg_i + r];
+            if (whole) {
+                ci = g.in_cnt[u];
+                co = g.out_cnt[u];
+            } else {
+                for (int e = g.in_head[u]; e >= 0; e = g.e_nin[e]) ci += (g.rank[g.e_from[e]] - beg_i >= 0);
+                for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) co += (g.rank[g.e_to[e]] - beg_i < n);
+            }
+            if (STATIC) {
+                band_static(A.f, g.hlen[beg_i + r] - h0, g.tlen[beg_i + r] - t0, m, wband, Bs, Be);
+                if (r == 0) Bs = 0;
+                bn = Be - Bs - 1;
+                bad |= bn < 0 || (r > 0 && ci > MAX_MULTI_PRED);
+                bn = max(bn, 0);
+            }
+            maxs[r] = r;
         }
-        int xi = ci;
-        long long xt = tbw, xs = spw;
+        int xi = ci, xo = co, xb = bn;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int yi = __shfl_up_sync(0xffffffffu, xi, o);
-            const long long yt = __shfl_up_sync(0xffffffffu, xt, o);
-            const long long ys = __shfl_up_sync(0xffffffffu, xs, o);
-            if (lane >= o) { xi += yi; xt += yt; xs += ys; }
+            const int yi = __shfl_up_sync(0xffffffffu, xi, o), yo = __shfl_up_sync(0xffffffffu, xo, o),
+                      yb = __shfl_up_sync(0xffffffffu, xb, o);
+            if (lane >= o) { xi += yi; xo += yo; xb += yb; }
         }
         if (r < n) {
             in_ptr[r + 1] = ci_c + xi;
-            rm.tb = tb_c + (xt - tbw);
-            rm.st = sp ? sp_c + (xs - spw) : -(int64_t)(r % (R > 0 ? R : 1)) - 1;
-            meta[r] = rm;
+            if (STATIC) {
+                rowi[r] = make_int4(Bs, Be, bn_c + xb - bn, 0);
+            } else {
+                out_ptr[r] = cur[r] = co_c + xo - co;
+            }
         }
         ci_c += __shfl_sync(0xffffffffu, xi, 31);
-        tb_c += __shfl_sync(0xffffffffu, xt, 31);
-        sp_c += __shfl_sync(0xffffffffu, xs, 31);
+        co_c += __shfl_sync(0xffffffffu, xo, 31);
+        bn_c += __shfl_sync(0xffffffffu, xb, 31);
     }
-    if (lane == 0) {
-        g.hdr[8] = (int32_t)(tb_c > INT_MAX ? INT_MAX : tb_c);   // DP output 4: record bytes
-        g.hdr[9] = (int32_t)(sp_c > INT_MAX ? INT_MAX : sp_c);   // DP output 5: spilled row-store entries
-    }
+    if (!STATIC && lane == 0) out_ptr[n] = co_c;
     if (__any_sync(0xffffffffu, bad)) return ST_DEGENERATE;
-    if (tb_c > L.tb_cap || sp_c > spill_cap) return ST_OOM;
+    if (bn_c > L.store_cap) return ST_OOM;
     __syncwarp();
-    // pass 2: predecessor lists in in-list order
+    const int R = A.sring_rows, RB = A.sring_blocks;
+    constexpr int BB = BLK * Cells<WIDE>::BYTES;
     for (int r = lane; r < n; r += 32) {
         const int u = g.rank_to_id[beg_i + r];
-        int k = in_ptr[r];
-        for (int e = g.in_head[u]; e >= 0; e = g.e_nin[e]) {
-            const int p = g.rank[g.e_from[e]] - beg_i;
-            if (p < 0) continue;
-            in_row[k] = p;
-            in_w[k] = g.e_w[e];
-            in_base[k] = p == 0 ? 4 : g.base[g.e_from[e]];
-            k++;
-        }
-    }
-    __syncwarp();
-    // pass 3: each row's predecessor records in the backtrack's priority order
-    // (in_weight descending, in-list position ascending; src/align.cpp:1601,
-    // 1637, 1708 keep the first maximum), so the fill can take "the first
-    // predecessor that satisfies a test" as the backtrack's choice.
-    // erec = {Bs | Be << 16, row-store location, in_weight | position << 16,
-    //         base | (in_weight >= ind/10) << 8}
-    for (int r = lane; r < n; r += 32) {
-        const int e0 = in_ptr[r], d = r == 0 ? 0 : in_ptr[r + 1] - e0;
-        const int ind = vind[r];
-        for (int k = 0; k < d; k++) {
-            const RowMeta pm = meta[in_row[e0 + k]];
-            const int w = in_w[e0 + k];
-            const int4 rec = make_int4(pm.Bs | (pm.Be << 16), (int32_t)pm.st, (w & 0xffff) | (k << 16),
-                                       (int)in_base[e0 + k] | ((w >= ind / 10) ? 256 : 0));
-            // insertion into the sorted prefix [e0, e0 + k)
-            int at = k;
-            while (at > 0) {
-                const int4 prev = erec[e0 + at - 1];
-                const int pw = prev.z & 0xffff;
-                if (pw >= w) break;  // strictly larger weight moves ahead; ties keep list order
-                erec[e0 + at] = prev;
-                at--;
-            }
-            erec[e0 + at] = rec;
-        }
-    }
-    __syncwarp();
-    // pass 4: row descriptors (the first predecessor record is the top-priority one)
-    for (int r = lane; r < n; r += 32) {
-        const RowMeta rm = meta[r];
         const int e0 = in_ptr[r];
-        const int d = r == 0 ? 0 : in_ptr[r + 1] - e0;
-        RowDesc rd;
-        rd.bsbe = rm.Bs | (rm.Be << 16);
-        rd.st = (int32_t)rm.st;
-        rd.tb = (int32_t)rm.tb;
-        rd.e0 = e0;
-        rd.d = d;
-        rd.ind = vind[r];
-        rd.prow0 = d >= 1 ? in_row[e0] : 0;
-        if (d >= 1) {
-            const int4 er = erec[e0];
-            rd.pbsbe = er.x; rd.pst = er.y; rd.pw = er.z & 0xffff; rd.pbase = er.w & 255;
-            rd.w1ok = (er.w >> 8) & 1;
-        } else {
-            rd.pbsbe = rd.pst = rd.pw = rd.pbase = 0;
-            rd.w1ok = 0;
+        int d = 0;
+        for (int e = g.in_head[u]; e >= 0;) {
+            const int from = g.e_from[e], w = g.e_w[e];
+            e = g.e_nin[e];
+            const int p = g.rank[from] - beg_i;
+            if (p < 0) continue;
+            // insertion by weight; ties keep list order
+            int at = e0 + d;
+            while (at > e0 && ed[at - 1].y < w) { ed[at] = ed[at - 1]; at--; }
+            ed[at] = make_int4((p << 4) | (p == 0 ? 4 : (int)g.base[from]), w, 0, 0);
+            d++;
+            atomicMax(&maxs[p], r);
+            if (!STATIC) out_row[atomicAdd(&cur[p], 1)] = r;
         }
-        desc[r] = rd;
+        const int least = g.ind[u] / 10;
+        for (int k = 0; k < d; k++) {
+            int4 x = ed[e0 + k];
+            if (x.y >= least) x.x |= 8;
+            if (STATIC) {
+                const int p = x.x >> 4;
+                const int4 pr = rowi[p];
+                const bool near = r - p < R && pr.y - pr.x - 1 <= RB;
+                fe[e0 + k] = make_int4(near ? (p & (R - 1)) * RB * BB : -1, (x.x & 7) * 0x01010101, pr.x, pr.y - 2 - pr.x);
+                x.y = pr.x; x.z = pr.y; x.w = pr.z;
+            }
+            ed[e0 + k] = x;
+        }
+        if (STATIC) {
+            const int4 ri = rowi[r];
+            const int eoff = e0 - in_ptr[r & ~(WSTG - 1)];
+            if (r == 0) d = 0;
+            fr[r] = make_int4(ri.x, ri.y - 2 - ri.x, ri.z,
+                              d | (eoff + d > WSTG_E ? FR_UNSTAGED : eoff << FR_EOFF));
+        } else {
+            ra[2 * r] = make_int4(e0, out_ptr[r], g.hlen[beg_i + r] - h0, g.tlen[beg_i + r] - t0);
+            ra[2 * r + 1] = make_int4(g.hlen[r] - h0, g.base[u], d, out_ptr[r + 1] - out_ptr[r]);
+        }
     }
     __syncwarp();
-    v.n = n;
-    v.in_ptr = in_ptr; v.in_row = in_row; v.in_w = in_w; v.in_base = in_base;
-    v.ind = vind;
     return ST_OK;
 }
 
-// Static-band DP fill of one alignment by one warp (see build_view_static).
-// Same recurrences and records as dp_fill (plain.cuh), specialised for the
-// batch:
-//  * row descriptors and predecessor records are staged into shared memory
-//    16 rows at a time (one coalesced round trip), so the row loop reads only
-//    shared memory: descriptors, predecessor blocks from the shared-memory
-//    ring of recent rows (global spill area for rows with distant
-//    successors), the query;
-//  * the horizontal gap recurrence in the form
-//    I[j] = o1 + (j-1)*e1 + max(K, max_{k<j} H0[k]-k*e1), K = NEG_INF+e1-o1,
-//    which also yields I[0] = NEG_INF;
-//  * records: predecessors arrive in the backtrack's priority order, so each
-//    choice (M1 with its weight threshold, M4, D open / extend) is the first
-//    predecessor passing its test; single-predecessor rows keep their blocks
-//    in registers between the two passes.
-constexpr int STAGE_ROWS = 16, STAGE_EDGES = 64;
-
-__device__ __forceinline__ RowDesc load_desc(const RowDesc* p) {
-    const int4* q = reinterpret_cast<const int4*>(p);
-    const int4 a = q[0], b = q[1], c = q[2];
-    RowDesc r;
-    r.bsbe = a.x; r.st = a.y; r.tb = a.z; r.e0 = a.w;
-    r.d = b.x; r.ind = b.y; r.w1ok = b.z; r.prow0 = b.w;
-    r.pbsbe = c.x; r.pst = c.y; r.pbase = c.z; r.pw = c.w;
-    return r;
-}
-
-__device__ __forceinline__ const int32_t* blk_src(const int32_t* ring, const int32_t* rs, int RB, int st) {
-    return st < 0 ? ring + (-st - 1) * RB * 16 : rs + st;
-}
-
-// One row of the warp fill: every chunk of 32 blocks (one block per lane) of
-// row i, whose descriptor is `cur` and whose predecessor records are
-// er_base[cur.e0 + k] in the backtrack's priority order. Predecessor blocks
-// come from blk_src (the shared-memory ring or the slot's row store). With
-// ARGMAX, each lane also keeps the first maximum of M over its cells.
-template <bool ARGMAX, bool TRACK>
-__device__ __forceinline__ void fill_row(const DpArgs& a, const RowDesc& cur, const int4* __restrict__ er_base,
-                                         const int32_t* ring, int RB, const uint8_t* __restrict__ qsm, int i,
-                                         int lane, int32_t& bestM, int& bestJ) {
-    const Scoring sc = a.sc;
-    const int32_t K = add32(add32(NEG_INF, sc.e1), -sc.o1);
-    const int Bs = cur.bsbe & 0xffff, Be = cur.bsbe >> 16, bn = Be - Bs - 1;
-    const int d = cur.d;
-    int32_t* dst = const_cast<int32_t*>(blk_src(ring, a.rs, RB, cur.st));
-    const int nch = (bn + 31) >> 5;
-    int32_t carryP = K, carryM = NEG_INF, carryI = NEG_INF;
-    for (int c = 0; c < nch; c++) {
-        const int b = c * 32 + lane;
-        const bool act = b < bn;
-        const int B = Bs + b;
-        const int j0 = b * BLK;
-        int32_t Mpre[BLK], Dv[BLK], H0[BLK], M[BLK], I[BLK];
-        // X, Y: with one predecessor, its M and D at this block (for the records);
-        // with several and TRACK, the record choices kept while the predecessors
-        // are read: X = m1 | m4 << 16 (first predecessors, in priority order,
-        // reaching the diagonal maximum), Y = dopen | dext << 16 (the vertical
-        // maximum); 511 = none
-        uint32_t X[BLK], Y[BLK];
-        int32_t cmprev = NEG_INF;
-        bool c_blk = false, c_prev = false, slow = !TRACK, slow0 = false;
-        uint32_t hm = 0;  // bit l: Mpre[l] >= Dv[l], then (after the scan) M[l] == Mpre[l]
-        uint32_t qlo = 0x04040404u, qhi = 0x04040404u;
-        const uint32_t xinit = (TRACK && d >= 2) ? 0x01ff01ffu : (uint32_t)NEG_INF;
+// The graph of the first read: source -> one node per base -> sink
+// (src/align.cpp:1747-1753), with the whole warp. Only on a graph without edges.
+__device__ int dg_first_read(DevGraph& g, const uint8_t* rd, int len, int lane) {
+    if (2 + len > g.NC || len + 1 > g.EC) return ST_CAPACITY;
+    for (int x = lane; x < len + 2; x += 32) {
+        // x: node id; edge x - 2 enters a base's node, edge len the sink
+        const int e_in = x == 0 ? -1 : x == 1 ? len : x - 2, e_out = x == 1 ? -1 : x == 0 ? 0 : x - 1;
+        const int b = x < 2 ? 4 : nt4_dev(rd[x - 2]);
+        g.base[x] = (uint8_t)b;
+        g.par[x] = x;
 #pragma unroll
-        for (int l = 0; l < BLK; l++) { Mpre[l] = NEG_INF; Dv[l] = NEG_INF; X[l] = Y[l] = xinit; }
-        if (act) {
-            const uint2 qw = *reinterpret_cast<const uint2*>(qsm + B * BLK);
-            qlo = qw.x;
-            qhi = qw.y;
-            if (i == 0 && b == 0) Mpre[0] = 0;
-            for (int k = 0; k < d; k++) {
-                int pbsbe, pst, pbase;
-                if (k == 0) { pbsbe = cur.pbsbe; pst = cur.pst; pbase = cur.pbase; }
-                else { const int4 er = er_base[cur.e0 + k]; pbsbe = er.x; pst = er.y; pbase = er.w & 255; }
-                const int pBs = pbsbe & 0xffff, pBe = pbsbe >> 16;
-                const int32_t* src = blk_src(ring, a.rs, RB, pst);
-                const PredMask mk = pred_mask(B, pBs, pBe);
-                int32_t Mb[BLK], Db[BLK];
-                int32_t mprev = NEG_INF;
-                if (mk.prev_in) mprev = src[(B - 1 - pBs) * 16 + 7];
-                if (mk.blk_in) {
-                    load_block16(src + (B - pBs) * 16, Mb, Db);
-                    if (TRACK && d >= 2) {
-                        // the maxima of pass1_pred, keeping the first predecessor (in
-                        // priority order) that reaches each final maximum
-                        const int4 erk = er_base[cur.e0 + k];
-                        const uint32_t pos = (uint32_t)erk.z >> 16;
-                        const uint32_t m1v = (erk.w & 256) ? pos : 510u;
-#pragma unroll
-                        for (int l = 0; l < BLK; l++) {
-                            const int32_t co = add32(Mb[l], sc.o1), ce = add32(Db[l], sc.e1);
-                            const int32_t nd = mx(Dv[l], mx(co, ce));
-                            if (nd > Dv[l]) {
-                                Y[l] = (co == nd ? pos : 511u) | ((ce == nd ? pos : 511u) << 16);
-                            } else {
-                                if ((Y[l] & 0xffffu) == 511u && co == nd) Y[l] = (Y[l] & 0xffff0000u) | pos;
-                                if ((Y[l] >> 16) == 511u && ce == nd) Y[l] = (Y[l] & 0xffffu) | (pos << 16);
-                            }
-                            Dv[l] = nd;
-                        }
-                        if (mk.diag) {
-#pragma unroll
-                            for (int l = 0; l < BLK; l++) {
-                                const int qc = (int)(((l < 4 ? qlo : qhi) >> (8 * (l & 3))) & 255);
-                                const bool bm = pbase == qc;
-                                const int32_t src0 = l == 0 ? (b == 0 ? NEG_INF : mprev) : Mb[l > 0 ? l - 1 : 0];
-                                const int32_t cand = add32(src0, bm ? sc.match : sc.mismatch);
-                                const bool tracked = l > 0 || b != 0;  // the backtrack tests this same value
-                                if (cand > Mpre[l]) {
-                                    X[l] = tracked ? ((bm ? m1v : 511u) | (pos << 16)) : 0x01ff01ffu;
-                                } else if (tracked && cand == Mpre[l]) {
-                                    if ((X[l] >> 16) == 511u) X[l] = (X[l] & 0xffffu) | (pos << 16);
-                                    if (bm && (X[l] & 0xffffu) == 511u) X[l] = (X[l] & 0xffff0000u) | m1v;
-                                }
-                                Mpre[l] = mx(Mpre[l], cand);
-                            }
-                        }
-                    } else {
-                        uint8_t qc8[BLK];
-#pragma unroll
-                        for (int l = 0; l < 4; l++) { qc8[l] = (uint8_t)(qlo >> (8 * l)); qc8[4 + l] = (uint8_t)(qhi >> (8 * l)); }
-                        pass1_pred(sc, mk, b == 0, pbase, Mb, Db, mprev, qc8, Mpre, Dv);
-                        if (d == 1) {
-#pragma unroll
-                            for (int l = 0; l < BLK; l++) { X[l] = (uint32_t)Mb[l]; Y[l] = (uint32_t)Db[l]; }
-                        }
-                    }
-                }
-                // where the backtrack's predecessor test and the fill's block-granular
-                // diagonal differ (a predecessor's band starting in this block, or ending
-                // just before it, or the row's first block), the choices are redone with
-                // the backtrack's own test: the whole block in the first case, cell 0 else
-                if (TRACK && d >= 2) {
-                    slow |= mk.blk_in && !mk.diag;
-                    slow0 |= mk.prev_in && !(mk.blk_in && mk.diag && b != 0);
-                }
-                if (d == 1) { cmprev = mprev; c_blk = mk.blk_in; c_prev = mk.prev_in; }
-            }
-        }
-        // prefix max of the scan keys across the warp
-        int32_t agg = INT_MIN;
-#pragma unroll
-        for (int l = 0; l < BLK; l++) {
-            H0[l] = mx(Mpre[l], Dv[l]);
-            if (TRACK && Mpre[l] >= Dv[l]) hm |= 1u << l;
-            agg = mx(agg, add32(H0[l], -(j0 + l) * sc.e1));
-        }
-        if (!act) agg = INT_MIN;
-        const int32_t incl = warp_incl_max(agg);
-        int32_t P = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) P = INT_MIN;
-        P = mx(P, carryP);
-        const int32_t chunk_total = __shfl_sync(0xffffffffu, incl, 31);
-        if (i == 0) {
-#pragma unroll
-            for (int l = 0; l < BLK; l++) { M[l] = H0[l]; I[l] = NEG_INF; }
-        } else {
-            int32_t run = P;
-#pragma unroll
-            for (int l = 0; l < BLK; l++) {
-                I[l] = add32(sc.o1 + (j0 + l - 1) * sc.e1, run);
-                M[l] = mx(H0[l], I[l]);
-                if (TRACK && H0[l] < I[l]) hm &= ~(1u << l);
-                run = mx(run, add32(H0[l], -(j0 + l) * sc.e1));
-            }
-        }
-        if (ARGMAX && act) {
-#pragma unroll
-            for (int l = 0; l < BLK; l++)
-                if (M[l] > bestM) { bestM = M[l]; bestJ = j0 + l; }  // first maximum of the row
-        }
-        const int32_t upM = __shfl_up_sync(0xffffffffu, M[BLK - 1], 1);
-        const int32_t upI = __shfl_up_sync(0xffffffffu, I[BLK - 1], 1);
-        const int32_t Ml0 = lane > 0 ? upM : carryM, Il0 = lane > 0 ? upI : carryI;
-        const int32_t nextM = __shfl_sync(0xffffffffu, M[BLK - 1], 31);
-        const int32_t nextI = __shfl_sync(0xffffffffu, I[BLK - 1], 31);
-        if (act) {
-            if (d <= 1) {
-                uint32_t lo = 0, hi = 0;
-#pragma unroll
-                for (int l = 0; l < BLK; l++) {
-                    const int32_t Ml = l > 0 ? M[l - 1] : Ml0, Il = l > 0 ? I[l - 1] : Il0;
-                    uint32_t r = own_flags(sc, j0 + l, M[l], Dv[l], I[l], Ml, Il);
-                    if (d == 1) {
-                        const int qc = (int)(((l < 4 ? qlo : qhi) >> (8 * (l & 3))) & 255);
-                        const bool inr = l == 0 ? c_prev : c_blk;
-                        const int32_t mv = l == 0 ? cmprev : (int32_t)X[l > 0 ? l - 1 : 0];
-                        const bool bm = cur.pbase == qc;
-                        const bool eqM = inr && M[l] == add32(mv, bm ? sc.match : sc.mismatch);
-                        if (eqM) r |= R_M4;
-                        if (eqM && bm && cur.w1ok) r |= R_M1;
-                        if (c_blk && Dv[l] == add32((int32_t)X[l], sc.o1)) r |= R_DOPEN;
-                        else if (c_blk && Dv[l] == add32((int32_t)Y[l], sc.e1)) r |= R_DEXT;
-                    }
-                    if (l < 4) lo |= r << (8 * l);
-                    else hi |= r << (8 * (l - 4));
-                }
-                *reinterpret_cast<uint2*>(a.tb + cur.tb + b * BLK) = make_uint2(lo, hi);
-            } else {
-                // choices per cell: m1 | m4 << 16, dopen | dext << 16 (511 = none,
-                // 510 = the best matching predecessor failed the weight threshold)
-                uint32_t* cm = X;
-                uint32_t* cd = Y;
-                if (!slow) {
-                    // tracked choices stand where M is the diagonal maximum itself
-#pragma unroll
-                    for (int l = 0; l < BLK; l++)
-                        if (!((hm >> l) & 1u)) cm[l] = 0x01ff01ffu;
-                    if (slow0) {
-                        // cell 0 by the backtrack's own test, over every predecessor
-                        uint32_t c0 = 0x01ff01ffu;
-                        const int qc = (int)(qlo & 255u);
-                        for (int k = 0; k < d; k++) {
-                            const int4 er = er_base[cur.e0 + k];
-                            const int pBs = er.x & 0xffff, pBe = er.x >> 16;
-                            if (!(B - 1 >= pBs && B - 1 <= pBe - 2)) continue;  // prev_in
-                            const int32_t mv = blk_src(ring, a.rs, RB, er.y)[(B - 1 - pBs) * 16 + 7];
-                            const uint32_t pos = (uint32_t)er.z >> 16;
-                            const bool bm = (er.w & 255) == qc;
-                            if (M[0] != add32(mv, bm ? sc.match : sc.mismatch)) continue;
-                            if ((c0 >> 16) == 511u) c0 = (c0 & 0xffffu) | (pos << 16);
-                            if (bm && (c0 & 0xffffu) == 511u) c0 = (c0 & 0xffff0000u) | ((er.w & 256) ? pos : 510u);
-                        }
-                        cm[0] = c0;
-                    }
-                }
-#pragma unroll
-                for (int l = 0; l < BLK; l++)
-                    if (slow) { cm[l] = 0x01ff01ffu; cd[l] = 0x01ff01ffu; }
-                for (int k = 0; k < (slow ? d : 0); k++) {
-                    const int4 er = er_base[cur.e0 + k];
-                    const int pBs = er.x & 0xffff, pBe = er.x >> 16;
-                    const int32_t* src = blk_src(ring, a.rs, RB, er.y);
-                    const PredMask mk = pred_mask(B, pBs, pBe);
-                    if (!(mk.blk_in || mk.prev_in)) continue;
-                    const uint32_t pos = (uint32_t)er.z >> 16;
-                    const int pbase = er.w & 255;
-                    const uint32_t m1v = (er.w & 256) ? pos : 510u;
-                    int32_t Mb[BLK], Db[BLK];
-                    int32_t mprev = NEG_INF;
-                    if (mk.prev_in) mprev = src[(B - 1 - pBs) * 16 + 7];
-                    if (mk.blk_in) load_block16(src + (B - pBs) * 16, Mb, Db);
-                    else {
-#pragma unroll
-                        for (int l = 0; l < BLK; l++) Mb[l] = Db[l] = NEG_INF;
-                    }
-#pragma unroll
-                    for (int l = 0; l < BLK; l++) {
-                        const int qc = (int)(((l < 4 ? qlo : qhi) >> (8 * (l & 3))) & 255);
-                        const bool inr = l == 0 ? mk.prev_in : mk.blk_in;
-                        const int32_t mv = l == 0 ? mprev : Mb[l > 0 ? l - 1 : 0];
-                        const bool bm = pbase == qc;
-                        const bool eqM = inr && M[l] == add32(mv, bm ? sc.match : sc.mismatch);
-                        if (eqM && (cm[l] >> 16) == 511u) cm[l] = (cm[l] & 0xffffu) | (pos << 16);
-                        if (eqM && bm && (cm[l] & 0xffffu) == 511u) cm[l] = (cm[l] & 0xffff0000u) | m1v;
-                        if (mk.blk_in) {
-                            if ((cd[l] & 0xffffu) == 511u && Dv[l] == add32(Mb[l], sc.o1))
-                                cd[l] = (cd[l] & 0xffff0000u) | pos;
-                            if ((cd[l] >> 16) == 511u && Dv[l] == add32(Db[l], sc.e1))
-                                cd[l] = (cd[l] & 0xffffu) | (pos << 16);
-                        }
-                    }
-                }
-                uint32_t r[BLK];
-#pragma unroll
-                for (int l = 0; l < BLK; l++) {
-                    const int32_t Ml = l > 0 ? M[l - 1] : Ml0, Il = l > 0 ? I[l - 1] : Il0;
-                    uint32_t w = own_flags(sc, j0 + l, M[l], Dv[l], I[l], Ml, Il) & 15u;
-                    uint32_t m1 = cm[l] & 0xffffu, m4 = cm[l] >> 16;
-                    if (m1 == 510u) m1 = W_NONE;
-                    uint32_t dd = cd[l] & 0xffffu;
-                    if (dd == 511u) {
-                        dd = cd[l] >> 16;
-                        if (dd != 511u) w |= W_DEXT;
-                    }
-                    r[l] = w | (m1 << W_M1_SHIFT) | (m4 << W_M4_SHIFT) | (dd << W_D_SHIFT);
-                }
-                uint4* tdst = reinterpret_cast<uint4*>(a.tb + cur.tb + b * BLK * 4);
-                tdst[0] = make_uint4(r[0], r[1], r[2], r[3]);
-                tdst[1] = make_uint4(r[4], r[5], r[6], r[7]);
-            }
-            store_block16(dst + b * 16, M, Dv);
-        }
-        carryP = mx(carryP, chunk_total);
-        carryM = nextM;
-        carryI = nextI;
-    }
-}
-
-// One row of the adaptive / full-band warp fill (dp_fill_warp_dyn): the chunk
-// loop of fill_row, with the predecessors' records `er` (backtrack priority
-// order, bands and row-store locations patched in) read once per chunk, and
-// the record choices of multi-predecessor rows kept in one pass
-// (dp_core.h track_d / track_m): per cell the running maximum of each kind
-// of term plus a 4-bit first position per choice, folded into one 16-bit
-// word (z) as soon as the predecessors are read:
-//   z bits 0..3 D choice (dopen, else dext; 15 none), bit 4 W_DEXT,
-//          8..11 m4, 12..15 m1 (15 none; gated by M == Mpre at the record).
-// Register roles by row kind: with one predecessor Mpre / Dv are the
-// diagonal / vertical maxima and pa / pb copies of its M / D block (for the
-// 1-byte records); with several, Mpre is the diagonal maximum, Dv the
-// maximum of M_p + o1, pb of D_p + e1 and pa of the matching diagonal terms
-// until the pass ends, when Dv becomes the vertical maximum.
-// Rows with more than TRACK_MAX_D predecessors, and blocks where the fill's
-// block-granular masks differ from the backtrack's per-cell test, take the
-// second pass over the predecessors (as fill_row does).
-template <bool ARGMAX>
-__device__ __forceinline__ void fill_row_dyn(const DpArgs& a, const RowDesc& cur, const int4* __restrict__ er,
-                                             const uint8_t* __restrict__ qsm, int i, int lane, int32_t& bestM,
-                                             int& bestJ) {
-    const Scoring sc = a.sc;
-    const int32_t K = add32(add32(NEG_INF, sc.e1), -sc.o1);
-    const int Bs = cur.bsbe & 0xffff, Be = cur.bsbe >> 16, bn = Be - Bs - 1;
-    const int d = cur.d;
-    const bool multi = d >= 2;
-    int32_t* dst = a.rs + cur.st;
-    const int nch = (bn + 31) >> 5;
-    int32_t carryP = K, carryM = NEG_INF, carryI = NEG_INF;
-    for (int c = 0; c < nch; c++) {
-        const int b = c * 32 + lane;
-        const bool act = b < bn;
-        const int B = Bs + b;
-        const int j0 = b * BLK;
-        int32_t Mpre[BLK], Dv[BLK], H0[BLK], M[BLK], I[BLK];
-        int32_t pa[BLK], pb[BLK];
-        uint32_t z2[BLK / 2];  // choice words: cell 2t in bits 0..15, cell 2t+1 in bits 16..31
-        int32_t cmprev = NEG_INF;
-        bool c_blk = false, c_prev = false, slow = d > TRACK_MAX_D, slow0 = false;
-        uint32_t f1lo = 0, f1hi = 0, m1lo = 0, m1hi = 0;  // one predecessor: record flags, see below
-        uint32_t hm = 0;  // bit l: Mpre[l] >= Dv[l], then (after the scan) M[l] == Mpre[l]
-        uint32_t qlo = 0x04040404u, qhi = 0x04040404u;
-        const int32_t minit = multi ? INT_MIN : NEG_INF;
-#pragma unroll
-        for (int l = 0; l < BLK; l++) Mpre[l] = Dv[l] = pa[l] = pb[l] = minit;
-#pragma unroll
-        for (int t = 0; t < BLK / 2; t++) z2[t] = 0xffffffffu;
-        if (act) {
-            const uint2 qw = *reinterpret_cast<const uint2*>(qsm + B * BLK);
-            qlo = qw.x;
-            qhi = qw.y;
-            if (i == 0 && b == 0) Mpre[0] = 0;
-        }
-        auto qc_at = [&](int l) { return (int)(((l < 4 ? qlo : qhi) >> (8 * (l & 3))) & 255u); };
-        if (act) {
-            for (int k = 0; k < d; k++) {
-                const int4 ek = er[k];
-                const int pBs = ek.x & 0xffff, pBe = ek.x >> 16;
-                const int32_t* src = a.rs + ek.y;
-                const int pbase = ek.w & 255;
-                const PredMask mk = pred_mask(B, pBs, pBe);
-                int32_t mprev = NEG_INF;
-                if (mk.prev_in) mprev = src[(B - 1 - pBs) * 16 + 7];
-                if (mk.blk_in) {
-                    int32_t Mb[BLK], Db[BLK];
-                    load_block16(src + (B - pBs) * 16, Mb, Db);
-                    if (multi) {
-                        const uint32_t pos = ((uint32_t)ek.z >> 16) & 15u;  // exact when d <= TRACK_MAX_D
-                        const uint32_t p1 = (ek.w & 256) ? pos : Y_NONE;
-#pragma unroll
-                        for (int l = 0; l < BLK; l++)
-                            track_d(sc, Mb[l], Db[l], pos, Dv[l], pb[l], z2[l >> 1], 16 * (l & 1));
-                        if (mk.diag) {
-                            // cell 0 of the row's first block reads NEG_INF (the lane quirk); the
-                            // backtrack never takes that term, so it records no position
-                            const bool first = b == 0;
-                            const bool bm0 = pbase == qc_at(0);
-                            track_m(add32(first ? NEG_INF : mprev, bm0 ? sc.match : sc.mismatch), bm0,
-                                    first ? Y_NONE : pos, first ? Y_NONE : p1, Mpre[0], pa[0], z2[0], 0);
-#pragma unroll
-                            for (int l = 1; l < BLK; l++) {
-                                const bool bm = pbase == qc_at(l);
-                                track_m(add32(Mb[l - 1], bm ? sc.match : sc.mismatch), bm, pos, p1, Mpre[l], pa[l],
-                                        z2[l >> 1], 16 * (l & 1));
-                            }
-                        }
-                    } else {
-                        // one predecessor: its terms and, while they are in registers, the
-                        // 1-byte record's predecessor flags (byte l of f1lo / f1hi): the
-                        // vertical choice (the fill's and the backtrack's vertical tests are
-                        // the same block test) and the diagonal one, which stands when
-                        // M == Mpre (checked after the scan) wherever the fill's diagonal
-                        // mask matches the backtrack's per-cell test (else slow: recomputed)
-#pragma unroll
-                        for (int l = 0; l < BLK; l++) {
-                            const int32_t ce = add32(Db[l], sc.e1), co = add32(Mb[l], sc.o1);
-                            const int32_t dv = mx(mx(NEG_INF, ce), co);
-                            Dv[l] = dv;
-                            const uint32_t fd = co == dv ? R_DOPEN : (ce == dv ? R_DEXT : 0u);
-                            if (l < 4) f1lo |= fd << (8 * l);
-                            else f1hi |= fd << (8 * (l - 4));
-                        }
-                        if (mk.diag) {
-#pragma unroll
-                            for (int l = 0; l < BLK; l++) {
-                                const bool bm = pbase == qc_at(l);
-                                const int32_t src0 = l == 0 ? (b == 0 ? NEG_INF : mprev) : Mb[l > 0 ? l - 1 : 0];
-                                const int32_t cand = add32(src0, bm ? sc.match : sc.mismatch);
-                                const int32_t mp = mx(NEG_INF, cand);
-                                Mpre[l] = mp;
-                                // cell 0 counts only where the backtrack tests the same value
-                                const bool tested = l > 0 || (mk.prev_in && b != 0);
-                                const uint32_t fm = (tested && cand == mp) ? (R_M4 | ((bm && cur.w1ok) ? R_M1 : 0u)) : 0u;
-                                if (l < 4) m1lo |= fm << (8 * l);
-                                else m1hi |= fm << (8 * (l - 4));
-                            }
-                        }
-                    }
-                }
-                if (multi) {
-                    slow |= mk.blk_in && !mk.diag;
-                    slow0 |= mk.prev_in && !(mk.blk_in && mk.diag && b != 0);
-                } else {
-                    cmprev = mprev; c_blk = mk.blk_in; c_prev = mk.prev_in;
-                    slow |= (mk.blk_in && !mk.diag) || (mk.prev_in && !(mk.blk_in && mk.diag && b != 0));
-                }
-            }
-        }
-        if (multi) {
-            // final maxima, and the choices folded into z (see above)
-#pragma unroll
-            for (int l = 0; l < BLK; l++) {
-                const int sh = 16 * (l & 1);
-                const uint32_t y = (z2[l >> 1] >> sh) & 0xffffu;
-                const int32_t mp = mx(NEG_INF, Mpre[l]);
-                const int32_t dv = mx(NEG_INF, mx(Dv[l], pb[l]));  // Dv: max of M_p + o1, pb: of D_p + e1
-                const bool okO = Dv[l] == dv, okE = pb[l] == dv;
-                uint32_t w = okO ? (y & 15u) : (okE ? (((y >> Y_E) & 15u) | W_DEXT) : Y_NONE);
-                w |= Mpre[l] == mp ? (y & 0x0f00u) : 0x0f00u;
-                w |= pa[l] == mp ? (y & 0xf000u) : 0xf000u;
-                z2[l >> 1] = (z2[l >> 1] & ~(0xffffu << sh)) | (w << sh);
-                Mpre[l] = mp;
-                Dv[l] = dv;
-            }
-        }
-        // prefix max of the scan keys across the warp
-        int32_t agg = INT_MIN;
-#pragma unroll
-        for (int l = 0; l < BLK; l++) {
-            H0[l] = mx(Mpre[l], Dv[l]);
-            if (Mpre[l] >= Dv[l]) hm |= 1u << l;
-            agg = mx(agg, add32(H0[l], -(j0 + l) * sc.e1));
-        }
-        if (!act) agg = INT_MIN;
-        const int32_t incl = warp_incl_max(agg);
-        int32_t P = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) P = INT_MIN;
-        P = mx(P, carryP);
-        const int32_t chunk_total = __shfl_sync(0xffffffffu, incl, 31);
-        if (i == 0) {
-#pragma unroll
-            for (int l = 0; l < BLK; l++) { M[l] = H0[l]; I[l] = NEG_INF; }
-        } else {
-            int32_t run = P;
-#pragma unroll
-            for (int l = 0; l < BLK; l++) {
-                I[l] = add32(sc.o1 + (j0 + l - 1) * sc.e1, run);
-                M[l] = mx(H0[l], I[l]);
-                if (H0[l] < I[l]) hm &= ~(1u << l);
-                run = mx(run, add32(H0[l], -(j0 + l) * sc.e1));
-            }
-        }
-        if (ARGMAX && act) {
-#pragma unroll
-            for (int l = 0; l < BLK; l++)
-                if (M[l] > bestM) { bestM = M[l]; bestJ = j0 + l; }  // first maximum of the row
-        }
-        const int32_t upM = __shfl_up_sync(0xffffffffu, M[BLK - 1], 1);
-        const int32_t upI = __shfl_up_sync(0xffffffffu, I[BLK - 1], 1);
-        const int32_t Ml0 = lane > 0 ? upM : carryM, Il0 = lane > 0 ? upI : carryI;
-        const int32_t nextM = __shfl_sync(0xffffffffu, M[BLK - 1], 31);
-        const int32_t nextI = __shfl_sync(0xffffffffu, I[BLK - 1], 31);
-        if (act) {
-            if (!multi) {
-                uint32_t lo = 0, hi = 0;
-#pragma unroll
-                for (int l = 0; l < BLK; l++) {
-                    const int32_t Ml = l > 0 ? M[l - 1] : Ml0, Il = l > 0 ? I[l - 1] : Il0;
-                    const uint32_t r = own_flags(sc, j0 + l, M[l], Dv[l], I[l], Ml, Il);
-                    if (l < 4) lo |= r << (8 * l);
-                    else hi |= r << (8 * (l - 4));
-                }
-                if (d == 1) {
-                    // the diagonal flags stand in cells where M == Mpre (byte mask of hm)
-                    const uint32_t hlo = ((hm & 15u) * 0x00204081u & 0x01010101u) * 0xffu;
-                    const uint32_t hhi = ((hm >> 4) * 0x00204081u & 0x01010101u) * 0xffu;
-                    lo |= f1lo | (m1lo & hlo);
-                    hi |= f1hi | (m1hi & hhi);
-                    if (slow) {
-                        // a block where the fill's diagonal mask and the backtrack's per-cell
-                        // test differ: the diagonal flags by the backtrack's own test
-                        const int pBs = cur.pbsbe & 0xffff;
-                        const int32_t* src = a.rs + cur.pst;
-                        int32_t Mb[BLK];
-#pragma unroll
-                        for (int l = 0; l < BLK; l++) Mb[l] = NEG_INF;
-                        if (c_blk) {
-                            const int4* q = reinterpret_cast<const int4*>(src + (B - pBs) * 16);
-                            const int4 u = q[0], v = q[1];
-                            Mb[0] = u.x; Mb[1] = u.y; Mb[2] = u.z; Mb[3] = u.w;
-                            Mb[4] = v.x; Mb[5] = v.y; Mb[6] = v.z; Mb[7] = v.w;
-                        }
-                        lo &= ~0x30303030u;
-                        hi &= ~0x30303030u;
-#pragma unroll
-                        for (int l = 0; l < BLK; l++) {
-                            const bool inr = l == 0 ? c_prev : c_blk;
-                            const int32_t mv = l == 0 ? cmprev : Mb[l > 0 ? l - 1 : 0];
-                            const bool bm = cur.pbase == qc_at(l);
-                            const bool eqM = inr && M[l] == add32(mv, bm ? sc.match : sc.mismatch);
-                            const uint32_t fm = eqM ? (R_M4 | ((bm && cur.w1ok) ? R_M1 : 0u)) : 0u;
-                            if (l < 4) lo |= fm << (8 * l);
-                            else hi |= fm << (8 * (l - 4));
-                        }
-                    }
-                }
-                *reinterpret_cast<uint2*>(a.tb + cur.tb + b * BLK) = make_uint2(lo, hi);
-            } else {
-                uint32_t r[BLK];
-                if (!slow) {
-                    uint32_t c0 = 0x01ff01ffu;
-                    if (slow0) {
-                        // cell 0 by the backtrack's own test, over every predecessor
-                        const int qc = qc_at(0);
-                        for (int k = 0; k < d; k++) {
-                            const int4 ek = er[k];
-                            const int pBs = ek.x & 0xffff, pBe = ek.x >> 16;
-                            if (!(B - 1 >= pBs && B - 1 <= pBe - 2)) continue;  // prev_in
-                            const int32_t mv = a.rs[ek.y + (B - 1 - pBs) * 16 + 7];
-                            const uint32_t pos = (uint32_t)ek.z >> 16;
-                            const bool bm = (ek.w & 255) == qc;
-                            if (M[0] != add32(mv, bm ? sc.match : sc.mismatch)) continue;
-                            if ((c0 >> 16) == 511u) c0 = (c0 & 0xffffu) | (pos << 16);
-                            if (bm && (c0 & 0xffffu) == 511u) c0 = (c0 & 0xffff0000u) | ((ek.w & 256) ? pos : 510u);
-                        }
-                    }
-#pragma unroll
-                    for (int l = 0; l < BLK; l++) {
-                        const int32_t Ml = l > 0 ? M[l - 1] : Ml0, Il = l > 0 ? I[l - 1] : Il0;
-                        const uint32_t own = own_flags(sc, j0 + l, M[l], Dv[l], I[l], Ml, Il) & 15u;
-                        const uint32_t w = (z2[l >> 1] >> (16 * (l & 1))) & 0xffffu;
-                        const bool h = (hm >> l) & 1u;
-                        const uint32_t n4 = (w >> Y_4) & 15u, n1 = (w >> Y_1) & 15u, nd = w & 15u;
-                        uint32_t m4 = (h && n4 != Y_NONE) ? n4 : W_NONE;
-                        uint32_t m1 = (h && n1 != Y_NONE) ? n1 : W_NONE;
-                        if (l == 0 && slow0) {
-                            m1 = c0 & 0xffffu;
-                            if (m1 == 510u) m1 = W_NONE;
-                            m4 = c0 >> 16;
-                        }
-                        const uint32_t dd = nd != Y_NONE ? nd : W_NONE;
-                        r[l] = own | (w & W_DEXT) | (m1 << W_M1_SHIFT) | (m4 << W_M4_SHIFT) | (dd << W_D_SHIFT);
-                    }
-                } else {
-                    // the diagonal choices by the backtrack's own test, over every predecessor;
-                    // the vertical choices in z stand (the fill's and the backtrack's vertical
-                    // tests are the same block test) unless the row has more predecessors
-                    // than z's 4-bit positions hold
-                    const bool dwide = d > TRACK_MAX_D;
-                    uint32_t cm[BLK], cd[BLK];
-#pragma unroll
-                    for (int l = 0; l < BLK; l++) cm[l] = cd[l] = 0x01ff01ffu;
-                    for (int k = 0; k < d; k++) {
-                        const int4 ek = er[k];
-                        const int pBs = ek.x & 0xffff, pBe = ek.x >> 16;
-                        const int32_t* src = a.rs + ek.y;
-                        const PredMask mk = pred_mask(B, pBs, pBe);
-                        if (!(mk.blk_in || mk.prev_in)) continue;
-                        const uint32_t pos = (uint32_t)ek.z >> 16;
-                        const int pbase = ek.w & 255;
-                        const uint32_t m1v = (ek.w & 256) ? pos : 510u;
-                        int32_t Mb[BLK];
-                        int32_t mprev = NEG_INF;
-                        if (mk.prev_in) mprev = src[(B - 1 - pBs) * 16 + 7];
-                        if (mk.blk_in) {
-                            const int4* q = reinterpret_cast<const int4*>(src + (B - pBs) * 16);
-                            const int4 u = q[0], v = q[1];
-                            Mb[0] = u.x; Mb[1] = u.y; Mb[2] = u.z; Mb[3] = u.w;
-                            Mb[4] = v.x; Mb[5] = v.y; Mb[6] = v.z; Mb[7] = v.w;
-                            if (dwide) {
-                                const int4 x = q[2], y = q[3];
-                                const int32_t Db[BLK] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-#pragma unroll
-                                for (int l = 0; l < BLK; l++) {
-                                    if ((cd[l] & 0xffffu) == 511u && Dv[l] == add32(Mb[l], sc.o1))
-                                        cd[l] = (cd[l] & 0xffff0000u) | pos;
-                                    if ((cd[l] >> 16) == 511u && Dv[l] == add32(Db[l], sc.e1))
-                                        cd[l] = (cd[l] & 0xffffu) | (pos << 16);
-                                }
-                            }
-                        } else {
-#pragma unroll
-                            for (int l = 0; l < BLK; l++) Mb[l] = NEG_INF;
-                        }
-#pragma unroll
-                        for (int l = 0; l < BLK; l++) {
-                            const bool inr = l == 0 ? mk.prev_in : mk.blk_in;
-                            const int32_t mv = l == 0 ? mprev : Mb[l > 0 ? l - 1 : 0];
-                            const bool bm = pbase == qc_at(l);
-                            const bool eqM = inr && M[l] == add32(mv, bm ? sc.match : sc.mismatch);
-                            if (eqM && (cm[l] >> 16) == 511u) cm[l] = (cm[l] & 0xffffu) | (pos << 16);
-                            if (eqM && bm && (cm[l] & 0xffffu) == 511u) cm[l] = (cm[l] & 0xffff0000u) | m1v;
-                        }
-                    }
-#pragma unroll
-                    for (int l = 0; l < BLK; l++) {
-                        const int32_t Ml = l > 0 ? M[l - 1] : Ml0, Il = l > 0 ? I[l - 1] : Il0;
-                        const uint32_t own = own_flags(sc, j0 + l, M[l], Dv[l], I[l], Ml, Il) & 15u;
-                        const uint32_t w = (z2[l >> 1] >> (16 * (l & 1))) & 0xffffu;
-                        uint32_t m1 = cm[l] & 0xffffu;
-                        if (m1 == 510u) m1 = W_NONE;
-                        const uint32_t m4 = cm[l] >> 16, nd = w & 15u;
-                        uint32_t dd = nd != Y_NONE ? nd : W_NONE, dext = w & W_DEXT;
-                        if (dwide) {
-                            dd = cd[l] & 0xffffu;
-                            dext = 0;
-                            if (dd == 511u) {
-                                dd = cd[l] >> 16;
-                                if (dd != 511u) dext = W_DEXT;
-                            }
-                        }
-                        r[l] = own | dext | (m1 << W_M1_SHIFT) | (m4 << W_M4_SHIFT) | (dd << W_D_SHIFT);
-                    }
-                }
-                uint4* tdst = reinterpret_cast<uint4*>(a.tb + cur.tb + b * BLK * 4);
-                tdst[0] = make_uint4(r[0], r[1], r[2], r[3]);
-                tdst[1] = make_uint4(r[4], r[5], r[6], r[7]);
-            }
-            store_block16(dst + b * 16, M, Dv);
-        }
-        carryP = mx(carryP, chunk_total);
-        carryM = nextM;
-        carryI = nextI;
-    }
-}
-
-__device__ void dp_fill_warp_static(const DpArgs& a, const RowDesc* __restrict__ desc, const int4* __restrict__ erec,
-                                    int32_t* ring, int RB, const uint8_t* qsm, unsigned char* stage, int lane) {
-    const int n = a.v.n, m = a.qlen + 1;
-    const Scoring sc = a.sc;
-    const int32_t K = add32(add32(NEG_INF, sc.e1), -sc.o1);
-    RowDesc* sdesc = reinterpret_cast<RowDesc*>(stage);
-    int4* serec = reinterpret_cast<int4*>(stage + STAGE_ROWS * sizeof(RowDesc));
-    int64_t cells = 0, ecells = 0;
-    for (int i0 = 0; i0 < n; i0 += STAGE_ROWS) {
-        const int cnt = min(STAGE_ROWS, n - i0);
-        // stage: descriptors of rows i0.., and their predecessor records when they fit
-        __syncwarp();
-        {
-            const int4* src = reinterpret_cast<const int4*>(desc + i0);
-            for (int x = lane; x < cnt * 3; x += 32) reinterpret_cast<int4*>(sdesc)[x] = src[x];
-        }
-        __syncwarp();
-        const int e_lo = sdesc[0].e0;
-        const int e_hi = sdesc[cnt - 1].e0 + sdesc[cnt - 1].d;
-        const bool staged = e_hi - e_lo <= STAGE_EDGES;
-        if (staged)
-            for (int e = lane; e < e_hi - e_lo; e += 32) serec[e] = erec[e_lo + e];
-        __syncwarp();
-        const int4* er_base = staged ? serec - e_lo : erec;
-        for (int i = i0; i < i0 + cnt; i++) {
-            const RowDesc cur = sdesc[i - i0];
-            const int64_t rc = (int64_t)((cur.bsbe >> 16) - (cur.bsbe & 0xffff) - 1) * BLK;
-            cells += rc;
-            ecells += rc * cur.d;
-            int32_t bm = 0;
-            int bj = 0;
-            fill_row<false, false>(a, cur, er_base, ring, RB, qsm, i, lane, bm, bj);
-            __syncwarp();
+        for (int k = 0; k < 5; k++) g.aligned[x * 5 + k] = k == b ? x : -1;
+        g.ind[x] = x != 0;
+        g.in_head[x] = g.in_tail[x] = g.hin[x] = e_in;
+        g.out_head[x] = g.out_tail[x] = g.hout[x] = e_out;
+        g.in_cnt[x] = x != 0;
+        g.out_cnt[x] = x != 1;
+        g.stamp[x] = 0;
+        if (x != 1) {  // the edge out of x
+            const int e = e_out;
+            g.e_from[e] = x;
+            g.e_to[e] = e == len ? 1 : e + 2;
+            g.e_w[e] = 1;
+            g.e_nin[e] = g.e_nout[e] = -1;
         }
     }
+    __syncwarp();
     if (lane == 0) {
-        const RowMeta last = a.meta[n - 1];
-        const int jm = m - last.Bs * BLK;
-        const int32_t* src = blk_src(ring, a.rs, RB, (int)last.st);
-        a.out[1] = src[(jm / BLK) * 16 + jm % BLK];
-        a.out[3] = (int32_t)(cells > INT_MAX ? INT_MAX : cells);
-        a.out[6] = (int32_t)(ecells > INT_MAX ? INT_MAX : ecells);
-        a.out[0] = ST_OK;
+        g.hdr[0] = len + 2;
+        g.hdr[1] = len + 1;
     }
     __syncwarp();
+    return ST_OK;
 }
 
-// Warp fill for bands known only row by row (adaptive band, -B; or the full
-// band, f = 0): the same chunk loop and records as the static fill
-// (fill_row), with each row's descriptor assembled when the row is reached:
-// its band from the adaptive state (row_band), its row-store location (a
-// full-width ring of ring_rows rows in the slot; rows with a successor
-// ring_rows or more rows ahead go to the spill area), its record offset (a
-// running sum), and its predecessor records with the predecessors' bands
-// and locations (staged in shared memory). After an adaptive row the warp
-// finds the first maximum of M and lane 0 updates the adaptive state
-// (src/align.cpp:1516-1568). out[4] / out[5]: record bytes and spilled
-// row-store entries used.
-constexpr int DYN_STAGE_EDGES = 128;
-__device__ void dp_fill_warp_dyn(const DpArgs& a, int4* __restrict__ erec, const int32_t* __restrict__ vmaxs,
-                                 const uint8_t* __restrict__ qsm, int4* sed, int32_t* upd, int lane) {
-    const int n = a.v.n, m = a.qlen + 1;
-    const bool adaptive = a.f > 0 && a.ab_band;
-    if (adaptive)
-        for (int r = lane; r < n; r += 32) adaptive_init_entry(a, r, m);
-    __syncwarp();
-    const int64_t ring_part = (int64_t)a.ring_rows * a.ring_blocks * 16;
-    int64_t st_next = ring_part, tb_next = 0, cells = 0, ecells = 0;
-    for (int i = 0; i < n; i++) {
-        int Bs, Be;
-        row_band(a, i, m, Bs, Be);
-        if (i == 0) Bs = 0;
-        const int bn = Be - Bs - 1;
-        const int e0 = a.v.in_ptr[i];
-        const int d = i == 0 ? 0 : a.v.in_ptr[i + 1] - e0;
-        const int bpc = d >= 2 ? 4 : 1;
-        const bool spill = a.ring_rows <= 0 || (vmaxs[i] - i >= a.ring_rows) || bn > a.ring_blocks;
-        const int64_t row_st = spill ? st_next : (int64_t)(i % a.ring_rows) * a.ring_blocks * 16;
-        int st = ST_OK;
-        if (bn < 0) st = ST_DEGENERATE;
-        else if (d > MAX_MULTI_PRED) st = ST_INDEGREE;
-        else if ((spill && row_st + (int64_t)bn * 16 > a.rs_cap) || tb_next + (int64_t)bn * BLK * bpc > a.tb_cap ||
-                 row_st > INT_MAX || tb_next > INT_MAX)
-            st = ST_OOM;
-        if (st != ST_OK) {
-            if (lane == 0) a.out[0] = st;
-            __syncwarp();
-            return;
-        }
-        if (spill) st_next = row_st + (int64_t)bn * 16;
-        if (lane == 0) {
-            RowMeta rm;
-            rm.Bs = Bs; rm.Be = Be; rm.st = row_st; rm.tb = tb_next;
-            a.meta[i] = rm;
-        }
-        // the adaptive update's inputs, copied while the row is filled
-        int ns = 0, base_i = 0, hql = 0;
-        bool pf = false;
-        if (adaptive && i >= 1) {
-            const int o0 = a.v.out_ptr[i];
-            ns = a.v.out_ptr[i + 1] - o0;
-            base_i = a.v.base[i];
-            hql = a.v.hq_loc[i];
-            pf = d <= 32 && ns <= 32;
-            if (pf) {
-                const int32_t* st_ = a.state;
-                if (lane < ns) {
-                    const int sr = a.v.out_row[o0 + lane];
-                    upd[UPD_SROW + lane] = sr;
-                    cp_async4(upd + UPD_SOL + lane, st_ + AB_OL * n + sr);
-                    cp_async4(upd + UPD_SOR + lane, st_ + AB_OR * n + sr);
-                    cp_async4(upd + UPD_SPL + lane, st_ + AB_PL * n + sr);
-                    cp_async4(upd + UPD_SPR + lane, st_ + AB_PR * n + sr);
-                    cp_async4(upd + UPD_SOW + lane, st_ + AB_OW * n + sr);
-                }
-                if (lane < 4) {
-                    const int arr = lane == 0 ? AB_SL : lane == 1 ? AB_OW : lane == 2 ? AB_OL : AB_OR;
-                    cp_async4(upd + UPD_OWN + lane, st_ + arr * n + i);
-                }
-            }
-        }
-        // predecessor records with the predecessors' bands and locations
-        int4* er = d <= DYN_STAGE_EDGES ? sed : erec + e0;
-        for (int k = lane; k < d; k += 32) {
-            int4 rec = erec[e0 + k];
-            if (pf) {
-                cp_async4(upd + UPD_PSL + k, a.state + AB_SL * n + rec.x);
-                cp_async4(upd + UPD_PMP + k, a.state + AB_MP * n + rec.x);
-            }
-            const RowMeta pm = a.meta[rec.x];
-            rec.x = pm.Bs | (pm.Be << 16);
-            rec.y = (int32_t)pm.st;
-            er[k] = rec;
-        }
-        if (pf) cp_async_commit_all();
-        __syncwarp();
-        RowDesc cur;
-        cur.bsbe = Bs | (Be << 16);
-        cur.st = (int32_t)row_st;
-        cur.tb = (int32_t)tb_next;
-        cur.e0 = 0;
-        cur.d = d;
-        cur.ind = a.v.ind[i];
-        if (d >= 1) {
-            const int4 r0 = er[0];
-            cur.pbsbe = r0.x; cur.pst = r0.y; cur.pbase = r0.w & 255; cur.pw = r0.z & 0xffff;
-            cur.w1ok = (r0.w >> 8) & 1;
-            cur.prow0 = 0;
-        } else {
-            cur.pbsbe = cur.pst = cur.pbase = cur.pw = cur.w1ok = cur.prow0 = 0;
-        }
-        int32_t bestM = INT_MIN;
-        int bestJ = 0;
-        if (adaptive) fill_row_dyn<true>(a, cur, er, qsm, i, lane, bestM, bestJ);
-        else fill_row_dyn<false>(a, cur, er, qsm, i, lane, bestM, bestJ);
-        cells += (int64_t)bn * BLK;
-        ecells += (int64_t)bn * BLK * d;
-        if (adaptive && i >= 1) {
-            // first maximum of the row: largest M, then smallest column
-            unsigned long long key = bestM == INT_MIN ? 0ull
-                                     : ((unsigned long long)((uint32_t)bestM ^ 0x80000000u) << 32) |
-                                           (unsigned long long)(0xffffffffu - (uint32_t)bestJ);
-            key = warp_max_u64(key);
-            const int max_j = bn > 0 ? (int)(0xffffffffu - (uint32_t)(key & 0xffffffffu)) : 0;
-            if (pf) {
-                cp_async_wait_all();
-                __syncwarp();
-                adaptive_update_pf(a, i, Bs, max_j, lane, upd, d, ns, base_i, hql, qsm);
-            } else {
-                adaptive_update_warp(a, i, Bs, max_j, lane);
-            }
-        }
-        tb_next = (tb_next + (int64_t)bn * BLK * bpc + 15) & ~(int64_t)15;
-        __syncwarp();
-    }
-    if (lane == 0) {
-        const RowMeta last = a.meta[n - 1];
-        const int jm = m - last.Bs * BLK;
-        a.out[1] = a.rs[last.st + (int64_t)(jm / BLK) * 16 + jm % BLK];
-        a.out[3] = (int32_t)(cells > INT_MAX ? INT_MAX : cells);
-        a.out[6] = (int32_t)(ecells > INT_MAX ? INT_MAX : ecells);
-        a.out[4] = (int32_t)tb_next;
-        a.out[5] = (int32_t)(st_next - ring_part);
-        a.out[0] = ST_OK;
-    }
-    __syncwarp();
-}
-
-// Backtrack over the records (src/align.cpp:1572-1736, same decisions as
-// backtrack_records) with the whole warp. The path mostly steps
-// (i, j) -> (i-1, j-1), so lane k preloads the descriptor of row i-k and its
-// record at column acj-k; the walk consumes lane t's values through shuffles
-// while the path stays on that diagonal and preloads again from wherever it
-// leaves it. All lanes run the walk (uniform control flow); lane 0 stores
-// the moves.
-__device__ int bt_warp_static(const RowDesc* __restrict__ desc, const int32_t* __restrict__ in_row,
-                              const uint8_t* __restrict__ in_base, const uint8_t* __restrict__ tb,
-                              const uint8_t* __restrict__ qs, int n, int m, int32_t* moves, int moves_cap,
-                              int32_t& nm_out, int lane) {
-    int i = n - 1, acj = m, op = ALL_OP, nm = 0;
-    int status = ST_OK;
-    while ((i > 0 || acj > 0) && status == ST_OK) {
-        const int i0 = i, a0 = acj;
-        // preload: lane k -> (i0 - k, a0 - k)
-        const int ri = i0 - lane, cj = a0 - lane;
-        int bsbe = 0, d = 0;
-        uint32_t rec = 0;
-        int qc = 4;
-        // predecessor row / base for the three choices a record can make (m1, m4, d)
-        int p1 = 0, b1 = 4, p4 = 0, b4 = 4, pd = 0;
-        if (ri >= 0) {
-            const RowDesc rd = load_desc(desc + ri);
-            bsbe = rd.bsbe; d = rd.d;
-            const int Bs = bsbe & 0xffff, Be = bsbe >> 16;
-            const int j = cj - Bs * BLK;
-            if (j >= 0 && j < (Be - Bs - 1) * BLK)
-                rec = d >= 2 ? *reinterpret_cast<const uint32_t*>(tb + rd.tb + j * 4) : (uint32_t)tb[rd.tb + j];
-            if (cj > 0) qc = qs[cj];
-            p1 = p4 = pd = rd.prow0;
-            b1 = b4 = rd.pbase;
-            if (d >= 2) {
-                const Rec r = decode_wide(rec);
-                if (r.m1 >= 0) { p1 = in_row[rd.e0 + r.m1]; b1 = in_base[rd.e0 + r.m1]; }
-                if (r.m4 >= 0) { p4 = in_row[rd.e0 + r.m4]; b4 = in_base[rd.e0 + r.m4]; }
-                if (r.dpos >= 0) pd = in_row[rd.e0 + r.dpos];
-            }
-        }
-        for (int t = 0; t < 32; t++) {
-            const int Bs_t = __shfl_sync(0xffffffffu, bsbe, t) & 0xffff;
-            const int Be_t = __shfl_sync(0xffffffffu, bsbe, t) >> 16;
-            const int d_t = __shfl_sync(0xffffffffu, d, t);
-            const uint32_t rec_t = __shfl_sync(0xffffffffu, rec, t);
-            const int qc_t = __shfl_sync(0xffffffffu, qc, t);
-            const int p1_t = __shfl_sync(0xffffffffu, p1, t), b1_t = __shfl_sync(0xffffffffu, b1, t);
-            const int p4_t = __shfl_sync(0xffffffffu, p4, t), b4_t = __shfl_sync(0xffffffffu, b4, t);
-            const int pd_t = __shfl_sync(0xffffffffu, pd, t);
-            if (acj > (Be_t - 1) * BLK || acj < Bs_t * BLK) { status = ST_BAND_ESCAPE; break; }
-            const int j = acj - Bs_t * BLK;
-            if (j >= (Be_t - Bs_t - 1) * BLK) { status = ST_BT_FAIL; break; }
-            if (nm + 1 > moves_cap) { status = ST_OOM; break; }
-            const Rec r = d_t >= 2 ? decode_wide(rec_t) : decode_small((uint8_t)rec_t);
-            int ni = i, na = acj;
-            bool moved = false;
-            if ((op & M_OP) && acj > 0 && r.m1 >= 0) {
-                if (lane == 0) moves[nm] = mv_pack(b1_t == qc_t ? MV_MATCH : MV_MISMATCH, p1_t, qc_t);
-                nm++;
-                op = ALL_OP; ni = p1_t; na = acj - 1; moved = true;
-            } else if ((op & D_OP) && (op == D_OP || r.eqMD) && r.dpos >= 0) {
-                ni = pd_t;
-                op = r.dext ? D_OP : (M_OP | I_OP);
-                moved = true;
-            } else if ((op & I_OP) && acj > 0 && j >= 1 && (op == I_OP || r.eqMI) && (r.iopen || r.iext)) {
-                if (lane == 0) moves[nm] = mv_pack(MV_INSERT, 0, qc_t);
-                nm++;
-                op = r.iopen ? (M_OP | D_OP) : I_OP;
-                na = acj - 1; moved = true;
-            } else if ((op & M_OP) && acj > 0 && r.m4 >= 0) {
-                if (lane == 0) moves[nm] = mv_pack(b4_t == qc_t ? MV_MATCH : MV_MISMATCH, p4_t, qc_t);
-                nm++;
-                op = ALL_OP; ni = p4_t; na = acj - 1; moved = true;
-            }
-            if (!moved) { status = ST_BT_FAIL; break; }
-            i = ni;
-            acj = na;
-            if (!(i > 0 || acj > 0)) break;
-            if (t + 1 >= 32 || i != i0 - (t + 1) || acj != a0 - (t + 1)) break;
-        }
-    }
-    nm_out = nm;
-    __syncwarp();
-    return status;
-}
-
-// Build the DP rows of window [rank(source), rank(sink)] with the whole warp.
-__device__ int build_view(DevGraph& g, char* s, const SlotLayout& L, WinView& v, int lane, bool recs) {
-    const int beg_i = g.rank[0], end_i = g.rank[1];
-    const int n = end_i - beg_i + 1;
-    int32_t* in_ptr = (int32_t*)(s + L.v_in_ptr);
-    int32_t* out_ptr = (int32_t*)(s + L.v_out_ptr);
-    int32_t* in_row = (int32_t*)(s + L.v_in_row);
-    int32_t* in_w = (int32_t*)(s + L.v_in_w);
-    uint8_t* in_base = (uint8_t*)(s + L.v_in_base);
-    int32_t* out_row = (int32_t*)(s + L.v_out_row);
-    uint8_t* vb = (uint8_t*)(s + L.v_base);
-    int32_t* vind = (int32_t*)(s + L.v_ind);
-    int32_t* hq = (int32_t*)(s + L.v_hq);
-    int32_t* hq_loc = (int32_t*)(s + L.v_hq_loc);
-    int32_t* tq = (int32_t*)(s + L.v_tq);
-    const int h0 = g.hlen[beg_i], t0 = g.tlen[end_i];
-    // pass 1: per-row counts and scalars
-    for (int r = lane; r < n; r += 32) {
-        const int u = g.rank_to_id[beg_i + r];
-        int ci = 0, co = 0;
-        for (int e = g.in_head[u]; e >= 0; e = g.e_nin[e]) ci += (g.rank[g.e_from[e]] - beg_i >= 0);
-        for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) co += (g.rank[g.e_to[e]] - beg_i < n);
-        in_ptr[r + 1] = ci;
-        out_ptr[r + 1] = co;
-        vb[r] = g.base[u];
-        vind[r] = g.ind[u];
-        hq[r] = g.hlen[beg_i + r] - h0;
-        hq_loc[r] = g.hlen[r] - h0;
-        tq[r] = g.tlen[beg_i + r] - t0;
-    }
-    __syncwarp();
-    // exclusive scans of the counts
-    int ci_carry = 0, co_carry = 0;
-    if (lane == 0) { in_ptr[0] = 0; out_ptr[0] = 0; }
-    for (int c0 = 0; c0 < n; c0 += 32) {
-        const int r = c0 + lane;
-        int ci = r < n ? in_ptr[r + 1] : 0, co = r < n ? out_ptr[r + 1] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int yi = __shfl_up_sync(0xffffffffu, ci, o), yo = __shfl_up_sync(0xffffffffu, co, o);
-            if (lane >= o) { ci += yi; co += yo; }
-        }
-        __syncwarp();
-        if (r < n) { in_ptr[r + 1] = ci + ci_carry; out_ptr[r + 1] = co + co_carry; }
-        ci_carry += __shfl_sync(0xffffffffu, ci, 31);
-        co_carry += __shfl_sync(0xffffffffu, co, 31);
-    }
-    __syncwarp();
-    // pass 2: fill the lists in in-list / out-list order
-    for (int r = lane; r < n; r += 32) {
-        const int u = g.rank_to_id[beg_i + r];
-        int k = in_ptr[r];
-        for (int e = g.in_head[u]; e >= 0; e = g.e_nin[e]) {
-            const int p = g.rank[g.e_from[e]] - beg_i;
-            if (p < 0) continue;
-            in_row[k] = p;
-            in_w[k] = g.e_w[e];
-            in_base[k] = p == 0 ? 4 : g.base[g.e_from[e]];
-            k++;
-        }
-        k = out_ptr[r];
-        for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) {
-            const int sr = g.rank[g.e_to[e]] - beg_i;
-            if (sr >= n) continue;
-            out_row[k++] = sr;
-        }
-    }
-    __syncwarp();
-    if (recs) {
-        // for the warp fill: each row's predecessor records in the backtrack's
-        // priority order (in_weight descending, in-list position ascending),
-        // erec = {predecessor row, 0, in_weight | position << 16,
-        //         base | (in_weight >= ind/10) << 8}; the fill patches in the
-        // predecessor's band and row-store location when it reaches the row.
-        // Also each row's furthest successor row (row-store placement).
-        int4* erec = (int4*)(s + L.v_pmeta);
-        int32_t* vmaxs = (int32_t*)(s + L.v_desc);
-        for (int r = lane; r < n; r += 32) {
-            const int e0 = in_ptr[r], d = r == 0 ? 0 : in_ptr[r + 1] - e0;
-            const int ind = vind[r];
-            for (int k = 0; k < d; k++) {
-                const int w = in_w[e0 + k];
-                const int4 rec = make_int4(in_row[e0 + k], 0, (w & 0xffff) | (k << 16),
-                                           (int)in_base[e0 + k] | ((w >= ind / 10) ? 256 : 0));
-                int at = k;
-                while (at > 0) {
-                    const int4 prev = erec[e0 + at - 1];
-                    if ((prev.z & 0xffff) >= w) break;  // ties keep list order
-                    erec[e0 + at] = prev;
-                    at--;
-                }
-                erec[e0 + at] = rec;
-            }
-            int maxs = r;
-            for (int k = out_ptr[r]; k < out_ptr[r + 1]; k++) maxs = max(maxs, out_row[k]);
-            vmaxs[r] = maxs;
-        }
-        __syncwarp();
-    }
-    v.n = n;
-    v.in_ptr = in_ptr; v.in_row = in_row; v.in_w = in_w; v.in_base = in_base;
-    v.base = vb; v.ind = vind; v.hq = hq; v.hq_loc = hq_loc; v.tq = tq;
-    v.out_ptr = out_ptr; v.out_row = out_row;
-    return beg_i;
-}
-
-template <bool STATIC>
-__device__ void process_window(const BatchArgs& A, char* s, DpArgs& a, unsigned char* wsm, int w, int lane) {
+template <bool STATIC, bool WIDE>
+__device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned char* wsm, int w, int lane) {
     const SlotLayout& L = A.L;
     DevGraph g = slot_graph(s, L);
     const int r0 = A.win_off[w], r1 = A.win_off[w + 1];
     const bool lens = A.f > 0;
-    constexpr bool static_band = STATIC;  // f > 0 && !ab_band (checked on the host)
     int status = ST_OK;
-    // the window's counters: in registers for the adaptive-band kernel; in the
-    // window's output slots (lane 0) for the static-band kernel, whose fill
-    // runs faster with the registers free (measured)
-    int64_t cells_r = 0, ecells_r = 0;
-    long long ph_r[NPHASE] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // the window's counters live in its output slots (lane 0): the fill needs the registers
     int64_t* const cells_g = A.cells + 2 * (int64_t)w;
     int64_t* const ph_g = A.phase + (int64_t)w * NPHASE;
-    if (STATIC && lane == 0) {
+    if (lane == 0) {
         cells_g[0] = cells_g[1] = 0;
         for (int k = 0; k < NPHASE; k++) ph_g[k] = 0;
     }
     long long tc = clock64();
     auto tick = [&](int k) {
         long long t = clock64();
-        if constexpr (STATIC) {
-            if (lane == 0) ph_g[k] += t - tc;
-        } else {
-            ph_r[k] += t - tc;
-        }
+        if (lane == 0) ph_g[k] += t - tc;
         tc = t;
-    };
-    auto add_cells = [&](int64_t c, int64_t e) {  // lane 0
-        if constexpr (STATIC) {
-            cells_g[0] += c;
-            cells_g[1] += e;
-        } else {
-            cells_r += c;
-            ecells_r += e;
-        }
     };
     for (int x = lane; x < L.NC; x += 32) { g.hlen[x] = 0; g.tlen[x] = 0; }
     if (lane == 0) {
@@ -1867,22 +817,29 @@ __device__ void process_window(const BatchArgs& A, char* s, DpArgs& a, unsigned 
         if (len > L.QC) { status = ST_CAPACITY; break; }
         const int nn0 = g.hdr[0];
         if (nn0 <= 2) {  // src/align.cpp:1747-1753: source + one new node per base
-            if (lane == 0) {
-                int nn = nn0, ne = g.hdr[1], anchored = 0, st = ST_OK;
-                for (int j = 0; j < len && st == ST_OK; j++) {
-                    const int cur = dg_add_node(g, nn, nt4_dev(rd[j]));
-                    if (cur < 0 || !dg_add_adj(g, ne, anchored, cur)) st = ST_CAPACITY;
-                    anchored = cur;
+            if (g.hdr[1] == 0) {
+                status = dg_first_read(g, rd, len, lane);
+            } else {
+                // after reads without bases: one edge at a time
+                if (lane == 0) {
+                    int nn = nn0, ne = g.hdr[1], anchored = 0, st = ST_OK;
+                    for (int j = 0; j < len && st == ST_OK; j++) {
+                        const int cur = dg_add_node(g, nn, nt4_dev(rd[j]));
+                        if (cur < 0 || !dg_add_adj(g, ne, anchored, cur)) st = ST_CAPACITY;
+                        anchored = cur;
+                    }
+                    if (st == ST_OK && !dg_add_adj(g, ne, anchored, 1)) st = ST_CAPACITY;
+                    g.hdr[0] = nn;
+                    g.hdr[1] = ne;
+                    g.hdr[2] = st;
                 }
-                if (st == ST_OK && !dg_add_adj(g, ne, anchored, 1)) st = ST_CAPACITY;
-                g.hdr[0] = nn;
-                g.hdr[1] = ne;
-                g.hdr[2] = st;
-                A.rstats[(int64_t)r * NRSTAT + 3] = nn;
-                A.rstats[(int64_t)r * NRSTAT + 6] = ne;
+                __syncwarp();
+                status = g.hdr[2];
             }
-            __syncwarp();
-            status = g.hdr[2];
+            if (lane == 0) {
+                A.rstats[(int64_t)r * NRSTAT + 3] = g.hdr[0];
+                A.rstats[(int64_t)r * NRSTAT + 6] = g.hdr[1];
+            }
             tick(PH_FUSE);
             if (status == ST_OK && r + 1 < r1)
                 dg_topsort_warp(g, g.hdr[0], g.hdr[1], lens, (uint16_t*)wsm, A.smem_per_warp, lane);
@@ -1891,128 +848,117 @@ __device__ void process_window(const BatchArgs& A, char* s, DpArgs& a, unsigned 
         }
         tick(PH_FUSE);
         // DP rows of the whole graph and the shifted query
-        WinView v;
-        int beg_i;
-        if constexpr (static_band) {
-            const int st = build_view_static(g, s, L, v, len + 1, A.f, A.b + (len + 1) / A.f, A.sring_rows,
-                                             A.sring_blocks, lane, beg_i);
-            if (st != ST_OK) { status = st; break; }
-        } else {
-            beg_i = build_view(g, s, L, v, lane, true);
-        }
+        int beg_i = 0, n = 0;
+        int st = build_rows<STATIC, WIDE>(g, s, A, a, len + 1, A.b + (A.f ? (len + 1) / A.f : 0), lane, n, beg_i);
+        if (STATIC && st != ST_OK) { status = st; break; }
         uint8_t* qs = (uint8_t*)(s + L.qs);
         const int64_t qsb = qs_bytes(len);
         for (int64_t x = lane; x < qsb; x += 32) qs[x] = (x >= 2 && x < len + 2) ? nt4_dev(rd[x - 2]) : 4;
         if (lane == 0) {
-            a.v = v;
-            a.qs = qs;
+            a.n = n;
             a.qlen = len;
-            a.ab_band = A.ab_band;
             a.f = A.f;
             a.w = A.b + (A.f ? (len + 1) / A.f : 0);
-            a.sc = A.sc;
-            a.meta = (RowMeta*)(s + L.meta);
+            a.k = A.k;
+            a.in_ptr = (const int32_t*)(s + L.v_in_ptr);
+            a.ed = (int4*)(s + L.v_ed);
+            a.fe = (int4*)(s + L.v_fe);
+            a.ra = (const int4*)(s + L.v_ra);
+            a.out_row = (const int32_t*)(s + L.v_out_row);
+            a.qs = qs;
+            a.rowi = (int4*)(s + L.v_rowi);
+            a.fr = (int4*)(s + L.v_fr);
             a.state = (int32_t*)(s + L.state);
-            a.rs = (int32_t*)(s + L.rs);
-            a.rs_cap = L.rs_cap;
-            a.ring_rows = L.ring_rows;
-            a.ring_blocks = L.ring_blocks;
-            a.tb = (uint8_t*)(s + L.tb);
-            a.tb_cap = L.tb_cap;
+            a.store = s + L.store;
+            a.store_cap = L.store_cap;
             a.moves = (int32_t*)(s + L.moves);
             a.moves_cap = L.NC + L.QC + 16;
-            a.out = g.hdr + 4;
         }
         __syncwarp();
-        if (v.n > L.NC) { status = ST_CAPACITY; break; }
+        if (n > L.NC) { status = ST_CAPACITY; break; }
         tick(PH_VIEW);
-        if constexpr (static_band) {
-            // the query goes after the row ring in this warp's shared memory
-            uint8_t* qsm = wsm + (size_t)A.sring_rows * A.sring_blocks * 64;
+        int64_t cells = 0;
+        if constexpr (STATIC) {
+            // shared memory: row ring, query, staged rows
+            const WarpRing ring{(unsigned)__cvta_generic_to_shared(wsm), A.sring_rows, A.sring_rows ? A.sring_blocks : 0};
+            uint8_t* qsm = wsm + (size_t)A.sring_rows * A.sring_blocks * BLK * Cells<WIDE>::BYTES;
             for (int64_t x = lane * 16; x < qsb; x += 32 * 16)
                 *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>(qs + x);
             __syncwarp();
-            unsigned char* stage = qsm + ((qsb + 15) & ~(int64_t)15);
-            dp_fill_warp_static(a, (const RowDesc*)(s + L.v_desc), (const int4*)(s + L.v_pmeta), (int32_t*)wsm,
-                                A.sring_blocks, qsm, stage, lane);
+            warp_fill_static<WIDE>(a, ring, qsm, qsm + ((qsb + 15) & ~(int64_t)15), lane);
         } else {
-            // shared memory: staged records, the update's inputs, and the query when it fits
+            // shared memory: staged records, state window, and the query when it fits
             const uint8_t* qf = qs;
-            int4* sed = reinterpret_cast<int4*>(wsm);
-            const int64_t sed_bytes = (int64_t)DYN_STAGE_EDGES * 16;
-            int32_t* upd = reinterpret_cast<int32_t*>(wsm + sed_bytes);
-            if (sed_bytes + UPD_BYTES + qsb <= A.smem_per_warp) {
-                uint8_t* qsm = wsm + sed_bytes + UPD_BYTES;
+            const int64_t used = WED * 16 + warp_state_bytes(A.state_rows);
+            if (used + qsb <= A.smem_per_warp) {
+                uint8_t* qsm = wsm + used;
                 for (int64_t x = lane * 16; x < qsb; x += 32 * 16)
                     *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>(qs + x);
                 qf = qsm;
             }
             __syncwarp();
-            dp_fill_warp_dyn(a, (int4*)(s + L.v_pmeta), (const int32_t*)(s + L.v_desc), qf, sed, upd, lane);
+            st = warp_fill_dyn<WIDE>(a, A.f > 0 && A.ab_band, wsm, A.state_rows, qf, lane, cells);
         }
         __syncwarp();
-        {
+        if (st == ST_OK) {
             // per-read band statistics
             int mbn = 0;
-            long long mid = 0;
-            for (int i = lane; i < v.n; i += 32) {
-                const RowMeta rm = ((const RowMeta*)(s + L.meta))[i];
-                mbn = max(mbn, rm.Be - rm.Bs - 1);
-                mid += (long long)(rm.Bs + rm.Be - 1) * (BLK / 2);
+            long long mid = 0, bns = 0, ebns = 0, rec = 0, sp = 0;
+            const int4* rowi = a.rowi;
+            const int32_t* in_ptr = a.in_ptr;
+            const int32_t* maxs = (const int32_t*)(s + L.v_maxs);
+            for (int i = lane; i < n; i += 32) {
+                const int4 ri = rowi[i];
+                const int bn = ri.y - ri.x - 1, d = i == 0 ? 0 : in_ptr[i + 1] - in_ptr[i];
+                mbn = max(mbn, bn);
+                mid += (long long)(ri.x + ri.y - 1) * (BLK / 2);
+                bns += bn;
+                ebns += (long long)bn * d;
+                rec += (bn * BLK * (d >= 2 ? 4 : 1) + 15) & ~15;
+                if (A.stat_rows == 0 || maxs[i] - i >= A.stat_rows || bn > A.stat_blocks) sp += bn * 16;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 mbn = max(mbn, __shfl_xor_sync(0xffffffffu, mbn, o));
                 mid += __shfl_xor_sync(0xffffffffu, mid, o);
+                bns += __shfl_xor_sync(0xffffffffu, bns, o);
+                ebns += __shfl_xor_sync(0xffffffffu, ebns, o);
+                rec += __shfl_xor_sync(0xffffffffu, rec, o);
+                sp += __shfl_xor_sync(0xffffffffu, sp, o);
             }
             if (lane == 0) {
                 int32_t* o = A.rstats + (int64_t)r * NRSTAT;
+                auto cap = [](long long x) { return (int32_t)(x > INT_MAX ? INT_MAX : x); };
                 o[0] = mbn;
-                o[1] = a.out[3];
-                o[2] = v.n;
-                o[7] = v.n > 0 ? (int32_t)(mid * 1000 / ((long long)v.n * (len + 1))) : 0;
-                o[4] = a.out[4];  // record bytes and spilled row-store entries
-                o[5] = a.out[5];
+                o[1] = cap(bns * BLK);
+                o[2] = n;
+                o[7] = n > 0 ? (int32_t)(mid * 1000 / ((long long)n * (len + 1))) : 0;
+                o[4] = cap(rec);  // record bytes (1 a cell, 4 in rows with several predecessors) and spilled entries
+                o[5] = cap(sp);
+                cells_g[0] += bns * BLK;
+                cells_g[1] += ebns * BLK;
             }
         }
         tick(PH_FILL);
-        if constexpr (static_band) {
-            int st = a.out[0];
-            int32_t nm = 0;
-            if (st == ST_OK)
-                st = bt_warp_static((const RowDesc*)(s + L.v_desc), a.v.in_row, a.v.in_base, a.tb, qs, v.n, len + 1,
-                                    a.moves, a.moves_cap, nm, lane);
-            if (lane == 0) {
-                add_cells(a.out[3], a.out[6]);
-                g.hdr[2] = st;
-                g.hdr[13] = nm;
-                g.hdr[12] = g.hdr[12] + 1;  // fusion stamp, increasing over the slot's lifetime
-            }
-        } else if (lane == 0) {
-            int st = a.out[0];
-            add_cells(a.out[3], a.out[6]);
-            int32_t nm = 0;
-            if (st == ST_OK) st = backtrack_records(a, len + 1, nm);
+        int32_t nm = 0;
+        if (st == ST_OK) st = team_backtrack<WIDE, 4>(a, (char*)wsm, A.smem_per_warp, lane, nm);
+        if (lane == 0) {
             g.hdr[2] = st;
             g.hdr[13] = nm;
-            g.hdr[12] = g.hdr[12] + 1;
+            g.hdr[12] = g.hdr[12] + 1;  // fusion stamp, increasing over the slot's lifetime
         }
         __syncwarp();
         tick(PH_BT);
-        {
-            int st = g.hdr[2];
-            const int nm = g.hdr[13];
-            if (st == ST_OK) {
-                st = dg_fuse_warp(g, a.moves, nm, beg_i, (int32_t*)(s + L.path), g.hdr[12], lane);
-                if (st == -1) {
-                    // sequential fusion (a path that repeats a node or an aligned sibling)
-                    st = ST_OK;
-                    if (lane == 0) st = dg_fuse_seq(g, a.moves, nm, beg_i);
-                    __syncwarp();
-                }
+        if (st == ST_OK) {
+            st = dg_fuse_warp(g, a.moves, nm, beg_i, (int32_t*)(s + L.path), g.hdr[12], lane);
+            if (st == -1) {
+                // sequential fusion (a path that repeats a node or an aligned sibling)
+                st = ST_OK;
+                if (lane == 0) st = dg_fuse_seq(g, a.moves, nm, beg_i);
+                __syncwarp();
             }
-            if (lane == 0) g.hdr[2] = st;
         }
+        if (lane == 0) g.hdr[2] = st;
         __syncwarp();
         status = g.hdr[2];
         if (lane == 0) {
@@ -2033,18 +979,13 @@ __device__ void process_window(const BatchArgs& A, char* s, DpArgs& a, unsigned 
         tick(PH_CONS);
         A.cons_len[w] = len < 0 ? 0 : len;
         A.status[w] = status;
-        if constexpr (!STATIC) {
-            cells_g[0] = cells_r;
-            cells_g[1] = ecells_r;
-            for (int k = 0; k < NPHASE; k++) ph_g[k] = ph_r[k];
-        }
     }
     __syncwarp();
 }
 
-template <int WARPS, bool STATIC, int MINB>
+template <int WARPS, bool STATIC, bool WIDE, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB) k_batch(BatchArgs A) {
-    __shared__ DpArgs s_args[WARPS];
+    __shared__ TeamJob s_args[WARPS];
     extern __shared__ __align__(16) unsigned char dsm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t slot = (int64_t)blockIdx.x * WARPS + warp;
@@ -2055,8 +996,18 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_batch(BatchArgs A) {
         if (lane == 0) idx = atomicAdd(A.counter, 1);
         idx = __shfl_sync(0xffffffffu, idx, 0);
         if (idx >= A.n_windows) break;
-        process_window<STATIC>(A, s, s_args[warp], wsm, A.order[idx], lane);
+        process_window<STATIC, WIDE>(A, s, s_args[warp], wsm, A.order[idx], lane);
     }
+}
+
+// Every build of the kernel by band kind, cell and register budget (blocks of 4
+// warps per SM).
+typedef void (*BatchKernel)(BatchArgs);
+BatchKernel batch_kernel(bool stat, bool wide, int blocks_per_sm) {
+    if (wide) return stat ? (BatchKernel)k_batch<4, true, true, 3> : (BatchKernel)k_batch<4, false, true, 3>;
+    if (blocks_per_sm >= 5) return stat ? (BatchKernel)k_batch<4, true, false, 5> : (BatchKernel)k_batch<4, false, false, 5>;
+    if (blocks_per_sm >= 4) return stat ? (BatchKernel)k_batch<4, true, false, 4> : (BatchKernel)k_batch<4, false, false, 4>;
+    return stat ? (BatchKernel)k_batch<4, true, false, 3> : (BatchKernel)k_batch<4, false, false, 3>;
 }
 
 }  // namespace
@@ -2169,8 +1120,9 @@ void BatchEngine::run() {
         std::vector<int32_t> nodes;
         std::vector<int64_t> tb, spill;
         std::vector<float> cost;
-        proposer_->plan(device_windows(), PROP_K, PROP_W, nodes, tb, spill, cost);
-        set_plan(nodes.data(), tb.data(), spill.data(), cost.data());
+        std::vector<int64_t> cells;
+        proposer_->plan(device_windows(), PROP_K, PROP_W, nodes, tb, spill, cost, cells);
+        set_plan(nodes.data(), tb.data(), spill.data(), cost.data(), cells.data());
         cuda_check(cudaEventRecord((cudaEvent_t)evp_, rs), "event");
     }
     if (n_reads_ > 0)
@@ -2185,12 +1137,10 @@ void BatchEngine::run() {
     if (!plan_nodes_.empty()) {
         Caps c;
         c.NC = 64;
-        c.tb_cap = 4096;
-        c.spill = 0;
+        c.cells = 4096;
         for (int w = 0; w < n_windows_; w++) {
             c.NC = std::max<int64_t>(c.NC, plan_nodes_[w]);
-            c.tb_cap = std::max(c.tb_cap, plan_tb_[w]);
-            c.spill = std::max(c.spill, plan_spill_[w]);
+            c.cells = std::max(c.cells, plan_cells_[w]);
         }
         c.NC = std::min<int64_t>(c.NC, 60000);
         launch(plan_order_.data(), n_windows_, c, PLAN_HEADROOM);
@@ -2243,23 +1193,29 @@ BatchEngine::Caps BatchEngine::default_caps(int scale) const {
     c.NC = (int32_t)std::max<int64_t>(NC64, 64);
     const int rb = ring_blocks();
     const int tb_blocks = adaptive ? std::min(m / BLK + 2, (std::min(m / BLK + 2, (4 * wb) / BLK + 4)) * scale) : rb;
-    c.tb_cap = (int64_t)c.NC * tb_blocks * BLK * 2 * std::min(scale, 2) + 4096;
-    const int64_t spill_rows = std::min<int64_t>(c.NC, std::max<int64_t>(c.NC / (adaptive ? 8 : 4), 64) * scale);
-    c.spill = spill_rows * rb * 16;
+    // static rows can be wider than tb_blocks where hlen and tlen disagree; adaptive rows of
+    // noisy reads widen past twice the initial band
+    c.cells = (int64_t)c.NC * tb_blocks * BLK;
+    c.cells = (adaptive ? c.cells * 3 / 2 : c.cells * std::min(scale, 2)) + 4096;
     return c;
 }
 
-void BatchEngine::set_plan(const int32_t* nodes, const int64_t* tb_bytes, const int64_t* spill, const float* cost) {
+void BatchEngine::set_plan(const int32_t* nodes, const int64_t* tb_bytes, const int64_t* spill, const float* cost,
+                           const int64_t* cells) {
     if (!nodes) {
         plan_nodes_.clear();
         plan_tb_.clear();
         plan_spill_.clear();
         plan_order_.clear();
+        plan_cells_.clear();
         return;
     }
     plan_nodes_.assign(nodes, nodes + n_windows_);
     plan_tb_.assign(tb_bytes, tb_bytes + n_windows_);
     plan_spill_.assign(spill, spill + n_windows_);
+    // the row store holds cells; a plan without a cell count bounds it by its record bytes (at least one a cell)
+    if (cells) plan_cells_.assign(cells, cells + n_windows_);
+    else plan_cells_ = plan_tb_;
     plan_order_.resize(n_windows_);
     std::iota(plan_order_.begin(), plan_order_.end(), 0);
     std::stable_sort(plan_order_.begin(), plan_order_.end(), [&](int a, int b) { return cost[a] > cost[b]; });
@@ -2274,37 +1230,45 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     const int32_t EC = 3 * NC;
     const int32_t QC = max_len_ + 8;
     const int ring_blocks = this->ring_blocks();
-    const int32_t ring_rows = 32;
-    const int64_t tb_cap = (caps.tb_cap + 4095) / 4096 * 4096;
-    const int64_t spill = (caps.spill + 63) / 64 * 64;
-    SlotLayout L = make_layout(NC, EC, QC, ring_rows, ring_blocks, spill, tb_cap, adaptive);
+    const bool stat = p_.f > 0 && !p_.ab_band;
+    const Scoring sc = scoring_of(p_);
+    // graphs hold at most 60,000 nodes
+    const bool wide = !cell_packable(sc, 60000, QC);
+    const int cell_bytes = wide ? Cells<true>::BYTES : Cells<false>::BYTES;
+    const int64_t store = (caps.cells * cell_bytes + 4095) / 4096 * 4096;
+    SlotLayout L = make_layout(NC, EC, QC, store, stat, adaptive, wide);
     const SlotLayout L_planned = L;
     const int warps = warps_per_block;
     const int smem_w = smem_per_warp;
     const size_t dyn = (size_t)warps * smem_w;
-    // static band: shared-memory ring of up to 8 rows of ring_blocks blocks
-    int sring_blocks = ring_blocks;
     const int qsm_bytes = (int)((qs_bytes(QC) + 15) / 16 * 16);
-    const int stage_bytes = STAGE_ROWS * (int)sizeof(RowDesc) + STAGE_EDGES * 16;
-    int sring_rows = std::min(8, (smem_w - qsm_bytes - stage_bytes) / std::max(1, sring_blocks * 64));
-    if (sring_rows < 2) sring_rows = 0;
-    if (p_.f > 0 && !p_.ab_band && qsm_bytes + stage_bytes > smem_w)
+    constexpr int kStageBytes = 1792;  // shared memory a static-band warp needs beside its query
+    static_assert(kStageBytes >= WSTG_BYTES && kStageBytes >= BtTile<true, 4>::PER_ROW * 2 + 16, "stage and backtrack tile");
+    if (stat && qsm_bytes + kStageBytes > smem_w)
         throw std::invalid_argument("reads too long for the batch kernel's shared memory; raise smem_per_warp");
-    if (!(p_.f > 0 && !p_.ab_band) && smem_w < DYN_STAGE_EDGES * 16 + UPD_BYTES)
-        throw std::invalid_argument("smem_per_warp too small for the adaptive-band fill");
+    constexpr int kDynBytes = 3136;  // the dynamic-band fill's records and its smallest state window
+    static_assert(kDynBytes >= WED * 16 + warp_state_bytes(32), "state window");
+    if (!stat && smem_w < kDynBytes) throw std::invalid_argument("smem_per_warp too small for the adaptive-band fill");
     if (smem_w % 16 != 0) throw std::invalid_argument("smem_per_warp must be a multiple of 16");
+    // static band: shared-memory ring of 2 to 16 rows of ring_blocks blocks
+    const int row_bytes = ring_blocks * BLK * cell_bytes;
+    int sring_rows = 16;
+    while (sring_rows >= 2 && sring_rows * row_bytes > smem_w - qsm_bytes - WSTG_BYTES) sring_rows /= 2;
+    if (sring_rows < 2) sring_rows = 0;
+    // dynamic bands: the largest state window that leaves room for the query, else the largest that fits
+    int state_rows = 128;
+    while (state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) + qsm_bytes > smem_w) state_rows /= 2;
+    if (WED * 16 + warp_state_bytes(state_rows) + qsm_bytes > smem_w)
+        for (state_rows = 128; state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) > smem_w;) state_rows /= 2;
+    // read statistics count spilled rows against a ring of 32 full-width rows (dynamic bands) or
+    // of up to 8 rows of 64 bytes a block in the warp's shared memory (static band)
+    int stat_rows = stat ? std::min(8, (smem_w - qsm_bytes - kStageBytes) / std::max(1, ring_blocks * 64)) : 32;
+    if (stat_rows < 2) stat_rows = 0;
     int occ = 0;
-    auto occ_of = [&](auto kern) {
-        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn), "smem attr");
-        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, warps * 32, dyn), "occupancy");
-    };
-    const bool stat = p_.f > 0 && !p_.ab_band;
+    const BatchKernel kern = batch_kernel(stat, wide, blocks_per_sm);
     if (warps != 4) throw std::invalid_argument("batch kernel is built for 4 warps per block");
-    // two register budgets: 3 blocks (12 warps) per SM at up to 168 registers, or
-    // 4 blocks (16 warps) per SM at up to 128 registers
-    const bool dense = blocks_per_sm >= 4;
-    if (stat) { if (dense) occ_of(k_batch<4, true, 4>); else occ_of(k_batch<4, true, 3>); }
-    else { if (dense) occ_of(k_batch<4, false, 4>); else occ_of(k_batch<4, false, 3>); }
+    cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn), "smem attr");
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, warps * 32, dyn), "occupancy");
     // every block must be resident at once (persistent kernel): never more than the occupancy allows
     const int per_sm = std::max(1, std::min(blocks_per_sm, occ));
     int blocks = sms * per_sm;
@@ -2321,9 +1285,8 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
         const double h = std::min(headroom, fit);
         if (h > 1.0) {
             const int32_t NCh = (int32_t)std::min<double>(60000.0, std::max(64.0, NC * h));
-            const int64_t tbh = ((int64_t)(tb_cap * h) + 4095) / 4096 * 4096;
-            const int64_t sph = ((int64_t)(spill * h) + 63) / 64 * 64;
-            L = make_layout(NCh, 3 * NCh, QC, ring_rows, ring_blocks, sph, tbh, adaptive);
+            const int64_t sth = ((int64_t)(store * h) + 4095) / 4096 * 4096;
+            L = make_layout(NCh, 3 * NCh, QC, sth, stat, adaptive, wide);
         }
     }
     const int64_t max_by_mem = (int64_t)(budget / (size_t)L.bytes) / warps;
@@ -2339,8 +1302,10 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
         d_slots_cap_ = 0;
         cuda_check(cudaMalloc(&d_slots_, slot_total), "cudaMalloc(batch slots)");
         d_slots_cap_ = slot_total;
-        // zeroed once: fusion stamps and slot headers start from a known state
-        cuda_check(cudaMemsetAsync(d_slots_, 0, d_slots_cap_, s), "memset slots");
+        // slot headers and fusion stamps start from zero (a stale stamp would only cost time: it
+        // sends a path to the sequential fusion)
+        cuda_check(cudaMemset2DAsync((char*)d_slots_ + L.hdr, L.bytes, 0, 64, slots, s), "memset headers");
+        cuda_check(cudaMemset2DAsync((char*)d_slots_ + L.stamp, L.bytes, 0, 4 * (size_t)L.NC, slots, s), "memset stamps");
     }
     stats.slots = (int32_t)slots;
     stats.slot_bytes = L.bytes;
@@ -2357,7 +1322,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     A.order = (const int32_t*)(d + off_order_);
     A.counter = (int32_t*)(d + off_ctr_);
     A.n_windows = count;
-    A.sc = scoring_of(p_);
+    A.k = cell_consts(sc);
     A.b = p_.b;
     A.f = p_.f;
     A.ab_band = p_.ab_band;
@@ -2365,7 +1330,10 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     A.L = L;
     A.smem_per_warp = smem_w;
     A.sring_rows = sring_rows;
-    A.sring_blocks = sring_blocks;
+    A.sring_blocks = ring_blocks;
+    A.state_rows = state_rows;
+    A.stat_rows = stat_rows;
+    A.stat_blocks = ring_blocks;
     A.cons = o + out_cons_;
     A.cons_stride = cons_stride_;
     A.cons_len = (int32_t*)(o + out_len_);
@@ -2376,14 +1344,13 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     // the work-counter reset and the persistent launch, recorded as a CUDA graph and
     // replayed while the launch (variant, grid, shared memory, arguments) is unchanged
     struct KKey {
-        bool stat, dense;
+        BatchKernel kern;
         int blocks;
         size_t dyn;
         BatchArgs A;
     } key;
     std::memset(&key, 0, sizeof key);
-    key.stat = stat;
-    key.dense = dense;
+    key.kern = kern;
     key.blocks = blocks;
     key.dyn = dyn;
     key.A = A;
@@ -2393,13 +1360,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
         cudaGraph_t gr = nullptr;
         cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
         cudaMemsetAsync(A.counter, 0, 4, s);
-        if (stat) {
-            if (dense) k_batch<4, true, 4><<<blocks, 4 * 32, dyn, s>>>(A);
-            else k_batch<4, true, 3><<<blocks, 4 * 32, dyn, s>>>(A);
-        } else {
-            if (dense) k_batch<4, false, 4><<<blocks, 4 * 32, dyn, s>>>(A);
-            else k_batch<4, false, 3><<<blocks, 4 * 32, dyn, s>>>(A);
-        }
+        kern<<<blocks, 4 * 32, dyn, s>>>(A);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(s, &gr);
         cuda_check(le, "k_batch launch");

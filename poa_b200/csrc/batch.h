@@ -75,7 +75,10 @@ class BatchEngine {
     // still runs the reference's band, and a window that outgrows its slot is
     // re-run with the default sizing (counted in stats.fallback). nullptr
     // clears the plan. Cleared by upload().
-    void set_plan(const int32_t* nodes, const int64_t* tb_bytes, const int64_t* spill, const float* cost);
+    // cells: band cells of the largest alignment, nullptr when the plan has
+    // none (its record bytes bound them).
+    void set_plan(const int32_t* nodes, const int64_t* tb_bytes, const int64_t* spill, const float* cost,
+                  const int64_t* cells = nullptr);
     DeviceWindows device_windows() const;
     // Plan every run() with this proposer first (nullptr: no proposer).
     void set_proposer(Proposer* p) { proposer_ = p; }
@@ -90,7 +93,7 @@ class BatchEngine {
     void read_stats(std::vector<int32_t>& out);
     BatchStats stats;
     int32_t warps_per_block = 4;
-    int32_t blocks_per_sm = 3;  // 3: 168-register build; >= 4: 128-register build (occupancy still caps it)
+    int32_t blocks_per_sm = 3;  // 3: 168-register build; 4: 128; >= 5: 96 (occupancy still caps it)
     int32_t smem_per_warp = 18432;  // shared-memory row ring + staging / topsort workspace per warp
     int32_t max_blocks = 0;         // cap on the persistent grid (0 = one wave of resident blocks)
 
@@ -98,8 +101,7 @@ class BatchEngine {
     void ensure(void** ptr, size_t* cap, size_t bytes);
     struct Caps {
         int32_t NC;      // graph nodes per slot
-        int64_t tb_cap;  // traceback record bytes
-        int64_t spill;   // spilled row-store entries (int32)
+        int64_t cells;   // band cells of one alignment
     };
     Caps default_caps(int scale) const;
     int ring_blocks() const;
@@ -121,7 +123,7 @@ class BatchEngine {
 
   private:
     std::vector<int32_t> plan_nodes_, plan_order_;
-    std::vector<int64_t> plan_tb_, plan_spill_;
+    std::vector<int64_t> plan_tb_, plan_spill_, plan_cells_;
     int device_;
     void* stream_ = nullptr;
     void* ev0_ = nullptr;

@@ -554,8 +554,9 @@ int poa_batch_propose(poa_ctx* ctx, poa_proposer* p) {
         std::vector<int32_t> nodes;
         std::vector<int64_t> tb, spill;
         std::vector<float> cost;
-        p->prop->plan(ctx->batch->device_windows(), kPropK, kPropW, nodes, tb, spill, cost);
-        ctx->batch->set_plan(nodes.data(), tb.data(), spill.data(), cost.data());
+        std::vector<int64_t> cells;
+        p->prop->plan(ctx->batch->device_windows(), kPropK, kPropW, nodes, tb, spill, cost, cells);
+        ctx->batch->set_plan(nodes.data(), tb.data(), spill.data(), cost.data(), cells.data());
     } catch (const std::exception& e) {
         return fail(ctx, POA_CUDA, e.what());
     }

@@ -431,12 +431,12 @@ __global__ void __launch_bounds__(FT_THREADS) k_features(const uint8_t* __restri
 __global__ void k_plan(const float* __restrict__ pred, const int32_t* __restrict__ read_len,
                        const int32_t* __restrict__ win_off, int n_windows, const float* __restrict__ extra,
                        int32_t* __restrict__ nodes_out, int64_t* __restrict__ tb_out, int64_t* __restrict__ spill_out,
-                       float* __restrict__ cost_out) {
+                       float* __restrict__ cost_out, int64_t* __restrict__ cells_out) {
     GRID_STRIDE(wi, n_windows) {
         const int w = (int)wi;
         const int r0 = win_off[w], r1 = win_off[w + 1];
         double nodes = r1 > r0 ? 2.0 + read_len[r0] : 2.0;
-        double maxtb = 0.0, maxrows = 0.0, cost = 0.0;
+        double maxtb = 0.0, maxcells = 0.0, maxrows = 0.0, cost = 0.0;
         for (int r = r0 + 1; r < r1; r++) {
             const float* y = pred + (int64_t)r * PROP_OUT;
             const double rows = nodes;
@@ -444,6 +444,7 @@ __global__ void k_plan(const float* __restrict__ pred, const int32_t* __restrict
             const double cells = fmin(fmax((double)y[1], 0.01), 1.0) * rows * m;
             const double bpc = fmin(fmax((double)y[2], 1.0), 4.0);
             maxtb = fmax(maxtb, cells * bpc);
+            maxcells = fmax(maxcells, cells);
             maxrows = fmax(maxrows, rows);
             cost += cells;
             nodes += fmax((double)y[0], 0.0) * read_len[r];
@@ -452,6 +453,7 @@ __global__ void k_plan(const float* __restrict__ pred, const int32_t* __restrict
         tb_out[w] = (int64_t)(maxtb * extra[X_TB_MARGIN]) + 4096;
         spill_out[w] = (int64_t)fmax((double)extra[X_SPILL_MIN], maxrows * extra[X_SPILL_PER_ROW]);
         cost_out[w] = (float)cost;
+        cells_out[w] = (int64_t)(maxcells * extra[X_TB_MARGIN]) + 4096;
     }
 }
 
@@ -794,7 +796,7 @@ void Proposer::features_prep(const DeviceWindows& dw, int k, int w, int& bits_ou
 }
 
 void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>& nodes, std::vector<int64_t>& tb,
-                    std::vector<int64_t>& spill, std::vector<float>& cost) {
+                    std::vector<int64_t>& spill, std::vector<float>& cost, std::vector<int64_t>& cells) {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     cudaStream_t s = (cudaStream_t)dw.stream;
     const int64_t nr = std::max<int64_t>(dw.n_reads, 1);
@@ -812,7 +814,7 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
         pred_bytes_ = pb;
     }
     const int nw = dw.n_windows;
-    const size_t need = up256(4 * (size_t)nw) + 3 * up256(8 * (size_t)nw);
+    const size_t need = up256(4 * (size_t)nw) + 4 * up256(8 * (size_t)nw);
     if (need > plan_bytes_) {
         if (d_plan_) cuda_check(cudaFree(d_plan_), "cudaFree");
         d_plan_ = nullptr;
@@ -823,6 +825,7 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
     tb.assign(nw, 0);
     spill.assign(nw, 0);
     cost.assign(nw, 0.f);
+    cells.assign(nw, 0);
     if (nw == 0) return;
     int bits = 0, grid = 0;
     features_prep(dw, k, w, bits, grid);
@@ -832,6 +835,7 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
     int64_t* dt = (int64_t*)(p + up256(4 * (size_t)nw));
     int64_t* ds = (int64_t*)(p + up256(4 * (size_t)nw) + up256(8 * (size_t)nw));
     float* dc = (float*)(p + up256(4 * (size_t)nw) + 2 * up256(8 * (size_t)nw));
+    int64_t* dl = (int64_t*)(p + up256(4 * (size_t)nw) + 3 * up256(8 * (size_t)nw));
     // features, inference and plan: ~10 launches per 4,096 reads, recorded once as a
     // CUDA graph per batch shape and replayed with one launch
     const GraphKey key{dw.seq, dw.read_off, dw.read_len, dw.win_off, dw.n_reads, nw, k, w, bits, grid,
@@ -844,7 +848,7 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
         try {
             features_launch(dw, k, w, bits, grid, d_feat_, s);
             predict_launch(d_feat_, dw.n_reads, d_pred_, s);
-            k_plan<<<grid_of(nw), 256, 0, s>>>(d_pred_, dw.read_len, dw.win_off, nw, d_extra_, dn, dt, ds, dc);
+            k_plan<<<grid_of(nw), 256, 0, s>>>(d_pred_, dw.read_len, dw.win_off, nw, d_extra_, dn, dt, ds, dc, dl);
             cuda_check(cudaGetLastError(), "k_plan");
         } catch (...) {
             cudaStreamEndCapture(s, &gr);
@@ -864,6 +868,7 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
     cuda_check(cudaMemcpyAsync(tb.data(), dt, 8 * (size_t)nw, cudaMemcpyDeviceToHost, s), "D2H plan");
     cuda_check(cudaMemcpyAsync(spill.data(), ds, 8 * (size_t)nw, cudaMemcpyDeviceToHost, s), "D2H plan");
     cuda_check(cudaMemcpyAsync(cost.data(), dc, 4 * (size_t)nw, cudaMemcpyDeviceToHost, s), "D2H plan");
+    cuda_check(cudaMemcpyAsync(cells.data(), dl, 8 * (size_t)nw, cudaMemcpyDeviceToHost, s), "D2H plan");
     cuda_check(cudaStreamSynchronize(s), "proposer plan");
 }
 

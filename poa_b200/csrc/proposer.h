@@ -81,7 +81,7 @@ class Proposer {
     // Features + inference + per-window plan on the device; the plan comes
     // back to the host (one value per window each).
     void plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>& nodes, std::vector<int64_t>& tb,
-              std::vector<int64_t>& spill, std::vector<float>& cost);
+              std::vector<int64_t>& spill, std::vector<float>& cost, std::vector<int64_t>& cells);
 
     float extra(int i) const { return host_w_[PROP_NPARAM + i]; }
 

@@ -227,19 +227,27 @@ struct TeamHdr {
     int4 ed[HDR_E];
 };
 
-// Backtrack tile: BT_ROWS rows around the walk, BT_BLK blocks of each, their
-// rows and predecessor records (team_backtrack).
-constexpr int BT_ROWS = 64, BT_BLK = 8, BT_E = 160;
+// Backtrack tile (team_backtrack): up to BT_ROWS rows around the walk, as many
+// as `bytes` of shared memory hold, BLKS blocks of each, their rows, their
+// predecessor records and where their heaviest predecessors lead.
+constexpr int BT_ROWS = 64;
 
-template <bool WIDE>
-struct BtSmem {
-    static constexpr int ROWB = BT_BLK * BLK * Cells<WIDE>::BYTES;
-    static constexpr int CELLS = 0;
-    static constexpr int ROW = CELLS + BT_ROWS * ROWB;      // int4 {Bs, Be, store block, first block of the tile row}
-    static constexpr int PTR = ROW + BT_ROWS * 16;          // int [BT_ROWS + 1], padded
-    static constexpr int ED = PTR + (BT_ROWS + 4) * 4;
-    static constexpr int JUMP = ED + BT_E * 16;             // uint8 [5][BT_ROWS]: the tile row 1, 2, 4, 8, 16 heaviest predecessors back
-    static constexpr int BYTES = JUMP + 5 * BT_ROWS;
+template <bool WIDE, int BLKS>
+struct BtTile {
+    static constexpr int ROWB = BLKS * BLK * Cells<WIDE>::BYTES;
+    static constexpr int PER_ROW = ROWB + 16 + 3 * 16 + 4 + 5;
+    int rows, E;              // rows and predecessor records
+    int row, ed, ptr, jump;   // byte offsets: int4 {Bs, Be, store block, first block of the tile row}; int4; int; uint8 [5][rows]
+    __host__ __device__ explicit BtTile(int bytes) {
+        const int r = (bytes - 16) / PER_ROW;
+        rows = r < BT_ROWS ? r : BT_ROWS;
+        E = 3 * rows;
+        row = rows * ROWB;
+        ed = row + rows * 16;
+        ptr = ed + E * 16;
+        jump = ptr + (rows + 4) * 4;
+    }
+    static constexpr int full() { return BT_ROWS * PER_ROW + 16; }
 };
 
 template <int W, bool ADAPT, bool WIDE>
@@ -253,7 +261,7 @@ struct TeamSmem {
     static constexpr int REST = BEST + 2 * W * 16;
     static constexpr int FILL =
         REST + (ADAPT ? 2 * (int)sizeof(TeamHdr) + SWIN * SW_INTS * 4 : 2 * (int)sizeof(TeamStage));
-    static constexpr int BYTES = FILL > BtSmem<WIDE>::BYTES ? FILL : BtSmem<WIDE>::BYTES;
+    static constexpr int BYTES = FILL > BtTile<WIDE, 8>::full() ? FILL : BtTile<WIDE, 8>::full();
     static constexpr int THREADS = 32 * (W + (ADAPT ? 1 : 0));
 };
 
@@ -894,12 +902,13 @@ __device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) 
 // M == I is decided only when it is asked for, by looking for the cell the
 // gap opened from: I[j] is the maximum over k < j of M[k] + o1 + (j - 1 - k) * e1
 // and never exceeds M[j]. Once in a gap the walk carries the gap's value.
-template <bool WIDE>
-static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* smem, int lane, int32_t& nmoves) {
+template <bool WIDE, int BT_BLK>
+static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* smem, int bytes, int lane, int32_t& nmoves) {
     typedef typename Cells<WIDE>::One One;
-    typedef BtSmem<WIDE> T;
+    const BtTile<WIDE, BT_BLK> T(bytes);
+    constexpr int ROWB = BtTile<WIDE, BT_BLK>::ROWB, BACK = BT_BLK - (BT_BLK >= 8 ? 3 : 2);  // blocks kept left of the walk's
     constexpr int32_t NEG = Cells<WIDE>::NEG;
-    constexpr int CB = Cells<WIDE>::BYTES, RL = T::ROWB / 16;  // 16-byte pieces of a tile row
+    constexpr int CB = Cells<WIDE>::BYTES, RL = ROWB / 16;  // 16-byte pieces of a tile row
     const CellK k = a.k;
     const One* store = reinterpret_cast<const One*>(a.store);
     const int4* rowi = a.rowi;
@@ -915,41 +924,41 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
     int32_t st = ST_OK;
     while (i > 0 || acj > 0) {
         int4 R = make_int4(0, 0, 0, 0);
-        if (i >= lo) R = lds128(sb + T::ROW + (i - lo) * 16);
+        if (i >= lo) R = lds128(sb + T.row + (i - lo) * 16);
         if (i < lo || (unsigned)((acj >> 3) - R.w) >= BT_BLK) {
             // the tile that ends with row i
-            lo = max(0, i - BT_ROWS + 1);
+            lo = max(0, i - T.rows + 1);
             const int cnt = i - lo + 1;
             const int dB = (acj >> 3) - rowi[i].x;
             __syncwarp();
             for (int r = lane; r < cnt; r += 32) {
                 int4 v = rowi[lo + r];
-                v.w = v.x + max(0, dB - (BT_BLK - 3));
-                *reinterpret_cast<int4*>(smem + T::ROW + r * 16) = v;
+                v.w = v.x + max(0, dB - BACK);
+                *reinterpret_cast<int4*>(smem + T.row + r * 16) = v;
             }
-            for (int r = lane; r <= cnt; r += 32) *reinterpret_cast<int32_t*>(smem + T::PTR + r * 4) = a.in_ptr[lo + r];
+            for (int r = lane; r <= cnt; r += 32) *reinterpret_cast<int32_t*>(smem + T.ptr + r * 4) = a.in_ptr[lo + r];
             __syncwarp();
-            e_lo = lds32(sb + T::PTR);
-            ne = min(lds32(sb + T::PTR + cnt * 4) - e_lo, BT_E);
-            for (int e = lane; e < ne; e += 32) cp_async16(smem + T::ED + e * 16, edg + e_lo + e);
+            e_lo = lds32(sb + T.ptr);
+            ne = min(lds32(sb + T.ptr + cnt * 4) - e_lo, T.E);
+            for (int e = lane; e < ne; e += 32) cp_async16(smem + T.ed + e * 16, edg + e_lo + e);
             for (int x = lane; x < cnt * RL; x += 32) {
                 const int r = x / RL, pc = x % RL;
-                const int4 v = *reinterpret_cast<const int4*>(smem + T::ROW + r * 16);
+                const int4 v = *reinterpret_cast<const int4*>(smem + T.row + r * 16);
                 const int blk = v.w + pc * 16 / (BLK * CB);
                 if (blk <= v.y - 2)
-                    cp_async16(smem + T::CELLS + r * T::ROWB + pc * 16,
+                    cp_async16(smem + r * ROWB + pc * 16,
                                a.store + ((int64_t)v.z + (v.w - v.x)) * (BLK * CB) + pc * 16);
             }
             cp_async_commit_all();
             cp_async_wait_all();
             __syncwarp();
-            uint8_t* jump = reinterpret_cast<uint8_t*>(smem + T::JUMP);
-            for (int r = lane; r < BT_ROWS; r += 32) {
+            uint8_t* jump = reinterpret_cast<uint8_t*>(smem + T.jump);
+            for (int r = lane; r < T.rows; r += 32) {
                 int to = 255;
                 if (r < cnt && lo + r > 0) {
-                    const int e = lds32(sb + T::PTR + r * 4) - e_lo, e1 = lds32(sb + T::PTR + r * 4 + 4) - e_lo;
+                    const int e = lds32(sb + T.ptr + r * 4) - e_lo, e1 = lds32(sb + T.ptr + r * 4 + 4) - e_lo;
                     if (e < e1 && e < ne) {
-                        const int p = lds32(sb + T::ED + e * 16) >> 4;
+                        const int p = lds32(sb + T.ed + e * 16) >> 4;
                         if (p >= lo) to = p - lo;
                     }
                 }
@@ -958,34 +967,34 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
 #pragma unroll
             for (int q = 1; q < 5; q++) {
                 __syncwarp();
-                for (int r = lane; r < BT_ROWS; r += 32) {
-                    const int h = jump[(q - 1) * BT_ROWS + r];
-                    jump[q * BT_ROWS + r] = h == 255 ? 255 : jump[(q - 1) * BT_ROWS + h];
+                for (int r = lane; r < T.rows; r += 32) {
+                    const int h = jump[(q - 1) * T.rows + r];
+                    jump[q * T.rows + r] = h == 255 ? 255 : jump[(q - 1) * T.rows + h];
                 }
             }
             __syncwarp();
-            R = lds128(sb + T::ROW + (i - lo) * 16);
+            R = lds128(sb + T.row + (i - lo) * 16);
         }
         if (op & M_OP) {
             // a run of matches with the heaviest predecessors
-            const uint8_t* jump = reinterpret_cast<const uint8_t*>(smem + T::JUMP);
+            const uint8_t* jump = reinterpret_cast<const uint8_t*>(smem + T.jump);
             int r = i - lo;
 #pragma unroll
             for (int q = 0; q < 5; q++)
-                if ((lane >> q) & 1) r = r == 255 ? 255 : jump[q * BT_ROWS + r];
+                if ((lane >> q) & 1) r = r == 255 ? 255 : jump[q * T.rows + r];
             const int c = acj - lane;
             bool ok = false;
             int32_t mv = 0;
             const int to = r == 255 ? 255 : jump[r];
             if (to != 255 && c > 0) {
-                const int4 A = lds128(sb + T::ROW + r * 16), P = lds128(sb + T::ROW + to * 16);
-                const int4 er = lds128(sb + T::ED + (lds32(sb + T::PTR + r * 4) - e_lo) * 16);
+                const int4 A = lds128(sb + T.row + r * 16), P = lds128(sb + T.row + to * 16);
+                const int4 er = lds128(sb + T.ed + (lds32(sb + T.ptr + r * 4) - e_lo) * 16);
                 const int qc = qs[c], bl = (c - 1) >> 3;
                 // both cells in their rows' bands and in the tile
                 if ((c >> 3) <= A.y - 2 && (unsigned)((c >> 3) - A.w) < BT_BLK && bl <= P.y - 2 && (unsigned)(bl - P.w) < BT_BLK &&
                     (er.x & 15) == (qc | 8)) {
-                    const int32_t x = One::lds(sb + T::CELLS + r * T::ROWB + (c - A.w * BLK) * CB).m();
-                    const int32_t y = One::lds(sb + T::CELLS + to * T::ROWB + (c - 1 - P.w * BLK) * CB).m();
+                    const int32_t x = One::lds(sb + r * ROWB + (c - A.w * BLK) * CB).m();
+                    const int32_t y = One::lds(sb + to * ROWB + (c - 1 - P.w * BLK) * CB).m();
                     ok = x == add32(y, k.match);
                     mv = mv_pack(MV_MATCH, lo + to, qc);
                 }
@@ -1006,9 +1015,9 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
         const int j = acj - Bs * BLK;
         if (j >= (Be - Bs - 1) * BLK) { st = ST_BT_FAIL; break; }
         if (nm + 1 > cap) { st = ST_OOM; break; }
-        const int e0 = lds32(sb + T::PTR + (i - lo) * 4) - e_lo;
-        const int d = i == 0 ? 0 : lds32(sb + T::PTR + (i - lo) * 4 + 4) - e_lo - e0;
-        const One cell = One::lds(sb + T::CELLS + (i - lo) * T::ROWB + (acj - R.w * BLK) * CB);
+        const int e0 = lds32(sb + T.ptr + (i - lo) * 4) - e_lo;
+        const int d = i == 0 ? 0 : lds32(sb + T.ptr + (i - lo) * 4 + 4) - e_lo - e0;
+        const One cell = One::lds(sb + (i - lo) * ROWB + (acj - R.w * BLK) * CB);
         const int qc = acj > 0 ? qs[acj] : 4;
         const int32_t M = cell.m();
         const bool eq_md = cell.eq_md(k);
@@ -1020,21 +1029,21 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
             int4 er = make_int4(0, 0, 0, 0);
             if (k0 + lane < d) {
                 const int e = e0 + k0 + lane;
-                if (e < ne) er = lds128(sb + T::ED + e * 16);
+                if (e < ne) er = lds128(sb + T.ed + e * 16);
                 else er = edg[e_lo + e];
                 const int p = er.x >> 4;
                 const int bl = (acj - 1) >> 3, bc = acj >> 3;
                 const bool inl = acj > 0 && bl >= er.y && bl <= er.z - 2;
                 const bool inc = bc >= er.y && bc <= er.z - 2;
                 int w0 = INT_MIN / 2;
-                if (p >= lo) w0 = lds32(sb + T::ROW + (p - lo) * 16 + 12);
+                if (p >= lo) w0 = lds32(sb + T.row + (p - lo) * 16 + 12);
                 One vl, vc;
                 if (inl) {
-                    if ((unsigned)(bl - w0) < BT_BLK) vl = One::lds(sb + T::CELLS + (p - lo) * T::ROWB + (acj - 1 - w0 * BLK) * CB);
+                    if ((unsigned)(bl - w0) < BT_BLK) vl = One::lds(sb + (p - lo) * ROWB + (acj - 1 - w0 * BLK) * CB);
                     else vl = store[(int64_t)er.w * BLK + (acj - 1 - er.y * BLK)];
                 }
                 if (inc) {
-                    if ((unsigned)(bc - w0) < BT_BLK) vc = One::lds(sb + T::CELLS + (p - lo) * T::ROWB + (acj - w0 * BLK) * CB);
+                    if ((unsigned)(bc - w0) < BT_BLK) vc = One::lds(sb + (p - lo) * ROWB + (acj - w0 * BLK) * CB);
                     else vc = store[(int64_t)er.w * BLK + (acj - er.y * BLK)];
                     eo = vc.d_opens(dv, k);
                     ex = vc.d_extends(dv, k);
@@ -1119,11 +1128,11 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
 }
 
 // Score, status and moves of a filled alignment (warp 0).
-template <bool WIDE>
-static __device__ void team_finish(const TeamJob& a, char* smem, int64_t cells, int lane) {
+template <bool WIDE, int BLKS>
+static __device__ void team_finish(const TeamJob& a, char* smem, int bytes, int64_t cells, int lane) {
     const int m = a.qlen + 1;
     int32_t nm = 0;
-    const int32_t st = team_backtrack<WIDE>(a, smem, lane, nm);
+    const int32_t st = team_backtrack<WIDE, BLKS>(a, smem, bytes, lane, nm);
     if (lane == 0) {
         const int4 last = a.rowi[a.n - 1];
         const int jm = m - last.x * BLK;
@@ -1178,7 +1187,7 @@ __global__ void __launch_bounds__(TeamSmem<W, ADAPT, WIDE>::THREADS, 1) k_align(
         }
         return;
     }
-    if (threadIdx.x < 32) team_finish<WIDE>(a, tsm, cells, threadIdx.x);
+    if (threadIdx.x < 32) team_finish<WIDE, 8>(a, tsm, S::BYTES, cells, threadIdx.x);
 }
 
 }  // namespace pb
