@@ -8,11 +8,15 @@
 // window: fusion (src/graph.cpp:170-235) is warp-parallel with stamp-based
 // conflict detection and a sequential fallback (dg_fuse_warp / dg_fuse_seq);
 // the LIFO topological sort (src/graph.cpp:21-128) runs its Kahn loop over a
-// shared-memory CSR copy, with hlen/tlen as depths by pointer jumping over
-// the warp; the window view of the DP rows, the shifted query, the fill and
-// the static-band backtrack use the whole warp; the adaptive-band backtrack
-// and the consensus (src/graph.cpp:294-351) are the reference's sequential
-// walks, run by lane 0.
+// shared-memory CSR copy, with hlen/tlen as depths by pointer jumping over the
+// warp; the DP rows (build_rows), the fill (warp.cuh) and the backtrack
+// (team.cuh) use the whole warp; the consensus (src/graph.cpp:294-351) is the
+// reference's sequential walk, run by lane 0.
+//
+// The graph steps are bound by the latency of dependent reads from a slot, so
+// they go over the edge array, not over the nodes' lists (coalesced, and a
+// node of high degree does not hold its warp up), and take several chunks of
+// 32 at a time so that their reads overlap.
 #include "batch.h"
 #include "proposer.h"
 
@@ -39,7 +43,7 @@ struct SlotLayout {
     int64_t hdr, base, par, aligned, ind, rank, in_head, in_tail, out_head, out_tail, in_cnt, out_cnt;
     int64_t e_from, e_to, e_w, e_nin, e_nout;
     int64_t rank_to_id, hlen, tlen, deg, stk, pre, score, hin, hout, stamp;
-    int64_t v_in_ptr, v_out_ptr, v_out_row, v_maxs, v_ed, v_fe, v_rowi, v_fr, v_ra;
+    int64_t v_in_ptr, v_out_ptr, v_out_row, v_maxs, v_ed, v_fe, v_deal, v_rowi, v_fr, v_ra;
     int64_t state, qs, moves, path, store;
     int64_t bytes;
 };
@@ -64,6 +68,7 @@ SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int64_t store_bytes, 
     L.v_in_ptr = take(n4 + 4);
     L.v_out_ptr = take(n4 + 4); L.v_out_row = take(e4); L.v_maxs = take(n4);
     L.v_ed = take(16 * (size_t)EC);
+    L.v_deal = take(16 * (size_t)EC);
     L.v_rowi = take(16 * (size_t)NC);
     if (stat) {
         L.v_fe = take(16 * (size_t)EC);
@@ -434,27 +439,58 @@ __device__ int dg_fuse_warp(DevGraph& g, const int32_t* moves, int nm, int beg_i
 // out-edge (pass 1, tlen: src/graph.cpp:103-121). Roots keep the value the
 // array already holds at their rank (the reference resizes the vector and
 // never writes there), except the sink, whose tlen is 1. Written back by rank.
+constexpr int GU = 4;  // chunks of 32 taken together
+
 template <typename T>
 __device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, T* P, T* Q, T* D, T* E, int lane) {
     const T none = (T)-1;
-    for (int u = lane; u < nn; u += 32) {
-        const int e = pass == 0 ? g.hin[u] : g.hout[u];
-        const int par = e < 0 ? -1 : (pass == 0 ? g.e_from[e] : g.e_to[e]);
-        P[u] = par < 0 ? none : (T)par;
-        D[u] = par >= 0 ? (T)1 : (T)((pass == 1 && u == 1) ? 1 : arr[g.rank[u]]);
+    const int32_t* heavy = pass == 0 ? g.hin : g.hout;
+    const int32_t* end = pass == 0 ? g.e_from : g.e_to;
+    for (int u0 = lane; u0 < nn; u0 += 32 * GU) {
+        int e[GU], par[GU], root[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) e[q] = u0 + 32 * q < nn ? heavy[u0 + 32 * q] : -1;
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int u = u0 + 32 * q;
+            par[q] = e[q] >= 0 ? end[e[q]] : -1;
+            root[q] = e[q] < 0 && u < nn && !(pass == 1 && u == 1) ? arr[g.rank[u]] : 1;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int u = u0 + 32 * q;
+            if (u >= nn) break;
+            P[u] = par[q] < 0 ? none : (T)par[q];
+            D[u] = (T)root[q];
+        }
     }
     __syncwarp();
     for (int it = 0; it < 40; it++) {
         bool moved = false;
-        for (int u = lane; u < nn; u += 32) {
-            const T p = P[u];
-            if (p != none) {
-                E[u] = (T)(D[u] + D[p]);
-                Q[u] = P[p];
-                moved = true;
-            } else {
-                E[u] = D[u];
-                Q[u] = none;
+        for (int u0 = lane; u0 < nn; u0 += 32 * GU) {
+            T p[GU], d[GU], pp[GU], dp[GU];
+#pragma unroll
+            for (int q = 0; q < GU; q++) {
+                const int u = u0 + 32 * q;
+                p[q] = u < nn ? P[u] : none;
+                d[q] = u < nn ? D[u] : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < GU; q++) {
+                pp[q] = none;
+                dp[q] = 0;
+                if (p[q] != none) {
+                    pp[q] = P[p[q]];
+                    dp[q] = D[p[q]];
+                    moved = true;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < GU; q++) {
+                const int u = u0 + 32 * q;
+                if (u >= nn) break;
+                E[u] = (T)(d[q] + dp[q]);
+                Q[u] = pp[q];
             }
         }
         __syncwarp();
@@ -462,162 +498,180 @@ __device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, T* P, T*
         t = D; D = E; E = t;
         if (!__any_sync(0xffffffffu, moved)) break;
     }
-    for (int u = lane; u < nn; u += 32) arr[g.rank[u]] = (int32_t)D[u];
+    for (int u0 = lane; u0 < nn; u0 += 32 * GU) {
+        int r[GU];
+        T d[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int u = u0 + 32 * q;
+            r[q] = u < nn ? g.rank[u] : 0;
+            d[q] = u < nn ? D[u] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++)
+            if (u0 + 32 * q < nn) arr[r[q]] = (int32_t)d[q];
+    }
     __syncwarp();
 }
 
-// Topological sort with the whole warp: the out-lists are copied into
-// shared memory as CSR (16-bit ids), the LIFO Kahn loop of
-// src/graph.cpp:61-85 then runs on lane 0 over shared memory only, and
-// hlen/tlen (src/graph.cpp:86-123) are depths in the heaviest-in-edge and
-// heaviest-out-edge forests, computed by pointer jumping across the warp
-// (double-buffered in the slot's scratch arrays). Graphs too large for the
-// shared-memory budget use the sequential global-memory version.
-// The same LIFO Kahn order for graphs whose 16-bit lists do not fit the warp's
-// shared memory: out-lists as int32 CSR in the slot's view arrays, in-degree
-// counters (8 bits) and the stack (16 bits) in shared memory. Returns false
-// when an in-degree exceeds 255 or the stack outgrows its space; the caller
-// then sorts on the global lists, which recomputes every rank.
-__device__ bool topsort_large(DevGraph& g, int nn, uint8_t* sm, int sm_bytes, int lane) {
-    int32_t* optr = g.csr_ptr;
-    int32_t* adj = g.csr_adj;
-    uint8_t* deg = sm;
-    uint16_t* stk = reinterpret_cast<uint16_t*>(sm + ((nn + 15) & ~15));
-    const int cap = (sm_bytes - ((nn + 15) & ~15)) / 2;
+// Out-lists as CSR in list order, which is edge-id order: the edges in order,
+// 32 at a time; lanes with the same start node take consecutive places. cur[u]
+// holds the first place of node u's list and ends at the last. An entry's
+// `one` bit says that the edge is its end node's only in-edge.
+template <typename A, typename CUR>
+__device__ void fill_out_csr(const DevGraph& g, int ne, A* adj, A one, CUR* cur, const uint8_t* deg, int lane) {
+    const unsigned lt = (1u << lane) - 1u;
+    for (int e0 = 0; e0 < ne; e0 += 32 * GU) {
+        int f[GU], t[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int e = e0 + 32 * q + lane;
+            f[q] = e < ne ? g.e_from[e] : -1 - lane;
+            t[q] = e < ne ? g.e_to[e] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            if (e0 + 32 * q >= ne) break;
+            const unsigned same = __match_any_sync(0xffffffffu, f[q]);
+            const int at = f[q] >= 0 ? (int)cur[f[q]] : 0;
+            __syncwarp();
+            if (f[q] >= 0) {
+                adj[at + __popc(same & lt)] = (A)(t[q] | (deg[t[q]] == 1 ? one : (A)0));
+                if ((same >> lane) == 1u) cur[f[q]] = (CUR)(at + __popc(same));
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Exclusive prefix sums of the out-degrees, and 8-bit in-degrees; false when
+// an in-degree exceeds 255.
+template <typename P, typename CUR>
+__device__ bool scan_degrees(const DevGraph& g, int nn, P* optr, CUR* cur, uint8_t* deg, int lane) {
     int carry = 0;
     bool big = false;
-    for (int c0 = 0; c0 < nn; c0 += 32) {
-        const int u = c0 + lane;
-        const int c = u < nn ? g.out_cnt[u] : 0;
-        int x = c;
+    for (int c0 = 0; c0 < nn; c0 += 32 * GU) {
+        int c[GU], ic[GU];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+        for (int q = 0; q < GU; q++) {
+            const int u = c0 + 32 * q + lane;
+            c[q] = u < nn ? g.out_cnt[u] : 0;
+            ic[q] = u < nn ? g.in_cnt[u] : 0;
         }
-        if (u < nn) optr[u] = carry + x - c;
-        carry += __shfl_sync(0xffffffffu, x, 31);
-    }
-    if (lane == 0) optr[nn] = carry;
-    for (int u = lane; u < nn; u += 32) {
-        int k = optr[u];
-        for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) adj[k++] = g.e_to[e];
-        const int ic = g.in_cnt[u];
-        big |= ic > 255;
-        deg[u] = (uint8_t)ic;
-    }
-    if (__any_sync(0xffffffffu, big)) return false;
-    // zero in-degree seeds in id order
-    int sp = 0;
-    bool over = false;
-    for (int c0 = 0; c0 < nn; c0 += 32) {
-        const int u = c0 + lane;
-        const bool z = u < nn && deg[u] == 0;
-        const unsigned msk = __ballot_sync(0xffffffffu, z);
-        over |= sp + __popc(msk) > cap;
-        if (z && !over) stk[sp + __popc(msk & ((1u << lane) - 1u))] = (uint16_t)u;
-        sp += __popc(msk);
-    }
-    __syncwarp();
-    if (over) return false;
-    int nr = 0;
-    if (lane == 0) {
-        while (sp && !over) {
-            const int u = stk[--sp];
-            g.rank[u] = nr;
-            g.rank_to_id[nr++] = u;
-            const int k1 = optr[u + 1];
-            for (int k = optr[u]; k < k1; k++) {
-                const int v = adj[k];
-                const int dv = deg[v] - 1;
-                deg[v] = (uint8_t)dv;
-                if (dv == 0) {
-                    if (sp >= cap) { over = true; break; }
-                    stk[sp++] = (uint16_t)v;
-                }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int u = c0 + 32 * q + lane;
+            int x = c[q];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
             }
+            if (u < nn) {
+                optr[u] = (P)(carry + x - c[q]);
+                cur[u] = (CUR)(carry + x - c[q]);
+                deg[u] = (uint8_t)ic[q];
+                big |= ic[q] > 255;
+            }
+            carry += __shfl_sync(0xffffffffu, x, 31);
         }
-        if (!over) g.hdr[3] = nr;
     }
-    over = __shfl_sync(0xffffffffu, over, 0);
-    __syncwarp();
-    return !over;
+    if (lane == 0) optr[nn] = (P)carry;
+    return !__any_sync(0xffffffffu, big);
 }
 
-__device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uint16_t* sm, int sm_bytes,
-                                int lane) {
-    const size_t need = 2 * ((size_t)nn + 1) + 2 * (size_t)ne + 4 * (size_t)nn + 16;
-    if (nn >= 65535 || ne >= 65535 || need > (size_t)sm_bytes) {
-        if (nn < 65535 && (size_t)nn + 16 + 2 * 256 <= (size_t)sm_bytes) {
-            if (topsort_large(g, nn, (uint8_t*)sm, sm_bytes, lane)) {
-                if (with_lens)
-                    for (int pass = 0; pass < 2; pass++)
-                        depth_jump<int32_t>(g, nn, pass, pass == 0 ? g.hlen : g.tlen, g.deg, g.stk, g.pre, g.score,
-                                            lane);
-                return;
+// The LIFO Kahn order (src/graph.cpp:61-85) on lane 0: zero in-degree nodes
+// seeded in id order, successors pushed in list order. The node on top of the
+// stack stays in a register; ord takes the order from its start and the rest
+// of the stack from its end (never more than n entries together). Returns the
+// number of ranks.
+template <typename P, typename A>
+__device__ int kahn_lifo(const P* optr, const A* adj, A one, uint8_t* deg, uint16_t* ord, int nn, int sp) {
+    int nr = 0, u = -1;
+    uint16_t* top = ord + nn - sp;  // the stack's top entry
+    uint16_t* const end = ord + nn;
+    while (true) {
+        if (u < 0) {
+            if (top == end) break;
+            u = *top++;
+        }
+        ord[nr++] = (uint16_t)u;
+        int k = (int)optr[u];
+        const int k1 = (int)optr[u + 1];
+        u = -1;
+        for (; k < k1; k++) {
+            const A x = adj[k];
+            const int v = (int)(x & (A)~one);
+            bool ready = (x & one) != 0;
+            if (!ready) {
+                const int dv = deg[v] - 1;
+                deg[v] = (uint8_t)dv;
+                ready = dv == 0;
+            }
+            if (ready) {
+                if (u >= 0) *--top = (uint16_t)u;
+                u = v;
             }
         }
+    }
+    return nr;
+}
+
+// Topological sort with the whole warp: out-lists as CSR (16 bits in shared
+// memory; 32 bits in the slot's view arrays for graphs that do not fit), the
+// Kahn loop on lane 0, ranks written in parallel, then hlen/tlen
+// (src/graph.cpp:86-123) as depths in the heaviest-in-edge and
+// heaviest-out-edge forests by pointer jumping (shared memory when it fits).
+// Graphs beyond the shared-memory budget, or with an in-degree above 255, use
+// the sequential global-memory version.
+__device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uint16_t* sm, int sm_bytes, int lane) {
+    auto up4 = [](size_t x) { return (x + 3) & ~(size_t)3; };
+    const size_t n_ord = up4(2 * (size_t)nn), n_deg = up4((size_t)nn), n_ptr = up4(2 * ((size_t)nn + 1));
+    uint16_t* ord = sm;
+    uint8_t* deg = (uint8_t*)sm + n_ord;
+    uint16_t* optr = (uint16_t*)(deg + n_deg);
+    uint16_t* adj = (uint16_t*)((uint8_t*)optr + n_ptr);
+    const bool small = nn < 32768 && ne < 65535 && n_ord + n_deg + n_ptr + 2 * (size_t)ne <= (size_t)sm_bytes;
+    const bool large = !small && nn < 65535 && n_ord + n_deg <= (size_t)sm_bytes;
+    bool ok = small || large;
+    if (ok) {
+        if (small) ok = scan_degrees(g, nn, optr, ord, deg, lane);
+        else ok = scan_degrees(g, nn, g.csr_ptr, g.deg, deg, lane);
+    }
+    if (!ok) {
         if (lane == 0) g.hdr[3] = dg_topsort(g, nn, with_lens);
         __syncwarp();
         return;
     }
-    uint16_t* optr = sm;
-    uint16_t* adj = optr + nn + 1;
-    uint16_t* deg = adj + ne;
-    uint16_t* stk = deg + nn;
-    int carry = 0;
-    for (int c0 = 0; c0 < nn; c0 += 32) {
-        const int u = c0 + lane;
-        const int c = u < nn ? g.out_cnt[u] : 0;
-        int x = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (u < nn) optr[u] = (uint16_t)(carry + x - c);
-        carry += __shfl_sync(0xffffffffu, x, 31);
-    }
-    if (lane == 0) optr[nn] = (uint16_t)carry;
-    for (int u = lane; u < nn; u += 32) {
-        int k = 0;
-        const int base_k = (int)optr[u];
-        for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) adj[base_k + k++] = (uint16_t)g.e_to[e];
-        deg[u] = (uint16_t)g.in_cnt[u];
-    }
     __syncwarp();
-    // zero in-degree seeds in id order
-    int sp = 0;
+    if (small) fill_out_csr(g, ne, adj, (uint16_t)0x8000, ord, deg, lane);
+    else fill_out_csr(g, ne, g.csr_adj, (int32_t)(1 << 30), g.deg, deg, lane);
+    // zero in-degree seeds: the last in id order on top
+    int seeds = 0;
     for (int c0 = 0; c0 < nn; c0 += 32) {
         const int u = c0 + lane;
         const bool z = u < nn && deg[u] == 0;
         const unsigned msk = __ballot_sync(0xffffffffu, z);
-        if (z) stk[sp + __popc(msk & ((1u << lane) - 1u))] = (uint16_t)u;
-        sp += __popc(msk);
+        if (z) ord[nn - 1 - seeds - __popc(msk & ((1u << lane) - 1u))] = (uint16_t)u;
+        seeds += __popc(msk);
     }
     __syncwarp();
+    int nr = 0;
     if (lane == 0) {
-        int nr = 0;
-        while (sp) {
-            const int u = stk[--sp];
-            g.rank[u] = nr;
-            g.rank_to_id[nr++] = u;
-            const int k1 = optr[u + 1];
-            for (int k = optr[u]; k < k1; k++) {
-                const int v = adj[k];
-                const int dv = deg[v] - 1;
-                deg[v] = (uint16_t)dv;
-                if (dv == 0) stk[sp++] = (uint16_t)v;
-            }
-        }
+        if (small) nr = kahn_lifo(optr, adj, (uint16_t)0x8000, deg, ord, nn, seeds);
+        else nr = kahn_lifo(g.csr_ptr, g.csr_adj, (int32_t)(1 << 30), deg, ord, nn, seeds);
         g.hdr[3] = nr;
+    }
+    nr = __shfl_sync(0xffffffffu, nr, 0);
+    __syncwarp();
+    for (int i = lane; i < nr; i += 32) {
+        const int u = ord[i];
+        g.rank_to_id[i] = u;
+        g.rank[u] = i;
     }
     __syncwarp();
     if (!with_lens) return;
-    // hlen / tlen: depths in the forests of heaviest in-edges (hin) and
-    // heaviest out-edges (hout), by pointer jumping; 16-bit arrays in shared
-    // memory when they fit, the slot's int32 scratch otherwise
-    const bool sm_ok = 8 * (size_t)nn + 16 <= (size_t)sm_bytes;
+    const bool sm_ok = nn < 65535 && 8 * (size_t)nn + 16 <= (size_t)sm_bytes;
     for (int pass = 0; pass < 2; pass++) {
         int32_t* arr = pass == 0 ? g.hlen : g.tlen;
         if (sm_ok) depth_jump<uint16_t>(g, nn, pass, arr, sm, sm + nn, sm + 2 * nn, sm + 3 * nn, lane);
@@ -629,14 +683,14 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
 // whole warp: in-edges in the backtrack's priority order (TeamJob::ed), and
 // for the static band, whose rows depend only on hlen / tlen, every row's
 // band, row-store place and fill header; for the dynamic bands the control
-// data of TeamJob::ra. One walk over the in-lists fills the out-edges too:
-// their order within a row does not matter to the band update (successors
-// are distinct rows).
+// data of TeamJob::ra. The edges are dealt to their rows in any order and then
+// placed by weight (descending) and edge id, which is list order; a row's
+// out-edges stay in any order (its successors are distinct rows, so the band
+// update does not depend on it).
 template <bool STATIC, bool WIDE>
-__device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, TeamJob& v, int m, int wband, int lane, int& n_out,
-                          int& beg_out) {
+__device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, int m, int wband, int lane, int& n_out, int& beg_out) {
     const SlotLayout& L = A.L;
-    const int beg_i = g.rank[0], end_i = g.rank[1];
+    const int beg_i = g.rank[0], end_i = g.rank[1], ne = g.hdr[1];
     const int n = end_i - beg_i + 1;
     beg_out = beg_i;
     n_out = n;
@@ -645,9 +699,11 @@ __device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, TeamJob& v, 
     int32_t* out_ptr = (int32_t*)(s + L.v_out_ptr);
     int32_t* out_row = (int32_t*)(s + L.v_out_row);
     int32_t* maxs = (int32_t*)(s + L.v_maxs);
-    int32_t* cur = (int32_t*)(s + L.deg);  // topsort scratch, free until the next sort
+    int32_t* ocur = (int32_t*)(s + L.deg);  // topsort scratch, free until the next sort
+    int32_t* icur = (int32_t*)(s + L.stk);
     int4* ed = (int4*)(s + L.v_ed);
     int4* fe = (int4*)(s + L.v_fe);
+    int4* dealt = (int4*)(s + L.v_deal);
     int4* rowi = (int4*)(s + L.v_rowi);
     int4* fr = (int4*)(s + L.v_fr);
     int4* ra = (int4*)(s + L.v_ra);
@@ -656,91 +712,139 @@ __device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, TeamJob& v, 
     bool bad = false;
     int ci_c = 0, co_c = 0, bn_c = 0;
     if (lane == 0) in_ptr[0] = 0;
-    for (int c0 = 0; c0 < n; c0 += 32) {
-        const int r = c0 + lane;
-        int ci = 0, co = 0, bn = 0, Bs = 0, Be = 1;
-        if (r < n) {
-            const int u = g.rank_to_id[beg_i + r];
-            if (whole) {
-                ci = g.in_cnt[u];
-                co = g.out_cnt[u];
-            } else {
-                for (int e = g.in_head[u]; e >= 0; e = g.e_nin[e]) ci += (g.rank[g.e_from[e]] - beg_i >= 0);
-                for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e]) co += (g.rank[g.e_to[e]] - beg_i < n);
+    for (int c0 = 0; c0 < n; c0 += 32 * GU) {
+        int u[GU], cis[GU], cos[GU], hl[GU], tl[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int r = c0 + 32 * q + lane;
+            u[q] = r < n ? g.rank_to_id[beg_i + r] : -1;
+            hl[q] = STATIC && r < n ? g.hlen[beg_i + r] : 0;
+            tl[q] = STATIC && r < n ? g.tlen[beg_i + r] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            cis[q] = cos[q] = 0;
+            if (u[q] >= 0) {
+                if (whole) {
+                    cis[q] = g.in_cnt[u[q]];
+                    cos[q] = g.out_cnt[u[q]];
+                } else {
+                    for (int e = g.in_head[u[q]]; e >= 0; e = g.e_nin[e]) cis[q] += (g.rank[g.e_from[e]] - beg_i >= 0);
+                    for (int e = g.out_head[u[q]]; e >= 0; e = g.e_nout[e]) cos[q] += (g.rank[g.e_to[e]] - beg_i < n);
+                }
             }
-            if (STATIC) {
-                band_static(A.f, g.hlen[beg_i + r] - h0, g.tlen[beg_i + r] - t0, m, wband, Bs, Be);
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int r = c0 + 32 * q + lane;
+            const int ci = cis[q], co = cos[q];
+            int bn = 0, Bs = 0, Be = 1;
+            if (STATIC && r < n) {
+                band_static(A.f, hl[q] - h0, tl[q] - t0, m, wband, Bs, Be);
                 if (r == 0) Bs = 0;
                 bn = Be - Bs - 1;
                 bad |= bn < 0 || (r > 0 && ci > MAX_MULTI_PRED);
                 bn = max(bn, 0);
             }
-            maxs[r] = r;
-        }
-        int xi = ci, xo = co, xb = bn;
+            int xi = ci, xo = STATIC ? bn : co;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int yi = __shfl_up_sync(0xffffffffu, xi, o), yo = __shfl_up_sync(0xffffffffu, xo, o),
-                      yb = __shfl_up_sync(0xffffffffu, xb, o);
-            if (lane >= o) { xi += yi; xo += yo; xb += yb; }
-        }
-        if (r < n) {
-            in_ptr[r + 1] = ci_c + xi;
-            if (STATIC) {
-                rowi[r] = make_int4(Bs, Be, bn_c + xb - bn, 0);
-            } else {
-                out_ptr[r] = cur[r] = co_c + xo - co;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int yi = __shfl_up_sync(0xffffffffu, xi, o), yo = __shfl_up_sync(0xffffffffu, xo, o);
+                if (lane >= o) { xi += yi; xo += yo; }
             }
+            if (r < n) {
+                in_ptr[r + 1] = ci_c + xi;
+                icur[r] = ci_c + xi - ci;
+                maxs[r] = r;
+                if (STATIC) rowi[r] = make_int4(Bs, Be, bn_c + xo - bn, 0);
+                else out_ptr[r] = ocur[r] = co_c + xo - co;
+            }
+            ci_c += __shfl_sync(0xffffffffu, xi, 31);
+            (STATIC ? bn_c : co_c) += __shfl_sync(0xffffffffu, xo, 31);
         }
-        ci_c += __shfl_sync(0xffffffffu, xi, 31);
-        co_c += __shfl_sync(0xffffffffu, xo, 31);
-        bn_c += __shfl_sync(0xffffffffu, xb, 31);
     }
     if (!STATIC && lane == 0) out_ptr[n] = co_c;
     if (__any_sync(0xffffffffu, bad)) return ST_DEGENERATE;
     if (bn_c > L.store_cap) return ST_OOM;
     __syncwarp();
+    // the edges to their rows: {weight, edge, record, row}
+    for (int e0 = lane; e0 < ne; e0 += 32 * GU) {
+        int f[GU], t[GU], w[GU], p[GU], r[GU], b[GU], at[GU], to[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int e = e0 + 32 * q;
+            f[q] = e < ne ? g.e_from[e] : -1;
+            t[q] = e < ne ? g.e_to[e] : 0;
+            w[q] = e < ne ? g.e_w[e] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            p[q] = f[q] >= 0 ? g.rank[f[q]] - beg_i : -1;
+            r[q] = f[q] >= 0 ? g.rank[t[q]] - beg_i : -1;
+            b[q] = f[q] >= 0 ? g.base[f[q]] : 0;
+            if (r[q] >= n) p[q] = -1;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++)
+            if (p[q] >= 0) {
+                at[q] = atomicAdd(&icur[r[q]], 1);
+                to[q] = STATIC ? 0 : atomicAdd(&ocur[p[q]], 1);
+                atomicMax(&maxs[p[q]], r[q]);
+            }
+#pragma unroll
+        for (int q = 0; q < GU; q++)
+            if (p[q] >= 0) {
+                dealt[at[q]] = make_int4(w[q], e0 + 32 * q, (p[q] << 4) | (p[q] == 0 ? 4 : b[q]), r[q]);
+                if (!STATIC) out_row[to[q]] = r[q];
+            }
+    }
+    __syncwarp();
     const int R = A.sring_rows, RB = A.sring_blocks;
     constexpr int BB = BLK * Cells<WIDE>::BYTES;
-    for (int r = lane; r < n; r += 32) {
-        const int u = g.rank_to_id[beg_i + r];
-        const int e0 = in_ptr[r];
-        int d = 0;
-        for (int e = g.in_head[u]; e >= 0;) {
-            const int from = g.e_from[e], w = g.e_w[e];
-            e = g.e_nin[e];
-            const int p = g.rank[from] - beg_i;
-            if (p < 0) continue;
-            // insertion by weight; ties keep list order
-            int at = e0 + d;
-            while (at > e0 && ed[at - 1].y < w) { ed[at] = ed[at - 1]; at--; }
-            ed[at] = make_int4((p << 4) | (p == 0 ? 4 : (int)g.base[from]), w, 0, 0);
-            d++;
-            atomicMax(&maxs[p], r);
-            if (!STATIC) out_row[atomicAdd(&cur[p], 1)] = r;
+    for (int k0 = lane; k0 < ci_c; k0 += 32 * GU) {
+        int4 x[GU], pr[GU];
+        int lo[GU], hi[GU], least[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) x[q] = k0 + 32 * q < ci_c ? dealt[k0 + 32 * q] : make_int4(0, 0, 0, 0);
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            lo[q] = in_ptr[x[q].w];
+            hi[q] = in_ptr[x[q].w + 1];
+            least[q] = g.rank_to_id[beg_i + x[q].w];
+            if (STATIC) pr[q] = rowi[x[q].z >> 4];
         }
-        const int least = g.ind[u] / 10;
-        for (int k = 0; k < d; k++) {
-            int4 x = ed[e0 + k];
-            if (x.y >= least) x.x |= 8;
+#pragma unroll
+        for (int q = 0; q < GU; q++) least[q] = g.ind[least[q]] / 10;
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            if (k0 + 32 * q >= ci_c) break;
+            int at = lo[q];
+            if (hi[q] - lo[q] > 1)
+                for (int k = lo[q]; k < hi[q]; k++) {
+                    const int2 y = *reinterpret_cast<const int2*>(&dealt[k]);
+                    at += y.x > x[q].x || (y.x == x[q].x && y.y < x[q].y);
+                }
+            int4 v = make_int4(x[q].z | (x[q].x >= least[q] ? 8 : 0), 0, 0, 0);
             if (STATIC) {
-                const int p = x.x >> 4;
-                const int4 pr = rowi[p];
-                const bool near = r - p < R && pr.y - pr.x - 1 <= RB;
-                fe[e0 + k] = make_int4(near ? (p & (R - 1)) * RB * BB : -1, (x.x & 7) * 0x01010101, pr.x, pr.y - 2 - pr.x);
-                x.y = pr.x; x.z = pr.y; x.w = pr.z;
+                const int p = v.x >> 4;
+                const bool near = x[q].w - p < R && pr[q].y - pr[q].x - 1 <= RB;
+                fe[at] = make_int4(near ? (p & (R - 1)) * RB * BB : -1, (v.x & 7) * 0x01010101, pr[q].x,
+                                   pr[q].y - 2 - pr[q].x);
+                v.y = pr[q].x; v.z = pr[q].y; v.w = pr[q].z;
             }
-            ed[e0 + k] = x;
+            ed[at] = v;
         }
+    }
+    for (int r = lane; r < n; r += 32) {
+        const int e0 = in_ptr[r], d = in_ptr[r + 1] - e0;
         if (STATIC) {
             const int4 ri = rowi[r];
             const int eoff = e0 - in_ptr[r & ~(WSTG - 1)];
-            if (r == 0) d = 0;
             fr[r] = make_int4(ri.x, ri.y - 2 - ri.x, ri.z,
-                              d | (eoff + d > WSTG_E ? FR_UNSTAGED : eoff << FR_EOFF));
+                              (r == 0 ? 0 : d) | (eoff + d > WSTG_E ? FR_UNSTAGED : eoff << FR_EOFF));
         } else {
             ra[2 * r] = make_int4(e0, out_ptr[r], g.hlen[beg_i + r] - h0, g.tlen[beg_i + r] - t0);
-            ra[2 * r + 1] = make_int4(g.hlen[r] - h0, g.base[u], d, out_ptr[r + 1] - out_ptr[r]);
+            ra[2 * r + 1] = make_int4(g.hlen[r] - h0, g.base[g.rank_to_id[beg_i + r]], d, out_ptr[r + 1] - out_ptr[r]);
         }
     }
     __syncwarp();
@@ -849,7 +953,7 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         tick(PH_FUSE);
         // DP rows of the whole graph and the shifted query
         int beg_i = 0, n = 0;
-        int st = build_rows<STATIC, WIDE>(g, s, A, a, len + 1, A.b + (A.f ? (len + 1) / A.f : 0), lane, n, beg_i);
+        int st = build_rows<STATIC, WIDE>(g, s, A, len + 1, A.b + (A.f ? (len + 1) / A.f : 0), lane, n, beg_i);
         if (STATIC && st != ST_OK) { status = st; break; }
         uint8_t* qs = (uint8_t*)(s + L.qs);
         const int64_t qsb = qs_bytes(len);
