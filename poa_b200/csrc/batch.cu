@@ -434,16 +434,17 @@ __device__ int dg_fuse_warp(DevGraph& g, const int32_t* moves, int nm, int beg_i
     return ST_OK;
 }
 
+constexpr int GU = 4;  // chunks of 32 taken together
+
 // Depth of every node in the forest where each node's parent is the far end
 // of its heaviest in-edge (pass 0, hlen: src/graph.cpp:86-101) or heaviest
 // out-edge (pass 1, tlen: src/graph.cpp:103-121). Roots keep the value the
 // array already holds at their rank (the reference resizes the vector and
 // never writes there), except the sink, whose tlen is 1. Written back by rank.
-constexpr int GU = 4;  // chunks of 32 taken together
-
-template <typename T>
-__device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, T* P, T* Q, T* D, T* E, int lane) {
-    const T none = (T)-1;
+// Pointer jumping in place: a word holds (ancestor, distance to it), 16 bits
+// each, so a word read while others change is a valid pair all the same.
+__device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, uint32_t* W, int lane) {
+    constexpr uint32_t NONE = 0xffffu;
     const int32_t* heavy = pass == 0 ? g.hin : g.hout;
     const int32_t* end = pass == 0 ? g.e_from : g.e_to;
     for (int u0 = lane; u0 < nn; u0 += 32 * GU) {
@@ -459,53 +460,36 @@ __device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, T* P, T*
 #pragma unroll
         for (int q = 0; q < GU; q++) {
             const int u = u0 + 32 * q;
-            if (u >= nn) break;
-            P[u] = par[q] < 0 ? none : (T)par[q];
-            D[u] = (T)root[q];
+            if (u < nn) W[u] = ((par[q] < 0 ? NONE : (uint32_t)par[q]) << 16) | (uint32_t)root[q];
         }
     }
     __syncwarp();
     for (int it = 0; it < 40; it++) {
         bool moved = false;
         for (int u0 = lane; u0 < nn; u0 += 32 * GU) {
-            T p[GU], d[GU], pp[GU], dp[GU];
+            uint32_t w[GU], a[GU];
 #pragma unroll
-            for (int q = 0; q < GU; q++) {
-                const int u = u0 + 32 * q;
-                p[q] = u < nn ? P[u] : none;
-                d[q] = u < nn ? D[u] : 0;
-            }
+            for (int q = 0; q < GU; q++) w[q] = u0 + 32 * q < nn ? W[u0 + 32 * q] : NONE << 16;
 #pragma unroll
-            for (int q = 0; q < GU; q++) {
-                pp[q] = none;
-                dp[q] = 0;
-                if (p[q] != none) {
-                    pp[q] = P[p[q]];
-                    dp[q] = D[p[q]];
+            for (int q = 0; q < GU; q++) a[q] = (w[q] >> 16) != NONE ? W[w[q] >> 16] : 0;
+#pragma unroll
+            for (int q = 0; q < GU; q++)
+                if ((w[q] >> 16) != NONE) {
+                    W[u0 + 32 * q] = a[q] + (w[q] & 0xffffu);
                     moved = true;
                 }
-            }
-#pragma unroll
-            for (int q = 0; q < GU; q++) {
-                const int u = u0 + 32 * q;
-                if (u >= nn) break;
-                E[u] = (T)(d[q] + dp[q]);
-                Q[u] = pp[q];
-            }
         }
         __syncwarp();
-        T* t = P; P = Q; Q = t;
-        t = D; D = E; E = t;
         if (!__any_sync(0xffffffffu, moved)) break;
     }
     for (int u0 = lane; u0 < nn; u0 += 32 * GU) {
         int r[GU];
-        T d[GU];
+        uint32_t d[GU];
 #pragma unroll
         for (int q = 0; q < GU; q++) {
             const int u = u0 + 32 * q;
             r[q] = u < nn ? g.rank[u] : 0;
-            d[q] = u < nn ? D[u] : 0;
+            d[q] = u < nn ? W[u] & 0xffffu : 0;
         }
 #pragma unroll
         for (int q = 0; q < GU; q++)
@@ -516,10 +500,9 @@ __device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, T* P, T*
 
 // Out-lists as CSR in list order, which is edge-id order: the edges in order,
 // 32 at a time; lanes with the same start node take consecutive places. cur[u]
-// holds the first place of node u's list and ends at the last. An entry's
-// `one` bit says that the edge is its end node's only in-edge.
+// holds the first place of node u's list and ends at the last.
 template <typename A, typename CUR>
-__device__ void fill_out_csr(const DevGraph& g, int ne, A* adj, A one, CUR* cur, const uint8_t* deg, int lane) {
+__device__ void fill_out_csr(const DevGraph& g, int ne, A* adj, CUR* cur, int lane) {
     const unsigned lt = (1u << lane) - 1u;
     for (int e0 = 0; e0 < ne; e0 += 32 * GU) {
         int f[GU], t[GU];
@@ -536,7 +519,7 @@ __device__ void fill_out_csr(const DevGraph& g, int ne, A* adj, A one, CUR* cur,
             const int at = f[q] >= 0 ? (int)cur[f[q]] : 0;
             __syncwarp();
             if (f[q] >= 0) {
-                adj[at + __popc(same & lt)] = (A)(t[q] | (deg[t[q]] == 1 ? one : (A)0));
+                adj[at + __popc(same & lt)] = (A)t[q];
                 if ((same >> lane) == 1u) cur[f[q]] = (CUR)(at + __popc(same));
             }
             __syncwarp();
@@ -580,39 +563,59 @@ __device__ bool scan_degrees(const DevGraph& g, int nn, P* optr, CUR* cur, uint8
     return !__any_sync(0xffffffffu, big);
 }
 
-// The LIFO Kahn order (src/graph.cpp:61-85) on lane 0: zero in-degree nodes
-// seeded in id order, successors pushed in list order. The node on top of the
-// stack stays in a register; ord takes the order from its start and the rest
-// of the stack from its end (never more than n entries together). Returns the
-// number of ranks.
+// The LIFO Kahn order (src/graph.cpp:61-85): zero in-degree nodes seeded in id
+// order, successors pushed in list order. The order itself is a serial chain;
+// the warp takes a node's out-edges at once (they end at distinct nodes) and
+// reads the lists' ends of every successor before it is known which one comes
+// next. The node on top of the stack stays in a register; ord takes the order
+// from its start and the rest of the stack from its end (never more than n
+// entries together). Returns the number of ranks.
 template <typename P, typename A>
-__device__ int kahn_lifo(const P* optr, const A* adj, A one, uint8_t* deg, uint16_t* ord, int nn, int sp) {
-    int nr = 0, u = -1;
-    uint16_t* top = ord + nn - sp;  // the stack's top entry
-    uint16_t* const end = ord + nn;
+__device__ int kahn_lifo(const P* optr, const A* adj, uint8_t* deg, uint16_t* ord, int nn, int sp, int lane) {
+    int nr = 0, top = nn - sp;  // ord[top]: the stack's top entry
+    int u = -1, k = 0, k1 = 0;
     while (true) {
         if (u < 0) {
-            if (top == end) break;
-            u = *top++;
+            if (top == nn) break;
+            u = ord[top++];
+            k = (int)optr[u];
+            k1 = (int)optr[u + 1];
         }
-        ord[nr++] = (uint16_t)u;
-        int k = (int)optr[u];
-        const int k1 = (int)optr[u + 1];
+        __syncwarp();
+        if (lane == 0) ord[nr] = (uint16_t)u;
+        nr++;
         u = -1;
-        for (; k < k1; k++) {
-            const A x = adj[k];
-            const int v = (int)(x & (A)~one);
-            bool ready = (x & one) != 0;
-            if (!ready) {
+        int n0 = 0, n1 = 0;
+        for (; k < k1; k += 32) {
+            bool ready = false;
+            int v = 0, v0 = 0, v1 = 0;
+            if (k + lane < k1) {
+                v = (int)adj[k + lane];
                 const int dv = deg[v] - 1;
-                deg[v] = (uint8_t)dv;
+                v0 = (int)optr[v];
+                v1 = (int)optr[v + 1];
                 ready = dv == 0;
+                deg[v] = (uint8_t)dv;
             }
-            if (ready) {
-                if (u >= 0) *--top = (uint16_t)u;
-                u = v;
+            const unsigned msk = __ballot_sync(0xffffffffu, ready);
+            if (!msk) continue;
+            if (u >= 0) {  // ready in the chunk before (more than 32 out-edges)
+                top--;
+                if (lane == 0) ord[top] = (uint16_t)u;
             }
+            const int last = 31 - __clz(msk);
+            const unsigned rest = msk & ~(1u << last);
+            if (rest) {
+                top -= __popc(rest);
+                if ((rest >> lane) & 1u) ord[top + __popc(rest >> 1 >> lane)] = (uint16_t)v;
+            }
+            u = __shfl_sync(0xffffffffu, v, last);
+            n0 = __shfl_sync(0xffffffffu, v0, last);
+            n1 = __shfl_sync(0xffffffffu, v1, last);
         }
+        k = n0;
+        k1 = n1;
+        __syncwarp();
     }
     return nr;
 }
@@ -631,7 +634,7 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
     uint8_t* deg = (uint8_t*)sm + n_ord;
     uint16_t* optr = (uint16_t*)(deg + n_deg);
     uint16_t* adj = (uint16_t*)((uint8_t*)optr + n_ptr);
-    const bool small = nn < 32768 && ne < 65535 && n_ord + n_deg + n_ptr + 2 * (size_t)ne <= (size_t)sm_bytes;
+    const bool small = nn < 65535 && ne < 65535 && n_ord + n_deg + n_ptr + 2 * (size_t)ne <= (size_t)sm_bytes;
     const bool large = !small && nn < 65535 && n_ord + n_deg <= (size_t)sm_bytes;
     bool ok = small || large;
     if (ok) {
@@ -644,8 +647,8 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
         return;
     }
     __syncwarp();
-    if (small) fill_out_csr(g, ne, adj, (uint16_t)0x8000, ord, deg, lane);
-    else fill_out_csr(g, ne, g.csr_adj, (int32_t)(1 << 30), g.deg, deg, lane);
+    if (small) fill_out_csr(g, ne, adj, ord, lane);
+    else fill_out_csr(g, ne, g.csr_adj, g.deg, lane);
     // zero in-degree seeds: the last in id order on top
     int seeds = 0;
     for (int c0 = 0; c0 < nn; c0 += 32) {
@@ -656,13 +659,9 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
         seeds += __popc(msk);
     }
     __syncwarp();
-    int nr = 0;
-    if (lane == 0) {
-        if (small) nr = kahn_lifo(optr, adj, (uint16_t)0x8000, deg, ord, nn, seeds);
-        else nr = kahn_lifo(g.csr_ptr, g.csr_adj, (int32_t)(1 << 30), deg, ord, nn, seeds);
-        g.hdr[3] = nr;
-    }
-    nr = __shfl_sync(0xffffffffu, nr, 0);
+    const int nr = small ? kahn_lifo(optr, adj, deg, ord, nn, seeds, lane)
+                         : kahn_lifo(g.csr_ptr, g.csr_adj, deg, ord, nn, seeds, lane);
+    if (lane == 0) g.hdr[3] = nr;
     __syncwarp();
     for (int i = lane; i < nr; i += 32) {
         const int u = ord[i];
@@ -671,12 +670,9 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
     }
     __syncwarp();
     if (!with_lens) return;
-    const bool sm_ok = nn < 65535 && 8 * (size_t)nn + 16 <= (size_t)sm_bytes;
-    for (int pass = 0; pass < 2; pass++) {
-        int32_t* arr = pass == 0 ? g.hlen : g.tlen;
-        if (sm_ok) depth_jump<uint16_t>(g, nn, pass, arr, sm, sm + nn, sm + 2 * nn, sm + 3 * nn, lane);
-        else depth_jump<int32_t>(g, nn, pass, arr, g.deg, g.stk, g.pre, g.score, lane);
-    }
+    uint32_t* W = 4 * (size_t)nn <= (size_t)sm_bytes ? reinterpret_cast<uint32_t*>(sm) : reinterpret_cast<uint32_t*>(g.deg);
+    depth_jump(g, nn, 0, g.hlen, W, lane);
+    depth_jump(g, nn, 1, g.tlen, W, lane);
 }
 
 // The DP rows of window [rank(source), rank(sink)] for one alignment, with the
@@ -1325,6 +1321,18 @@ void BatchEngine::set_plan(const int32_t* nodes, const int64_t* tb_bytes, const 
     std::stable_sort(plan_order_.begin(), plan_order_.end(), [&](int a, int b) { return cost[a] > cost[b]; });
 }
 
+// Shared memory per warp of a launch over `count` windows: what was configured,
+// or the default where that fills the GPU; with fewer windows the blocks that
+// share an SM divide it, so that larger graphs are sorted in shared memory
+// (16-bit lists: ~9 bytes a node; 18 KB hold ~2,000 nodes, 48 KB ~5,000).
+int BatchEngine::shared_per_warp(int32_t count, int warps, int sms) const {
+    if (smem_set) return smem_per_warp;
+    const int blocks = (count + warps - 1) / warps;
+    const int per_sm = std::max(1, (blocks + sms - 1) / sms);
+    const int share = (220 * 1024 / per_sm / warps - 256) / 16 * 16;
+    return std::max(smem_per_warp, std::min(share, 48 * 1024));
+}
+
 void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps, double headroom) {
     cudaStream_t s = (cudaStream_t)stream_;
     int sms = 0;
@@ -1343,7 +1351,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     SlotLayout L = make_layout(NC, EC, QC, store, stat, adaptive, wide);
     const SlotLayout L_planned = L;
     const int warps = warps_per_block;
-    const int smem_w = smem_per_warp;
+    const int smem_w = shared_per_warp(count, warps, sms);
     const size_t dyn = (size_t)warps * smem_w;
     const int qsm_bytes = (int)((qs_bytes(QC) + 15) / 16 * 16);
     constexpr int kStageBytes = 1792;  // shared memory a static-band warp needs beside its query

@@ -95,6 +95,7 @@ class BatchEngine {
     int32_t warps_per_block = 4;
     int32_t blocks_per_sm = 3;  // 3: 168-register build; 4: 128; >= 5: 96 (occupancy still caps it)
     int32_t smem_per_warp = 18432;  // shared-memory row ring + staging / topsort workspace per warp
+    bool smem_set = false;          // smem_per_warp was configured: used as it is
     int32_t max_blocks = 0;         // cap on the persistent grid (0 = one wave of resident blocks)
 
   private:
@@ -104,6 +105,7 @@ class BatchEngine {
         int64_t cells;   // band cells of one alignment
     };
     Caps default_caps(int scale) const;
+    int shared_per_warp(int32_t count, int warps, int sms) const;
     int ring_blocks() const;
     // one persistent launch over `count` windows (ids) with slots of the given
     // capacities, grown by up to `headroom` when memory allows every resident warp one

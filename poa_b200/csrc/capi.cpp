@@ -391,6 +391,7 @@ int poa_batch_config(poa_ctx* ctx, int32_t key, int64_t value) {
             if (value < 1024 || value > 48 * 1024 || value % 16 != 0)
                 return fail(ctx, POA_BAD_ARG, "smem per warp: 1024..49152 bytes, a multiple of 16");
             ctx->batch->smem_per_warp = (int32_t)value;
+            ctx->batch->smem_set = true;
             break;
         default: return fail(ctx, POA_BAD_ARG, "unknown key");
     }
