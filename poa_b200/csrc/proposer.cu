@@ -1,9 +1,7 @@
 // proposer.cu - features, network (training and inference) and window plan of
 // the learned band proposer; see proposer.h for what it predicts and why.
 //
-// Everything here is hand-written CUDA: a tiled BF16 x BF16 -> FP32 GEMM for
-// the convolutions (as im2col products) and the dense layers, small
-// elementwise kernels for im2col / col2im, ReLU masks, pooling, the loss and
+// Everything here is hand-written CUDA: the network kernel (prop_net.cuh),
 // Adam, the minimizer feature kernel and the plan kernel.
 #include "proposer.h"
 
@@ -19,6 +17,7 @@
 
 #include "batch.h"
 #include "gpu_engine.h"
+#include "prop_net.cuh"
 #include "sketch.h"
 
 namespace pb {
@@ -27,15 +26,13 @@ namespace {
 typedef __nv_bfloat16 bf16;
 
 constexpr int T = PROP_BINS;
-constexpr int KC1 = PROP_KW * PROP_CIN;  // im2col width of layer 1
-constexpr int KC = PROP_KW * PROP_CH;    // im2col width of layers 2, 3
-// parameter offsets (floats)
-constexpr int OW1 = 0, OB1 = OW1 + PROP_CH * KC1;
-constexpr int OW2 = OB1 + PROP_CH, OB2 = OW2 + PROP_CH * KC;
-constexpr int OW3 = OB2 + PROP_CH, OB3 = OW3 + PROP_CH * KC;
-constexpr int OW4 = OB3 + PROP_CH, OB4 = OW4 + PROP_CH * PROP_CH;
-constexpr int OW5 = OB4 + PROP_CH, OB5 = OW5 + PROP_OUT * PROP_CH;
-static_assert(OB5 + PROP_OUT == PROP_NPARAM, "parameter layout");
+using net::OB5;
+using net::OW1;
+using net::OW2;
+using net::OW3;
+using net::OW4;
+using net::OW5;
+constexpr int KC1 = net::KC1, KC = net::KC;
 // extras
 constexpr int X_MEAN = 0, X_STD = 4, X_NODE_MARGIN = 8, X_TB_MARGIN = 9, X_SPILL_PER_ROW = 10, X_SPILL_MIN = 11;
 
@@ -43,199 +40,13 @@ inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // ---------------------------------------------------------------------------
-// GEMM: C[M][N] = A x B (+ bias[n]) (ReLU), FP32 accumulation of BF16 operands.
-// A element (m,k) = TA ? A[k*lda + m] : A[m*lda + k];
-// B element (k,n) = TB ? B[n*ldb + k] : B[k*ldb + n].
-// 64x64 tile per CTA of 256 threads (4x4 outputs each), K in steps of 16.
-constexpr int GT = 64, GK = 16;
-
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_gemm(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B, int ldb,
-                                              float* __restrict__ C, bf16* __restrict__ Cb, int ldc, int64_t M, int N,
-                                              int64_t K, const float* __restrict__ bias, int relu) {
-    __shared__ float As[GK][GT + 4];
-    __shared__ float Bs[GK][GT + 4];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t m0 = (int64_t)blockIdx.x * GT;
-    const int n0 = blockIdx.y * GT;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-    for (int64_t k0 = 0; k0 < K; k0 += GK) {
-        for (int e = tid; e < GT * GK; e += 256) {
-            int mm, kk;
-            if (TA) { mm = e % GT; kk = e / GT; } else { kk = e % GK; mm = e / GK; }
-            const int64_t gm = m0 + mm, gk = k0 + kk;
-            float v = 0.f;
-            if (gm < M && gk < K) v = __bfloat162float(TA ? A[gk * lda + gm] : A[gm * lda + gk]);
-            As[kk][mm] = v;
-        }
-        for (int e = tid; e < GT * GK; e += 256) {
-            int nn, kk;
-            if (TB) { kk = e % GK; nn = e / GK; } else { nn = e % GT; kk = e / GT; }
-            const int gn = n0 + nn;
-            const int64_t gk = k0 + kk;
-            float v = 0.f;
-            if (gn < N && gk < K) v = __bfloat162float(TB ? B[(int64_t)gn * ldb + gk] : B[gk * ldb + gn]);
-            Bs[kk][nn] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int64_t gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            float v = acc[i][j];
-            if (bias) v += bias[gn];
-            if (relu) v = fmaxf(v, 0.f);
-            if (C) C[gm * ldc + gn] = v;
-            if (Cb) Cb[gm * ldc + gn] = __float2bfloat16(v);
-        }
-    }
-}
-
-template <bool TA, bool TB>
-void gemm(cudaStream_t s, const bf16* A, int lda, const bf16* B, int ldb, float* C, bf16* Cb, int ldc, int64_t M,
-          int N, int64_t K, const float* bias, int relu) {
-    if (M <= 0 || N <= 0) return;
-    dim3 grid((unsigned)cdiv(M, GT), (unsigned)cdiv(N, GT));
-    k_gemm<TA, TB><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, Cb, ldc, M, N, K, bias, relu);
-}
-
-// ---------------------------------------------------------------------------
 // elementwise kernels (grid-stride)
 #define GRID_STRIDE(i, n) for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
 inline unsigned grid_of(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), 148 * 16)); }
 
-// Xc[r][k*C + c] = x[r + k - 1][c] when bin t + k - 1 of the same read is in range
-__global__ void k_im2col(const bf16* __restrict__ x, bf16* __restrict__ xc, int64_t rows, int C) {
-    const int KCw = PROP_KW * C;
-    GRID_STRIDE(i, rows * KCw) {
-        const int c = (int)(i % C);
-        const int k = (int)((i / C) % PROP_KW);
-        const int64_t r = i / KCw;
-        const int tt = (int)(r % T) + k - 1;
-        xc[i] = (tt >= 0 && tt < T) ? x[(r + k - 1) * C + c] : __float2bfloat16(0.f);
-    }
-}
-
-// dy[r][c] = (sum_k dxc[r - k + 1][k*C + c]) * (y[r][c] > 0), as BF16
-__global__ void k_col2im_relu(const float* __restrict__ dxc, const bf16* __restrict__ y, bf16* __restrict__ dy,
-                              int64_t rows, int C) {
-    const int KCw = PROP_KW * C;
-    GRID_STRIDE(i, rows * C) {
-        const int c = (int)(i % C);
-        const int64_t r = i / C;
-        const int t = (int)(r % T);
-        float s = 0.f;
-#pragma unroll
-        for (int k = 0; k < PROP_KW; k++) {
-            const int tt = t - k + 1;
-            if (tt >= 0 && tt < T) s += dxc[(r - k + 1) * KCw + k * C + c];
-        }
-        dy[i] = __float2bfloat16(__bfloat162float(y[i]) > 0.f ? s : 0.f);
-    }
-}
-
-// h[b][c] = mean over bins of y[b*T + t][c]
-__global__ void k_pool(const bf16* __restrict__ y, bf16* __restrict__ h, int64_t nb) {
-    GRID_STRIDE(i, nb * PROP_CH) {
-        const int c = (int)(i % PROP_CH);
-        const int64_t b = i / PROP_CH;
-        float s = 0.f;
-        for (int t = 0; t < T; t++) s += __bfloat162float(y[(b * T + t) * PROP_CH + c]);
-        h[i] = __float2bfloat16(s * (1.f / T));
-    }
-}
-
-// dy[b*T + t][c] = dh[b][c] / T * (y > 0)
-__global__ void k_unpool_relu(const float* __restrict__ dh, const bf16* __restrict__ y, bf16* __restrict__ dy,
-                              int64_t nb) {
-    GRID_STRIDE(i, nb * T * PROP_CH) {
-        const int c = (int)(i % PROP_CH);
-        const int64_t b = i / ((int64_t)T * PROP_CH);
-        const float g = dh[b * PROP_CH + c] * (1.f / T);
-        dy[i] = __float2bfloat16(__bfloat162float(y[i]) > 0.f ? g : 0.f);
-    }
-}
-
-// out = d * (y > 0) as BF16
-__global__ void k_relu_mask(const float* __restrict__ d, const bf16* __restrict__ y, bf16* __restrict__ out, int64_t n) {
-    GRID_STRIDE(i, n) out[i] = __float2bfloat16(__bfloat162float(y[i]) > 0.f ? d[i] : 0.f);
-}
-
 __global__ void k_to_bf16(const float* __restrict__ x, bf16* __restrict__ y, int64_t n) {
     GRID_STRIDE(i, n) y[i] = __float2bfloat16(x[i]);
-}
-
-// training batch: rows idx[0..nb) of X (host layout [n][T][CIN]) and of the
-// standardised targets
-__global__ void k_gather(const float* __restrict__ X, const float* __restrict__ Y, const int32_t* __restrict__ idx,
-                         int nb, const float* __restrict__ extra, bf16* __restrict__ xb, float* __restrict__ yb) {
-    GRID_STRIDE(i, (int64_t)nb * T * PROP_CIN) {
-        const int64_t b = i / (T * PROP_CIN);
-        xb[i] = __float2bfloat16(X[(int64_t)idx[b] * T * PROP_CIN + i % (T * PROP_CIN)]);
-    }
-    GRID_STRIDE(i, (int64_t)nb * PROP_OUT) {
-        const int64_t b = i / PROP_OUT;
-        const int o = (int)(i % PROP_OUT);
-        yb[i] = (Y[(int64_t)idx[b] * PROP_OUT + o] - extra[X_MEAN + o]) / extra[X_STD + o];
-    }
-}
-
-// mean squared error over nb x 4 outputs; gradient as BF16; loss summed into *loss
-__global__ void k_loss(const float* __restrict__ o, const float* __restrict__ y, bf16* __restrict__ dob, int nb,
-                       float* __restrict__ loss) {
-    __shared__ float red[256];
-    float acc = 0.f;
-    const float scale = 1.f / (float)(nb * PROP_OUT);
-    for (int i = threadIdx.x; i < nb * PROP_OUT; i += blockDim.x) {
-        const float d = o[i] - y[i];
-        acc += d * d * scale;
-        dob[i] = __float2bfloat16(2.f * d * scale);
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
-        if ((int)threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *loss += red[0];
-}
-
-// g[n] = sum over rows of d[r][n]; one CTA per column
-__global__ void k_colsum(const bf16* __restrict__ d, int64_t rows, int N, float* __restrict__ g) {
-    __shared__ float red[256];
-    const int n = blockIdx.x;
-    float acc = 0.f;
-    for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) acc += __bfloat162float(d[r * N + n]);
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
-        if ((int)threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) g[n] = red[0];
 }
 
 // Adam on the FP32 master weights, refreshing the BF16 copy
@@ -250,14 +61,6 @@ __global__ void k_adam(float* __restrict__ w, bf16* __restrict__ wb, const float
         const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
         w[i] = wi;
         wb[i] = __float2bfloat16(wi);
-    }
-}
-
-// raw outputs: y * std + mean
-__global__ void k_destd(const float* __restrict__ o, const float* __restrict__ extra, float* __restrict__ y, int64_t n) {
-    GRID_STRIDE(i, n * PROP_OUT) {
-        const int k = (int)(i % PROP_OUT);
-        y[i] = o[i] * extra[X_STD + k] + extra[X_MEAN + k];
     }
 }
 
@@ -459,48 +262,12 @@ __global__ void k_plan(const float* __restrict__ pred, const int32_t* __restrict
 
 }  // namespace
 
-// ---------------------------------------------------------------------------
-// activations of one forward/backward pass over nb reads
-struct Act {
-    bf16 *x0, *xc1, *y1, *xc2, *y2, *xc3, *y3, *h, *z, *dob, *dzb, *dy3, *dy2, *dy1;
-    float *o, *yt, *dz, *dh, *dxc, *loss;
-};
-
-static size_t act_layout(int64_t nb, Act* a, char* base) {
-    const int64_t R = nb * T;
-    size_t o = 0;
-    auto take = [&](size_t bytes) { size_t r = o; o = up256(o + bytes); return base ? base + r : nullptr; };
-    Act t;
-    t.x0 = (bf16*)take(2 * R * PROP_CIN);
-    t.xc1 = (bf16*)take(2 * R * KC1);
-    t.y1 = (bf16*)take(2 * R * PROP_CH);
-    t.xc2 = (bf16*)take(2 * R * KC);
-    t.y2 = (bf16*)take(2 * R * PROP_CH);
-    t.xc3 = (bf16*)take(2 * R * KC);
-    t.y3 = (bf16*)take(2 * R * PROP_CH);
-    t.h = (bf16*)take(2 * nb * PROP_CH);
-    t.z = (bf16*)take(2 * nb * PROP_CH);
-    t.o = (float*)take(4 * nb * PROP_OUT);
-    t.yt = (float*)take(4 * nb * PROP_OUT);
-    t.dob = (bf16*)take(2 * nb * PROP_OUT);
-    t.dz = (float*)take(4 * nb * PROP_CH);
-    t.dzb = (bf16*)take(2 * nb * PROP_CH);
-    t.dh = (float*)take(4 * nb * PROP_CH);
-    t.dy3 = (bf16*)take(2 * R * PROP_CH);
-    t.dxc = (float*)take(4 * R * KC);
-    t.dy2 = (bf16*)take(2 * R * PROP_CH);
-    t.dy1 = (bf16*)take(2 * R * PROP_CH);
-    t.loss = (float*)take(64);
-    if (a) *a = t;
-    return o;
-}
-
 Proposer::Proposer(int device) : device_(device) {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     host_w_.assign(PROP_NWEIGHTS, 0.f);
     cuda_check(cudaMalloc(&d_w_, 4 * (size_t)PROP_NPARAM), "cudaMalloc(proposer)");
     cuda_check(cudaMalloc(&d_wb_, 2 * (size_t)PROP_NPARAM), "cudaMalloc(proposer)");
-    cuda_check(cudaMalloc(&d_g_, 4 * (size_t)PROP_NPARAM), "cudaMalloc(proposer)");
+    cuda_check(cudaMalloc(&d_g_, 4 * (size_t)(PROP_NPARAM + 1)), "cudaMalloc(proposer)");
     cuda_check(cudaMalloc(&d_m_, 4 * (size_t)PROP_NPARAM), "cudaMalloc(proposer)");
     cuda_check(cudaMalloc(&d_v_, 4 * (size_t)PROP_NPARAM), "cudaMalloc(proposer)");
     cuda_check(cudaMalloc(&d_extra_, 4 * (size_t)PROP_NEXTRA), "cudaMalloc(proposer)");
@@ -528,7 +295,7 @@ Proposer::Proposer(int device) : device_(device) {
 Proposer::~Proposer() {
     cudaSetDevice(device_);
     if (graph_exec_) cudaGraphExecDestroy((cudaGraphExec_t)graph_exec_);
-    for (void* p : {(void*)d_w_, (void*)d_wb_, (void*)d_g_, (void*)d_m_, (void*)d_v_, (void*)d_extra_, d_act_, d_tab_,
+    for (void* p : {(void*)d_w_, (void*)d_wb_, (void*)d_g_, (void*)d_m_, (void*)d_v_, (void*)d_extra_, (void*)d_part_, d_io_, d_tab_,
                     d_plan_, (void*)d_feat_, (void*)d_pred_})
         if (p) cudaFree(p);
 }
@@ -561,32 +328,43 @@ void Proposer::get_weights(float* w) const {
     std::memcpy(w + PROP_NPARAM, host_w_.data() + PROP_NPARAM, 4 * (size_t)PROP_NEXTRA);
 }
 
-void Proposer::ensure(int64_t nb) {
-    if (nb <= cap_) return;
-    if (d_act_) cuda_check(cudaFree(d_act_), "cudaFree");
-    d_act_ = nullptr;
-    act_bytes_ = act_layout(nb, nullptr, nullptr);
-    cuda_check(cudaMalloc(&d_act_, act_bytes_), "cudaMalloc(proposer activations)");
-    cap_ = nb;
+void* Proposer::io(size_t bytes) {
+    if (bytes > io_bytes_) {
+        if (d_io_) cuda_check(cudaFree(d_io_), "cudaFree");
+        d_io_ = nullptr;
+        io_bytes_ = 0;
+        cuda_check(cudaMalloc(&d_io_, bytes), "cudaMalloc(proposer batch)");
+        io_bytes_ = bytes;
+    }
+    return d_io_;
 }
 
-// forward over nb reads whose BF16 inputs are in act.x0; outputs (standardised) in act.o
-void Proposer::forward(const float*, int64_t nb, void* stream) {
+// CTAs of the network kernel for n reads: one per SM at most (a CTA holds the
+// weights and a tile in most of an SM's shared memory), persistent over tiles
+int Proposer::net_grid(int64_t n) const {
+    int sms = 0;
+    cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "attr");
+    return (int)std::min<int64_t>(cdiv(n, net::RT), sms);
+}
+
+// Loss (added to the word after the gradient) and gradient of reads idx[0 .. n)
+// of device arrays X, Y into d_g_.
+void Proposer::loss_and_gradient(const float* X, const float* Y, const int32_t* idx, int64_t n, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    Act a;
-    act_layout(cap_, &a, (char*)d_act_);
-    const bf16* W = (const bf16*)d_wb_;
-    const int64_t R = nb * T;
-    k_im2col<<<grid_of(R * KC1), 256, 0, s>>>(a.x0, a.xc1, R, PROP_CIN);
-    gemm<false, true>(s, a.xc1, KC1, W + OW1, KC1, nullptr, a.y1, PROP_CH, R, PROP_CH, KC1, d_w_ + OB1, 1);
-    k_im2col<<<grid_of(R * KC), 256, 0, s>>>(a.y1, a.xc2, R, PROP_CH);
-    gemm<false, true>(s, a.xc2, KC, W + OW2, KC, nullptr, a.y2, PROP_CH, R, PROP_CH, KC, d_w_ + OB2, 1);
-    k_im2col<<<grid_of(R * KC), 256, 0, s>>>(a.y2, a.xc3, R, PROP_CH);
-    gemm<false, true>(s, a.xc3, KC, W + OW3, KC, nullptr, a.y3, PROP_CH, R, PROP_CH, KC, d_w_ + OB3, 1);
-    k_pool<<<grid_of(nb * PROP_CH), 256, 0, s>>>(a.y3, a.h, nb);
-    gemm<false, true>(s, a.h, PROP_CH, W + OW4, PROP_CH, nullptr, a.z, PROP_CH, nb, PROP_CH, PROP_CH, d_w_ + OB4, 1);
-    gemm<false, true>(s, a.z, PROP_CH, W + OW5, PROP_CH, a.o, nullptr, PROP_OUT, nb, PROP_OUT, PROP_CH, d_w_ + OB5, 0);
-    cuda_check(cudaGetLastError(), "proposer forward");
+    const int grid = net_grid(n);
+    if (grid > part_ctas_) {
+        if (d_part_) cuda_check(cudaFree(d_part_), "cudaFree");
+        d_part_ = nullptr;
+        part_ctas_ = 0;
+        cuda_check(cudaMalloc(&d_part_, 4 * (size_t)net::PART * grid), "cudaMalloc(proposer sums)");
+        part_ctas_ = grid;
+    }
+    cuda_check(cudaFuncSetAttribute(net::k_net<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(net::Smem)),
+               "smem attr (k_net)");
+    net::k_net<true><<<grid, net::THREADS, sizeof(net::Smem), s>>>(X, Y, idx, n, (const bf16*)d_wb_, d_w_, d_extra_, nullptr,
+                                                                  d_part_);
+    net::k_net_sum<<<(unsigned)cdiv(PROP_NPARAM + 1, 128), 128, 0, s>>>(d_part_, grid, d_g_, d_g_ + PROP_NPARAM);
+    cuda_check(cudaGetLastError(), "proposer gradient");
 }
 
 float Proposer::train(const float* X, const float* Y, int64_t n, int epochs, int batch, float lr, uint64_t seed,
@@ -614,9 +392,6 @@ float Proposer::train(const float* X, const float* Y, int64_t n, int epochs, int
     cuda_check(cudaMalloc(&dIdx, 4 * (size_t)n), "cudaMalloc(train idx)");
     cuda_check(cudaMemcpy(dX, X, 4 * (size_t)n * T * PROP_CIN, cudaMemcpyHostToDevice), "H2D X");
     cuda_check(cudaMemcpy(dY, Y, 4 * (size_t)n * PROP_OUT, cudaMemcpyHostToDevice), "H2D Y");
-    ensure(batch);
-    Act a;
-    act_layout(cap_, &a, (char*)d_act_);
     std::vector<int32_t> idx(n);
     std::iota(idx.begin(), idx.end(), 0);
     std::mt19937_64 rng(seed);
@@ -625,12 +400,11 @@ float Proposer::train(const float* X, const float* Y, int64_t n, int epochs, int
     for (int ep = 0; ep < epochs; ep++) {
         std::shuffle(idx.begin(), idx.end(), rng);
         cuda_check(cudaMemcpy(dIdx, idx.data(), 4 * (size_t)n, cudaMemcpyHostToDevice), "H2D idx");
-        cuda_check(cudaMemset(a.loss, 0, 4), "memset loss");
+        cuda_check(cudaMemset(d_g_ + PROP_NPARAM, 0, 4), "memset loss");
         int nbatches = 0;
         for (int64_t b0 = 0; b0 < n; b0 += batch) {
-            const int nb = (int)std::min<int64_t>(batch, n - b0);
-            k_gather<<<grid_of((int64_t)nb * T * PROP_CIN), 256, 0, s>>>(dX, dY, dIdx + b0, nb, d_extra_, a.x0, a.yt);
-            loss_and_gradient(nb, s);
+            const int64_t nb = std::min<int64_t>(batch, n - b0);
+            loss_and_gradient(dX, dY, dIdx + b0, nb, s);
             step++;
             const float b1 = 0.9f, b2 = 0.999f;
             k_adam<<<grid_of(PROP_NPARAM), 256, 0, s>>>(d_w_, (bf16*)d_wb_, d_g_, d_m_, d_v_, PROP_NPARAM, lr, b1, b2,
@@ -640,7 +414,7 @@ float Proposer::train(const float* X, const float* Y, int64_t n, int epochs, int
             nbatches++;
         }
         float lsum = 0.f;
-        cuda_check(cudaMemcpy(&lsum, a.loss, 4, cudaMemcpyDeviceToHost), "D2H loss");
+        cuda_check(cudaMemcpy(&lsum, d_g_ + PROP_NPARAM, 4, cudaMemcpyDeviceToHost), "D2H loss");
         last = lsum / (float)std::max(nbatches, 1);
         if (losses) losses[ep] = last;
     }
@@ -650,107 +424,47 @@ float Proposer::train(const float* X, const float* Y, int64_t n, int epochs, int
     return last;
 }
 
-// Loss and parameter gradient of one batch whose BF16 inputs are in act.x0 and
-// standardised targets in act.yt: forward, MSE (summed into act.loss), then
-// the backward GEMMs, col2im / unpooling with the ReLU masks and the bias
-// column sums into d_g_.
-void Proposer::loss_and_gradient(int nb, void* stream) {
-    cudaStream_t s = (cudaStream_t)stream;
-    Act a;
-    act_layout(cap_, &a, (char*)d_act_);
-    const bf16* W = (const bf16*)d_wb_;
-    const int64_t R = (int64_t)nb * T;
-    forward(nullptr, nb, s);
-    k_loss<<<1, 256, 0, s>>>(a.o, a.yt, a.dob, nb, a.loss);
-    // output layer
-    gemm<true, false>(s, a.dob, PROP_OUT, a.z, PROP_CH, d_g_ + OW5, nullptr, PROP_CH, PROP_OUT, PROP_CH, nb,
-                      nullptr, 0);
-    k_colsum<<<PROP_OUT, 256, 0, s>>>(a.dob, nb, PROP_OUT, d_g_ + OB5);
-    gemm<false, false>(s, a.dob, PROP_OUT, W + OW5, PROP_CH, a.dz, nullptr, PROP_CH, nb, PROP_CH, PROP_OUT,
-                       nullptr, 0);
-    k_relu_mask<<<grid_of((int64_t)nb * PROP_CH), 256, 0, s>>>(a.dz, a.z, a.dzb, (int64_t)nb * PROP_CH);
-    // hidden dense layer
-    gemm<true, false>(s, a.dzb, PROP_CH, a.h, PROP_CH, d_g_ + OW4, nullptr, PROP_CH, PROP_CH, PROP_CH, nb,
-                      nullptr, 0);
-    k_colsum<<<PROP_CH, 256, 0, s>>>(a.dzb, nb, PROP_CH, d_g_ + OB4);
-    gemm<false, false>(s, a.dzb, PROP_CH, W + OW4, PROP_CH, a.dh, nullptr, PROP_CH, nb, PROP_CH, PROP_CH,
-                       nullptr, 0);
-    k_unpool_relu<<<grid_of(R * PROP_CH), 256, 0, s>>>(a.dh, a.y3, a.dy3, nb);
-    // conv 3
-    gemm<true, false>(s, a.dy3, PROP_CH, a.xc3, KC, d_g_ + OW3, nullptr, KC, PROP_CH, KC, R, nullptr, 0);
-    k_colsum<<<PROP_CH, 256, 0, s>>>(a.dy3, R, PROP_CH, d_g_ + OB3);
-    gemm<false, false>(s, a.dy3, PROP_CH, W + OW3, KC, a.dxc, nullptr, KC, R, KC, PROP_CH, nullptr, 0);
-    k_col2im_relu<<<grid_of(R * PROP_CH), 256, 0, s>>>(a.dxc, a.y2, a.dy2, R, PROP_CH);
-    // conv 2
-    gemm<true, false>(s, a.dy2, PROP_CH, a.xc2, KC, d_g_ + OW2, nullptr, KC, PROP_CH, KC, R, nullptr, 0);
-    k_colsum<<<PROP_CH, 256, 0, s>>>(a.dy2, R, PROP_CH, d_g_ + OB2);
-    gemm<false, false>(s, a.dy2, PROP_CH, W + OW2, KC, a.dxc, nullptr, KC, R, KC, PROP_CH, nullptr, 0);
-    k_col2im_relu<<<grid_of(R * PROP_CH), 256, 0, s>>>(a.dxc, a.y1, a.dy1, R, PROP_CH);
-    // conv 1 (no input gradient)
-    gemm<true, false>(s, a.dy1, PROP_CH, a.xc1, KC1, d_g_ + OW1, nullptr, KC1, PROP_CH, KC1, R, nullptr, 0);
-    k_colsum<<<PROP_CH, 256, 0, s>>>(a.dy1, R, PROP_CH, d_g_ + OB1);
-    cuda_check(cudaGetLastError(), "proposer backward");
-}
-
 float Proposer::gradient(const float* X, const float* Y, int64_t n, float* grad) {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     if (n <= 0 || n > 4096) throw std::invalid_argument("proposer: gradient batch must hold 1..4096 reads");
-    float *dX = nullptr, *dY = nullptr;
-    int32_t* dIdx = nullptr;
-    cuda_check(cudaMalloc(&dX, 4 * (size_t)n * T * PROP_CIN), "cudaMalloc(grad X)");
-    cuda_check(cudaMalloc(&dY, 4 * (size_t)n * PROP_OUT), "cudaMalloc(grad Y)");
-    cuda_check(cudaMalloc(&dIdx, 4 * (size_t)n), "cudaMalloc(grad idx)");
-    std::vector<int32_t> idx(n);
-    std::iota(idx.begin(), idx.end(), 0);
+    const size_t xb = up256(4 * (size_t)n * T * PROP_CIN);
+    float* dX = (float*)io(xb + 4 * (size_t)n * PROP_OUT);
+    float* dY = (float*)((char*)dX + xb);
     cuda_check(cudaMemcpy(dX, X, 4 * (size_t)n * T * PROP_CIN, cudaMemcpyHostToDevice), "H2D X");
     cuda_check(cudaMemcpy(dY, Y, 4 * (size_t)n * PROP_OUT, cudaMemcpyHostToDevice), "H2D Y");
-    cuda_check(cudaMemcpy(dIdx, idx.data(), 4 * (size_t)n, cudaMemcpyHostToDevice), "H2D idx");
-    ensure(n);
-    Act a;
-    act_layout(cap_, &a, (char*)d_act_);
-    cuda_check(cudaMemset(a.loss, 0, 4), "memset loss");
-    k_gather<<<grid_of(n * T * PROP_CIN), 256>>>(dX, dY, dIdx, (int)n, d_extra_, a.x0, a.yt);
-    loss_and_gradient((int)n, nullptr);
-    float loss = 0.f;
-    cuda_check(cudaMemcpy(grad, d_g_, 4 * (size_t)PROP_NPARAM, cudaMemcpyDeviceToHost), "D2H grad");
-    cuda_check(cudaMemcpy(&loss, a.loss, 4, cudaMemcpyDeviceToHost), "D2H loss");
-    cudaFree(dX);
-    cudaFree(dY);
-    cudaFree(dIdx);
-    return loss;
+    cuda_check(cudaMemsetAsync(d_g_ + PROP_NPARAM, 0, 4, nullptr), "memset loss");
+    loss_and_gradient(dX, dY, nullptr, n, nullptr);
+    std::vector<float> h(PROP_NPARAM + 1);
+    cuda_check(cudaMemcpy(h.data(), d_g_, 4 * (size_t)(PROP_NPARAM + 1), cudaMemcpyDeviceToHost), "D2H grad");
+    std::memcpy(grad, h.data(), 4 * (size_t)PROP_NPARAM);
+    return h[PROP_NPARAM];
 }
-
-constexpr int64_t PREDICT_CHUNK = 4096;
 
 void Proposer::predict_device(const float* dX, int64_t n, float* dY, void* stream) {
-    ensure(std::min<int64_t>(std::max<int64_t>(n, 1), PREDICT_CHUNK));
-    predict_launch(dX, n, dY, stream);
-}
-
-// the inference launches only (buffers already sized by ensure)
-void Proposer::predict_launch(const float* dX, int64_t n, float* dY, void* stream) {
-    cudaStream_t s = (cudaStream_t)stream;
-    Act a;
-    act_layout(cap_, &a, (char*)d_act_);
-    for (int64_t b0 = 0; b0 < n; b0 += cap_) {
-        const int64_t nb = std::min<int64_t>(cap_, n - b0);
-        k_to_bf16<<<grid_of(nb * T * PROP_CIN), 256, 0, s>>>(dX + b0 * T * PROP_CIN, a.x0, nb * T * PROP_CIN);
-        forward(nullptr, nb, s);
-        k_destd<<<grid_of(nb * PROP_OUT), 256, 0, s>>>(a.o, d_extra_, dY + b0 * PROP_OUT, nb);
-    }
+    if (n <= 0) return;
+    cuda_check(cudaFuncSetAttribute(net::k_net<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(net::Smem)),
+               "smem attr (k_net)");
+    net::k_net<false><<<net_grid(n), net::THREADS, sizeof(net::Smem), (cudaStream_t)stream>>>(
+        dX, nullptr, nullptr, n, (const bf16*)d_wb_, d_w_, d_extra_, dY, nullptr);
     cuda_check(cudaGetLastError(), "proposer predict");
 }
 
+// Host arrays go through the object's device buffer a chunk at a time (16 K
+// reads, 16 MiB), so it stays small whatever the call.
+constexpr int64_t PREDICT_CHUNK = 16384;
+
 void Proposer::predict_host(const float* X, int64_t n, float* Y) {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
-    float *dX = nullptr, *dY = nullptr;
-    cuda_check(cudaMalloc(&dX, 4 * (size_t)std::max<int64_t>(n, 1) * T * PROP_CIN), "cudaMalloc(predict X)");
-    cuda_check(cudaMalloc(&dY, 4 * (size_t)std::max<int64_t>(n, 1) * PROP_OUT), "cudaMalloc(predict Y)");
-    cuda_check(cudaMemcpy(dX, X, 4 * (size_t)n * T * PROP_CIN, cudaMemcpyHostToDevice), "H2D X");
-    predict_device(dX, n, dY, nullptr);
-    cuda_check(cudaMemcpy(Y, dY, 4 * (size_t)n * PROP_OUT, cudaMemcpyDeviceToHost), "D2H Y");
-    cudaFree(dX);
-    cudaFree(dY);
+    const int64_t cap = std::min<int64_t>(std::max<int64_t>(n, 1), PREDICT_CHUNK);
+    const size_t xb = up256(4 * (size_t)cap * T * PROP_CIN);
+    float* dX = (float*)io(xb + 4 * (size_t)cap * PROP_OUT);
+    float* dY = (float*)((char*)dX + xb);
+    for (int64_t b0 = 0; b0 < n; b0 += cap) {
+        const int64_t nb = std::min<int64_t>(cap, n - b0);
+        cuda_check(cudaMemcpy(dX, X + b0 * T * PROP_CIN, 4 * (size_t)nb * T * PROP_CIN, cudaMemcpyHostToDevice), "H2D X");
+        predict_device(dX, nb, dY, nullptr);
+        cuda_check(cudaMemcpy(Y + b0 * PROP_OUT, dY, 4 * (size_t)nb * PROP_OUT, cudaMemcpyDeviceToHost), "D2H Y");
+    }
 }
 
 void Proposer::features(const DeviceWindows& dw, int k, int w, float* dX, void* stream) {
@@ -829,17 +543,16 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
     if (nw == 0) return;
     int bits = 0, grid = 0;
     features_prep(dw, k, w, bits, grid);
-    ensure(std::min<int64_t>(std::max<int64_t>(dw.n_reads, 1), PREDICT_CHUNK));
     char* p = (char*)d_plan_;
     int32_t* dn = (int32_t*)p;
     int64_t* dt = (int64_t*)(p + up256(4 * (size_t)nw));
     int64_t* ds = (int64_t*)(p + up256(4 * (size_t)nw) + up256(8 * (size_t)nw));
     float* dc = (float*)(p + up256(4 * (size_t)nw) + 2 * up256(8 * (size_t)nw));
     int64_t* dl = (int64_t*)(p + up256(4 * (size_t)nw) + 3 * up256(8 * (size_t)nw));
-    // features, inference and plan: ~10 launches per 4,096 reads, recorded once as a
-    // CUDA graph per batch shape and replayed with one launch
+    // features, inference and plan: recorded once as a CUDA graph per batch shape and
+    // replayed with one launch
     const GraphKey key{dw.seq, dw.read_off, dw.read_len, dw.win_off, dw.n_reads, nw, k, w, bits, grid,
-                       d_feat_, d_pred_, d_plan_, d_tab_, d_act_, cap_, s};
+                       d_feat_, d_pred_, d_plan_, d_tab_, s};
     if (!graph_exec_ || std::memcmp(&key, &graph_key_, sizeof key) != 0) {
         if (graph_exec_) cudaGraphExecDestroy((cudaGraphExec_t)graph_exec_);
         graph_exec_ = nullptr;
@@ -847,7 +560,7 @@ void Proposer::plan(const DeviceWindows& dw, int k, int w, std::vector<int32_t>&
         cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
         try {
             features_launch(dw, k, w, bits, grid, d_feat_, s);
-            predict_launch(d_feat_, dw.n_reads, d_pred_, s);
+            predict_device(d_feat_, dw.n_reads, d_pred_, s);
             k_plan<<<grid_of(nw), 256, 0, s>>>(d_pred_, dw.read_len, dw.win_off, nw, d_extra_, dn, dt, ds, dc, dl);
             cuda_check(cudaGetLastError(), "k_plan");
         } catch (...) {

@@ -91,32 +91,30 @@ class Proposer {
         const void *seq, *read_off, *read_len, *win_off;
         int64_t n_reads;
         int32_t n_windows, k, w, bits, grid;
-        const void *feat, *pred, *plan, *tab, *act;
-        int64_t cap;
+        const void *feat, *pred, *plan, *tab;
         const void* stream;
     };
     void features_prep(const DeviceWindows& dw, int k, int w, int& bits, int& grid);
     void features_launch(const DeviceWindows& dw, int k, int w, int bits, int grid, float* dX, void* stream);
-    void predict_launch(const float* dX, int64_t n, float* dY, void* stream);
     void* graph_exec_ = nullptr;
     GraphKey graph_key_{};
-    void ensure(int64_t batch_reads);
-    void forward(const float* dX, int64_t n, void* stream);
-    void loss_and_gradient(int nb, void* stream);
+    void* io(size_t bytes);
+    int net_grid(int64_t n) const;
+    void loss_and_gradient(const float* X, const float* Y, const int32_t* idx, int64_t n, void* stream);
     void upload_bf16(void* stream);
     int device_;
     std::vector<float> host_w_;
     // device parameters
     float* d_w_ = nullptr;        // FP32 master
     uint16_t* d_wb_ = nullptr;    // BF16 copy (GEMM operands)
-    float* d_g_ = nullptr;        // gradients
+    float* d_g_ = nullptr;        // gradients, then the loss
     float* d_m_ = nullptr;        // Adam first moment
     float* d_v_ = nullptr;        // Adam second moment
     float* d_extra_ = nullptr;    // the PROP_NEXTRA floats
-    // activations for up to cap_ reads
-    int64_t cap_ = 0;
-    void* d_act_ = nullptr;
-    size_t act_bytes_ = 0;
+    float* d_part_ = nullptr;     // per-CTA gradient sums
+    int part_ctas_ = 0;
+    void* d_io_ = nullptr;        // a host call's batch (predict: a chunk of 16 K reads at most)
+    size_t io_bytes_ = 0;
     // feature scratch: per-CTA hash tables
     void* d_tab_ = nullptr;
     size_t tab_bytes_ = 0;
