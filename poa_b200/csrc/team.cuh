@@ -34,15 +34,18 @@
 // Adaptive band: row i + 1's band depends on row i's first maximum. The first
 // maximum of M is the first maximum of H0 = max(diagonal, vertical) (a gap
 // never exceeds the cell it opens from), so it is published with the same
-// barrier; an extra warp, which owns no columns, then updates the band state
-// and prepares the next row's header while the others finalise the row.
+// barrier; two more warps, which own no columns, update the band state and
+// prepare the next row's header while the others finalise the row.
+//
+// The row before is nearly always a predecessor; its cells stay in registers,
+// so a row with no other predecessor reads no cells at all.
 //
 // Measured on a B200, DP kernels of one run, record fill -> this one: 10 reads
-// of 16,569 bp, static band, 346 -> 151 ms (fill 1,550 cycles per row of ~1,050
-// cells, backtrack 325 cycles per move); 24 reads of 443 bp 31 -> 12 ms; 10
-// reads of 5 kb at 10 % error, adaptive band, 308 -> 118 ms (2,900 cycles per
-// row). What is left is latency: ~230 dependent instructions per warp and row,
-// two cycles of each waiting on the instruction before it.
+// of 16,569 bp, static band, 346 -> 132 ms (fill ~1,350 cycles per row of ~1,050
+// cells, backtrack 325 cycles per move); 24 reads of 443 bp 31 -> 11.6 ms; 10
+// reads of 5 kb at 10 % error, adaptive band, 308 -> 107 ms; 840 seeded
+// sub-windows 94 -> 33 ms. What is left is latency: ~215 mostly dependent
+// instructions per warp and row.
 #pragma once
 #include "plain.cuh"
 
@@ -190,7 +193,7 @@ struct TeamJob {
     // | its base as the DP sees it; y, z, w = its band and row-store block,
     // filled in here
     int4* ed;
-    int4* fe;                // [edges] the same for the fill: {ring offset or -1, base in every byte, Bs, last block - Bs}
+    int4* fe;                // [edges] the same for the fill, the row before left out: {ring offset, or ~row-store block; base in every byte; Bs; last block - Bs}
     const int32_t *hq, *tq;  // [n] static band
     const int4* ra;          // [2 n] adaptive band: {first in-edge, first out-edge, hq, tq}, {hq_loc, base, d, successors}
     const int32_t* out_row;  // adaptive band: successor rows in out-list order
@@ -214,17 +217,18 @@ constexpr int HDR_E = 32;       // predecessor records in an adaptive row's head
 constexpr int SWIN = 256;       // rows of the adaptive state window (a power of two), half of them ahead
 constexpr int SW_INTS = 12;     // {Pl, Pr, Ol, Or, Ow, Sl, Mp, -, Bs, Be, tb, -}
 enum { SW_PL = 0, SW_PR, SW_OL, SW_OR, SW_OW, SW_SL, SW_MP, SW_BS = 8, SW_BE, SW_TB };
-// flags in a row header's last word: d in the low 10 bits
-enum { FR_D = 1023, FR_GENERAL = 1 << 10, FR_UNSTAGED = 1 << 11, FR_EOFF = 16 };
+// flags in a row header's last word: listed predecessors in the low 10 bits;
+// FR_PREV: the row before is a predecessor too, its base above FR_PBASE
+enum { FR_D = 1023, FR_GENERAL = 1 << 10, FR_UNSTAGED = 1 << 11, FR_PREV = 1 << 12, FR_PBASE = 13, FR_EOFF = 16 };
 
 struct TeamStage {
     int4 row[STG];
     int4 ed[STG_E];
 };
 struct TeamHdr {
-    int4 h;        // as TeamJob::fr
-    int4 g;        // {first in-edge, status, -, -}
-    int4 ed[HDR_E];
+    int4 h;        // {Bs, last block - Bs, row-store block, FR_GENERAL | status << FR_EOFF}
+    int4 g;        // {first in-edge, predecessors, flags and count of the fill's list, -}
+    int4 ed[HDR_E];  // the fill's list, as TeamJob::fe
 };
 
 // Backtrack tile (team_backtrack): up to BT_ROWS rows around the walk, as many
@@ -252,9 +256,11 @@ struct BtTile {
 
 template <int W, bool ADAPT, bool WIDE>
 struct TeamSmem {
-    static constexpr int TR = W <= 6 && !WIDE ? 32 : 16;           // rows of the ring (a power of two)
     static constexpr int CELLB = TC * Cells<WIDE>::BYTES;          // bytes per thread and row
     static constexpr int ROWB = 32 * W * CELLB;
+    // rows of the ring (a power of two): noisy graphs have predecessors tens of rows back, and
+    // one read from the row store costs as much as a row
+    static constexpr int TR = ROWB * 64 <= 196608 ? 64 : ROWB * 32 <= 196608 ? 32 : 16;
     static constexpr int RING = TR * ROWB;
     static constexpr int PUB = RING;                               // int4 [2][W]
     static constexpr int BEST = PUB + 2 * W * 16;                  // int4 [2][W]
@@ -262,22 +268,27 @@ struct TeamSmem {
     static constexpr int FILL =
         REST + (ADAPT ? 2 * (int)sizeof(TeamHdr) + SWIN * SW_INTS * 4 : 2 * (int)sizeof(TeamStage));
     static constexpr int BYTES = FILL > BtTile<WIDE, 8>::full() ? FILL : BtTile<WIDE, 8>::full();
-    static constexpr int THREADS = 32 * (W + (ADAPT ? 1 : 0));
+    static constexpr int THREADS = 32 * (W + (ADAPT ? 2 : 0));
 };
 
 // Named barriers: 1 the whole team, 2 the compute warps' maxima (they arrive,
-// the control warp waits), 3 the compute warps.
+// the state warp waits), 3 the compute warps.
 template <int ID, int NT>
 __device__ __forceinline__ void bar_sync() { asm volatile("barrier.sync %0, %1;" ::"n"(ID), "n"(NT) : "memory"); }
 template <int ID, int NT>
 __device__ __forceinline__ void bar_arrive() { asm volatile("barrier.arrive %0, %1;" ::"n"(ID), "n"(NT) : "memory"); }
 
-// inclusive prefix maximum over the warp (a lane without a source gets its own
-// value back, which a maximum does not mind)
+// Inclusive prefix maximum over the warp in three rounds of independent
+// shuffles (a lane without a source gets its own value back, which a maximum
+// does not mind).
 __device__ __forceinline__ int32_t scan_max(int32_t v) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) v = mx(v, __shfl_up_sync(0xffffffffu, v, o));
-    return v;
+    const int32_t a = __shfl_up_sync(0xffffffffu, v, 1), b = __shfl_up_sync(0xffffffffu, v, 2),
+                  c = __shfl_up_sync(0xffffffffu, v, 3);
+    v = mx(mx(v, a), mx(b, c));
+    const int32_t d = __shfl_up_sync(0xffffffffu, v, 4), e = __shfl_up_sync(0xffffffffu, v, 8),
+                  f = __shfl_up_sync(0xffffffffu, v, 12);
+    v = mx(mx(v, d), mx(e, f));
+    return mx(v, __shfl_up_sync(0xffffffffu, v, 16));
 }
 
 __device__ __forceinline__ int strips_of(int Bs, int Be) { return ((Be - 2) >> 4) - (Bs >> 4) + 1; }
@@ -341,16 +352,19 @@ __device__ int team_rows_static(const TeamJob& a, int64_t* s_part, unsigned long
         if (i == 0 || ri.y - ri.x - 1 <= 0 || strips_of(ri.x, ri.y) > W) fl |= FR_GENERAL;
         if (eoff + d > STG_E) fl |= FR_UNSTAGED;
         else fl |= eoff << FR_EOFF;
-        a.fr[i] = make_int4(ri.x, ri.y - 2 - ri.x, ri.z, fl);
+        int x = e0;
         for (int e = e0; e < e0 + d; e++) {
             int4 v = a.ed[e];
             const int p = v.x >> 4;
             const int4 pr = a.rowi[p];
             v.y = pr.x; v.z = pr.y; v.w = pr.z;
             a.ed[e] = v;
-            const bool near = i - p < S::TR && strips_of(pr.x, pr.y) <= W;
-            a.fe[e] = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : -1, (v.x & 7) * 0x01010101, pr.x, pr.y - 2 - pr.x);
+            const bool lap1 = pr.y - pr.x - 1 > 0 && strips_of(pr.x, pr.y) <= W;
+            if (lap1 && p == i - 1 && !(fl & FR_GENERAL)) fl += FR_PREV - 1 + ((v.x & 7) << FR_PBASE);
+            else a.fe[x++] = make_int4(lap1 && i - p < S::TR ? (p & (S::TR - 1)) * S::ROWB : ~pr.z, (v.x & 7) * 0x01010101, pr.x,
+                                      pr.y - 2 - pr.x);
         }
+        a.fr[i] = make_int4(ri.x, ri.y - 2 - ri.x, ri.z, fl);
     }
     __syncthreads();
     return ST_OK;
@@ -385,7 +399,10 @@ struct TeamRow {
     int col0 = 0, B = 0, Bz = 0;    // its first column, block (and that block, or a large value for block 0: no diagonal mask there)
     uint32_t qw = 0;                // query codes of the thread's columns
     int qn = 4;                     // code of the column after them (adaptive band)
-    int32_t edge = NEG;             // static band: M left of this warp's strip in the previous row
+    // the row before, when it fits the team's columns: band, this thread's M and vertical
+    // terms (NEG outside the band), M left of the thread's columns
+    int pBs = 0, pspan = -1;
+    int32_t pm[4] = {C::NEG, C::NEG, C::NEG, C::NEG}, pe[4] = {C::NEG, C::NEG, C::NEG, C::NEG}, pleft = C::NEG;
     unsigned xp = 0;                // byte offset of the published summaries' half in use
 
     __device__ TeamRow(char* sm, const TeamJob& job)
@@ -401,19 +418,26 @@ struct TeamRow {
         const bool in = col0 + 8 <= (int)qs_bytes(a.qlen);
         qw = in ? *reinterpret_cast<const uint32_t*>(a.qs + col0) : 0x04040404u;
         if (ADAPT) qn = in ? a.qs[col0 + 4] : 4;
+        // the row before had other columns here, if any
+#pragma unroll
+        for (int l = 0; l < 4; l++) pm[l] = pe[l] = NEG;
     }
 
-    // One predecessor's terms. in: the block is in its band; src: cells; left: M of the cell before them.
-    __device__ __forceinline__ void fold(const C& pc, int32_t left, bool diag, uint32_t x, int32_t* P, int32_t* V) const {
+    // diagonal terms of one predecessor: m its M, left the M before them
+    __device__ __forceinline__ void diagonal(const int32_t* m, int32_t left, bool diag, uint32_t x, int32_t* P) const {
         // packed cells: a term pushed far below NEG drops out of the maximum
         const int32_t sm = diag || WIDE ? k.match : -(1 << 23), sx = diag || WIDE ? k.mismatch : -(1 << 23);
 #pragma unroll
         for (int l = 0; l < 4; l++) {
-            const int32_t src = l == 0 ? left : pc.m(l > 0 ? l - 1 : 0);
-            const int32_t cand = src + ((x & (255u << (8 * l))) == 0 ? sm : sx);
+            const int32_t cand = (l == 0 ? left : m[l > 0 ? l - 1 : 0]) + ((x & (255u << (8 * l))) == 0 ? sm : sx);
             if (!WIDE || diag) P[l] = mx(P[l], cand);
-            V[l] = mx(V[l], pc.v(l, k));
         }
+    }
+    __device__ __forceinline__ void fold(const C& pc, int32_t left, bool diag, uint32_t x, int32_t* P, int32_t* V) const {
+        const int32_t m[4] = {pc.m(0), pc.m(1), pc.m(2), pc.m(3)};
+        diagonal(m, left, diag, x, P);
+#pragma unroll
+        for (int l = 0; l < 4; l++) V[l] = mx(V[l], pc.v(l, k));
     }
 
     // prefix maximum within the warp and its summary; base: -(column in the row's band) * e1
@@ -447,31 +471,45 @@ struct TeamRow {
     __device__ __forceinline__ void put_maximum(const int4& best) const {
         if (lane == 0) sts128(sb + S::BEST + xp + wid * 16, best);
         __syncwarp();
-        bar_arrive<2, S::THREADS>();
+        bar_arrive<2, 32 * (W + 1)>();
     }
-    __device__ __forceinline__ void finish(C& o, int i, const int32_t* H, const int32_t* V, const int32_t* key, int32_t run) const {
-        if (i == 0) {
-#pragma unroll
-            for (int l = 0; l < 4; l++) o.set(l, H[l], V[l], k);
-            return;
-        }
+    // M of the thread's cells (into H) from the prefix maximum `run` left of them
+    __device__ __forceinline__ void gaps(int32_t* H, const int32_t* key, int32_t run) const {
         const int32_t g = k.o1 - k.e1;
-        o.set(0, mx(H[0], run + g), V[0], k);
+        H[0] = mx(H[0], run + g);
         run = mx(run, key[0]);
-        o.set(1, mx(H[1], run + (g + k.e1)), V[1], k);
+        H[1] = mx(H[1], run + (g + k.e1));
         run = mx(run, key[1]);
-        o.set(2, mx(H[2], run + (g + 2 * k.e1)), V[2], k);
+        H[2] = mx(H[2], run + (g + 2 * k.e1));
         run = mx(run, key[2]);
-        o.set(3, mx(H[3], run + (g + 3 * k.e1)), V[3], k);
+        H[3] = mx(H[3], run + (g + 3 * k.e1));
+    }
+    // stores the thread's cells and keeps the row as the row before of the next;
+    // edge: M of the cell left of the strip
+    __device__ __forceinline__ void keep(int i, const int4& h, bool act, const int32_t* M, const int32_t* V, int rel, int32_t edge) {
+        if (act) {
+            C o;
+#pragma unroll
+            for (int l = 0; l < 4; l++) o.set(l, M[l], V[l], k);
+            o.sts(sb + (i & (S::TR - 1)) * S::ROWB + own);
+            o.store(store + ((int64_t)h.z * BLK + rel) * C::BYTES);
+        }
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            pm[l] = M[l];
+            pe[l] = act ? mx(add32(M[l], k.o1), add32(V[l], k.e1)) : NEG;
+        }
+        pleft = __shfl_up_sync(0xffffffffu, M[3], 1);
+        if (lane == 0) pleft = edge;
     }
     __device__ __forceinline__ void sync_row() const {
         if (ADAPT) bar_sync<3, 32 * W>();
         else bar_sync<1, S::THREADS>();
     }
 
-    // A row that fits the team's columns (i > 0). ed_at(e): fill record; far(e): its TeamJob::ed record.
-    template <class EdAt, class Far, class After>
-    __device__ __forceinline__ void row(int i, int4 h, EdAt ed_at, Far far, After after_barrier) {
+    // A row that fits the team's columns (i > 0). ed_at(e): the e-th listed record.
+    template <class EdAt, class After>
+    __device__ __forceinline__ void row(int i, int4 h, EdAt ed_at, After after_barrier) {
         const int Bs = h.x, span = h.y, d = h.w & FR_D;
         const int S0 = Bs >> 4, S1 = (Bs + span) >> 4;
         if ((unsigned)(s_cur - S0) >= (unsigned)W) {
@@ -483,29 +521,34 @@ struct TeamRow {
         const bool act = on && (unsigned)(B - Bs) <= (unsigned)span;
         const bool first = B == Bs && !(lane & 1);  // column 0 of the row's first block reads NEG_INF
         int32_t P[4], V[4], H[4], key[4], ex = LOW, base = 0;
-        __syncwarp();
         if (on) {
 #pragma unroll
             for (int l = 0; l < 4; l++) P[l] = V[l] = NEG;
+            if (h.w & FR_PREV) {
+                // diag: the fill's block mask for the diagonal (src/align.cpp:1467)
+                const bool diag = (unsigned)(B - pBs) <= (unsigned)pspan && Bz > pBs;
+                diagonal(pm, first ? NEG : pleft, diag, qw ^ (((uint32_t)h.w >> FR_PBASE & 7u) * 0x01010101u), P);
+#pragma unroll
+                for (int l = 0; l < 4; l++) V[l] = mx(NEG, pe[l]);
+            }
+            if (d > 0) __syncwarp();  // the ring's words of the lanes to the left
             for (int e = 0; e < d; e++) {
                 const int4 er = ed_at(e);
                 const bool in = (unsigned)(B - er.z) <= (unsigned)er.w;
-                const bool diag = in && Bz > er.z;  // the fill's block mask for the diagonal (src/align.cpp:1467)
+                const bool diag = in && Bz > er.z;
                 C pc;
                 int32_t left;
                 if (er.x >= 0) {
                     pc.lds(sb + er.x + own);
                     left = C::lds_m(sb + er.x + leftw);
-                    if (!ADAPT && lane == 0 && er.x == (int)(((i - 1) & (S::TR - 1)) * S::ROWB)) left = edge;
                     if (!in) pc.none();
                 } else {
-                    const int4 fe = far(e);
-                    const char* src = store + ((int64_t)fe.w * BLK + (col0 - fe.y * BLK)) * C::BYTES;
+                    const char* src = store + ((int64_t)~er.x * BLK + (col0 - er.z * BLK)) * C::BYTES;
                     pc.none();
                     left = NEG;
                     if (in && act) {
                         pc.load(src);
-                        if (B > fe.y || (lane & 1)) left = C::load_m(src - C::BYTES);
+                        if (B > er.z || (lane & 1)) left = C::load_m(src - C::BYTES);
                     }
                 }
                 if (first) left = NEG;
@@ -526,23 +569,20 @@ struct TeamRow {
         }
         sync_row();
         after_barrier();
+        pBs = Bs;
+        pspan = span;
         if (on) {
             const int4 pv = lane < W ? lds128(sb + S::PUB + xp + lane * 16) : make_int4(LOW, LOW, NEG, INT_MAX);
             const int4 L = lds128(sb + S::PUB + xp + (wid == 0 ? W - 1 : wid - 1) * 16);
             const int32_t Pl = mx(K, __reduce_max_sync(0xffffffffu, pv.w < s_cur - 1 ? pv.x : LOW));
-            const bool hasl = s_cur > S0;
-            const int32_t Pr = hasl ? mx(Pl, L.x) : Pl;
-            if (!ADAPT && lane == 0) {
-                // M of the cell left of the strip, for the next row
-                const int32_t I = add32(k.o1 + (rel - 2) * k.e1, mx(Pl, L.y));
-                edge = mx(L.z, I);
-            }
-            if (act) {
-                C o;
-                finish(o, i, H, V, key, mx(Pr, ex) - base);
-                o.sts(sb + (i & (S::TR - 1)) * S::ROWB + own);
-                o.store(store + ((int64_t)h.z * BLK + rel) * C::BYTES);
-            }
+            const int32_t Pr = s_cur > S0 ? mx(Pl, L.x) : Pl;
+            // M of the cell left of the strip (lane 0's), from its warp's summary
+            const int32_t edge = mx(L.z, add32(k.o1 + (rel - 2) * k.e1, mx(Pl, L.y)));
+            gaps(H, key, mx(Pr, ex) - base);
+            keep(i, h, act, H, V, rel, edge);
+        } else {
+#pragma unroll
+            for (int l = 0; l < 4; l++) pe[l] = NEG;
         }
         xp ^= W * 16;
     }
@@ -596,23 +636,27 @@ struct TeamRow {
             sync_row();
             const int4 pv = lane < W ? lds128(sb + S::PUB + xp + lane * 16) : make_int4(LOW, LOW, NEG, INT_MAX);
             const int32_t P0 = mx(carry, __reduce_max_sync(0xffffffffu, pv.w < s ? pv.x : LOW));
+            const int32_t Pl = mx(K, __reduce_max_sync(0xffffffffu, pv.w < s - 1 ? pv.x : LOW));
             carry = mx(carry, __reduce_max_sync(0xffffffffu, pv.x));
             if (on) {
-                if (!ADAPT && S1 - S0 < W) {
-                    // M of the cell left of the strip, for the next row
-                    const int32_t Pl = mx(K, __reduce_max_sync(0xffffffffu, pv.w < s - 1 ? pv.x : LOW));
+                if (i > 0) gaps(H, key, mx(P0, ex) - base);
+                if (S1 - S0 < W) {
                     const int4 L = lds128(sb + S::PUB + xp + (wid == 0 ? W - 1 : wid - 1) * 16);
-                    edge = i == 0 ? L.z : mx(L.z, add32(k.o1 + (rel - lane * TC - 2) * k.e1, mx(Pl, L.y)));
-                }
-                if (act) {
+                    keep(i, h, act, H, V, rel, i == 0 ? L.z : mx(L.z, add32(k.o1 + (rel - 2) * k.e1, mx(Pl, L.y))));
+                } else if (act) {
                     C o;
-                    finish(o, i, H, V, key, mx(P0, ex) - base);
-                    if (S1 - S0 < W) o.sts(sb + (i & (S::TR - 1)) * S::ROWB + own);
+#pragma unroll
+                    for (int l = 0; l < 4; l++) o.set(l, H[l], V[l], k);
                     o.store(store + ((int64_t)h.z * BLK + rel) * C::BYTES);
                 }
+            } else {
+#pragma unroll
+                for (int l = 0; l < 4; l++) pe[l] = NEG;
             }
             xp ^= W * 16;
         }
+        pBs = Bs;
+        pspan = h.y;
         if (!ADAPT) sync_row();
     }
 };
@@ -640,61 +684,62 @@ __device__ void team_fill_static(const TeamJob& a, char* smem) {
         } else {
             const int4 hc = h;
             const unsigned ed = cur + STG * 16 + (hc.w >> FR_EOFF) * 16;
-            const int4* far = a.ed;
-            t.row(i, hc,
-                  [&](int e) { return hc.w & FR_UNSTAGED ? a.fe[a.in_ptr[i] + e] : lds128(ed + e * 16); },
-                  [&](int e) { return far[a.in_ptr[i] + e]; }, [&]() { h = lds128(nxt); });
+            t.row(i, hc, [&](int e) { return hc.w & FR_UNSTAGED ? a.fe[a.in_ptr[i] + e] : lds128(ed + e * 16); },
+                  [&]() { h = lds128(nxt); });
         }
     }
     __syncthreads();
 }
 
-// The adaptive band's serial part (src/align.cpp:1433-1444, 1516-1568) on the
-// control warp. Its state lives in a shared-memory window of SWIN rows around
-// the current one (successors up to SWIN / 2 - 2 rows ahead, predecessors up to
-// SWIN / 2 behind), in global memory beyond it. Everything that does not need
-// row i's maximum is fetched while the other warps fill the row.
+// The adaptive band's serial part (src/align.cpp:1433-1444, 1516-1568) on two
+// warps of its own. The state warp turns a row's maximum into the next row's
+// band; the records warp prepares the next row's predecessor records. Rows' state
+// and places live in a shared-memory window of SWIN rows around the current one
+// (successors up to SWIN / 2 - 2 rows ahead, predecessors up to SWIN / 2
+// behind), in global memory beyond it. Between the row's maxima and the next
+// header there is only what depends on them; everything else runs while the
+// other warps fill the row. (As one warp the two took 2,400 cycles a row.)
+constexpr int AHEAD = SWIN / 2 - 1;
+
 template <int W, bool WIDE>
-__device__ void team_control(const TeamJob& a, char* smem, int64_t& cells_out) {
+__device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
     typedef TeamSmem<W, true, WIDE> S;
     TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
     int32_t* win = reinterpret_cast<int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
-    const int4* bests = reinterpret_cast<const int4*>(smem + S::BEST);
+    const unsigned bests = (unsigned)__cvta_generic_to_shared(smem + S::BEST);
     const int lane = threadIdx.x & 31;
-    const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n];
-    constexpr int AHEAD = SWIN / 2 - 1;
+    const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n], bw = a.w;
+    const int4* ra = a.ra;
+    const int4* ed = a.ed;
+    const int32_t* out_row = a.out_row;
+    int32_t* state = a.state;
+    const int64_t store_cap = a.store_cap;
     auto slot = [&](int r) { return win + (r & (SWIN - 1)) * SW_INTS; };
-    int4 ra0 = a.ra[0], ra1 = a.ra[1];  // row i
+    int4 ra0 = ra[0], ra1 = ra[1];                // row i
     int4 rb0 = make_int4(0, 0, 0, 0), rb1 = rb0;  // row i + 1
-    if (n > 1) { rb0 = a.ra[2]; rb1 = a.ra[3]; }
+    if (n > 1) { rb0 = ra[2]; rb1 = ra[3]; }
     int Bs, Be;
-    band_adaptive(ra0.z, ra0.w, m, a.w, m, 0, 0, 0, 0, Bs, Be);
+    band_adaptive(ra0.z, ra0.w, m, bw, m, 0, 0, 0, 0, Bs, Be);
     Bs = 0;
     int64_t tb = 0, cells = 0;
-    auto put_header = [&](int i, int d, int e0) {
+    // the header's band, place, and (last word) GENERAL or a failed status
+    auto put_header = [&](int i, int d) {
         const int bn = Be - Bs - 1;
         int st = ST_OK;
         if (bn < 0) st = ST_DEGENERATE;
         else if (d > MAX_MULTI_PRED) st = ST_INDEGREE;
-        else if (tb + bn > a.store_cap || tb + bn > INT_MAX) st = ST_OOM;
-        if (lane == 0) {
-            TeamHdr& h = hdr[i & 1];
-            const bool gen = i == 0 || bn <= 0 || strips_of(Bs, Be) > W;
-            h.h = make_int4(Bs, Be - 2 - Bs, (int)tb, (d & FR_D) | (gen ? FR_GENERAL : 0));
-            h.g = make_int4(e0, st, 0, 0);
-            if (st == ST_OK) a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
-            int32_t* w = slot(i);
-            w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
-        }
+        else if (tb + bn > store_cap || tb + bn > INT_MAX) st = ST_OOM;
+        const bool gen = i == 0 || bn <= 0 || strips_of(Bs, Be) > W;
+        if (lane == 0) hdr[i & 1].h = make_int4(Bs, Be - 2 - Bs, (int)tb, (gen ? FR_GENERAL : 0) | (st << FR_EOFF));
         return st;
     };
-    int st = put_header(0, 0, 0);
-    int edx = 0, edx_n = 0;     // row i's and row i + 1's predecessor records (x), one per lane
-    int succ = -1, succ_n = -1; // row i's and row i + 1's successors, one per lane
-    if (lane < ra1.w) succ = a.out_row[ra0.y + lane];
+    int st = put_header(0, 0);
+    int edx = 0, edx_n = 0;      // row i's and row i + 1's predecessor records (x), one per lane
+    int succ = -1, succ_n = -1;  // their successors, one per lane
+    if (lane < ra1.w) succ = out_row[ra0.y + lane];
     if (n > 1) {
-        if (lane < rb1.z) edx_n = a.ed[rb0.x + lane].x;
-        if (lane < rb1.w) succ_n = a.out_row[rb0.y + lane];
+        if (lane < rb1.z) edx_n = ed[rb0.x + lane].x;
+        if (lane < rb1.w) succ_n = out_row[rb0.y + lane];
     }
     int32_t pend = 0;  // state entering the window, one int per lane (8)
     __syncwarp();
@@ -708,93 +753,81 @@ __device__ void team_control(const TeamJob& a, char* smem, int64_t& cells_out) {
         }
         const int bn = Be - Bs - 1;
         const int d = i == 0 ? 0 : ra1.z, ns = ra1.w;
-        // the state that entered the window after the previous row
-        if (i > 0 && i - 1 + AHEAD < n && lane < 8) slot(i - 1 + AHEAD)[lane] = pend;
+        if (lane == 0) {
+            a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
+            int32_t* w = slot(i);
+            w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
+        }
         // loads two rows ahead
         int4 rc0 = rb0, rc1 = rb1;
         int edx_2 = 0, succ_2 = -1;
         if (i + 2 < n) {
-            rc0 = a.ra[2 * (i + 2)];
-            rc1 = a.ra[2 * (i + 2) + 1];
+            rc0 = ra[2 * (i + 2)];
+            rc1 = ra[2 * (i + 2) + 1];
             // (the in-window in-edges and out-edges are the same edges: E of each)
             const int e2 = rb0.x + rb1.z, o2 = rb0.y + rb1.w;
-            if (e2 + lane < E) edx_2 = a.ed[e2 + lane].x;
-            if (o2 + lane < E) succ_2 = a.out_row[o2 + lane];
-        }
-        __syncwarp();
-        // row i + 1's predecessor records
-        const int dn = i + 1 < n ? rb1.z : 0;
-        if (i + 1 < n) {
-            TeamHdr& h = hdr[(i + 1) & 1];
-            for (int k0 = 0; k0 < dn; k0 += 32) {
-                const int kk = k0 + lane;
-                if (kk < dn) {
-                    int4 v;
-                    v.x = k0 == 0 ? edx_n : a.ed[rb0.x + kk].x;
-                    const int p = v.x >> 4;
-                    if (i - p < AHEAD) {
-                        const int32_t* w = slot(p);
-                        v.y = w[SW_BS]; v.z = w[SW_BE]; v.w = w[SW_TB];
-                    } else {
-                        const int4 q = a.rowi[p];
-                        v.y = q.x; v.z = q.y; v.w = q.z;
-                    }
-                    const bool near = i + 1 - p < S::TR && strips_of(v.y, v.z) <= W;
-                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : -1, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
-                    if (kk < HDR_E) h.ed[kk] = f;
-                    else a.fe[rb0.x + kk] = f;
-                    a.ed[rb0.x + kk] = v;
-                }
-            }
+            if (e2 + lane < E) edx_2 = ed[e2 + lane].x;
+            if (o2 + lane < E) succ_2 = out_row[o2 + lane];
         }
         // row i's predecessors' slopes and maxima (their rows are done), its own
         // state and the next row's
         int psl = 0, pmp = INT_MIN / 2;
         if (i > 0 && lane < d && d <= 32) {
             const int p = edx >> 4;
-            const int32_t* w = i - p < AHEAD ? slot(p) : a.state + 8 * (int64_t)p;
+            const int32_t* w = i - p < AHEAD ? slot(p) : state + 8 * (int64_t)p;
             psl = w[SW_SL];
             pmp = w[SW_MP];
         }
-        const int max_psl = __reduce_max_sync(0xffffffffu, psl);
+        int max_psl = psl, pmp0 = pmp;
+        if (d > 1) {
+            max_psl = __reduce_max_sync(0xffffffffu, psl);
+        } else {
+            max_psl = __shfl_sync(0xffffffffu, psl, 0);
+            pmp0 = __shfl_sync(0xffffffffu, pmp, 0);
+        }
         int32_t* own = slot(i);
         int sl = own[SW_SL], ow = own[SW_OW], ol = own[SW_OL], orr = own[SW_OR];
         const int32_t* nw = slot(i + 1);
         int nPl = nw[SW_PL], nPr = nw[SW_PR], nOl = nw[SW_OL], nOr = nw[SW_OR], nOw = nw[SW_OW];
         bool to_next = __any_sync(0xffffffffu, lane < ns && succ == i + 1);
         for (int k0 = 32; k0 < ns; k0 += 32)
-            to_next |= __any_sync(0xffffffffu, k0 + lane < ns && a.out_row[ra0.y + k0 + lane] == i + 1);
+            to_next |= __any_sync(0xffffffffu, k0 + lane < ns && out_row[ra0.y + k0 + lane] == i + 1);
         // the row's maxima: published in the last lap's half of the summaries
         const int nst = bn > 0 ? strips_of(Bs, Be) : 0;
         const int laps = nst > W ? (nst + W - 1) / W : 1;
         xp = (xp + laps - 1) & 1;
-        bar_sync<2, S::THREADS>();
+        // the state that entered the window after the previous row (its load had the time since)
+        if (i > 0 && i - 1 + AHEAD < n && lane < 8) slot(i - 1 + AHEAD)[lane] = pend;
+        __syncwarp();
+        bar_sync<2, 32 * (W + 1)>();
+        int acj = 0;
         if (i >= 1) {
-            const int4 bw = lane < W ? bests[xp * W + lane] : make_int4(INT_MIN, INT_MAX, 4, 0);
-            const int32_t best = __reduce_max_sync(0xffffffffu, bw.x);
-            const int key = __reduce_min_sync(0xffffffffu, lane < W && bw.x == best ? bw.y * 8 + bw.z : INT_MAX);
-            const int acj = bn > 0 ? key >> 3 : Bs * BLK;
+            const int4 bq = lane < W ? lds128(bests + (xp * W + lane) * 16) : make_int4(INT_MIN, 0, 0, 0);
+            const int32_t best = __reduce_max_sync(0xffffffffu, bq.x);
+            const int key = __reduce_min_sync(0xffffffffu, bq.x == best ? bq.y * 8 + bq.z : INT_MAX);
+            acj = bn > 0 ? key >> 3 : Bs * BLK;
             const int code = bn > 0 ? key & 7 : (int)a.qs[acj + 1];
             int sl_best = INT_MIN, max_slp = 0;
-            bool is_match = false;
             if (ra1.y == code) {  // cur.base == seq[max_acj]
-                if (d <= 32) {
-                    max_slp = max_psl;
+                max_slp = max_psl;
+                if (d <= 1) {
+                    if (pmp0 + 1 == acj) sl_best = max_psl + 1;
+                } else if (d <= 32) {
                     sl_best = __reduce_max_sync(0xffffffffu, pmp + 1 == acj ? psl + 1 : INT_MIN);
                 } else {
                     for (int kk = lane; kk < d; kk += 32) {
-                        const int p = a.ed[ra0.x + kk].x >> 4;
-                        const int32_t* w = i - p < AHEAD ? slot(p) : a.state + 8 * (int64_t)p;
+                        const int p = ed[ra0.x + kk].x >> 4;
+                        const int32_t* w = i - p < AHEAD ? slot(p) : state + 8 * (int64_t)p;
                         max_slp = max(max_slp, w[SW_SL]);
                         if (w[SW_MP] + 1 == acj) sl_best = max(sl_best, w[SW_SL] + 1);
                     }
                     max_slp = __reduce_max_sync(0xffffffffu, max_slp);
                     sl_best = __reduce_max_sync(0xffffffffu, sl_best);
                 }
-                is_match = sl_best != INT_MIN;
             }
+            const bool is_match = sl_best != INT_MIN;
             if (is_match) sl = mx(sl, sl_best);
-            if (!is_match && max_slp < 30) ow = mn(ow + max_slp + 1, 5 * a.w);
+            else if (max_slp < 30) ow = mn(ow + max_slp + 1, 5 * bw);
             if (sl >= 30) {
                 ol = orr = acj - ra1.x;
                 ow = 0;
@@ -806,23 +839,26 @@ __device__ void team_control(const TeamJob& a, char* smem, int64_t& cells_out) {
                 nPr = mx(nPr, acj + 1);
                 nOw = ow ? mx(nOw, ow) : ow;
             }
-            cells += (int64_t)bn * BLK;
-            tb += bn;
-            if (i + 1 < n) {
-                band_adaptive(rb0.z, rb0.w, m, a.w, nPl, nPr, nOl, nOr, nOw, Bs, Be);
-                st = put_header(i + 1, dn, rb0.x);
-            }
-            bar_sync<1, S::THREADS>();  // header i + 1; row i's cells
+        }
+        cells += (int64_t)bn * BLK;
+        tb += bn;
+        if (i + 1 < n) {
+            band_adaptive(rb0.z, rb0.w, m, bw, nPl, nPr, nOl, nOr, nOw, Bs, Be);
+            st = put_header(i + 1, rb1.z);
+        }
+        __syncwarp();
+        bar_sync<1, S::THREADS>();  // header i + 1; row i's cells
+        if (i >= 1) {
             if (lane == 0) {
                 own[SW_SL] = sl; own[SW_MP] = acj;
-                int32_t* gs = a.state + 8 * (int64_t)i;
+                int32_t* gs = state + 8 * (int64_t)i;
                 gs[SW_SL] = sl; gs[SW_MP] = acj;
             }
             for (int k0 = 0; k0 < ns; k0 += 32) {
                 const int kk = k0 + lane;
                 if (kk < ns) {
-                    const int sr = k0 == 0 ? succ : a.out_row[ra0.y + kk];
-                    int32_t* w = sr - i < AHEAD ? slot(sr) : a.state + 8 * (int64_t)sr;
+                    const int sr = k0 == 0 ? succ : out_row[ra0.y + kk];
+                    int32_t* w = sr - i < AHEAD ? slot(sr) : state + 8 * (int64_t)sr;
                     w[SW_OL] = sl >= 30 ? ol : mn(w[SW_OL], ol);
                     w[SW_OR] = sl >= 30 ? orr : mx(w[SW_OR], orr);
                     w[SW_PL] = mn(w[SW_PL], acj);
@@ -830,23 +866,82 @@ __device__ void team_control(const TeamJob& a, char* smem, int64_t& cells_out) {
                     w[SW_OW] = ow ? mx(w[SW_OW], ow) : ow;
                 }
             }
-        } else {
-            cells += (int64_t)bn * BLK;
-            tb += bn;
-            if (n > 1) {
-                band_adaptive(rb0.z, rb0.w, m, a.w, nPl, nPr, nOl, nOr, nOw, Bs, Be);
-                st = put_header(1, dn, rb0.x);
-            }
-            bar_sync<1, S::THREADS>();
         }
         __syncwarp();
         xp ^= 1;
-        if (i + AHEAD < n && lane < 8) pend = a.state[8 * (int64_t)(i + AHEAD) + lane];
+        if (i + AHEAD < n && lane < 8) pend = state[8 * (int64_t)(i + AHEAD) + lane];
         ra0 = rb0; ra1 = rb1; rb0 = rc0; rb1 = rc1;
         edx = edx_n; edx_n = edx_2;
         succ = succ_n; succ_n = succ_2;
     }
     cells_out = cells;
+}
+
+// Row i + 1's records while row i is filled: every predecessor's band and place
+// (TeamJob::ed), and the fill's list, without row i when that fits the team's
+// columns (TeamHdr).
+template <int W, bool WIDE>
+__device__ void team_records(const TeamJob& a, char* smem) {
+    typedef TeamSmem<W, true, WIDE> S;
+    TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
+    const int32_t* win = reinterpret_cast<const int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
+    const unsigned hb = (unsigned)__cvta_generic_to_shared(hdr);
+    const int lane = threadIdx.x & 31;
+    const int n = a.n, E = a.in_ptr[n];
+    int4* ed = a.ed;
+    int4* fe = a.fe;
+    const int32_t* in_ptr = a.in_ptr;
+    // row i + 1: first in-edge, end, and the records (x) one per lane; row i + 2's are fetched a row ahead
+    int e0 = n > 1 ? in_ptr[1] : 0, e1 = n > 1 ? in_ptr[2] : 0, e2 = n > 2 ? in_ptr[3] : e1;
+    int x = e0 + lane < E ? ed[e0 + lane].x : 0;
+    if (lane == 0) hdr[0].g = make_int4(0, 0, 0, 0);
+    __syncwarp();
+    bar_sync<1, S::THREADS>();  // header 0
+    for (int i = 0; i < n; i++) {
+        const int4 h = lds128(hb + (i & 1) * (unsigned)sizeof(TeamHdr));
+        if (h.w >> FR_EOFF) return;
+        const int x2 = e1 + lane < E ? ed[e1 + lane].x : 0;
+        const int e3 = i + 4 <= n ? in_ptr[i + 4] : e2;
+        if (i + 1 < n) {
+            TeamHdr& o = hdr[(i + 1) & 1];
+            const int Bs = h.x, Be = h.x + h.y + 2, dn = e1 - e0;
+            const bool lap1 = h.y >= 0 && strips_of(Bs, Be) <= W;
+            int prev = 0;
+            for (int k0 = 0; k0 < dn; k0 += 32) {
+                const int kk = k0 + lane;
+                int4 v = make_int4(-1, 0, 0, 0);
+                if (kk < dn) {
+                    v.x = k0 == 0 ? x : ed[e0 + kk].x;
+                    const int p = v.x >> 4;
+                    if (p == i) {
+                        v.y = Bs; v.z = Be; v.w = h.z;
+                    } else if (i - p < AHEAD) {
+                        const int32_t* w = win + (p & (SWIN - 1)) * SW_INTS;
+                        v.y = w[SW_BS]; v.z = w[SW_BE]; v.w = w[SW_TB];
+                    } else {
+                        const int4 q = a.rowi[p];
+                        v.y = q.x; v.z = q.y; v.w = q.z;
+                    }
+                    ed[e0 + kk] = v;
+                }
+                const unsigned pmask = __ballot_sync(0xffffffffu, lap1 && (v.x >> 4) == i);
+                if (kk < dn && !((pmask >> lane) & 1u)) {
+                    const int p = v.x >> 4, at = kk - (prev != 0 || (pmask & ((1u << lane) - 1u)) != 0);
+                    const bool near = i + 1 - p < S::TR && v.z - v.y - 1 > 0 && strips_of(v.y, v.z) <= W;
+                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : ~v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+                    if (at < HDR_E) o.ed[at] = f;
+                    else fe[e0 + at] = f;
+                }
+                if (pmask) prev = FR_PREV | ((__shfl_sync(0xffffffffu, v.x, __ffs(pmask) - 1) & 7) << FR_PBASE);
+            }
+            // {first in-edge, predecessors, the fill's flags and count, -}
+            if (lane == 0) o.g = make_int4(e0, dn, (dn - (prev != 0)) | prev, 0);
+        }
+        __syncwarp();
+        bar_sync<1, S::THREADS>();  // header i + 1
+        e0 = e1; e1 = e2; e2 = e3;
+        x = x2;
+    }
 }
 
 template <int W, bool WIDE>
@@ -859,21 +954,26 @@ __device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) 
     for (int x = tid; x < SWIN * SW_INTS; x += S::THREADS) win[x] = x % SW_INTS == SW_PL ? m : 0;
     if (tid == 0) a.out[0] = ST_OK;
     bar_sync<1, S::THREADS>();
-    if (tid >= 32 * W) {
-        team_control<W, WIDE>(a, smem, cells);
+    if (tid >= 32 * (W + 1)) {
+        team_records<W, WIDE>(a, smem);
+    } else if (tid >= 32 * W) {
+        team_state<W, WIDE>(a, smem, cells);
     } else {
         TeamRow<W, true, WIDE> t(smem, a);
         const unsigned hb = (unsigned)__cvta_generic_to_shared(hdr);
         bar_sync<1, S::THREADS>();  // header 0
         for (int i = 0; i < n; i++) {
             const unsigned hc = hb + (i & 1) * (unsigned)sizeof(TeamHdr);
-            const int4 h = lds128(hc), g = lds128(hc + 16);
-            if (g.y != ST_OK) break;
-            if (h.w & FR_GENERAL)
+            int4 h = lds128(hc);
+            const int4 g = lds128(hc + 16);
+            if (h.w >> FR_EOFF) break;
+            if (h.w & FR_GENERAL) {
+                h.w |= g.y;
                 t.general(i, h, a.ed + g.x);
-            else
-                t.row(i, h, [&](int e) { return e < HDR_E ? lds128(hc + 32 + e * 16) : a.fe[g.x + e]; },
-                      [&](int e) { return a.ed[g.x + e]; }, [] {});
+            } else {
+                h.w = g.z;
+                t.row(i, h, [&](int e) { return e < HDR_E ? lds128(hc + 32 + e * 16) : a.fe[g.x + e]; }, [] {});
+            }
             bar_sync<1, S::THREADS>();  // row i's cells, header i + 1
         }
     }
@@ -1171,7 +1271,7 @@ __global__ void __launch_bounds__(TeamSmem<W, ADAPT, WIDE>::THREADS, 1) k_align(
     int st;
     if constexpr (ADAPT) {
         st = team_fill_adaptive<W, WIDE>(a, tsm, cells);
-        if (threadIdx.x == 32 * W) s_cells = cells;
+        if (threadIdx.x == 32 * W) s_cells = cells;  // the state warp's
         __syncthreads();
         cells = s_cells;
     } else {
