@@ -48,7 +48,8 @@ struct SlotLayout {
     int64_t bytes;
 };
 
-SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int64_t store_bytes, bool stat, bool adaptive, bool wide) {
+SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int64_t store_bytes, bool stat, bool adaptive, bool wide,
+                       bool team) {
     SlotLayout L;
     std::memset(&L, 0, sizeof L);
     L.NC = NC; L.EC = EC; L.QC = QC;
@@ -70,8 +71,8 @@ SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int64_t store_bytes, 
     L.v_ed = take(16 * (size_t)EC);
     L.v_deal = take(16 * (size_t)EC);
     L.v_rowi = take(16 * (size_t)NC);
+    if (stat || team) L.v_fe = take(16 * (size_t)EC);
     if (stat) {
-        L.v_fe = take(16 * (size_t)EC);
         L.v_fr = take(16 * (size_t)NC);
     } else {
         L.v_ra = take(32 * (size_t)NC);
@@ -824,7 +825,7 @@ __device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, int m, int w
             if (STATIC) {
                 const int p = v.x >> 4;
                 const bool near = x[q].w - p < R && pr[q].y - pr[q].x - 1 <= RB;
-                fe[at] = make_int4(near ? (p & (R - 1)) * RB * BB : -1, (v.x & 7) * 0x01010101, pr[q].x,
+                fe[at] = make_int4(near ? (p & (R - 1)) * RB * BB : ~pr[q].z, (v.x & 7) * 0x01010101, pr[q].x,
                                    pr[q].y - 2 - pr[q].x);
                 v.y = pr[q].x; v.z = pr[q].y; v.w = pr[q].z;
             }
@@ -882,7 +883,10 @@ __device__ int dg_first_read(DevGraph& g, const uint8_t* rd, int len, int lane) 
     return ST_OK;
 }
 
-template <bool STATIC, bool WIDE>
+// TEAM > 0 (adaptive band): the window belongs to a block of TEAM + 2 warps; this
+// is warp 0's part, which runs everything but the fill alone (k_batch_team).
+constexpr int TEAM_RING = 98304;  // two blocks of up to 8 warps' columns per SM
+template <bool STATIC, bool WIDE, int TEAM, int U>
 __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned char* wsm, int w, int lane) {
     const SlotLayout& L = A.L;
     DevGraph g = slot_graph(s, L);
@@ -973,6 +977,7 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
             a.store_cap = L.store_cap;
             a.moves = (int32_t*)(s + L.moves);
             a.moves_cap = L.NC + L.QC + 16;
+            a.out = g.hdr + 4;
         }
         __syncwarp();
         if (n > L.NC) { status = ST_CAPACITY; break; }
@@ -980,24 +985,29 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         int64_t cells = 0;
         if constexpr (STATIC) {
             // shared memory: row ring, query, staged rows
-            const WarpRing ring{(unsigned)__cvta_generic_to_shared(wsm), A.sring_rows, A.sring_rows ? A.sring_blocks : 0};
+            const WarpRing ring{(unsigned)__cvta_generic_to_shared(wsm), A.sring_rows, A.sring_rows ? A.sring_blocks : 0, -1};
             uint8_t* qsm = wsm + (size_t)A.sring_rows * A.sring_blocks * BLK * Cells<WIDE>::BYTES;
             for (int64_t x = lane * 16; x < qsb; x += 32 * 16)
                 *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>(qs + x);
             __syncwarp();
             warp_fill_static<WIDE>(a, ring, qsm, qsm + ((qsb + 15) & ~(int64_t)15), lane);
+        } else if constexpr (TEAM > 0) {
+            bar_sync<4, 32 * (TEAM + 2)>();  // the job
+            st = team_fill_adaptive<TEAM, WIDE, TEAM_RING>(a, (char*)wsm, cells);
         } else {
             // shared memory: staged records, state window, and the query when it fits
             const uint8_t* qf = qs;
-            const int64_t used = WED * 16 + warp_state_bytes(A.state_rows);
+            int64_t used = WED * 16 + warp_state_bytes(A.state_rows);
             if (used + qsb <= A.smem_per_warp) {
                 uint8_t* qsm = wsm + used;
                 for (int64_t x = lane * 16; x < qsb; x += 32 * 16)
                     *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>(qs + x);
                 qf = qsm;
+                used += (qsb + 15) & ~(int64_t)15;
             }
             __syncwarp();
-            st = warp_fill_dyn<WIDE>(a, A.f > 0 && A.ab_band, wsm, A.state_rows, qf, lane, cells);
+            st = warp_fill_dyn<WIDE, U>(a, A.f > 0 && A.ab_band, wsm, A.state_rows, wsm + used,
+                                     (int)((A.smem_per_warp - used) / (BLK * Cells<WIDE>::BYTES)), qf, lane, cells);
         }
         __syncwarp();
         if (st == ST_OK) {
@@ -1041,7 +1051,7 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         }
         tick(PH_FILL);
         int32_t nm = 0;
-        if (st == ST_OK) st = team_backtrack<WIDE, 4>(a, (char*)wsm, A.smem_per_warp, lane, nm);
+        if (st == ST_OK) st = team_backtrack<WIDE, TEAM ? 8 : 4>(a, (char*)wsm, A.smem_per_warp, lane, nm);
         if (lane == 0) {
             g.hdr[2] = st;
             g.hdr[13] = nm;
@@ -1096,16 +1106,63 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_batch(BatchArgs A) {
         if (lane == 0) idx = atomicAdd(A.counter, 1);
         idx = __shfl_sync(0xffffffffu, idx, 0);
         if (idx >= A.n_windows) break;
-        process_window<STATIC, WIDE>(A, s, s_args[warp], wsm, A.order[idx], lane);
+        process_window<STATIC, WIDE, 0, MINB <= 2 ? 2 : 1>(A, s, s_args[warp], wsm, A.order[idx], lane);
     }
+}
+
+// The adaptive band with few windows: a block of W + 2 warps per window. Warp 0
+// runs the window; for each alignment's fill the others join it.
+template <int W>
+__global__ void __launch_bounds__(32 * (W + 2), 2) k_batch_team(BatchArgs A) {
+    __shared__ TeamJob job;
+    __shared__ int s_run;
+    extern __shared__ __align__(16) unsigned char dsm[];
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x >= 32) {
+        while (true) {
+            bar_sync<4, 32 * (W + 2)>();
+            if (!s_run) return;
+            int64_t cells = 0;
+            team_fill_adaptive<W, false, TEAM_RING>(job, (char*)dsm, cells);
+        }
+    }
+    if (lane == 0) s_run = 1;
+    char* s = A.slots + (int64_t)blockIdx.x * A.L.bytes;
+    while (true) {
+        int idx = 0;
+        if (lane == 0) idx = atomicAdd(A.counter, 1);
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        if (idx >= A.n_windows) break;
+        process_window<false, false, W, 1>(A, s, job, dsm, A.order[idx], lane);
+    }
+    __syncwarp();
+    if (lane == 0) s_run = 0;
+    __syncwarp();
+    bar_sync<4, 32 * (W + 2)>();
 }
 
 // Every build of the kernel by band kind, cell and register budget (blocks of 4
 // warps per SM).
 typedef void (*BatchKernel)(BatchArgs);
+struct TeamKernel {
+    BatchKernel kern;
+    int threads, smem;
+};
+template <int W>
+TeamKernel team_kernel_of() {
+    return {(BatchKernel)k_batch_team<W>, 32 * (W + 2), TeamSmem<W, true, false, TEAM_RING>::BYTES};
+}
+TeamKernel team_kernel(int cols) {
+    const int strips = (cols + STRIP - 1) / STRIP;
+    if (strips <= 2) return team_kernel_of<2>();
+    if (strips <= 4) return team_kernel_of<4>();
+    if (strips <= 6) return team_kernel_of<6>();
+    return team_kernel_of<8>();
+}
 BatchKernel batch_kernel(bool stat, bool wide, int blocks_per_sm) {
     if (wide) return stat ? (BatchKernel)k_batch<4, true, true, 3> : (BatchKernel)k_batch<4, false, true, 3>;
     if (blocks_per_sm >= 5) return stat ? (BatchKernel)k_batch<4, true, false, 5> : (BatchKernel)k_batch<4, false, false, 5>;
+    if (blocks_per_sm <= 2 && !stat) return (BatchKernel)k_batch<4, false, false, 2>;  // two chunks of a row at a time
     if (blocks_per_sm >= 4) return stat ? (BatchKernel)k_batch<4, true, false, 4> : (BatchKernel)k_batch<4, false, false, 4>;
     return stat ? (BatchKernel)k_batch<4, true, false, 3> : (BatchKernel)k_batch<4, false, false, 3>;
 }
@@ -1348,11 +1405,21 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     const bool wide = !cell_packable(sc, 60000, QC);
     const int cell_bytes = wide ? Cells<true>::BYTES : Cells<false>::BYTES;
     const int64_t store = (caps.cells * cell_bytes + 4095) / 4096 * 4096;
-    SlotLayout L = make_layout(NC, EC, QC, store, stat, adaptive, wide);
+    // Adaptive windows: a warp's row costs ~7,000 cycles however few windows there are, a
+    // team's ~1,800 with two teams to an SM. Measured, warps -> teams (kernel): windows of
+    // 150-900 bp, 240: 122 -> 75 ms, 740: 140 -> 80, 1,184: 151 -> 99; 1,000-2,000 bp, 400:
+    // 120 -> 78, 740: 121 -> 112, 1,024: 129 -> 152; 300-400 bp, 1,184: 24 -> 31. Teams up to
+    // 5 windows per SM.
+    const bool team = adaptive && !wide && !smem_set && count <= team_windows_per_sm * sms;
+    const int wband = p_.b + (p_.f ? (max_len_ + 1) / p_.f : 0);
+    TeamKernel tk{};
+    if (team) tk = team_kernel(std::min(((max_len_ + 1) / BLK + 1) * BLK, 6 * wband + STRIP));
+    SlotLayout L = make_layout(NC, EC, QC, store, stat, adaptive, wide, team);
     const SlotLayout L_planned = L;
-    const int warps = warps_per_block;
-    const int smem_w = shared_per_warp(count, warps, sms);
+    const int warps = team ? 1 : warps_per_block;  // windows per block
+    const int smem_w = team ? tk.smem : shared_per_warp(count, warps, sms);
     const size_t dyn = (size_t)warps * smem_w;
+    const int threads = team ? tk.threads : warps * 32;
     const int qsm_bytes = (int)((qs_bytes(QC) + 15) / 16 * 16);
     constexpr int kStageBytes = 1792;  // shared memory a static-band warp needs beside its query
     static_assert(kStageBytes >= WSTG_BYTES && kStageBytes >= BtTile<true, 4>::PER_ROW * 2 + 16, "stage and backtrack tile");
@@ -1377,10 +1444,12 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     int stat_rows = stat ? std::min(8, (smem_w - qsm_bytes - kStageBytes) / std::max(1, ring_blocks * 64)) : 32;
     if (stat_rows < 2) stat_rows = 0;
     int occ = 0;
-    const BatchKernel kern = batch_kernel(stat, wide, blocks_per_sm);
-    if (warps != 4) throw std::invalid_argument("batch kernel is built for 4 warps per block");
+    // windows that leave two blocks to an SM run the build with twice the registers
+    const int want_per_sm = std::min<int64_t>(blocks_per_sm, ((int64_t)(count + warps - 1) / warps + sms - 1) / sms);
+    const BatchKernel kern = team ? tk.kern : batch_kernel(stat, wide, want_per_sm);
+    if (!team && warps != 4) throw std::invalid_argument("batch kernel is built for 4 warps per block");
     cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn), "smem attr");
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, warps * 32, dyn), "occupancy");
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, dyn), "occupancy");
     // every block must be resident at once (persistent kernel): never more than the occupancy allows
     const int per_sm = std::max(1, std::min(blocks_per_sm, occ));
     int blocks = sms * per_sm;
@@ -1398,7 +1467,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
         if (h > 1.0) {
             const int32_t NCh = (int32_t)std::min<double>(60000.0, std::max(64.0, NC * h));
             const int64_t sth = ((int64_t)(store * h) + 4095) / 4096 * 4096;
-            L = make_layout(NCh, 3 * NCh, QC, sth, stat, adaptive, wide);
+            L = make_layout(NCh, 3 * NCh, QC, sth, stat, adaptive, wide, team);
         }
     }
     const int64_t max_by_mem = (int64_t)(budget / (size_t)L.bytes) / warps;
@@ -1472,7 +1541,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
         cudaGraph_t gr = nullptr;
         cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
         cudaMemsetAsync(A.counter, 0, 4, s);
-        kern<<<blocks, 4 * 32, dyn, s>>>(A);
+        kern<<<blocks, threads, dyn, s>>>(A);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(s, &gr);
         cuda_check(le, "k_batch launch");

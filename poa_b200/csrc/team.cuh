@@ -254,13 +254,15 @@ struct BtTile {
     static constexpr int full() { return BT_ROWS * PER_ROW + 16; }
 };
 
-template <int W, bool ADAPT, bool WIDE>
+// RING_MAX: shared memory for the ring of rows (one CTA per SM by default).
+constexpr int RING_ALONE = 196608;
+template <int W, bool ADAPT, bool WIDE, int RING_MAX = RING_ALONE>
 struct TeamSmem {
     static constexpr int CELLB = TC * Cells<WIDE>::BYTES;          // bytes per thread and row
     static constexpr int ROWB = 32 * W * CELLB;
     // rows of the ring (a power of two): noisy graphs have predecessors tens of rows back, and
     // one read from the row store costs as much as a row
-    static constexpr int TR = ROWB * 64 <= 196608 ? 64 : ROWB * 32 <= 196608 ? 32 : 16;
+    static constexpr int TR = ROWB * 64 <= RING_MAX ? 64 : ROWB * 32 <= RING_MAX ? 32 : 16;
     static constexpr int RING = TR * ROWB;
     static constexpr int PUB = RING;                               // int4 [2][W]
     static constexpr int BEST = PUB + 2 * W * 16;                  // int4 [2][W]
@@ -383,10 +385,10 @@ __device__ __forceinline__ void team_stage(const TeamJob& a, TeamStage& st, int 
 }
 
 // The fill of one row by a column-owning thread; see the file comment.
-template <int W, bool ADAPT, bool WIDE>
+template <int W, bool ADAPT, bool WIDE, int RING_MAX = RING_ALONE>
 struct TeamRow {
     typedef Cells<WIDE> C;
-    typedef TeamSmem<W, ADAPT, WIDE> S;
+    typedef TeamSmem<W, ADAPT, WIDE, RING_MAX> S;
     static constexpr int32_t NEG = C::NEG;
     static constexpr int32_t LOW = WIDE ? INT_MIN : -(1 << 30);
     const TeamJob& a;
@@ -701,9 +703,9 @@ __device__ void team_fill_static(const TeamJob& a, char* smem) {
 // other warps fill the row. (As one warp the two took 2,400 cycles a row.)
 constexpr int AHEAD = SWIN / 2 - 1;
 
-template <int W, bool WIDE>
+template <int W, bool WIDE, int RING_MAX = RING_ALONE>
 __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
-    typedef TeamSmem<W, true, WIDE> S;
+    typedef TeamSmem<W, true, WIDE, RING_MAX> S;
     TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
     int32_t* win = reinterpret_cast<int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
     const unsigned bests = (unsigned)__cvta_generic_to_shared(smem + S::BEST);
@@ -880,9 +882,9 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
 // Row i + 1's records while row i is filled: every predecessor's band and place
 // (TeamJob::ed), and the fill's list, without row i when that fits the team's
 // columns (TeamHdr).
-template <int W, bool WIDE>
+template <int W, bool WIDE, int RING_MAX = RING_ALONE>
 __device__ void team_records(const TeamJob& a, char* smem) {
-    typedef TeamSmem<W, true, WIDE> S;
+    typedef TeamSmem<W, true, WIDE, RING_MAX> S;
     TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
     const int32_t* win = reinterpret_cast<const int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
     const unsigned hb = (unsigned)__cvta_generic_to_shared(hdr);
@@ -944,9 +946,9 @@ __device__ void team_records(const TeamJob& a, char* smem) {
     }
 }
 
-template <int W, bool WIDE>
+template <int W, bool WIDE, int RING_MAX = RING_ALONE>
 __device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) {
-    typedef TeamSmem<W, true, WIDE> S;
+    typedef TeamSmem<W, true, WIDE, RING_MAX> S;
     const int tid = threadIdx.x, n = a.n, m = a.qlen + 1;
     int32_t* win = reinterpret_cast<int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
     TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
@@ -955,11 +957,11 @@ __device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) 
     if (tid == 0) a.out[0] = ST_OK;
     bar_sync<1, S::THREADS>();
     if (tid >= 32 * (W + 1)) {
-        team_records<W, WIDE>(a, smem);
+        team_records<W, WIDE, RING_MAX>(a, smem);
     } else if (tid >= 32 * W) {
-        team_state<W, WIDE>(a, smem, cells);
+        team_state<W, WIDE, RING_MAX>(a, smem, cells);
     } else {
-        TeamRow<W, true, WIDE> t(smem, a);
+        TeamRow<W, true, WIDE, RING_MAX> t(smem, a);
         const unsigned hb = (unsigned)__cvta_generic_to_shared(hdr);
         bar_sync<1, S::THREADS>();  // header 0
         for (int i = 0; i < n; i++) {

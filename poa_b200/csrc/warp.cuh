@@ -8,7 +8,8 @@
 // go to the slot's row store, 32 bytes per block; with the static band the
 // last rows are also kept in a shared-memory ring (two planes of 16 bytes per
 // block, so any shift between a row's band and its predecessor's reads without
-// bank conflicts).
+// bank conflicts). With the dynamic bands the ring is a circular buffer of blocks
+// that holds as many of the last rows as fit, whatever their width.
 //
 // Measured on a B200 against the record fill it replaced (kernel time):
 // 8,000 polishing windows 651 -> 339 ms, 1,024 windows of 2,000 bp at 15 %
@@ -27,106 +28,143 @@ constexpr int warp_state_bytes(int rows) { return rows * SW_INTS * 4; }
 
 struct WarpRing {
     unsigned at;  // shared memory address
-    int rows;     // a power of two, or 0: no ring
-    int blocks;   // per row
+    int rows;     // static band: a power of two, or 0: no ring
+    int blocks;   // static band: per row
+    int cur;      // dynamic bands: the current row's first block, or -1: not kept
 };
+enum { RING_STATIC = 1, RING_DYN = 2 };
 
-// One row. ed_at(e): {x, base in every byte, Bs, last block - Bs}, x the
-// predecessor's ring offset (RING, -1: not in the ring, far(e) has its row-store
-// block) or its row-store block. With ARGMAX, best / best_col become the row's
-// first maximum.
-template <bool WIDE, bool RING, bool ARGMAX, class EdAt, class Far>
+// One row. ed_at(e): {ring offset, or ~row-store block; base in every byte; Bs;
+// last block - Bs}. With ARGMAX, best / best_col become the row's first maximum.
+// U chunks are taken together: a chunk is ~300 mostly dependent instructions, so
+// two of them in flight hide each other's latency where the registers allow it
+// (rows of several chunks, few warps per SM).
+//
+// The gap term of cell l is I[l] = max(I[l-1] + e1, H0[l-1] + o1): within a
+// block one dependent step per cell, first from nothing for the block's own
+// contribution, then from the prefix over the lanes.
+template <bool WIDE, int RING, bool ARGMAX, int U, class EdAt>
 __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span, int tb, int d, const uint8_t* qs,
-                                         const WarpRing& ring, char* store, int lane, EdAt ed_at, Far far, int32_t& best,
+                                         const WarpRing& ring, char* store, int lane, EdAt ed_at, int32_t& best,
                                          int& best_col) {
     typedef Cells<WIDE> C;
     constexpr int32_t NEG = C::NEG;
     constexpr int32_t LOW = WIDE ? INT_MIN : -(1 << 30);
     constexpr int HB = 4 * C::BYTES, BB = 2 * HB;  // bytes per half block and block
-    const int32_t g = k.o1 - k.e1;
-    int32_t carry = add32(add32(NEG, k.e1), -k.o1);  // the gap term's floor: NEG_INF extended from column 0
-    for (int c0 = 0; c0 <= span; c0 += 32) {
-        const int b = c0 + lane, B = Bs + b;
-        const bool act = b <= span;
-        const int Bz = B == 0 ? INT_MAX : B;
-        const uint2 qw = act ? *reinterpret_cast<const uint2*>(qs + (int64_t)B * BLK) : make_uint2(0x04040404u, 0x04040404u);
-        int32_t P[8], V[8];
+    // gap terms are kept as their value at column 0 (minus j * e1); the floor: NEG_INF extended from column 0
+    int32_t carry = NEG;
+    // row 0 has no gap terms: they start, and open, below everything
+    constexpr int32_t BELOW = WIDE ? -2000000000 : -(1 << 30);
+    const int32_t open = i == 0 && !WIDE ? BELOW : k.o1;
+    for (int c0 = 0; c0 <= span; c0 += 32 * U) {
+        int32_t H[U][8], V[U][8], out[U];
+        uint2 qw[U];
+        bool act[U];
 #pragma unroll
-        for (int l = 0; l < 8; l++) P[l] = V[l] = NEG;
-        if (i == 0 && B == 0) P[0] = 0;
+        for (int u = 0; u < U; u++) {
+            const int b = c0 + 32 * u + lane;
+            act[u] = b <= span;
+            qw[u] = act[u] ? *reinterpret_cast<const uint2*>(qs + (int64_t)(Bs + b) * BLK) : make_uint2(0x04040404u, 0x04040404u);
+#pragma unroll
+            for (int l = 0; l < 8; l++) H[u][l] = V[u][l] = NEG;
+            if (i == 0 && Bs + b == 0) H[u][0] = 0;
+        }
         for (int e = 0; e < d; e++) {
             const int4 er = ed_at(e);
-            const int pb = B - er.z;
-            const bool in = act && (unsigned)pb <= (unsigned)er.w;
-            const bool diag = in && Bz > er.z;  // the fill's block mask for the diagonal (src/align.cpp:1467)
-            C lo, hi;
-            lo.none();
-            hi.none();
-            int32_t left0 = NEG;  // lane 0: the cell before the chunk
-            const bool l0 = lane == 0 && c0 > 0 && in && pb > 0;
-            if (RING && er.x >= 0) {
-                const unsigned src = ring.at + er.x + pb * HB;
-                if (in) { lo.lds(src); hi.lds(src + ring.blocks * HB); }
-                if (l0) left0 = C::lds_m(src + ring.blocks * HB - C::BYTES);
-            } else {
-                const char* src = store + ((int64_t)(RING ? far(e) : er.x) + pb) * BB;
-                if (in) { lo.load(src); hi.load(src + HB); }
-                if (l0) left0 = C::load_m(src - C::BYTES);
+            C lo[U], hi[U];
+            int32_t left0[U];  // lane 0: the cell before the chunk (NEG_INF before the row's first block)
+            bool in[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int b = c0 + 32 * u + lane, pb = Bs + b - er.z;
+                in[u] = act[u] && (unsigned)pb <= (unsigned)er.w;
+                left0[u] = NEG;
+                const bool l0 = lane == 0 && c0 + u > 0 && in[u] && pb > 0;
+                if (er.x >= 0) {
+                    const unsigned src = ring.at + er.x + pb * HB;
+                    const int plane = (RING == RING_STATIC ? ring.blocks : er.w + 1) * HB;
+                    if (in[u]) { lo[u].lds(src); hi[u].lds(src + plane); }
+                    else { lo[u].none(); hi[u].none(); }
+                    if (l0) left0[u] = C::lds_m(src + plane - C::BYTES);
+                } else {
+                    const char* src = store + ((int64_t)~er.x + pb) * BB;
+                    if (in[u]) { lo[u].load(src); hi[u].load(src + HB); }
+                    else { lo[u].none(); hi[u].none(); }
+                    if (l0) left0[u] = C::load_m(src - C::BYTES);
+                }
             }
-            int32_t left = __shfl_up_sync(0xffffffffu, hi.m(3), 1);
-            if (lane == 0) left = left0;  // (NEG_INF before the row's first block)
-            const int32_t sm = diag || WIDE ? k.match : -(1 << 23), sx = diag || WIDE ? k.mismatch : -(1 << 23);
-            const uint32_t x0 = qw.x ^ (uint32_t)er.y, x1 = qw.y ^ (uint32_t)er.y;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int B = Bs + c0 + 32 * u + lane;
+                // the fill's block mask for the diagonal (src/align.cpp:1467)
+                const bool diag = in[u] && (B > er.z || B == 0);
+                int32_t left = __shfl_up_sync(0xffffffffu, hi[u].m(3), 1);
+                if (lane == 0) left = left0[u];
+                const int32_t sm = diag || WIDE ? k.match : -(1 << 23), sx = diag || WIDE ? k.mismatch : -(1 << 23);
+                const uint32_t x0 = qw[u].x ^ (uint32_t)er.y, x1 = qw[u].y ^ (uint32_t)er.y;
+#pragma unroll
+                for (int l = 0; l < 8; l++) {
+                    const int32_t src = l == 0 ? left : l <= 4 ? lo[u].m(l > 0 ? l - 1 : 0) : hi[u].m(l - 5);
+                    const int32_t cand = src + (((l < 4 ? x0 : x1) & (255u << (8 * (l & 3)))) == 0 ? sm : sx);
+                    if (!WIDE || diag) H[u][l] = mx(H[u][l], cand);
+                    V[u][l] = mx(V[u][l], l < 4 ? lo[u].v(l & 3, k) : hi[u].v(l & 3, k));
+                }
+            }
+        }
+        // H0; what the block passes on by itself; the row's maximum
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+#pragma unroll
+            for (int l = 0; l < 8; l++) H[u][l] = mx(H[u][l], V[u][l]);
+            int32_t t = add32(H[u][0], k.o1);
+#pragma unroll
+            for (int l = 1; l < 8; l++) t = mx(add32(t, k.e1), add32(H[u][l], k.o1));
+            out[u] = act[u] ? t - ((c0 + 32 * u + lane + 1) * BLK) * k.e1 : LOW;
+            if (ARGMAX) {
+                // the first maximum of H0 is the row's first maximum (a gap never exceeds the cell it opens from)
+                const int32_t lm = act[u] ? mx(mx(mx(H[u][0], H[u][1]), mx(H[u][2], H[u][3])),
+                                               mx(mx(H[u][4], H[u][5]), mx(H[u][6], H[u][7]))) : INT_MIN;
+                const int32_t wm = __reduce_max_sync(0xffffffffu, lm);
+                if (wm > best) {
+                    best = wm;
+                    int l = 7;
+#pragma unroll
+                    for (int q = 6; q >= 0; q--) l = H[u][q] == wm ? q : l;
+                    best_col = __shfl_sync(0xffffffffu, (Bs + c0 + 32 * u + lane) * BLK + l,
+                                           __ffs(__ballot_sync(0xffffffffu, lm == wm)) - 1);
+                }
+            }
+        }
+        int32_t incl[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) incl[u] = scan_max(out[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int b = c0 + 32 * u + lane;
+            int32_t ex = __shfl_up_sync(0xffffffffu, incl[u], 1);
+            if (lane == 0) ex = LOW;
+            int32_t I = mx(carry, ex) + (b * BLK) * k.e1;
+            carry = mx(carry, __shfl_sync(0xffffffffu, incl[u], 31));
+            if (i == 0) I = BELOW;
+            C lo, hi;
 #pragma unroll
             for (int l = 0; l < 8; l++) {
-                const int32_t src = l == 0 ? left : l <= 4 ? lo.m(l > 0 ? l - 1 : 0) : hi.m(l - 5);
-                const int32_t cand = src + (((l < 4 ? x0 : x1) & (255u << (8 * (l & 3)))) == 0 ? sm : sx);
-                if (!WIDE || diag) P[l] = mx(P[l], cand);
-                V[l] = mx(V[l], l < 4 ? lo.v(l & 3, k) : hi.v(l & 3, k));
+                const int32_t h = H[u][l], M = mx(h, I);
+                if (l < 4) lo.set(l & 3, M, V[u][l], k);
+                else hi.set(l & 3, M, V[u][l], k);
+                I = mx(add32(I, k.e1), WIDE && i == 0 ? BELOW : add32(h, open));
             }
-        }
-        int32_t H[8], key[8];
-#pragma unroll
-        for (int l = 0; l < 8; l++) {
-            H[l] = mx(P[l], V[l]);
-            key[l] = H[l] - l * k.e1;
-        }
-        const int32_t base = -(b * BLK) * k.e1;
-        int32_t top = mx(mx(mx(key[0], key[1]), mx(key[2], key[3])), mx(mx(key[4], key[5]), mx(key[6], key[7])));
-        const int32_t incl = scan_max(act ? top + base : LOW);
-        int32_t ex = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) ex = LOW;
-        if (ARGMAX) {
-            // the first maximum of H0 is the row's first maximum (a gap never exceeds the cell it opens from)
-            const int32_t lm = act ? mx(mx(mx(H[0], H[1]), mx(H[2], H[3])), mx(mx(H[4], H[5]), mx(H[6], H[7]))) : INT_MIN;
-            const int32_t wm = __reduce_max_sync(0xffffffffu, lm);
-            if (wm > best) {
-                best = wm;
-                int l = 7;
-#pragma unroll
-                for (int t = 6; t >= 0; t--) l = H[t] == wm ? t : l;
-                best_col = __shfl_sync(0xffffffffu, B * BLK + l, __ffs(__ballot_sync(0xffffffffu, lm == wm)) - 1);
+            if (act[u]) {
+                if (RING == RING_STATIC ? span < ring.blocks : ring.cur >= 0) {
+                    const unsigned at = RING == RING_STATIC ? (i & (ring.rows - 1)) * (unsigned)(ring.blocks * BB) : ring.cur * BB;
+                    const unsigned dst = ring.at + at + b * HB;
+                    lo.sts(dst);
+                    hi.sts(dst + (RING == RING_STATIC ? ring.blocks : span + 1) * HB);
+                }
+                char* dst = store + ((int64_t)tb + b) * BB;
+                lo.store(dst);
+                hi.store(dst + HB);
             }
-        }
-        int32_t run = mx(carry, ex) - base;
-        carry = mx(carry, __shfl_sync(0xffffffffu, incl, 31));
-        C lo, hi;
-#pragma unroll
-        for (int l = 0; l < 8; l++) {
-            const int32_t M = i == 0 ? H[l] : mx(H[l], run + (g + l * k.e1));
-            if (l < 4) lo.set(l & 3, M, V[l], k);
-            else hi.set(l & 3, M, V[l], k);
-            run = mx(run, key[l]);
-        }
-        if (act) {
-            if (RING && span < ring.blocks) {
-                const unsigned dst = ring.at + (i & (ring.rows - 1)) * (unsigned)(ring.blocks * BB) + b * HB;
-                lo.sts(dst);
-                hi.sts(dst + ring.blocks * HB);
-            }
-            char* dst = store + ((int64_t)tb + b) * BB;
-            lo.store(dst);
-            hi.store(dst + HB);
         }
     }
 }
@@ -154,15 +192,12 @@ __device__ void warp_fill_static(const TeamJob& a, const WarpRing& ring, const u
             const unsigned ed = stg + WSTG * 16 + (h.w >> FR_EOFF) * 16;
             const int i = i0 + x;
             const int4* fe = a.fe;
-            const int4* far = a.ed;
             if (h.w & FR_UNSTAGED)
-                warp_row<WIDE, true, false>(k, i, h.x, h.y, h.z, h.w & FR_D, qsm, ring, store, lane,
-                                            [&](int e) { return fe[a.in_ptr[i] + e]; },
-                                            [&](int e) { return far[a.in_ptr[i] + e].w; }, bm, bc);
+                warp_row<WIDE, RING_STATIC, false, 1>(k, i, h.x, h.y, h.z, h.w & FR_D, qsm, ring, store, lane,
+                                                   [&](int e) { return fe[a.in_ptr[i] + e]; }, bm, bc);
             else
-                warp_row<WIDE, true, false>(k, i, h.x, h.y, h.z, h.w & FR_D, qsm, ring, store, lane,
-                                            [&](int e) { return lds128(ed + e * 16); },
-                                            [&](int e) { return far[a.in_ptr[i] + e].w; }, bm, bc);
+                warp_row<WIDE, RING_STATIC, false, 1>(k, i, h.x, h.y, h.z, h.w & FR_D, qsm, ring, store, lane,
+                                                   [&](int e) { return lds128(ed + e * 16); }, bm, bc);
             __syncwarp();
         }
     }
@@ -171,11 +206,12 @@ __device__ void warp_fill_static(const TeamJob& a, const WarpRing& ring, const u
 // Adaptive band (-B) or full band (f = 0): bands known row by row. The band
 // state's serial part is team_control's, on the same warp: inputs that do not
 // need row i's maximum are fetched before the row is filled, the state of
-// nearby rows lives in a shared-memory window of `wrows` rows (a power of two).
-// Returns a status (uniform).
-template <bool WIDE>
-__device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm, int wrows, const uint8_t* qf, int lane,
-                             int64_t& cells_out) {
+// nearby rows lives in a shared-memory window of `wrows` rows (a power of two),
+// their cells in a buffer of rcap blocks at `rbuf`. Returns a status (uniform).
+enum { SW_RPOS = 7, SW_RAT = 11 };  // a kept row: its position in the stream of kept blocks, its first block in the buffer
+template <bool WIDE, int U>
+__device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm, int wrows, unsigned char* rbuf, int rcap,
+                             const uint8_t* qf, int lane, int64_t& cells_out) {
     const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n];
     const CellK k = a.k;
     char* const store = a.store;
@@ -202,7 +238,9 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
         if (lane < rb1.z) edx_n = a.ed[rb0.x + lane].x;
         if (lane < rb1.w) succ_n = a.out_row[rb0.y + lane];
     }
-    const WarpRing none{0, 0, 0};
+    constexpr int BB = BLK * Cells<WIDE>::BYTES;
+    WarpRing ring{(unsigned)__cvta_generic_to_shared(rbuf), 0, 0, -1};
+    int rpos = 0, rat = 0;  // end of the stream of kept blocks; its place in the buffer
     int32_t pend = 0;  // state entering the window, one int per lane (8)
     for (int i = 0; i < n; i++) {
         const int bn = Be - Bs - 1;
@@ -222,10 +260,19 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
             if (e2 + lane < E) edx_2 = a.ed[e2 + lane].x;
             if (o2 + lane < E) succ_2 = a.out_row[o2 + lane];
         }
+        // the row's place in the buffer: whole, so the end of the buffer may stay empty
+        ring.cur = -1;
+        if (bn > 0 && bn <= rcap) {
+            if (rat + bn > rcap) { rpos += rcap - rat; rat = 0; }
+            ring.cur = rat;
+            rat += bn;
+            rpos += bn;
+        }
         if (lane == 0) {
             a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
             int32_t* w = slot(i);
             w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
+            w[SW_RPOS] = rpos - bn; w[SW_RAT] = ring.cur;
         }
         // row i's predecessor records; their slopes and maxima
         int psl = 0, pmp = INT_MIN / 2;
@@ -235,16 +282,18 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
                 int4 v;
                 v.x = k0 == 0 ? edx : a.ed[ra0.x + kk].x;
                 const int p = v.x >> 4;
+                int from = -1;  // its first block in the buffer, unless written over by now
                 if (i - p < AHEAD) {
                     const int32_t* w = slot(p);
                     v.y = w[SW_BS]; v.z = w[SW_BE]; v.w = w[SW_TB];
+                    if (rpos - w[SW_RPOS] <= rcap) from = w[SW_RAT];
                     if (k0 == 0) { psl = w[SW_SL]; pmp = w[SW_MP]; }
                 } else {
                     const int4 q = a.rowi[p];
                     v.y = q.x; v.z = q.y; v.w = q.z;
                     if (adaptive && k0 == 0) { psl = a.state[8 * (int64_t)p + SW_SL]; pmp = a.state[8 * (int64_t)p + SW_MP]; }
                 }
-                if (kk < WED) sed[kk] = make_int4(v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+                if (kk < WED) sed[kk] = make_int4(from >= 0 ? from * BB : ~v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
                 a.ed[ra0.x + kk] = v;
             }
         }
@@ -257,13 +306,16 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
         auto ed_at = [&](int e) {
             if (e < WED) return lds128(seda + e * 16);
             const int4 v = ed[e];
-            return make_int4(v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+            return make_int4(~v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
         };
-        auto far = [](int) { return 0; };
         int32_t best = INT_MIN;
         int acj = Bs * BLK;
-        if (adaptive) warp_row<WIDE, false, true>(k, i, Bs, bn - 1, (int)tb, d, qf, none, store, lane, ed_at, far, best, acj);
-        else warp_row<WIDE, false, false>(k, i, Bs, bn - 1, (int)tb, d, qf, none, store, lane, ed_at, far, best, acj);
+        if (U > 1 && adaptive && bn > 32)
+            warp_row<WIDE, RING_DYN, true, U>(k, i, Bs, bn - 1, (int)tb, d, qf, ring, store, lane, ed_at, best, acj);
+        else if (adaptive)
+            warp_row<WIDE, RING_DYN, true, 1>(k, i, Bs, bn - 1, (int)tb, d, qf, ring, store, lane, ed_at, best, acj);
+        else
+            warp_row<WIDE, RING_DYN, false, 1>(k, i, Bs, bn - 1, (int)tb, d, qf, ring, store, lane, ed_at, best, acj);
         cells += (int64_t)bn * BLK;
         tb += bn;
         if (adaptive) {
