@@ -123,7 +123,8 @@ struct DevGraph {
     int32_t *e_from, *e_to, *e_w, *e_nin, *e_nout;
     int32_t *rank_to_id, *hlen, *tlen, *deg, *stk, *pre, *score;
     int32_t *hin, *hout, *stamp;  // heaviest in/out edge (first max in list order); fusion stamps
-    int32_t *csr_ptr, *csr_adj;   // topsort scratch: the view's out-lists, free until the view is rebuilt
+    int32_t *csr_ptr, *csr_adj;   // topsort scratch: the rows' out-lists, free until the rows are rebuilt
+    void *scratch8, *scratch8b;   // consensus scratch, 8 bytes a node each: the rows' records
     int32_t NC, EC;
 };
 
@@ -143,6 +144,7 @@ __device__ DevGraph slot_graph(char* s, const SlotLayout& L) {
     g.score = (int32_t*)(s + L.score);
     g.hin = (int32_t*)(s + L.hin); g.hout = (int32_t*)(s + L.hout); g.stamp = (int32_t*)(s + L.stamp);
     g.csr_ptr = (int32_t*)(s + L.v_out_ptr); g.csr_adj = (int32_t*)(s + L.v_out_row);
+    g.scratch8 = s + L.v_rowi; g.scratch8b = s + L.v_ed;
     g.NC = L.NC; g.EC = L.EC;
     return g;
 }
@@ -274,6 +276,136 @@ __device__ int dg_consensus(DevGraph& g, int nn, char* out, int cap) {
     return len;
 }
 
+// build_consensus with the whole warp: the same predecessors and scores as the
+// serial walk, which processes nodes in topological order, keeping of each
+// node's heaviest in-edges the first whose start has the largest score. Only
+// nodes whose heaviest weight is tied need scores to choose, so: take the first
+// heaviest edge everywhere, sum the scores along the chosen edges by pointer
+// jumping, let the tied nodes choose again with those scores, and repeat until
+// no choice changes. Choices that agree with the scores they give are the serial
+// ones (by induction along the topological order). Serial after 12 rounds.
+//  pre: chosen edge per node; W: {ancestor, score up to it} words, 8 bytes a node.
+__device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap, unsigned char* sm, int sm_bytes, int lane) {
+    constexpr int CU = 4;
+    if (nn <= 2) {
+        int len = 0;
+        if (lane == 0) len = dg_consensus(g, nn, out, cap);
+        return __shfl_sync(0xffffffffu, len, 0);
+    }
+    // int2 per node; a slot's deg and stk arrays are not contiguous, so large graphs use the row arrays
+    int2* W = 8 * (size_t)nn <= (size_t)sm_bytes ? reinterpret_cast<int2*>(sm) : reinterpret_cast<int2*>(g.scratch8);
+    int32_t* pre = g.pre;
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(g.scratch8b);
+    int32_t* ties = g.csr_adj;
+    for (int u = lane; u < nn; u += 32) pre[u] = g.hin[u];
+    // edges that tie with their end node's heaviest (list order is edge order: hin is the first)
+    int nt = 0;
+    for (int e0 = 0; e0 < ne; e0 += 32 * CU) {
+        int v[CU], w[CU], h[CU];
+#pragma unroll
+        for (int q = 0; q < CU; q++) {
+            const int e = e0 + 32 * q + lane;
+            v[q] = e < ne ? g.e_to[e] : 0;
+            w[q] = e < ne ? g.e_w[e] : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < CU; q++) h[q] = w[q] >= 0 ? g.hin[v[q]] : -1;
+#pragma unroll
+        for (int q = 0; q < CU; q++) {
+            const int e = e0 + 32 * q + lane;
+            const bool tie = h[q] >= 0 && h[q] != e && g.e_w[h[q]] == w[q];
+            const unsigned msk = __ballot_sync(0xffffffffu, tie);
+            if (tie) ties[nt + __popc(msk & ((1u << lane) - 1u))] = e;
+            nt += __popc(msk);
+        }
+    }
+    __syncwarp();
+    bool settled = false;
+    for (int round = 0; round < 12 && !settled; round++) {
+        for (int u0 = lane; u0 < nn; u0 += 32 * CU) {
+            int e[CU], f[CU], w[CU];
+#pragma unroll
+            for (int q = 0; q < CU; q++) e[q] = u0 + 32 * q < nn ? pre[u0 + 32 * q] : -1;
+#pragma unroll
+            for (int q = 0; q < CU; q++) {
+                f[q] = e[q] >= 0 ? g.e_from[e[q]] : -1;
+                w[q] = e[q] >= 0 ? g.e_w[e[q]] : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < CU; q++)
+                if (u0 + 32 * q < nn) W[u0 + 32 * q] = make_int2(f[q], w[q]);
+        }
+        __syncwarp();
+        for (int it = 0; it < 40; it++) {
+            bool moved = false;
+            for (int u0 = lane; u0 < nn; u0 += 32 * CU) {
+                int2 x[CU], a[CU];
+#pragma unroll
+                for (int q = 0; q < CU; q++) x[q] = u0 + 32 * q < nn ? W[u0 + 32 * q] : make_int2(-1, 0);
+#pragma unroll
+                for (int q = 0; q < CU; q++) a[q] = x[q].x >= 0 ? W[x[q].x] : make_int2(-1, 0);
+#pragma unroll
+                for (int q = 0; q < CU; q++)
+                    if (x[q].x >= 0) {
+                        W[u0 + 32 * q] = make_int2(a[q].x, a[q].y + x[q].y);
+                        moved = true;
+                    }
+            }
+            __syncwarp();
+            if (!__any_sync(0xffffffffu, moved)) break;
+        }
+        // tied nodes choose: the largest score, then the first edge
+        bool changed = false;
+        for (int t = lane; t < nt; t += 32) {
+            const int v = g.e_to[ties[t]], h = g.hin[v];
+            key[v] = ((unsigned long long)(uint32_t)W[g.e_from[h]].y << 32) | (uint32_t)(0x7fffffff - h);
+        }
+        __syncwarp();
+        for (int t = lane; t < nt; t += 32) {
+            const int e = ties[t];
+            atomicMax(&key[g.e_to[e]], ((unsigned long long)(uint32_t)W[g.e_from[e]].y << 32) | (uint32_t)(0x7fffffff - e));
+        }
+        __syncwarp();
+        for (int t = lane; t < nt; t += 32) {
+            const int v = g.e_to[ties[t]], e = 0x7fffffff - (int)(uint32_t)__ldcg(&key[v]);
+            if (pre[v] != e) changed = true;
+        }
+        __syncwarp();
+        for (int t = lane; t < nt; t += 32) {
+            const int v = g.e_to[ties[t]];
+            pre[v] = 0x7fffffff - (int)(uint32_t)__ldcg(&key[v]);
+        }
+        __syncwarp();
+        settled = !__any_sync(0xffffffffu, changed);
+    }
+    int len = 0;
+    if (!settled) {
+        if (lane == 0) len = dg_consensus(g, nn, out, cap);
+        return __shfl_sync(0xffffffffu, len, 0);
+    }
+    // the path back from the sink, then its bases
+    for (int u0 = lane; u0 < nn; u0 += 32 * CU) {
+        int e[CU];
+#pragma unroll
+        for (int q = 0; q < CU; q++) e[q] = u0 + 32 * q < nn ? pre[u0 + 32 * q] : -1;
+#pragma unroll
+        for (int q = 0; q < CU; q++)
+            if (u0 + 32 * q < nn) W[u0 + 32 * q].x = e[q] >= 0 ? g.e_from[e[q]] : 0;
+    }
+    __syncwarp();
+    int32_t* path = g.stk;
+    if (lane == 0)
+        for (int id = W[1].x; id != 0; id = W[id].x) path[len++] = id;
+    len = __shfl_sync(0xffffffffu, len, 0);
+    __syncwarp();
+    if (len > cap) return -1;
+    for (int i = lane; i < len; i += 32) {
+        const int b = g.base[path[i]];
+        out[len - 1 - i] = b == 0 ? 'A' : b == 1 ? 'C' : b == 2 ? 'G' : b == 3 ? 'T' : 'N';
+    }
+    return len;
+}
+
 // Sequential fusion of one backtrack path (lane 0): the reference's order of
 // node creation and edge insertion, one element at a time.
 __device__ int dg_fuse_seq(DevGraph& g, const int32_t* moves, int nm, int beg_i) {
@@ -390,19 +522,43 @@ __device__ int dg_fuse_warp(DevGraph& g, const int32_t* moves, int nm, int beg_i
     // edges: pair t joins path[t] -> path[t+1] (the last one -> sink)
     int new_edges = 0;
     bool efull = false;
+    constexpr int FU = 4;  // chunks whose edges are looked up together
+    int us[FU], vs[FU], fs[FU];
     for (int c0 = 0; c0 < nm; c0 += 32) {
-        const int t = c0 + lane;
-        int u = -1, v = -1, found = -1;
-        bool need = false;
-        if (t < nm) {
-            u = path[t];
-            v = t + 1 < nm ? path[t + 1] : 1;
-            if (u != v) {
-                for (int e = g.out_head[u]; e >= 0; e = g.e_nout[e])
-                    if (g.e_to[e] == v) { found = e; break; }
-                need = found < 0;
+        const int t = c0 + lane, f = (c0 >> 5) % FU;
+        if (f == 0) {
+            int e[FU];
+#pragma unroll
+            for (int q = 0; q < FU; q++) {
+                const int x = t + 32 * q;
+                us[q] = x < nm ? path[x] : -1;
+                vs[q] = x < nm ? (x + 1 < nm ? path[x + 1] : 1) : -1;
+                fs[q] = -1;
+            }
+#pragma unroll
+            for (int q = 0; q < FU; q++) e[q] = us[q] != vs[q] ? g.out_head[us[q]] : -1;
+            bool more = true;
+            while (more) {
+                more = false;
+                int to[FU], nx[FU];
+#pragma unroll
+                for (int q = 0; q < FU; q++) {
+                    to[q] = e[q] >= 0 ? g.e_to[e[q]] : -1;
+                    nx[q] = e[q] >= 0 ? g.e_nout[e[q]] : -1;
+                }
+#pragma unroll
+                for (int q = 0; q < FU; q++) {
+                    if (e[q] >= 0 && to[q] == vs[q]) { fs[q] = e[q]; nx[q] = -1; }
+                    e[q] = nx[q];
+                    more |= nx[q] >= 0;
+                }
             }
         }
+        int u = -1, v = -1, found = -1;
+#pragma unroll
+        for (int q = 0; q < FU; q++)
+            if (f == q) { u = us[q]; v = vs[q]; found = fs[q]; }
+        const bool need = u != v && found < 0;
         const unsigned msk = __ballot_sync(0xffffffffu, need);
         if (t < nm && u != v) {
             g.ind[v]++;
@@ -621,6 +777,71 @@ __device__ int kahn_lifo(const P* optr, const A* adj, uint8_t* deg, uint16_t* or
     return nr;
 }
 
+__device__ __forceinline__ int lds_u16(unsigned a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ int lds_u8(unsigned a) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return (int)v;
+}
+__device__ __forceinline__ void sts_u16(unsigned a, int v) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
+}
+__device__ __forceinline__ void sts_u8(unsigned a, int v) {
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// kahn_lifo over 16-bit lists in shared memory, by their shared-memory
+// addresses: the loop is a serial chain, so every instruction of it counts
+// (with generic pointers 425 cycles a node).
+__device__ int kahn_lifo_shared(unsigned optr, unsigned adj, unsigned deg, unsigned ord, int nn, int sp, int lane) {
+    int nr = 0, top = nn - sp, u = -1, k = 0, k1 = 0;
+    const unsigned above = 0xfffffffeu << lane;  // the lanes above this one
+    while (true) {
+        if (u < 0) {
+            if (top == nn) break;
+            u = lds_u16(ord + 2 * top);
+            top++;
+            k = lds_u16(optr + 2 * u);
+            k1 = lds_u16(optr + 2 * u + 2);
+        }
+        sts_u16(ord + 2 * nr, u);  // every lane, the same word
+        nr++;
+        u = -1;
+        int n0 = 0, n1 = 0;
+        for (; k < k1; k += 32) {
+            // lanes beyond the list repeat its last entry, without effect
+            const bool has = k + lane < k1;
+            const int v = lds_u16(adj + 2 * min(k + lane, k1 - 1));
+            const int dv = lds_u8(deg + v) - 1;
+            const int v0 = lds_u16(optr + 2 * v), v1 = lds_u16(optr + 2 * v + 2);
+            const unsigned msk = __ballot_sync(0xffffffffu, has && dv == 0);
+            if (has) sts_u8(deg + v, dv);
+            if (!msk) continue;
+            if (u >= 0) {  // ready in the chunk before (more than 32 out-edges)
+                top--;
+                sts_u16(ord + 2 * top, u);
+            }
+            const int last = 31 - __clz(msk);
+            const unsigned rest = msk ^ (1u << last);
+            if (rest) {
+                top -= __popc(rest);
+                if ((rest >> lane) & 1u) sts_u16(ord + 2 * (top + __popc(rest & above)), v);
+                __syncwarp();
+            }
+            u = __shfl_sync(0xffffffffu, v, last);
+            n0 = __shfl_sync(0xffffffffu, v0, last);
+            n1 = __shfl_sync(0xffffffffu, v1, last);
+        }
+        k = n0;
+        k1 = n1;
+    }
+    return nr;
+}
+
 // Topological sort with the whole warp: out-lists as CSR (16 bits in shared
 // memory; 32 bits in the slot's view arrays for graphs that do not fit), the
 // Kahn loop on lane 0, ranks written in parallel, then hlen/tlen
@@ -660,7 +881,8 @@ __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uin
         seeds += __popc(msk);
     }
     __syncwarp();
-    const int nr = small ? kahn_lifo(optr, adj, deg, ord, nn, seeds, lane)
+    auto sa = [](const void* p) { return (unsigned)__cvta_generic_to_shared(p); };
+    const int nr = small ? kahn_lifo_shared(sa(optr), sa(adj), sa(deg), sa(ord), nn, seeds, lane)
                          : kahn_lifo(g.csr_ptr, g.csr_adj, deg, ord, nn, seeds, lane);
     if (lane == 0) g.hdr[3] = nr;
     __syncwarp();
@@ -1080,13 +1302,13 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
             dg_topsort_warp(g, g.hdr[0], g.hdr[1], lens, (uint16_t*)wsm, A.smem_per_warp, lane);
         tick(PH_SORT);
     }
+    int len = -1;
+    if (status == ST_OK)
+        len = dg_consensus_warp(g, g.hdr[0], g.hdr[1], A.cons + (int64_t)w * A.cons_stride, A.cons_stride, wsm,
+                                A.smem_per_warp, lane);
+    tick(PH_CONS);
     if (lane == 0) {
-        int len = -1;
-        if (status == ST_OK) {
-            len = dg_consensus(g, g.hdr[0], A.cons + (int64_t)w * A.cons_stride, A.cons_stride);
-            if (len < 0) status = ST_CAPACITY;
-        }
-        tick(PH_CONS);
+        if (status == ST_OK && len < 0) status = ST_CAPACITY;
         A.cons_len[w] = len < 0 ? 0 : len;
         A.status[w] = status;
     }
@@ -1454,27 +1676,29 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     const int per_sm = std::max(1, std::min(blocks_per_sm, occ));
     int blocks = sms * per_sm;
     if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
-    // and the slots must fit the device-memory budget (75 % of what is free, counting our own slots)
-    size_t free_b = 0, total_b = 0;
-    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-    const size_t budget = (size_t)(0.75 * (double)(free_b + d_slots_cap_));
-    if (headroom > 1.0) {
-        // planned capacities: grow every slot by up to `headroom` while every resident
-        // warp still gets one, so a window a little beyond the plan still fits
-        const int want = std::max(1, std::min(blocks, (count + warps - 1) / warps));
-        const double fit = 0.97 * (double)budget / ((double)want * warps * (double)L_planned.bytes);
-        const double h = std::min(headroom, fit);
-        if (h > 1.0) {
-            const int32_t NCh = (int32_t)std::min<double>(60000.0, std::max(64.0, NC * h));
-            const int64_t sth = ((int64_t)(store * h) + 4095) / 4096 * 4096;
-            L = make_layout(NCh, 3 * NCh, QC, sth, stat, adaptive, wide, team);
+    blocks = std::max(1, std::min(blocks, (count + warps - 1) / warps));
+    auto planned = [&](double h) {
+        // planned capacities grown by `h`, so a window a little beyond the plan still fits
+        const int32_t NCh = (int32_t)std::min<double>(60000.0, std::max(64.0, NC * h));
+        const int64_t sth = ((int64_t)(store * h) + 4095) / 4096 * 4096;
+        return make_layout(NCh, 3 * NCh, QC, sth, stat, adaptive, wide, team);
+    };
+    if (headroom > 1.0) L = planned(headroom);
+    if ((size_t)L.bytes * blocks * warps > d_slots_cap_) {
+        // the slots must fit the device-memory budget: 75 % of what is free, counting our own
+        size_t free_b = 0, total_b = 0;
+        cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+        const size_t budget = (size_t)(0.75 * (double)(free_b + d_slots_cap_));
+        if (headroom > 1.0) {
+            // no more headroom than leaves every resident warp a slot
+            const double fit = 0.97 * (double)budget / ((double)blocks * warps * (double)L_planned.bytes);
+            const double h = std::min(headroom, fit);
+            L = h > 1.0 ? planned(h) : L_planned;
         }
+        const int64_t max_by_mem = (int64_t)(budget / (size_t)L.bytes) / warps;
+        if (max_by_mem < 1) throw std::runtime_error("not enough device memory for one batch slot");
+        blocks = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, max_by_mem));
     }
-    const int64_t max_by_mem = (int64_t)(budget / (size_t)L.bytes) / warps;
-    if (max_by_mem < 1) throw std::runtime_error("not enough device memory for one batch slot");
-    blocks = (int)std::min<int64_t>(blocks, max_by_mem);
-    blocks = std::min(blocks, (count + warps - 1) / warps);
-    blocks = std::max(blocks, 1);
     const int64_t slots = (int64_t)blocks * warps;
     const size_t slot_total = (size_t)(slots * L.bytes);
     if (slot_total > d_slots_cap_) {
