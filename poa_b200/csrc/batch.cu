@@ -1639,7 +1639,16 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     SlotLayout L = make_layout(NC, EC, QC, store, stat, adaptive, wide, team);
     const SlotLayout L_planned = L;
     const int warps = team ? 1 : warps_per_block;  // windows per block
-    const int smem_w = team ? tk.smem : shared_per_warp(count, warps, sms);
+    int per_sm_max = blocks_per_sm;
+    int smem_w = team ? tk.smem : shared_per_warp(count, warps, sms);
+    // a full GPU of short static-band windows: 4 blocks per SM with 13.75 KB a warp (8,000
+    // polishing windows 225 ms; 3 blocks with 18 KB 240, 5 with 11 KB 256), as long as the
+    // ring keeps 8 rows
+    if (stat && !smem_set && !blocks_set && count > 3 * warps * sms &&
+        8 * ring_blocks * BLK * cell_bytes + (int)qs_bytes(QC) + 16 + 1792 <= 14080) {
+        per_sm_max = 4;
+        smem_w = 14080;
+    }
     const size_t dyn = (size_t)warps * smem_w;
     const int threads = team ? tk.threads : warps * 32;
     const int qsm_bytes = (int)((qs_bytes(QC) + 15) / 16 * 16);
@@ -1667,13 +1676,13 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     if (stat_rows < 2) stat_rows = 0;
     int occ = 0;
     // windows that leave two blocks to an SM run the build with twice the registers
-    const int want_per_sm = std::min<int64_t>(blocks_per_sm, ((int64_t)(count + warps - 1) / warps + sms - 1) / sms);
+    const int want_per_sm = std::min<int64_t>(per_sm_max, ((int64_t)(count + warps - 1) / warps + sms - 1) / sms);
     const BatchKernel kern = team ? tk.kern : batch_kernel(stat, wide, want_per_sm);
     if (!team && warps != 4) throw std::invalid_argument("batch kernel is built for 4 warps per block");
     cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn), "smem attr");
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, dyn), "occupancy");
     // every block must be resident at once (persistent kernel): never more than the occupancy allows
-    const int per_sm = std::max(1, std::min(blocks_per_sm, occ));
+    const int per_sm = std::max(1, std::min(per_sm_max, occ));
     int blocks = sms * per_sm;
     if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
     blocks = std::max(1, std::min(blocks, (count + warps - 1) / warps));

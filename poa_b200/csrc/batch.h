@@ -95,6 +95,7 @@ class BatchEngine {
     int32_t warps_per_block = 4;
     int32_t blocks_per_sm = 3;  // 3: 168-register build; 4: 128; >= 5: 96 (occupancy still caps it)
     int32_t smem_per_warp = 18432;  // shared-memory row ring + staging / topsort workspace per warp
+    bool blocks_set = false;        // blocks_per_sm was configured: used as it is
     bool smem_set = false;          // smem_per_warp was configured: used as it is
     int32_t team_windows_per_sm = 5;  // adaptive band: up to this many windows per SM run as teams of warps
     int32_t max_blocks = 0;         // cap on the persistent grid (0 = one wave of resident blocks)

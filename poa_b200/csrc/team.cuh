@@ -119,12 +119,12 @@ template <> struct Cells<false> {
     static __device__ __forceinline__ int32_t lds_m(unsigned a) { return lds32(a) >> 8; }
     static __device__ __forceinline__ int32_t load_m(const void* p) { return *reinterpret_cast<const int32_t*>(p) >> 8; }
     __device__ __forceinline__ int32_t m(int l) const { return c[l] >> 8; }
-    // the vertical term max(M + o1, D + e1)
+    // vertical terms are kept less o1: max(M + o1, D + e1) - o1
     __device__ __forceinline__ int32_t v(int l, const CellK& k) const {
-        return (c[l] >> 8) + (int32_t)((uint32_t)c[l] & k.qmask) + k.o1;
+        return (c[l] >> 8) + (int32_t)((uint32_t)c[l] & k.qmask);
     }
-    __device__ __forceinline__ void set(int l, int32_t M, int32_t D, const CellK& k) {
-        c[l] = (int32_t)((uint32_t)M << 8) + mx(D - M + k.gq, 0);
+    __device__ __forceinline__ void set(int l, int32_t M, int32_t V, const CellK& k) {
+        c[l] = (int32_t)((uint32_t)M << 8) + mx(V - M + (k.gq + k.o1), 0);
     }
     // one cell of the row store, for the backtrack
     struct One {
@@ -169,10 +169,8 @@ template <> struct Cells<true> {
     static __device__ __forceinline__ int32_t lds_m(unsigned a) { return lds32(a); }
     static __device__ __forceinline__ int32_t load_m(const void* p) { return *reinterpret_cast<const int32_t*>(p); }
     __device__ __forceinline__ int32_t m(int l) const { return M_[l]; }
-    __device__ __forceinline__ int32_t v(int l, const CellK& k) const {
-        return mx(add32(M_[l], k.o1), add32(D_[l], k.e1));
-    }
-    __device__ __forceinline__ void set(int l, int32_t M, int32_t D, const CellK&) { M_[l] = M; D_[l] = D; }
+    __device__ __forceinline__ int32_t v(int l, const CellK& k) const { return mx(M_[l], D_[l] + (k.e1 - k.o1)); }
+    __device__ __forceinline__ void set(int l, int32_t M, int32_t V, const CellK& k) { M_[l] = M; D_[l] = V + k.o1; }
     struct One {
         int32_t M, D;
         static __device__ __forceinline__ One lds(unsigned a) { return One{lds32(a), lds32(a + 4)}; }
@@ -402,15 +400,20 @@ struct TeamRow {
     uint32_t qw = 0;                // query codes of the thread's columns
     int qn = 4;                     // code of the column after them (adaptive band)
     // the row before, when it fits the team's columns: band, this thread's M and vertical
-    // terms (NEG outside the band), M left of the thread's columns
+    // terms (VNEG outside the band), M left of the thread's columns
     int pBs = 0, pspan = -1;
-    int32_t pm[4] = {C::NEG, C::NEG, C::NEG, C::NEG}, pe[4] = {C::NEG, C::NEG, C::NEG, C::NEG}, pleft = C::NEG;
+    const int32_t VNEG;             // NEG_INF as a vertical term (less o1)
+    int32_t pm[4], pe[4], pleft = C::NEG;
     unsigned xp = 0;                // byte offset of the published summaries' half in use
 
     __device__ TeamRow(char* sm, const TeamJob& job)
         : a(job), k(job.k), store(job.store), sb((unsigned)__cvta_generic_to_shared(sm)),
           own(threadIdx.x * S::CELLB), leftw((threadIdx.x == 0 ? 32 * W : threadIdx.x) * S::CELLB - C::BYTES),
-          lane(threadIdx.x & 31), wid(threadIdx.x >> 5), K(add32(add32(C::NEG, job.k.e1), -job.k.o1)) {}
+          lane(threadIdx.x & 31), wid(threadIdx.x >> 5), K(add32(add32(C::NEG, job.k.e1), -job.k.o1)),
+          VNEG(C::NEG - job.k.o1) {
+#pragma unroll
+        for (int l = 0; l < 4; l++) { pm[l] = NEG; pe[l] = VNEG; }
+    }
 
     __device__ __forceinline__ void take_strip(int s) {
         s_cur = s;
@@ -422,7 +425,7 @@ struct TeamRow {
         if (ADAPT) qn = in ? a.qs[col0 + 4] : 4;
         // the row before had other columns here, if any
 #pragma unroll
-        for (int l = 0; l < 4; l++) pm[l] = pe[l] = NEG;
+        for (int l = 0; l < 4; l++) { pm[l] = NEG; pe[l] = VNEG; }
     }
 
     // diagonal terms of one predecessor: m its M, left the M before them
@@ -499,7 +502,7 @@ struct TeamRow {
 #pragma unroll
         for (int l = 0; l < 4; l++) {
             pm[l] = M[l];
-            pe[l] = act ? mx(add32(M[l], k.o1), add32(V[l], k.e1)) : NEG;
+            pe[l] = act ? mx(M[l], add32(V[l], k.e1)) : VNEG;
         }
         pleft = __shfl_up_sync(0xffffffffu, M[3], 1);
         if (lane == 0) pleft = edge;
@@ -525,13 +528,13 @@ struct TeamRow {
         int32_t P[4], V[4], H[4], key[4], ex = LOW, base = 0;
         if (on) {
 #pragma unroll
-            for (int l = 0; l < 4; l++) P[l] = V[l] = NEG;
+            for (int l = 0; l < 4; l++) { P[l] = NEG; V[l] = VNEG; }
             if (h.w & FR_PREV) {
                 // diag: the fill's block mask for the diagonal (src/align.cpp:1467)
                 const bool diag = (unsigned)(B - pBs) <= (unsigned)pspan && Bz > pBs;
                 diagonal(pm, first ? NEG : pleft, diag, qw ^ (((uint32_t)h.w >> FR_PBASE & 7u) * 0x01010101u), P);
 #pragma unroll
-                for (int l = 0; l < 4; l++) V[l] = mx(NEG, pe[l]);
+                for (int l = 0; l < 4; l++) V[l] = mx(VNEG, pe[l]);
             }
             if (d > 0) __syncwarp();  // the ring's words of the lanes to the left
             for (int e = 0; e < d; e++) {
@@ -557,7 +560,7 @@ struct TeamRow {
                 fold(pc, left, diag, qw ^ (uint32_t)er.y, P, V);
             }
 #pragma unroll
-            for (int l = 0; l < 4; l++) H[l] = mx(P[l], V[l]);
+            for (int l = 0; l < 4; l++) H[l] = mx(P[l], add32(V[l], k.o1));
             if (ADAPT) {
                 int4 best = make_int4(INT_MIN, 0, 0, 0);
                 maximum(act, H, best);
@@ -584,7 +587,7 @@ struct TeamRow {
             keep(i, h, act, H, V, rel, edge);
         } else {
 #pragma unroll
-            for (int l = 0; l < 4; l++) pe[l] = NEG;
+            for (int l = 0; l < 4; l++) pe[l] = VNEG;
         }
         xp ^= W * 16;
     }
@@ -610,7 +613,7 @@ struct TeamRow {
                 act = B >= Bs && B <= Bs + h.y;
                 rel = col0 - Bs * BLK;
 #pragma unroll
-                for (int l = 0; l < 4; l++) P[l] = V[l] = NEG;
+                for (int l = 0; l < 4; l++) { P[l] = NEG; V[l] = VNEG; }
                 if (i == 0 && col0 == 0) P[0] = 0;
                 for (int e = 0; e < d; e++) {
                     const int4 fe = ed[e];
@@ -627,7 +630,7 @@ struct TeamRow {
                     fold(pc, left, diag, qw ^ (uint32_t)((fe.x & 7) * 0x01010101), P, V);
                 }
 #pragma unroll
-                for (int l = 0; l < 4; l++) H[l] = mx(P[l], V[l]);
+                for (int l = 0; l < 4; l++) H[l] = mx(P[l], add32(V[l], k.o1));
                 base = -rel * k.e1;
                 publish(act, H, base, key, ex);
                 if (ADAPT) maximum(act, H, best);
@@ -653,7 +656,7 @@ struct TeamRow {
                 }
             } else {
 #pragma unroll
-                for (int l = 0; l < 4; l++) pe[l] = NEG;
+                for (int l = 0; l < 4; l++) pe[l] = VNEG;
             }
             xp ^= W * 16;
         }

@@ -66,7 +66,7 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
             act[u] = b <= span;
             qw[u] = act[u] ? *reinterpret_cast<const uint2*>(qs + (int64_t)(Bs + b) * BLK) : make_uint2(0x04040404u, 0x04040404u);
 #pragma unroll
-            for (int l = 0; l < 8; l++) H[u][l] = V[u][l] = NEG;
+            for (int l = 0; l < 8; l++) { H[u][l] = NEG; V[u][l] = NEG - k.o1; }
             if (i == 0 && Bs + b == 0) H[u][0] = 0;
         }
         for (int e = 0; e < d; e++) {
@@ -115,10 +115,10 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
 #pragma unroll
         for (int u = 0; u < U; u++) {
 #pragma unroll
-            for (int l = 0; l < 8; l++) H[u][l] = mx(H[u][l], V[u][l]);
-            int32_t t = add32(H[u][0], k.o1);
+            for (int l = 0; l < 8; l++) H[u][l] = mx(H[u][l], add32(V[u][l], k.o1));
+            int32_t t = add32(H[u][0], open);
 #pragma unroll
-            for (int l = 1; l < 8; l++) t = mx(add32(t, k.e1), add32(H[u][l], k.o1));
+            for (int l = 1; l < 8; l++) t = mx(add32(t, k.e1), add32(H[u][l], open));
             out[u] = act[u] ? t - ((c0 + 32 * u + lane + 1) * BLK) * k.e1 : LOW;
             if (ARGMAX) {
                 // the first maximum of H0 is the row's first maximum (a gap never exceeds the cell it opens from)
