@@ -78,7 +78,7 @@ SlotLayout make_layout(int32_t NC, int32_t EC, int32_t QC, int64_t store_bytes, 
         L.v_ra = take(32 * (size_t)NC);
     }
     L.state = take(adaptive ? 32 * (size_t)NC : 64);
-    L.qs = take((size_t)qs_bytes(QC) + 64);
+    L.qs = take(3 * (size_t)qs_bytes(QC) / 2 + 96);  // bytes, then nibbles
     L.moves = take(4 * ((size_t)NC + QC + 16));
     L.path = take(4 * ((size_t)NC + QC + 16));
     L.store = take((size_t)L.store_cap * bb);
@@ -1047,8 +1047,8 @@ __device__ int build_rows(DevGraph& g, char* s, const BatchArgs& A, int m, int w
             if (STATIC) {
                 const int p = v.x >> 4;
                 const bool near = x[q].w - p < R && pr[q].y - pr[q].x - 1 <= RB;
-                fe[at] = make_int4(near ? (p & (R - 1)) * RB * BB : ~pr[q].z, (v.x & 7) * 0x01010101, pr[q].x,
-                                   pr[q].y - 2 - pr[q].x);
+                const int2 band = rec_band(pr[q].x, pr[q].y);
+                fe[at] = make_int4(near ? (p & (R - 1)) * (RB + 2) * BB : ~pr[q].z, row_score<WIDE>(A.k, v.x & 7), band.x, band.y);
                 v.y = pr[q].x; v.z = pr[q].y; v.w = pr[q].z;
             }
             ed[at] = v;
@@ -1179,7 +1179,22 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         if (STATIC && st != ST_OK) { status = st; break; }
         uint8_t* qs = (uint8_t*)(s + L.qs);
         const int64_t qsb = qs_bytes(len);
-        for (int64_t x = lane; x < qsb; x += 32) qs[x] = (x >= 2 && x < len + 2) ? nt4_dev(rd[x - 2]) : 4;
+        // the query's codes as bytes, and as nibbles (eight columns a word) for the warp fill
+        uint32_t* qn = (uint32_t*)(qs + ((qsb + 15) & ~(int64_t)15));
+        for (int64_t x0 = 8 * (int64_t)lane; x0 < qsb; x0 += 8 * 32) {
+            uint32_t lo = 0, hi = 0, nib = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int64_t x = x0 + q;
+                const uint32_t c = (x >= 2 && x < len + 2) ? nt4_dev(rd[x - 2]) : 4u;
+                if (q < 4) lo |= c << (8 * q);
+                else hi |= c << (8 * (q - 4));
+                nib |= c << (4 * q);
+            }
+            *reinterpret_cast<uint2*>(qs + x0) = make_uint2(lo, hi);
+            qn[x0 >> 3] = nib;
+        }
+        const int64_t qnb = ((qsb >> 1) + 15) & ~(int64_t)15;
         if (lane == 0) {
             a.n = n;
             a.qlen = len;
@@ -1208,24 +1223,24 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         if constexpr (STATIC) {
             // shared memory: row ring, query, staged rows
             const WarpRing ring{(unsigned)__cvta_generic_to_shared(wsm), A.sring_rows, A.sring_rows ? A.sring_blocks : 0, -1};
-            uint8_t* qsm = wsm + (size_t)A.sring_rows * A.sring_blocks * BLK * Cells<WIDE>::BYTES;
-            for (int64_t x = lane * 16; x < qsb; x += 32 * 16)
-                *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>(qs + x);
+            unsigned char* qsm = wsm + (size_t)A.sring_rows * (A.sring_rows ? A.sring_blocks + 2 : 0) * BLK * Cells<WIDE>::BYTES;
+            for (int64_t x = lane * 16; x < qnb; x += 32 * 16)
+                *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>((const char*)qn + x);
             __syncwarp();
-            warp_fill_static<WIDE>(a, ring, qsm, qsm + ((qsb + 15) & ~(int64_t)15), lane);
+            warp_fill_static<WIDE>(a, ring, (const uint32_t*)qsm, qsm + qnb, lane);
         } else if constexpr (TEAM > 0) {
             bar_sync<4, 32 * (TEAM + 2)>();  // the job
             st = team_fill_adaptive<TEAM, WIDE, TEAM_RING>(a, (char*)wsm, cells);
         } else {
             // shared memory: staged records, state window, and the query when it fits
-            const uint8_t* qf = qs;
+            const uint32_t* qf = qn;
             int64_t used = WED * 16 + warp_state_bytes(A.state_rows);
-            if (used + qsb <= A.smem_per_warp) {
-                uint8_t* qsm = wsm + used;
-                for (int64_t x = lane * 16; x < qsb; x += 32 * 16)
-                    *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>(qs + x);
-                qf = qsm;
-                used += (qsb + 15) & ~(int64_t)15;
+            if (used + qnb <= A.smem_per_warp) {
+                unsigned char* qsm = wsm + used;
+                for (int64_t x = lane * 16; x < qnb; x += 32 * 16)
+                    *reinterpret_cast<uint4*>(qsm + x) = *reinterpret_cast<const uint4*>((const char*)qn + x);
+                qf = (const uint32_t*)qsm;
+                used += qnb;
             }
             __syncwarp();
             st = warp_fill_dyn<WIDE, U>(a, A.f > 0 && A.ab_band, wsm, A.state_rows, wsm + used,
@@ -1645,13 +1660,14 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     // polishing windows 225 ms; 3 blocks with 18 KB 240, 5 with 11 KB 256), as long as the
     // ring keeps 8 rows
     if (stat && !smem_set && !blocks_set && count > 3 * warps * sms &&
-        8 * ring_blocks * BLK * cell_bytes + (int)qs_bytes(QC) + 16 + 1792 <= 14080) {
+        8 * (ring_blocks + 2) * BLK * cell_bytes + (int)qs_bytes(QC) + 16 + 1792 <= 14080) {
         per_sm_max = 4;
         smem_w = 14080;
     }
     const size_t dyn = (size_t)warps * smem_w;
     const int threads = team ? tk.threads : warps * 32;
     const int qsm_bytes = (int)((qs_bytes(QC) + 15) / 16 * 16);
+    const int qn_bytes = (int)((qs_bytes(QC) / 2 + 15) / 16 * 16);  // the query as nibbles
     constexpr int kStageBytes = 1792;  // shared memory a static-band warp needs beside its query
     static_assert(kStageBytes >= WSTG_BYTES && kStageBytes >= BtTile<true, 4>::PER_ROW * 2 + 16, "stage and backtrack tile");
     if (stat && qsm_bytes + kStageBytes > smem_w)
@@ -1661,14 +1677,14 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     if (!stat && smem_w < kDynBytes) throw std::invalid_argument("smem_per_warp too small for the adaptive-band fill");
     if (smem_w % 16 != 0) throw std::invalid_argument("smem_per_warp must be a multiple of 16");
     // static band: shared-memory ring of 2 to 16 rows of ring_blocks blocks
-    const int row_bytes = ring_blocks * BLK * cell_bytes;
+    const int row_bytes = (ring_blocks + 2) * BLK * cell_bytes;
     int sring_rows = 16;
-    while (sring_rows >= 2 && sring_rows * row_bytes > smem_w - qsm_bytes - WSTG_BYTES) sring_rows /= 2;
+    while (sring_rows >= 2 && sring_rows * row_bytes > smem_w - qn_bytes - WSTG_BYTES) sring_rows /= 2;
     if (sring_rows < 2) sring_rows = 0;
     // dynamic bands: the largest state window that leaves room for the query, else the largest that fits
     int state_rows = 128;
-    while (state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) + qsm_bytes > smem_w) state_rows /= 2;
-    if (WED * 16 + warp_state_bytes(state_rows) + qsm_bytes > smem_w)
+    while (state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) + qn_bytes > smem_w) state_rows /= 2;
+    if (WED * 16 + warp_state_bytes(state_rows) + qn_bytes > smem_w)
         for (state_rows = 128; state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) > smem_w;) state_rows /= 2;
     // read statistics count spilled rows against a ring of 32 full-width rows (dynamic bands) or
     // of up to 8 rows of 64 bytes a block in the warp's shared memory (static band)

@@ -74,7 +74,15 @@ PB_HD bool cell_packable(const Scoring& s, int64_t n, int64_t m) {
         const int64_t a = v[k] < 0 ? -v[k] : v[k];
         if (a > big) big = a;
     }
-    return big < (1 << 20) && (n + m + 2) * big < (1 << 20) && (int64_t)s.e1 - s.o1 <= 255;
+    const bool bytes = s.match >= -128 && s.match <= 127 && s.mismatch >= -128 && s.mismatch <= 127;  // score_table
+    return bytes && big < (1 << 20) && (n + m + 2) * big < (1 << 20) && (int64_t)s.e1 - s.o1 <= 255;
+}
+
+// Scores of a predecessor's base against query codes 0..3, one byte each; code 4
+// (N) matches base 4 only, whose table is the mismatch in every byte.
+PB_HD uint32_t score_table(const CellK& k, int base) {
+    const uint32_t x = ((uint32_t)k.mismatch & 255u) * 0x01010101u;
+    return base < 4 ? x ^ ((((uint32_t)k.match ^ (uint32_t)k.mismatch) & 255u) << (8 * base)) : x;
 }
 
 constexpr int32_t PACK_NEG = -(1 << 22);
@@ -291,6 +299,12 @@ __device__ __forceinline__ int32_t scan_max(int32_t v) {
     return mx(v, __shfl_up_sync(0xffffffffu, v, 16));
 }
 
+// A predecessor's band as the fill's records hold it, {Bs, last block - Bs}: an
+// empty band as one block that no row reaches.
+__device__ __forceinline__ int2 rec_band(int Bs, int Be) {
+    return Be - 2 - Bs >= 0 ? make_int2(Bs, Be - 2 - Bs) : make_int2(1 << 29, 0);
+}
+
 __device__ __forceinline__ int strips_of(int Bs, int Be) { return ((Be - 2) >> 4) - (Bs >> 4) + 1; }
 
 // Static band: every row's band and place in the row store, its header for
@@ -361,8 +375,11 @@ __device__ int team_rows_static(const TeamJob& a, int64_t* s_part, unsigned long
             a.ed[e] = v;
             const bool lap1 = pr.y - pr.x - 1 > 0 && strips_of(pr.x, pr.y) <= W;
             if (lap1 && p == i - 1 && !(fl & FR_GENERAL)) fl += FR_PREV - 1 + ((v.x & 7) << FR_PBASE);
-            else a.fe[x++] = make_int4(lap1 && i - p < S::TR ? (p & (S::TR - 1)) * S::ROWB : ~pr.z, (v.x & 7) * 0x01010101, pr.x,
-                                      pr.y - 2 - pr.x);
+            else {
+                const int2 band = rec_band(pr.x, pr.y);
+                a.fe[x++] = make_int4(lap1 && i - p < S::TR ? (p & (S::TR - 1)) * S::ROWB : ~pr.z, (v.x & 7) * 0x01010101, band.x,
+                                      band.y);
+            }
         }
         a.fr[i] = make_int4(ri.x, ri.y - 2 - ri.x, ri.z, fl);
     }
@@ -933,7 +950,8 @@ __device__ void team_records(const TeamJob& a, char* smem) {
                 if (kk < dn && !((pmask >> lane) & 1u)) {
                     const int p = v.x >> 4, at = kk - (prev != 0 || (pmask & ((1u << lane) - 1u)) != 0);
                     const bool near = i + 1 - p < S::TR && v.z - v.y - 1 > 0 && strips_of(v.y, v.z) <= W;
-                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : ~v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+                    const int2 band = rec_band(v.y, v.z);
+                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : ~v.w, (v.x & 7) * 0x01010101, band.x, band.y);
                     if (at < HDR_E) o.ed[at] = f;
                     else fe[e0 + at] = f;
                 }

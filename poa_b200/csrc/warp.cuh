@@ -26,25 +26,49 @@ constexpr int WED = 32;                // an adaptive row's predecessor records 
 // shared memory of the adaptive fill: records, then the state window
 constexpr int warp_state_bytes(int rows) { return rows * SW_INTS * 4; }
 
+// Shared-memory copies of rows. A row's blocks lie between two blocks of
+// unreachable cells, so a lane outside a predecessor's band reads those instead
+// of taking another path.
 struct WarpRing {
     unsigned at;  // shared memory address
     int rows;     // static band: a power of two, or 0: no ring
-    int blocks;   // static band: per row
-    int cur;      // dynamic bands: the current row's first block, or -1: not kept
+    int blocks;   // static band: blocks per row
+    int cur;      // dynamic bands: the current row's first block (of its pads), or -1: not kept
 };
 enum { RING_STATIC = 1, RING_DYN = 2 };
+constexpr int warp_ring_row_blocks(int blocks) { return blocks + 2; }
 
-// One row. ed_at(e): {ring offset, or ~row-store block; base in every byte; Bs;
-// last block - Bs}. With ARGMAX, best / best_col become the row's first maximum.
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
+    return d;
+}
+// byte l of x, sign-extended
+template <int l>
+__device__ __forceinline__ int32_t sbyte(uint32_t x) { return (int32_t)prmt(x, x, 0x8880u + 0x1111u * l); }
+
+// The query for the warp fill: codes as nibbles, eight columns a word.
+// qcode: the code of one column.
+__device__ __forceinline__ int qcode(const uint32_t* qn, int col) { return (int)(qn[col >> 3] >> (4 * (col & 7))) & 15; }
+
+// a record's base as warp_row takes it
+template <bool WIDE>
+__device__ __forceinline__ int row_score(const CellK& k, int base) { return WIDE ? base : (int)score_table(k, base); }
+
+// One row. ed_at(e): {ring offset, or ~row-store block; base (WIDE) or score
+// table; Bs; last block - Bs}. With ARGMAX, best / best_col become the row's first maximum.
 // U chunks are taken together: a chunk is ~300 mostly dependent instructions, so
 // two of them in flight hide each other's latency where the registers allow it
 // (rows of several chunks, few warps per SM).
+//
+// The query codes are byte selectors: one PRMT turns a predecessor's score table
+// into the scores of four cells.
 //
 // The gap term of cell l is I[l] = max(I[l-1] + e1, H0[l-1] + o1): within a
 // block one dependent step per cell, first from nothing for the block's own
 // contribution, then from the prefix over the lanes.
 template <bool WIDE, int RING, bool ARGMAX, int U, class EdAt>
-__device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span, int tb, int d, const uint8_t* qs,
+__device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span, int tb, int d, const uint32_t* qn,
                                          const WarpRing& ring, char* store, int lane, EdAt ed_at, int32_t& best,
                                          int& best_col) {
     typedef Cells<WIDE> C;
@@ -58,13 +82,13 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
     const int32_t open = i == 0 && !WIDE ? BELOW : k.o1;
     for (int c0 = 0; c0 <= span; c0 += 32 * U) {
         int32_t H[U][8], V[U][8], out[U];
-        uint2 qw[U];
+        uint32_t qw[U];
         bool act[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int b = c0 + 32 * u + lane;
             act[u] = b <= span;
-            qw[u] = act[u] ? *reinterpret_cast<const uint2*>(qs + (int64_t)(Bs + b) * BLK) : make_uint2(0x04040404u, 0x04040404u);
+            qw[u] = qn[Bs + min(b, span)];
 #pragma unroll
             for (int l = 0; l < 8; l++) { H[u][l] = NEG; V[u][l] = NEG - k.o1; }
             if (i == 0 && Bs + b == 0) H[u][0] = 0;
@@ -74,25 +98,31 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
             C lo[U], hi[U];
             int32_t left0[U];  // lane 0: the cell before the chunk (NEG_INF before the row's first block)
             bool in[U];
+            if (er.x >= 0) {
+                const int plane = (RING == RING_STATIC ? ring.blocks + 2 : er.w + 3) * HB;
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int b = c0 + 32 * u + lane, pb = Bs + b - er.z;
-                in[u] = act[u] && (unsigned)pb <= (unsigned)er.w;
-                left0[u] = NEG;
-                const bool l0 = lane == 0 && c0 + u > 0 && in[u] && pb > 0;
-                if (er.x >= 0) {
-                    const unsigned src = ring.at + er.x + pb * HB;
-                    const int plane = (RING == RING_STATIC ? ring.blocks : er.w + 1) * HB;
-                    if (in[u]) { lo[u].lds(src); hi[u].lds(src + plane); }
-                    else { lo[u].none(); hi[u].none(); }
-                    if (l0) left0[u] = C::lds_m(src + plane - C::BYTES);
-                } else {
+                for (int u = 0; u < U; u++) {
+                    const int pb = Bs + c0 + 32 * u + lane - er.z;
+                    in[u] = (unsigned)pb <= (unsigned)er.w;
+                    const unsigned src = ring.at + er.x + (min(max(pb, -1), er.w + 1) + 1) * HB;
+                    lo[u].lds(src);
+                    hi[u].lds(src + plane);
+                    left0[u] = NEG;
+                    if (c0 + u > 0) left0[u] = C::lds_m(ring.at + er.x + plane + (min(max(pb - 1, -1), er.w + 1) + 1) * HB + HB - C::BYTES);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int pb = Bs + c0 + 32 * u + lane - er.z;
+                    in[u] = act[u] && (unsigned)pb <= (unsigned)er.w;
                     const char* src = store + ((int64_t)~er.x + pb) * BB;
+                    left0[u] = NEG;
                     if (in[u]) { lo[u].load(src); hi[u].load(src + HB); }
                     else { lo[u].none(); hi[u].none(); }
-                    if (l0) left0[u] = C::load_m(src - C::BYTES);
+                    if (lane == 0 && c0 + u > 0 && in[u] && pb > 0) left0[u] = C::load_m(src - C::BYTES);
                 }
             }
+            const uint32_t tabn = WIDE ? 0u : (uint32_t)(er.y == (int)score_table(k, 4) ? k.match : k.mismatch);
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int B = Bs + c0 + 32 * u + lane;
@@ -100,15 +130,27 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
                 const bool diag = in[u] && (B > er.z || B == 0);
                 int32_t left = __shfl_up_sync(0xffffffffu, hi[u].m(3), 1);
                 if (lane == 0) left = left0[u];
-                const int32_t sm = diag || WIDE ? k.match : -(1 << 23), sx = diag || WIDE ? k.mismatch : -(1 << 23);
-                const uint32_t x0 = qw[u].x ^ (uint32_t)er.y, x1 = qw[u].y ^ (uint32_t)er.y;
+                if (diag) {
+                    if constexpr (WIDE) {
 #pragma unroll
-                for (int l = 0; l < 8; l++) {
-                    const int32_t src = l == 0 ? left : l <= 4 ? lo[u].m(l > 0 ? l - 1 : 0) : hi[u].m(l - 5);
-                    const int32_t cand = src + (((l < 4 ? x0 : x1) & (255u << (8 * (l & 3)))) == 0 ? sm : sx);
-                    if (!WIDE || diag) H[u][l] = mx(H[u][l], cand);
-                    V[u][l] = mx(V[u][l], l < 4 ? lo[u].v(l & 3, k) : hi[u].v(l & 3, k));
+                        for (int l = 0; l < 8; l++) {
+                            const int32_t src = l == 0 ? left : l <= 4 ? lo[u].m(l > 0 ? l - 1 : 0) : hi[u].m(l - 5);
+                            H[u][l] = mx(H[u][l], src + ((int)((qw[u] >> (4 * l)) & 15u) == er.y ? k.match : k.mismatch));
+                        }
+                    } else {
+                        const uint32_t s0 = prmt((uint32_t)er.y, tabn, qw[u]), s1 = prmt((uint32_t)er.y, tabn, qw[u] >> 16);
+                        H[u][0] = mx(H[u][0], left + sbyte<0>(s0));
+                        H[u][1] = mx(H[u][1], lo[u].m(0) + sbyte<1>(s0));
+                        H[u][2] = mx(H[u][2], lo[u].m(1) + sbyte<2>(s0));
+                        H[u][3] = mx(H[u][3], lo[u].m(2) + sbyte<3>(s0));
+                        H[u][4] = mx(H[u][4], lo[u].m(3) + sbyte<0>(s1));
+                        H[u][5] = mx(H[u][5], hi[u].m(0) + sbyte<1>(s1));
+                        H[u][6] = mx(H[u][6], hi[u].m(1) + sbyte<2>(s1));
+                        H[u][7] = mx(H[u][7], hi[u].m(2) + sbyte<3>(s1));
+                    }
                 }
+#pragma unroll
+                for (int l = 0; l < 8; l++) V[u][l] = mx(V[u][l], l < 4 ? lo[u].v(l & 3, k) : hi[u].v(l & 3, k));
             }
         }
         // H0; what the block passes on by itself; the row's maximum
@@ -156,10 +198,22 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
             }
             if (act[u]) {
                 if (RING == RING_STATIC ? span < ring.blocks : ring.cur >= 0) {
-                    const unsigned at = RING == RING_STATIC ? (i & (ring.rows - 1)) * (unsigned)(ring.blocks * BB) : ring.cur * BB;
-                    const unsigned dst = ring.at + at + b * HB;
+                    const unsigned at = RING == RING_STATIC ? (i & (ring.rows - 1)) * (unsigned)((ring.blocks + 2) * BB) : ring.cur * BB;
+                    const unsigned dst = ring.at + at + (b + 1) * HB, plane = (RING == RING_STATIC ? ring.blocks + 2 : span + 3) * HB;
                     lo.sts(dst);
-                    hi.sts(dst + (RING == RING_STATIC ? ring.blocks : span + 1) * HB);
+                    hi.sts(dst + plane);
+                    if (b == span) {
+                        C pad;
+                        pad.none();
+                        pad.sts(dst + HB);
+                        pad.sts(dst + plane + HB);
+                    }
+                    if (RING == RING_DYN && b == 0) {  // (the static ring's are written once)
+                        C pad;
+                        pad.none();
+                        pad.sts(dst - HB);
+                        pad.sts(dst + plane - HB);
+                    }
                 }
                 char* dst = store + ((int64_t)tb + b) * BB;
                 lo.store(dst);
@@ -171,13 +225,20 @@ __device__ __forceinline__ void warp_row(const CellK& k, int i, int Bs, int span
 
 // Static band: rows and records staged WSTG rows at a time.
 template <bool WIDE>
-__device__ void warp_fill_static(const TeamJob& a, const WarpRing& ring, const uint8_t* qsm, unsigned char* stage, int lane) {
+__device__ void warp_fill_static(const TeamJob& a, const WarpRing& ring, const uint32_t* qsm, unsigned char* stage, int lane) {
     const int n = a.n;
     const CellK k = a.k;
     char* const store = a.store;
     const unsigned stg = (unsigned)__cvta_generic_to_shared(stage);
     int32_t bm = 0;
     int bc = 0;
+    {
+        // the blocks before the ring's rows
+        constexpr int HB = 4 * Cells<WIDE>::BYTES;
+        Cells<WIDE> pad;
+        pad.none();
+        for (int x = lane; x < 2 * ring.rows; x += 32) pad.sts(ring.at + x * (ring.blocks + 2) * HB);
+    }
     for (int i0 = 0; i0 < n; i0 += WSTG) {
         const int cnt = min(WSTG, n - i0);
         const int e0 = a.in_ptr[i0], ne = min(a.in_ptr[i0 + cnt] - e0, WSTG_E);
@@ -211,7 +272,7 @@ __device__ void warp_fill_static(const TeamJob& a, const WarpRing& ring, const u
 enum { SW_RPOS = 7, SW_RAT = 11 };  // a kept row: its position in the stream of kept blocks, its first block in the buffer
 template <bool WIDE, int U>
 __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm, int wrows, unsigned char* rbuf, int rcap,
-                             const uint8_t* qf, int lane, int64_t& cells_out) {
+                             const uint32_t* qf, int lane, int64_t& cells_out) {
     const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n];
     const CellK k = a.k;
     char* const store = a.store;
@@ -262,17 +323,17 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
         }
         // the row's place in the buffer: whole, so the end of the buffer may stay empty
         ring.cur = -1;
-        if (bn > 0 && bn <= rcap) {
-            if (rat + bn > rcap) { rpos += rcap - rat; rat = 0; }
+        if (bn > 0 && bn + 2 <= rcap) {
+            if (rat + bn + 2 > rcap) { rpos += rcap - rat; rat = 0; }
             ring.cur = rat;
-            rat += bn;
-            rpos += bn;
+            rat += bn + 2;
+            rpos += bn + 2;
         }
         if (lane == 0) {
             a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
             int32_t* w = slot(i);
             w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
-            w[SW_RPOS] = rpos - bn; w[SW_RAT] = ring.cur;
+            w[SW_RPOS] = rpos - bn - 2; w[SW_RAT] = ring.cur;
         }
         // row i's predecessor records; their slopes and maxima
         int psl = 0, pmp = INT_MIN / 2;
@@ -293,7 +354,8 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
                     v.y = q.x; v.z = q.y; v.w = q.z;
                     if (adaptive && k0 == 0) { psl = a.state[8 * (int64_t)p + SW_SL]; pmp = a.state[8 * (int64_t)p + SW_MP]; }
                 }
-                if (kk < WED) sed[kk] = make_int4(from >= 0 ? from * BB : ~v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+                const int2 band = rec_band(v.y, v.z);
+                if (kk < WED) sed[kk] = make_int4(from >= 0 ? from * BB : ~v.w, row_score<WIDE>(k, v.x & 7), band.x, band.y);
                 a.ed[ra0.x + kk] = v;
             }
         }
@@ -306,7 +368,8 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
         auto ed_at = [&](int e) {
             if (e < WED) return lds128(seda + e * 16);
             const int4 v = ed[e];
-            return make_int4(~v.w, (v.x & 7) * 0x01010101, v.y, v.z - 2 - v.y);
+            const int2 band = rec_band(v.y, v.z);
+            return make_int4(~v.w, row_score<WIDE>(k, v.x & 7), band.x, band.y);
         };
         int32_t best = INT_MIN;
         int acj = Bs * BLK;
@@ -322,7 +385,7 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
             if (i >= 1) {  // src/align.cpp:1516-1568
                 int sl_best = INT_MIN, max_slp = 0;
                 bool is_match = false;
-                if (ra1.y == (int)qf[acj + 1]) {  // cur.base == seq[max_acj]
+                if (ra1.y == qcode(qf, acj + 1)) {  // cur.base == seq[max_acj]
                     max_slp = psl;
                     sl_best = pmp + 1 == acj ? psl + 1 : INT_MIN;
                     for (int kk = 32 + lane; kk < d; kk += 32) {
