@@ -777,23 +777,6 @@ __device__ int kahn_lifo(const P* optr, const A* adj, uint8_t* deg, uint16_t* or
     return nr;
 }
 
-__device__ __forceinline__ int lds_u16(unsigned a) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ int lds_u8(unsigned a) {
-    uint32_t v;
-    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return (int)v;
-}
-__device__ __forceinline__ void sts_u16(unsigned a, int v) {
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
-}
-__device__ __forceinline__ void sts_u8(unsigned a, int v) {
-    asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-
 // kahn_lifo over 16-bit lists in shared memory, by their shared-memory
 // addresses: the loop is a serial chain, so every instruction of it counts
 // (with generic pointers 425 cycles a node).
@@ -1288,7 +1271,7 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         }
         tick(PH_FILL);
         int32_t nm = 0;
-        if (st == ST_OK) st = team_backtrack<WIDE, TEAM ? 8 : 4>(a, (char*)wsm, A.smem_per_warp, lane, nm);
+        if (st == ST_OK) st = team_backtrack<WIDE, TEAM ? 8 : 4, TEAM || U == 2>(a, (char*)wsm, A.smem_per_warp, lane, nm);
         if (lane == 0) {
             g.hdr[2] = st;
             g.hdr[13] = nm;

@@ -47,6 +47,8 @@
 // sub-windows 94 -> 33 ms. What is left is latency: ~215 mostly dependent
 // instructions per warp and row.
 #pragma once
+#include <type_traits>
+
 #include "plain.cuh"
 
 namespace pb {
@@ -103,6 +105,23 @@ __device__ __forceinline__ int32_t lds32(unsigned a) {
 }
 __device__ __forceinline__ void sts128(unsigned a, int4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+__device__ __forceinline__ int lds_u16(unsigned a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ int lds_u8(unsigned a) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return (int)v;
+}
+__device__ __forceinline__ void sts_u16(unsigned a, int v) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
+}
+__device__ __forceinline__ void sts_u8(unsigned a, int v) {
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 template <bool WIDE> struct Cells;
@@ -1025,7 +1044,16 @@ __device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) 
 // M == I is decided only when it is asked for, by looking for the cell the
 // gap opened from: I[j] is the maximum over k < j of M[k] + o1 + (j - 1 - k) * e1
 // and never exceeds M[j]. Once in a gap the walk carries the gap's value.
-template <bool WIDE, int BT_BLK>
+//
+// Loading a tile was the walk's largest part (10,400 cycles for 64 rows, most of
+// it one row's chain of address arithmetic after another): two rows a lane, the
+// rows' cells 8 passes in flight and the jump tables from registers through
+// 32-bit shared-memory addresses take 6,300. The search for a gap's origin goes
+// 128 columns and then 384 at a time: 2,860 -> 1,300 cycles on 12 kb rows.
+// ROOMY: builds with the registers for that. Those that share the SM with three
+// or four more CTAs of 4 warps keep 2 passes and 128 columns: full unrolling
+// spills there (5,000 polishing windows: 233 ms against 209; before, 214).
+template <bool WIDE, int BT_BLK, bool ROOMY = true>
 static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* smem, int bytes, int lane, int32_t& nmoves) {
     typedef typename Cells<WIDE>::One One;
     const BtTile<WIDE, BT_BLK> T(bytes);
@@ -1054,61 +1082,82 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
             const int cnt = i - lo + 1;
             const int dB = (acj >> 3) - rowi[i].x;
             __syncwarp();
-            for (int r = lane; r < cnt; r += 32) {
-                int4 v = rowi[lo + r];
-                v.w = v.x + max(0, dB - BACK);
-                *reinterpret_cast<int4*>(smem + T.row + r * 16) = v;
+            // rows and list ends: two rows a lane
+            int4 v[2];
+            int ends[3];
+#pragma unroll
+            for (int q = 0; q < 2; q++) v[q] = lane + 32 * q < cnt ? rowi[lo + lane + 32 * q] : make_int4(0, 0, 0, 0);
+#pragma unroll
+            for (int q = 0; q < 3; q++) ends[q] = lane + 32 * q <= cnt ? a.in_ptr[lo + lane + 32 * q] : 0;
+            e_lo = __shfl_sync(0xffffffffu, ends[0], 0);
+            {
+                const int x0 = __shfl_sync(0xffffffffu, ends[0], cnt & 31), x1 = __shfl_sync(0xffffffffu, ends[1], cnt & 31),
+                          x2 = __shfl_sync(0xffffffffu, ends[2], cnt & 31);
+                ne = min((cnt < 32 ? x0 : cnt < 64 ? x1 : x2) - e_lo, T.E);
             }
-            for (int r = lane; r <= cnt; r += 32) *reinterpret_cast<int32_t*>(smem + T.ptr + r * 4) = a.in_ptr[lo + r];
-            __syncwarp();
-            e_lo = lds32(sb + T.ptr);
-            ne = min(lds32(sb + T.ptr + cnt * 4) - e_lo, T.E);
             for (int e = lane; e < ne; e += 32) cp_async16(smem + T.ed + e * 16, edg + e_lo + e);
-            for (int x = lane; x < cnt * RL; x += 32) {
-                const int r = x / RL, pc = x % RL;
-                const int4 v = *reinterpret_cast<const int4*>(smem + T.row + r * 16);
-                const int blk = v.w + pc * 16 / (BLK * CB);
-                if (blk <= v.y - 2)
-                    cp_async16(smem + r * ROWB + pc * 16,
-                               a.store + ((int64_t)v.z + (v.w - v.x)) * (BLK * CB) + pc * 16);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                v[q].w = v[q].x + max(0, dB - BACK);
+                if (lane + 32 * q < cnt) sts128(sb + T.row + (lane + 32 * q) * 16, v[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                if (lane + 32 * q <= cnt) *reinterpret_cast<int32_t*>(smem + T.ptr + (lane + 32 * q) * 4) = ends[q];
+            __syncwarp();
+            constexpr int RPI = 32 / RL, TU = ROOMY ? 8 : 2;  // rows a pass takes, passes in flight
+            for (int r0 = lane / RL; r0 < cnt; r0 += RPI * TU) {
+                int4 w[TU];
+#pragma unroll
+                for (int q = 0; q < TU; q++) w[q] = r0 + RPI * q < cnt ? lds128(sb + T.row + (r0 + RPI * q) * 16) : make_int4(0, 0, 0, 0);
+#pragma unroll
+                for (int q = 0; q < TU; q++) {
+                    const int r = r0 + RPI * q, pc = lane % RL;
+                    if (r < cnt && w[q].w + pc * 16 / (BLK * CB) <= w[q].y - 2)
+                        cp_async16(smem + r * ROWB + pc * 16, a.store + ((int64_t)w[q].z + (w[q].w - w[q].x)) * (BLK * CB) + pc * 16);
+                }
             }
             cp_async_commit_all();
             cp_async_wait_all();
             __syncwarp();
-            uint8_t* jump = reinterpret_cast<uint8_t*>(smem + T.jump);
-            for (int r = lane; r < T.rows; r += 32) {
-                int to = 255;
+            // where the heaviest predecessors lead, 1, 2, 4, 8 and 16 steps back
+            int to[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int r = lane + 32 * q;
+                to[q] = 255;
                 if (r < cnt && lo + r > 0) {
                     const int e = lds32(sb + T.ptr + r * 4) - e_lo, e1 = lds32(sb + T.ptr + r * 4 + 4) - e_lo;
                     if (e < e1 && e < ne) {
                         const int p = lds32(sb + T.ed + e * 16) >> 4;
-                        if (p >= lo) to = p - lo;
+                        if (p >= lo) to[q] = p - lo;
                     }
                 }
-                jump[r] = (uint8_t)to;
+                if (r < T.rows) sts_u8(sb + T.jump + r, to[q]);
             }
 #pragma unroll
-            for (int q = 1; q < 5; q++) {
+            for (int x = 1; x < 5; x++) {
                 __syncwarp();
-                for (int r = lane; r < T.rows; r += 32) {
-                    const int h = jump[(q - 1) * T.rows + r];
-                    jump[q * T.rows + r] = h == 255 ? 255 : jump[(q - 1) * T.rows + h];
-                }
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    to[q] = to[q] == 255 ? 255 : lds_u8(sb + T.jump + (x - 1) * T.rows + to[q]);
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    if (lane + 32 * q < T.rows) sts_u8(sb + T.jump + x * T.rows + lane + 32 * q, to[q]);
             }
             __syncwarp();
             R = lds128(sb + T.row + (i - lo) * 16);
         }
         if (op & M_OP) {
             // a run of matches with the heaviest predecessors
-            const uint8_t* jump = reinterpret_cast<const uint8_t*>(smem + T.jump);
             int r = i - lo;
 #pragma unroll
             for (int q = 0; q < 5; q++)
-                if ((lane >> q) & 1) r = r == 255 ? 255 : jump[q * T.rows + r];
+                if (((lane >> q) & 1) && r != 255) r = lds_u8(sb + T.jump + q * T.rows + r);
             const int c = acj - lane;
             bool ok = false;
             int32_t mv = 0;
-            const int to = r == 255 ? 255 : jump[r];
+            const int to = r == 255 ? 255 : lds_u8(sb + T.jump + r);
             if (to != 255 && c > 0) {
                 const int4 A = lds128(sb + T.row + r * 16), P = lds128(sb + T.row + to * 16);
                 const int4 er = lds128(sb + T.ed + (lds32(sb + T.ptr + r * 4) - e_lo) * 16);
@@ -1212,15 +1261,23 @@ static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* sm
                 if (i == 0) {
                     in_gap = M == NEG;
                 } else {
-                    for (int x0 = j - 1; x0 >= 0 && !in_gap; x0 -= 128) {
+                    // 128 columns, then more at a time (a round trip to the row store each)
+                    constexpr int FAR = ROOMY ? 12 : 4;
+                    auto look = [&](int x0, auto n) {
+                        One c[decltype(n)::value];
                         bool hit = false;
 #pragma unroll
-                        for (int u = 0; u < 4; u++) {
+                        for (int u = 0; u < decltype(n)::value; u++)
+                            if (x0 - 32 * u - lane >= 0) c[u] = row[x0 - 32 * u - lane];
+#pragma unroll
+                        for (int u = 0; u < decltype(n)::value; u++) {
                             const int x = x0 - 32 * u - lane;
-                            if (x >= 0) hit |= add32(row[x].m(), k.o1 + (j - 1 - x) * k.e1) == v;
+                            if (x >= 0) hit |= add32(c[u].m(), k.o1 + (j - 1 - x) * k.e1) == v;
                         }
-                        in_gap = __any_sync(0xffffffffu, hit);
-                    }
+                        return __any_sync(0xffffffffu, hit) != 0;
+                    };
+                    in_gap = look(j - 1, std::integral_constant<int, 4>());
+                    for (int x0 = j - 129; x0 >= 0 && !in_gap; x0 -= 32 * FAR) in_gap = look(x0, std::integral_constant<int, FAR>());
                     in_gap = in_gap || add32(NEG, j * k.e1) == v;
                 }
             }
