@@ -1271,7 +1271,7 @@ __device__ void process_window(const BatchArgs& A, char* s, TeamJob& a, unsigned
         }
         tick(PH_FILL);
         int32_t nm = 0;
-        if (st == ST_OK) st = team_backtrack<WIDE, TEAM ? 8 : 4, TEAM || U == 2>(a, (char*)wsm, A.smem_per_warp, lane, nm);
+        if (st == ST_OK) st = team_backtrack<WIDE, TEAM ? 8 : 4, TEAM || (U > 1)>(a, (char*)wsm, A.smem_per_warp, lane, nm);
         if (lane == 0) {
             g.hdr[2] = st;
             g.hdr[13] = nm;

@@ -269,18 +269,18 @@ __device__ void warp_fill_static(const TeamJob& a, const WarpRing& ring, const u
 // need row i's maximum are fetched before the row is filled, the state of
 // nearby rows lives in a shared-memory window of `wrows` rows (a power of two),
 // their cells in a buffer of rcap blocks at `rbuf`. Returns a status (uniform).
-enum { SW_RPOS = 7, SW_RAT = 11 };  // a kept row: its position in the stream of kept blocks, its first block in the buffer
 template <bool WIDE, int U>
 __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm, int wrows, unsigned char* rbuf, int rcap,
                              const uint32_t* qf, int lane, int64_t& cells_out) {
     const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n];
     const CellK k = a.k;
     char* const store = a.store;
-    int4* sed = reinterpret_cast<int4*>(wsm);
     const unsigned seda = (unsigned)__cvta_generic_to_shared(wsm);
     int32_t* win = reinterpret_cast<int32_t*>(wsm + WED * 16);
     const int wmask = wrows - 1, AHEAD = wrows / 2 - 1;
-    auto slot = [&](int r) { return win + (r & wmask) * SW_INTS; };
+    const unsigned wina = seda + WED * 16;
+    // row r's state: {Pl, Pr, Ol, Or}, {Ow, Sl, Mp, rpos}, {Bs, Be, tb, rat}
+    auto slot = [&](int r) { return wina + (r & wmask) * (SW_INTS * 4); };
     if (adaptive)
         for (int64_t x = lane; x < 8 * (int64_t)n; x += 32) a.state[x] = (x & 7) == SW_PL ? m : 0;
     for (int x = lane; x < wrows * SW_INTS; x += 32) win[x] = x % SW_INTS == SW_PL ? m : 0;
@@ -294,6 +294,8 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
     Bs = 0;
     int64_t tb = 0, cells = 0;
     int edx = 0, edx_n = 0, succ = -1, succ_n = -1;
+    int4 far = make_int4(0, 0, 0, 0);  // the row's predecessors beyond the window, one per lane: row,
+    int2 far_s = make_int2(0, 0);      // slope and maximum
     if (lane < ra1.w) succ = a.out_row[ra0.y + lane];
     if (n > 1) {
         if (lane < rb1.z) edx_n = a.ed[rb0.x + lane].x;
@@ -302,15 +304,12 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
     constexpr int BB = BLK * Cells<WIDE>::BYTES;
     WarpRing ring{(unsigned)__cvta_generic_to_shared(rbuf), 0, 0, -1};
     int rpos = 0, rat = 0;  // end of the stream of kept blocks; its place in the buffer
-    int32_t pend = 0;  // state entering the window, one int per lane (8)
     for (int i = 0; i < n; i++) {
         const int bn = Be - Bs - 1;
         const int d = i == 0 ? 0 : ra1.z, ns = ra1.w;
         if (bn < 0) return ST_DEGENERATE;
         if (d > MAX_MULTI_PRED) return ST_INDEGREE;
         if (tb + bn > a.store_cap || tb + bn > INT_MAX) return ST_OOM;
-        // the state that entered the window after the previous row
-        if (adaptive && i > 0 && i - 1 + AHEAD < n && lane < 8) slot(i - 1 + AHEAD)[lane] = pend;
         int4 rc0 = rb0, rc1 = rb1;
         int edx_2 = 0, succ_2 = -1;
         if (i + 2 < n) {
@@ -320,6 +319,18 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
             const int e2 = rb0.x + rb1.z, o2 = rb0.y + rb1.w;
             if (e2 + lane < E) edx_2 = a.ed[e2 + lane].x;
             if (o2 + lane < E) succ_2 = a.out_row[o2 + lane];
+        }
+        int32_t pend = 0;  // state entering the window, one int per lane (8)
+        if (adaptive && i >= 1 && i - 1 + AHEAD < n && lane < 8) pend = a.state[8 * (int64_t)(i - 1 + AHEAD) + lane];
+        // the next row's predecessors beyond the window, whose rows are done
+        int4 far_n = make_int4(0, 0, 0, 0);
+        int2 far_sn = make_int2(0, 0);
+        if (lane < rb1.z && i + 1 - (edx_n >> 4) >= AHEAD) {
+            far_n = a.rowi[edx_n >> 4];
+            if (adaptive) {
+                const int32_t* w = a.state + 8 * (int64_t)(edx_n >> 4);
+                far_sn = make_int2(w[SW_SL], w[SW_MP]);
+            }
         }
         // the row's place in the buffer: whole, so the end of the buffer may stay empty
         ring.cur = -1;
@@ -331,39 +342,34 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
         }
         if (lane == 0) {
             a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
-            int32_t* w = slot(i);
-            w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
-            w[SW_RPOS] = rpos - bn - 2; w[SW_RAT] = ring.cur;
+            sts128(slot(i) + 32, make_int4(Bs, Be, (int)tb, ring.cur));
+            sts32(slot(i) + 28, rpos - bn - 2);
         }
         // row i's predecessor records; their slopes and maxima
         int psl = 0, pmp = INT_MIN / 2;
-        for (int k0 = 0; k0 < d; k0 += 32) {
-            const int kk = k0 + lane;
-            if (kk < d) {
-                int4 v;
-                v.x = k0 == 0 ? edx : a.ed[ra0.x + kk].x;
-                const int p = v.x >> 4;
-                int from = -1;  // its first block in the buffer, unless written over by now
-                if (i - p < AHEAD) {
-                    const int32_t* w = slot(p);
-                    v.y = w[SW_BS]; v.z = w[SW_BE]; v.w = w[SW_TB];
-                    if (rpos - w[SW_RPOS] <= rcap) from = w[SW_RAT];
-                    if (k0 == 0) { psl = w[SW_SL]; pmp = w[SW_MP]; }
-                } else {
-                    const int4 q = a.rowi[p];
-                    v.y = q.x; v.z = q.y; v.w = q.z;
-                    if (adaptive && k0 == 0) { psl = a.state[8 * (int64_t)p + SW_SL]; pmp = a.state[8 * (int64_t)p + SW_MP]; }
-                }
-                const int2 band = rec_band(v.y, v.z);
-                if (kk < WED) sed[kk] = make_int4(from >= 0 ? from * BB : ~v.w, row_score<WIDE>(k, v.x & 7), band.x, band.y);
-                a.ed[ra0.x + kk] = v;
-            }
+        auto put_record = [&](int kk, int x, int4 q, int from) {  // q: {Bs, Be, tb}; from: its first block in the buffer, or -1
+            const int2 band = rec_band(q.x, q.y);
+            if (kk < WED) sts128(seda + kk * 16, make_int4(from >= 0 ? from * BB : ~q.z, row_score<WIDE>(k, x & 7), band.x, band.y));
+            a.ed[ra0.x + kk] = make_int4(x, q.x, q.y, q.z);
+        };
+        if (lane < d) {
+            const int p = edx >> 4;
+            const bool near = i - p < AHEAD;
+            const int4 w = lds128(slot(p) + 16), q = lds128(slot(p) + 32);
+            psl = near ? w.y : far_s.x;
+            pmp = near ? w.z : far_s.y;
+            // (written over in the buffer by now?)
+            put_record(lane, edx, near ? q : far, near && rpos - w.w <= rcap ? q.w : -1);
+        }
+        for (int kk = 32 + lane; kk < d; kk += 32) {
+            const int x = a.ed[ra0.x + kk].x;
+            put_record(kk, x, a.rowi[x >> 4], -1);
         }
         __syncwarp();
-        int32_t* own = slot(i);
-        const int32_t* nw = slot(i + 1);
-        int sl = own[SW_SL], ow = own[SW_OW], ol = own[SW_OL], orr = own[SW_OR];
-        int nPl = nw[SW_PL], nPr = nw[SW_PR], nOl = nw[SW_OL], nOr = nw[SW_OR], nOw = nw[SW_OW];
+        const int4 own0 = lds128(slot(i)), own1 = lds128(slot(i) + 16), nw = lds128(slot(i + 1));
+        int sl = own1.y, ow = own1.x, ol = own0.z, orr = own0.w;
+        int nPl = nw.x, nPr = nw.y, nOl = nw.z, nOr = nw.w, nOw = lds32(slot(i + 1) + 16);
+        const int max_psl = adaptive ? __reduce_max_sync(0xffffffffu, psl) : 0;
         const int4* ed = a.ed + ra0.x;
         auto ed_at = [&](int e) {
             if (e < WED) return lds128(seda + e * 16);
@@ -383,19 +389,25 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
         tb += bn;
         if (adaptive) {
             if (i >= 1) {  // src/align.cpp:1516-1568
+                // the state that enters the window (asked for before the row was filled)
+                if (i - 1 + AHEAD < n && lane < 8) sts32(slot(i - 1 + AHEAD) + 4 * lane, pend);
+                __syncwarp();
                 int sl_best = INT_MIN, max_slp = 0;
                 bool is_match = false;
                 if (ra1.y == qcode(qf, acj + 1)) {  // cur.base == seq[max_acj]
-                    max_slp = psl;
-                    sl_best = pmp + 1 == acj ? psl + 1 : INT_MIN;
-                    for (int kk = 32 + lane; kk < d; kk += 32) {
-                        const int p = ed[kk].x >> 4;
-                        const int32_t* w = i - p < AHEAD ? slot(p) : a.state + 8 * (int64_t)p;
-                        max_slp = max(max_slp, w[SW_SL]);
-                        if (w[SW_MP] + 1 == acj) sl_best = max(sl_best, w[SW_SL] + 1);
+                    max_slp = max_psl;
+                    sl_best = __reduce_max_sync(0xffffffffu, pmp + 1 == acj ? psl + 1 : INT_MIN);
+                    if (d > 32) {
+                        for (int kk = 32 + lane; kk < d; kk += 32) {
+                            const int p = ed[kk].x >> 4;
+                            const int4 w = i - p < AHEAD ? lds128(slot(p) + 16)
+                                                         : *reinterpret_cast<const int4*>(a.state + 8 * (int64_t)p + 4);
+                            max_slp = max(max_slp, w.y);
+                            if (w.z + 1 == acj) sl_best = max(sl_best, w.y + 1);
+                        }
+                        max_slp = __reduce_max_sync(0xffffffffu, max_slp);
+                        sl_best = __reduce_max_sync(0xffffffffu, sl_best);
                     }
-                    max_slp = __reduce_max_sync(0xffffffffu, max_slp);
-                    sl_best = __reduce_max_sync(0xffffffffu, sl_best);
                     is_match = sl_best != INT_MIN;
                 }
                 if (is_match) sl = mx(sl, sl_best);
@@ -404,19 +416,30 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
                     ol = orr = acj - ra1.x;
                     ow = 0;
                 }
-                bool to_next = false;
-                for (int k0 = 0; k0 < ns; k0 += 32) {
-                    const int kk = k0 + lane;
-                    int sr = -1;
-                    if (kk < ns) {
-                        sr = k0 == 0 ? succ : a.out_row[ra0.y + kk];
-                        int32_t* w = sr - i < AHEAD ? slot(sr) : a.state + 8 * (int64_t)sr;
-                        w[SW_OL] = sl >= 30 ? ol : mn(w[SW_OL], ol);
-                        w[SW_OR] = sl >= 30 ? orr : mx(w[SW_OR], orr);
-                        w[SW_PL] = mn(w[SW_PL], acj);
-                        w[SW_PR] = mx(w[SW_PR], acj + 1);
-                        w[SW_OW] = ow ? mx(w[SW_OW], ow) : ow;
+                auto put_state = [&](int sr) {
+                    const bool near = sr - i < AHEAD;
+                    int32_t* gs = a.state + 8 * (int64_t)sr;
+                    int4 w = lds128(slot(sr));
+                    int sow = lds32(slot(sr) + 16);
+                    if (!near) {
+                        w = *reinterpret_cast<const int4*>(gs);
+                        sow = gs[SW_OW];
                     }
+                    w = make_int4(mn(w.x, acj), mx(w.y, acj + 1), sl >= 30 ? ol : mn(w.z, ol), sl >= 30 ? orr : mx(w.w, orr));
+                    sow = ow ? mx(sow, ow) : ow;
+                    if (near) {
+                        sts128(slot(sr), w);
+                        sts32(slot(sr) + 16, sow);
+                    } else {
+                        *reinterpret_cast<int4*>(gs) = w;
+                        gs[SW_OW] = sow;
+                    }
+                };
+                if (lane < ns) put_state(succ);
+                bool to_next = __any_sync(0xffffffffu, lane < ns && succ == i + 1);
+                for (int k0 = 32; k0 < ns; k0 += 32) {
+                    const int sr = k0 + lane < ns ? a.out_row[ra0.y + k0 + lane] : -1;
+                    if (sr >= 0) put_state(sr);
                     to_next |= __any_sync(0xffffffffu, sr == i + 1);
                 }
                 if (to_next) {
@@ -427,7 +450,8 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
                     nOw = ow ? mx(nOw, ow) : ow;
                 }
                 if (lane == 0) {
-                    own[SW_SL] = sl; own[SW_MP] = acj;
+                    sts32(slot(i) + 20, sl);
+                    sts32(slot(i) + 24, acj);
                     a.state[8 * (int64_t)i + SW_SL] = sl;
                     a.state[8 * (int64_t)i + SW_MP] = acj;
                 }
@@ -435,9 +459,9 @@ __device__ int warp_fill_dyn(const TeamJob& a, bool adaptive, unsigned char* wsm
             if (i + 1 < n) band_adaptive(rb0.z, rb0.w, m, a.w, nPl, nPr, nOl, nOr, nOw, Bs, Be);
         }
         __syncwarp();
-        if (adaptive && i + AHEAD < n && lane < 8) pend = a.state[8 * (int64_t)(i + AHEAD) + lane];
         ra0 = rb0; ra1 = rb1; rb0 = rc0; rb1 = rc1;
         edx = edx_n; edx_n = edx_2;
+        far = far_n; far_s = far_sn;
         succ = succ_n; succ_n = succ_2;
     }
     cells_out = cells;
