@@ -747,7 +747,7 @@ template <int W, bool WIDE, int RING_MAX = RING_ALONE>
 __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
     typedef TeamSmem<W, true, WIDE, RING_MAX> S;
     TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
-    int32_t* win = reinterpret_cast<int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
+    const unsigned win = (unsigned)__cvta_generic_to_shared(smem + S::REST + 2 * sizeof(TeamHdr));
     const unsigned bests = (unsigned)__cvta_generic_to_shared(smem + S::BEST);
     const int lane = threadIdx.x & 31;
     const int n = a.n, m = a.qlen + 1, E = a.in_ptr[n], bw = a.w;
@@ -756,7 +756,8 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
     const int32_t* out_row = a.out_row;
     int32_t* state = a.state;
     const int64_t store_cap = a.store_cap;
-    auto slot = [&](int r) { return win + (r & (SWIN - 1)) * SW_INTS; };
+    // row r's state: {Pl, Pr, Ol, Or}, {Ow, Sl, Mp, -}, {Bs, Be, tb, -}
+    auto slot = [&](int r) { return win + (r & (SWIN - 1)) * (SW_INTS * 4); };
     int4 ra0 = ra[0], ra1 = ra[1];                // row i
     int4 rb0 = make_int4(0, 0, 0, 0), rb1 = rb0;  // row i + 1
     if (n > 1) { rb0 = ra[2]; rb1 = ra[3]; }
@@ -783,7 +784,7 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
         if (lane < rb1.z) edx_n = ed[rb0.x + lane].x;
         if (lane < rb1.w) succ_n = out_row[rb0.y + lane];
     }
-    int32_t pend = 0;  // state entering the window, one int per lane (8)
+    int2 far_s = make_int2(0, 0);  // row i's predecessors beyond the window: slope and maximum, one per lane
     __syncwarp();
     bar_sync<1, S::THREADS>();  // header 0
     int xp = 0;
@@ -797,9 +798,10 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
         const int d = i == 0 ? 0 : ra1.z, ns = ra1.w;
         if (lane == 0) {
             a.rowi[i] = make_int4(Bs, Be, (int)tb, 0);
-            int32_t* w = slot(i);
-            w[SW_BS] = Bs; w[SW_BE] = Be; w[SW_TB] = (int)tb;
+            sts128(slot(i) + 32, make_int4(Bs, Be, (int)tb, 0));
         }
+        int32_t pend = 0;  // state entering the window, one int per lane (8)
+        if (i > 0 && i - 1 + AHEAD < n && lane < 8) pend = state[8 * (int64_t)(i - 1 + AHEAD) + lane];
         // loads two rows ahead
         int4 rc0 = rb0, rc1 = rb1;
         int edx_2 = 0, succ_2 = -1;
@@ -811,14 +813,19 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
             if (e2 + lane < E) edx_2 = ed[e2 + lane].x;
             if (o2 + lane < E) succ_2 = out_row[o2 + lane];
         }
+        int2 far_n = make_int2(0, 0);
+        if (lane < rb1.z && i + 1 - (edx_n >> 4) >= AHEAD) {
+            const int32_t* w = state + 8 * (int64_t)(edx_n >> 4);
+            far_n = make_int2(w[SW_SL], w[SW_MP]);
+        }
         // row i's predecessors' slopes and maxima (their rows are done), its own
         // state and the next row's
         int psl = 0, pmp = INT_MIN / 2;
-        if (i > 0 && lane < d && d <= 32) {
+        if (lane < d) {
             const int p = edx >> 4;
-            const int32_t* w = i - p < AHEAD ? slot(p) : state + 8 * (int64_t)p;
-            psl = w[SW_SL];
-            pmp = w[SW_MP];
+            const int4 w = lds128(slot(p) + 16);
+            psl = i - p < AHEAD ? w.y : far_s.x;
+            pmp = i - p < AHEAD ? w.z : far_s.y;
         }
         int max_psl = psl, pmp0 = pmp;
         if (d > 1) {
@@ -827,10 +834,9 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
             max_psl = __shfl_sync(0xffffffffu, psl, 0);
             pmp0 = __shfl_sync(0xffffffffu, pmp, 0);
         }
-        int32_t* own = slot(i);
-        int sl = own[SW_SL], ow = own[SW_OW], ol = own[SW_OL], orr = own[SW_OR];
-        const int32_t* nw = slot(i + 1);
-        int nPl = nw[SW_PL], nPr = nw[SW_PR], nOl = nw[SW_OL], nOr = nw[SW_OR], nOw = nw[SW_OW];
+        const int4 own0 = lds128(slot(i)), own1 = lds128(slot(i) + 16), nw = lds128(slot(i + 1));
+        int sl = own1.y, ow = own1.x, ol = own0.z, orr = own0.w;
+        int nPl = nw.x, nPr = nw.y, nOl = nw.z, nOr = nw.w, nOw = lds32(slot(i + 1) + 16);
         bool to_next = __any_sync(0xffffffffu, lane < ns && succ == i + 1);
         for (int k0 = 32; k0 < ns; k0 += 32)
             to_next |= __any_sync(0xffffffffu, k0 + lane < ns && out_row[ra0.y + k0 + lane] == i + 1);
@@ -838,8 +844,8 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
         const int nst = bn > 0 ? strips_of(Bs, Be) : 0;
         const int laps = nst > W ? (nst + W - 1) / W : 1;
         xp = (xp + laps - 1) & 1;
-        // the state that entered the window after the previous row (its load had the time since)
-        if (i > 0 && i - 1 + AHEAD < n && lane < 8) slot(i - 1 + AHEAD)[lane] = pend;
+        // the state that enters the window
+        if (i > 0 && i - 1 + AHEAD < n && lane < 8) sts32(slot(i - 1 + AHEAD) + 4 * lane, pend);
         __syncwarp();
         bar_sync<2, 32 * (W + 1)>();
         int acj = 0;
@@ -859,9 +865,10 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
                 } else {
                     for (int kk = lane; kk < d; kk += 32) {
                         const int p = ed[ra0.x + kk].x >> 4;
-                        const int32_t* w = i - p < AHEAD ? slot(p) : state + 8 * (int64_t)p;
-                        max_slp = max(max_slp, w[SW_SL]);
-                        if (w[SW_MP] + 1 == acj) sl_best = max(sl_best, w[SW_SL] + 1);
+                        const int4 w = i - p < AHEAD ? lds128(slot(p) + 16)
+                                                     : *reinterpret_cast<const int4*>(state + 8 * (int64_t)p + 4);
+                        max_slp = max(max_slp, w.y);
+                        if (w.z + 1 == acj) sl_best = max(sl_best, w.y + 1);
                     }
                     max_slp = __reduce_max_sync(0xffffffffu, max_slp);
                     sl_best = __reduce_max_sync(0xffffffffu, sl_best);
@@ -892,26 +899,36 @@ __device__ void team_state(const TeamJob& a, char* smem, int64_t& cells_out) {
         bar_sync<1, S::THREADS>();  // header i + 1; row i's cells
         if (i >= 1) {
             if (lane == 0) {
-                own[SW_SL] = sl; own[SW_MP] = acj;
+                sts32(slot(i) + 20, sl);
+                sts32(slot(i) + 24, acj);
                 int32_t* gs = state + 8 * (int64_t)i;
                 gs[SW_SL] = sl; gs[SW_MP] = acj;
             }
-            for (int k0 = 0; k0 < ns; k0 += 32) {
-                const int kk = k0 + lane;
-                if (kk < ns) {
-                    const int sr = k0 == 0 ? succ : out_row[ra0.y + kk];
-                    int32_t* w = sr - i < AHEAD ? slot(sr) : state + 8 * (int64_t)sr;
-                    w[SW_OL] = sl >= 30 ? ol : mn(w[SW_OL], ol);
-                    w[SW_OR] = sl >= 30 ? orr : mx(w[SW_OR], orr);
-                    w[SW_PL] = mn(w[SW_PL], acj);
-                    w[SW_PR] = mx(w[SW_PR], acj + 1);
-                    w[SW_OW] = ow ? mx(w[SW_OW], ow) : ow;
+            auto put_state = [&](int sr) {
+                const bool near = sr - i < AHEAD;
+                int32_t* gs = state + 8 * (int64_t)sr;
+                int4 w = lds128(slot(sr));
+                int sow = lds32(slot(sr) + 16);
+                if (!near) {
+                    w = *reinterpret_cast<const int4*>(gs);
+                    sow = gs[SW_OW];
                 }
-            }
+                w = make_int4(mn(w.x, acj), mx(w.y, acj + 1), sl >= 30 ? ol : mn(w.z, ol), sl >= 30 ? orr : mx(w.w, orr));
+                sow = ow ? mx(sow, ow) : ow;
+                if (near) {
+                    sts128(slot(sr), w);
+                    sts32(slot(sr) + 16, sow);
+                } else {
+                    *reinterpret_cast<int4*>(gs) = w;
+                    gs[SW_OW] = sow;
+                }
+            };
+            if (lane < ns) put_state(succ);
+            for (int kk = 32 + lane; kk < ns; kk += 32) put_state(out_row[ra0.y + kk]);
         }
         __syncwarp();
         xp ^= 1;
-        if (i + AHEAD < n && lane < 8) pend = state[8 * (int64_t)(i + AHEAD) + lane];
+        far_s = far_n;
         ra0 = rb0; ra1 = rb1; rb0 = rc0; rb1 = rc1;
         edx = edx_n; edx_n = edx_2;
         succ = succ_n; succ_n = succ_2;
@@ -926,7 +943,7 @@ template <int W, bool WIDE, int RING_MAX = RING_ALONE>
 __device__ void team_records(const TeamJob& a, char* smem) {
     typedef TeamSmem<W, true, WIDE, RING_MAX> S;
     TeamHdr* hdr = reinterpret_cast<TeamHdr*>(smem + S::REST);
-    const int32_t* win = reinterpret_cast<const int32_t*>(smem + S::REST + 2 * sizeof(TeamHdr));
+    const unsigned win = (unsigned)__cvta_generic_to_shared(smem + S::REST + 2 * sizeof(TeamHdr));
     const unsigned hb = (unsigned)__cvta_generic_to_shared(hdr);
     const int lane = threadIdx.x & 31;
     const int n = a.n, E = a.in_ptr[n];
@@ -949,34 +966,29 @@ __device__ void team_records(const TeamJob& a, char* smem) {
             const int Bs = h.x, Be = h.x + h.y + 2, dn = e1 - e0;
             const bool lap1 = h.y >= 0 && strips_of(Bs, Be) <= W;
             int prev = 0;
-            for (int k0 = 0; k0 < dn; k0 += 32) {
-                const int kk = k0 + lane;
-                int4 v = make_int4(-1, 0, 0, 0);
-                if (kk < dn) {
-                    v.x = k0 == 0 ? x : ed[e0 + kk].x;
-                    const int p = v.x >> 4;
-                    if (p == i) {
-                        v.y = Bs; v.z = Be; v.w = h.z;
-                    } else if (i - p < AHEAD) {
-                        const int32_t* w = win + (p & (SWIN - 1)) * SW_INTS;
-                        v.y = w[SW_BS]; v.z = w[SW_BE]; v.w = w[SW_TB];
-                    } else {
-                        const int4 q = a.rowi[p];
-                        v.y = q.x; v.z = q.y; v.w = q.z;
-                    }
-                    ed[e0 + kk] = v;
+            auto put = [&](int k0, int vx) {
+                const int kk = k0 + lane, p = vx >> 4;
+                const bool has = kk < dn, own = has && p == i;
+                int4 q = make_int4(0, 0, 0, 0);  // its band and place
+                if (has) {
+                    q = lds128(win + (p & (SWIN - 1)) * (SW_INTS * 4) + 32);
+                    if (i - p >= AHEAD) q = a.rowi[p];
+                    if (own) q = make_int4(Bs, Be, h.z, 0);
+                    ed[e0 + kk] = make_int4(vx, q.x, q.y, q.z);
                 }
-                const unsigned pmask = __ballot_sync(0xffffffffu, lap1 && (v.x >> 4) == i);
-                if (kk < dn && !((pmask >> lane) & 1u)) {
-                    const int p = v.x >> 4, at = kk - (prev != 0 || (pmask & ((1u << lane) - 1u)) != 0);
-                    const bool near = i + 1 - p < S::TR && v.z - v.y - 1 > 0 && strips_of(v.y, v.z) <= W;
-                    const int2 band = rec_band(v.y, v.z);
-                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : ~v.w, (v.x & 7) * 0x01010101, band.x, band.y);
+                const unsigned pmask = __ballot_sync(0xffffffffu, lap1 && own);
+                if (has && !((pmask >> lane) & 1u)) {
+                    const int at = kk - (prev != 0 || (pmask & ((1u << lane) - 1u)) != 0);
+                    const bool near = i + 1 - p < S::TR && q.y - q.x - 1 > 0 && strips_of(q.x, q.y) <= W;
+                    const int2 band = rec_band(q.x, q.y);
+                    const int4 f = make_int4(near ? (p & (S::TR - 1)) * S::ROWB : ~q.z, (vx & 7) * 0x01010101, band.x, band.y);
                     if (at < HDR_E) o.ed[at] = f;
                     else fe[e0 + at] = f;
                 }
-                if (pmask) prev = FR_PREV | ((__shfl_sync(0xffffffffu, v.x, __ffs(pmask) - 1) & 7) << FR_PBASE);
-            }
+                if (pmask) prev = FR_PREV | ((__shfl_sync(0xffffffffu, vx, __ffs(pmask) - 1) & 7) << FR_PBASE);
+            };
+            if (dn > 0) put(0, x);
+            for (int k0 = 32; k0 < dn; k0 += 32) put(k0, k0 + lane < dn ? ed[e0 + k0 + lane].x : 0);
             // {first in-edge, predecessors, the fill's flags and count, -}
             if (lane == 0) o.g = make_int4(e0, dn, (dn - (prev != 0)) | prev, 0);
         }
