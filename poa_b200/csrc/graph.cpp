@@ -36,6 +36,7 @@ int Graph::add_node(uint8_t base) {  // node_t ctor, include/node.h:16-22
     for (int k = 0; k < 5; k++) v.aligned[k] = -1;
     v.aligned[base] = v.id;
     node.push_back(std::move(v));
+    reads.emplace_back();
     return (int)node.size() - 1;
 }
 
@@ -43,19 +44,13 @@ int Graph::add_node(uint8_t base) {  // node_t ctor, include/node.h:16-22
 // new edges append (in-list / out-list order is insertion order).
 void Graph::add_adj(int seq_id, int from, int to, int cur_pos) {
     if (from == to) return;
-    Node& f = node[from];
-    bool ok = false;
-    for (size_t i = 0; i < f.out.size(); i++)
-        if (f.out[i] == to) { f.out_w[i]++; ok = true; break; }
-    if (!ok) { f.out.push_back(to); f.out_w.push_back(1); }
+    node[from].out.add(to);
+    NodeReads& f = reads[from];
     if (f.ids.empty() || f.ids.back() != seq_id) f.ids.push_back(seq_id);
 
-    Node& t = node[to];
-    t.ind++;
-    ok = false;
-    for (size_t i = 0; i < t.in.size(); i++)
-        if (t.in[i] == from) { t.in_w[i]++; ok = true; break; }
-    if (!ok) { t.in.push_back(from); t.in_w.push_back(1); }
+    node[to].ind++;
+    node[to].in.add(from);
+    NodeReads& t = reads[to];
     if (t.ids.empty() || t.ids.back() != seq_id) {
         t.ids.push_back(seq_id);
         t.idp.push_back(cur_pos);
@@ -99,7 +94,7 @@ void Graph::topsort(bool with_lens, bool seeding, int op) {
             if (v.par_id != v.id) continue;
             int s = 0;
             for (int k = 0; k < 5; k++)
-                if (v.aligned[k] >= 0) s += (int)node[v.aligned[k]].in.size();
+                if (v.aligned[k] >= 0) s += node[v.aligned[k]].in.size();
             deg[i] = s;
             if (s == 0) stk.push_back(i);
         }
@@ -112,8 +107,8 @@ void Graph::topsort(bool with_lens, bool seeding, int op) {
                 int sid = node[u].aligned[k];
                 if (sid < 0) continue;
                 node[sid].rank = node[u].rank;
-                for (int32_t o : node[sid].out) {
-                    int v = node[o].par_id;
+                for (const Edge& o : node[sid].out) {
+                    int v = node[o.id].par_id;
                     if (--deg[v] == 0) stk.push_back(v);
                 }
             }
@@ -123,7 +118,7 @@ void Graph::topsort(bool with_lens, bool seeding, int op) {
     }
     // src/graph.cpp:61-85: Kahn with a LIFO stack, zero in-degree nodes seeded in id order
     for (int i = 0; i < N; i++) {
-        deg[i] = (int32_t)node[i].in.size();
+        deg[i] = node[i].in.size();
         if (deg[i] == 0) stk.push_back(i);
     }
     while (!stk.empty()) {
@@ -131,8 +126,8 @@ void Graph::topsort(bool with_lens, bool seeding, int op) {
         stk.pop_back();
         node[u].rank = (int32_t)rank.size();
         rank.push_back(u);
-        for (int32_t v : node[u].out)
-            if (--deg[v] == 0) stk.push_back(v);
+        for (const Edge& o : node[u].out)
+            if (--deg[o.id] == 0) stk.push_back(o.id);
     }
     is_topsorted = true;
     if (with_lens) {  // src/graph.cpp:86-123: heaviest-edge depth from source / to sink
@@ -140,18 +135,18 @@ void Graph::topsort(bool with_lens, bool seeding, int op) {
         for (size_t i = 0; i < rank.size(); i++) {
             const Node& cur = node[rank[i]];
             int wmax = -1, max_pre = -1;
-            for (size_t k = 0; k < cur.in.size(); k++)
-                if (cur.in_w[k] > wmax) { wmax = cur.in_w[k]; max_pre = node[cur.in[k]].rank; }
-            if (max_pre != -1) hlen[cur.rank] = hlen[max_pre] + 1;
+            for (const Edge& e : cur.in)
+                if (e.w > wmax) { wmax = e.w; max_pre = e.id; }
+            if (max_pre != -1) hlen[cur.rank] = hlen[node[max_pre].rank] + 1;
         }
         tlen.resize(N);
         tlen[node[1].rank] = 1;
         for (int i = (int)rank.size() - 1; i >= 0; i--) {
             const Node& cur = node[rank[i]];
             int wmax = -1, max_suc = -1;
-            for (size_t k = 0; k < cur.out.size(); k++)
-                if (cur.out_w[k] > wmax) { wmax = cur.out_w[k]; max_suc = node[cur.out[k]].rank; }
-            if (max_suc != -1) tlen[cur.rank] = tlen[max_suc] + 1;
+            for (const Edge& e : cur.out)
+                if (e.w > wmax) { wmax = e.w; max_suc = e.id; }
+            if (max_suc != -1) tlen[cur.rank] = tlen[node[max_suc].rank] + 1;
         }
     }
     if (seeding) build_consensus(false);  // src/graph.cpp:127
@@ -163,23 +158,23 @@ void Graph::build_consensus(bool need_coverages) {
     const int N = (int)node.size();
     std::vector<int32_t> deg(N), pre(N, 0), score(N, 0), q;
     q.reserve(N);
-    for (int i = 0; i < N; i++) deg[i] = (int32_t)node[i].in.size();
+    for (int i = 0; i < N; i++) deg[i] = node[i].in.size();
     q.push_back(0);
     for (size_t h = 0; h < q.size(); h++) {
         int u = q[h];
         const Node& cur = node[u];
         if (u != 0) {
             int wmax = -1, max_pre = -1;
-            for (size_t k = 0; k < cur.in.size(); k++) {
-                int pr = node[cur.in[k]].id, wk = cur.in_w[k];
+            for (const Edge& e : cur.in) {
+                int pr = e.id, wk = e.w;
                 if (wk > wmax || (wk == wmax && score[pr] > score[max_pre])) { wmax = wk; max_pre = pr; }
             }
             pre[u] = max_pre;
             score[u] = score[max_pre] + wmax;
         }
         if (u == 1) break;
-        for (int32_t v : cur.out)
-            if (--deg[v] == 0) q.push_back(v);
+        for (const Edge& o : cur.out)
+            if (--deg[o.id] == 0) q.push_back(o.id);
     }
     if (need_coverages) coverages.clear();
     cons.clear();
@@ -190,8 +185,8 @@ void Graph::build_consensus(bool need_coverages) {
         cons_pos_to_id.push_back(cur.id);
         if (need_coverages) {
             int in_w = 0, out_w = 0;
-            for (int32_t x : cur.in_w) in_w += x;
-            for (int32_t x : cur.out_w) out_w += x;
+            for (const Edge& e : cur.in) in_w += e.w;
+            for (const Edge& e : cur.out) out_w += e.w;
             coverages.push_back(std::max(in_w, out_w));
         }
     }
@@ -209,7 +204,7 @@ std::vector<std::string> Graph::msa_rows(int nseq) const {
     for (size_t i = 2; i < node.size(); i++) {
         int rk = node[node[i].par_id].rank;
         if (rk - 1 < 0 || rk - 1 >= nc) continue;
-        for (int32_t id : node[i].ids)
+        for (int32_t id : reads[i].ids)
             if (id >= 0 && id < nseq) rows[id][rk - 1] = kNt256[node[i].base];
     }
     return rows;
@@ -243,18 +238,18 @@ void build_window(const Graph& g, int beg_id, int end_id, bool with_lens, HostWi
             w.tq[r] = g.tlen[beg_i + r] - g.tlen[end_i];
         }
         int deg = 0;
-        for (size_t k = 0; k < v.in.size(); k++) {
-            int p = g.node[v.in[k]].rank - beg_i;
+        for (const Edge& e : v.in) {
+            int p = g.node[e.id].rank - beg_i;
             if (p < 0) continue;  // src/align.cpp:1451-1452
             w.in_row.push_back(p);
-            w.in_w.push_back(v.in_w[k]);
-            w.in_base.push_back(p == 0 ? 4 : g.node[v.in[k]].base);  // src/align.cpp:1453
+            w.in_w.push_back(e.w);
+            w.in_base.push_back(p == 0 ? 4 : g.node[e.id].base);  // src/align.cpp:1453
             deg++;
         }
         w.max_indeg = std::max(w.max_indeg, deg);
         w.in_ptr[r + 1] = (int32_t)w.in_row.size();
-        for (int32_t o : v.out) {
-            int s = g.node[o].rank - beg_i;
+        for (const Edge& o : v.out) {
+            int s = g.node[o.id].rank - beg_i;
             if (s >= n) continue;  // src/align.cpp:1550-1551
             w.out_row.push_back(s);
         }
@@ -296,7 +291,7 @@ void Graph::gfa_text(const std::vector<int32_t>& read_len, const std::vector<std
     if (n <= 2) return;
     const int nseq = (int)read_len.size();
     std::vector<int32_t> deg(n);
-    for (int i = 0; i < n; i++) deg[i] = (int32_t)node[i].in.size();
+    for (int i = 0; i < n; i++) deg[i] = node[i].in.size();
     std::vector<std::vector<int32_t>> paths(nseq);
     for (int i = 0; i < nseq; i++) paths[i].assign(read_len[rid_to_ord[i]], 0);
     out += "H\tVN:Z:1.0\n";
@@ -309,15 +304,16 @@ void Graph::gfa_text(const std::vector<int32_t>& read_len, const std::vector<std
         const Node& v = node[cur];
         if (cur != 0) {
             out += "S\t" + std::to_string(cur - 1) + "\t" + kNt256[v.base] + "\n";
-            for (int32_t pre : v.in)
-                if (pre != 0) out += "L\t" + std::to_string(pre - 1) + "\t+\t" + std::to_string(cur - 1) + "\t+\t0M\n";
-            for (size_t k = 0; k < v.ids.size() && k < v.idp.size(); k++) {
-                const int id = v.ids[k], pos = v.idp[k];
+            for (const Edge& e : v.in)
+                if (e.id != 0) out += "L\t" + std::to_string(e.id - 1) + "\t+\t" + std::to_string(cur - 1) + "\t+\t0M\n";
+            const NodeReads& rd = reads[cur];
+            for (size_t k = 0; k < rd.ids.size() && k < rd.idp.size(); k++) {
+                const int id = rd.ids[k], pos = rd.idp[k];
                 if (id >= 0 && id < nseq && pos >= 0 && pos < (int)paths[id].size()) paths[id][pos] = cur - 1;
             }
         }
-        for (int32_t o : v.out)
-            if (--deg[o] == 0) fifo.push_back(o);
+        for (const Edge& o : v.out)
+            if (--deg[o.id] == 0) fifo.push_back(o.id);
     }
     for (int i = 0; i < nseq; i++) {
         out += "P\t";
