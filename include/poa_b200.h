@@ -246,7 +246,9 @@ int poa_align_noalloc(const poa_dev_window* w, const uint8_t* q_dev, int32_t qle
  * per SM upper bound (the occupancy calculator still caps it), 1 = maximum
  * number of blocks in total (0 = no cap), 2 = shared memory per warp in
  * bytes, a multiple of 16 (row ring, staged records, query,
- * topsort workspace). Takes effect at the next run. */
+ * topsort workspace). Unset, the engine chooses both for the batch: small
+ * adaptive batches run a team of warps per window, static-band batches that
+ * fill the GPU 4 blocks per SM. Takes effect at the next run. */
 int poa_batch_config(poa_ctx* ctx, int32_t key, int64_t value);
 
 /* The measured int32 add+max rate of `device` (no counterpart in the

@@ -5,7 +5,7 @@
 
 Needs a GPU. For one workload it times the persistent batch kernel under each
 candidate launch shape (the knobs of ``poa_batch_config``: blocks per SM,
-i.e. the 168- or 128-register build, and shared memory per warp, which
+i.e. the 168-, 128- or 96-register build, and shared memory per warp, which
 trades the static-band row ring and staging against L1 capacity) on a seeded
 sample of the workload's windows, and records the fastest shape, with every
 measurement, in a JSON file that ``bench.py`` and ``Context.batch_autotuned``
@@ -33,7 +33,7 @@ WORKLOADS = {
     "learned_band": ("learned_band_windows", ["-B"], 2664, 605, True),
     "polishing": ("polishing_windows", [], 20000, 604, False),
 }
-CANDIDATES = [(3, 18432), (3, 16384), (3, 12288), (3, 10240), (4, 12288), (4, 10240)]
+CANDIDATES = [(3, 18432), (3, 16384), (3, 12288), (3, 10240), (4, 14080), (4, 12288), (4, 10240)]
 
 
 def tune(workload: str, windows: int = 0, repeats: int = 1, log=print) -> dict:

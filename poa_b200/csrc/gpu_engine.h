@@ -1,6 +1,6 @@
 // gpu_engine.h - runs poa() calls on the GPU: packs window views and queries
 // into one pinned staging buffer, uploads it with a single copy, launches
-// one CTA per alignment (plain.cuh) and reads back scores and moves.
+// one CTA per alignment (team.cuh) and reads back scores and moves.
 #pragma once
 #include <stdint.h>
 

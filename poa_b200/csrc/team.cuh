@@ -741,6 +741,9 @@ __device__ void team_fill_static(const TeamJob& a, char* smem) {
 // behind), in global memory beyond it. Between the row's maxima and the next
 // header there is only what depends on them; everything else runs while the
 // other warps fill the row. (As one warp the two took 2,400 cycles a row.)
+// Lists are one pass for up to 32 entries that reads the window whatever the row,
+// the state 16 bytes at a time: as loops around the near / far branch the noisy 5 kb
+// graph's kernel took 101 ms, now 92.
 constexpr int AHEAD = SWIN / 2 - 1;
 
 template <int W, bool WIDE, int RING_MAX = RING_ALONE>
@@ -1065,7 +1068,7 @@ __device__ int team_fill_adaptive(const TeamJob& a, char* smem, int64_t& cells) 
 // 128 columns and then 384 at a time: 2,860 -> 1,300 cycles on 12 kb rows.
 // ROOMY: builds with the registers for that. Those that share the SM with three
 // or four more CTAs of 4 warps keep 2 passes and 128 columns: full unrolling
-// spills there (5,000 polishing windows: 233 ms against 209; before, 214).
+// spills there (8,000 polishing windows: 233 ms against 209; before, 214).
 template <bool WIDE, int BT_BLK, bool ROOMY = true>
 static __device__ __noinline__ int32_t team_backtrack(const TeamJob& a, char* smem, int bytes, int lane, int32_t& nmoves) {
     typedef typename Cells<WIDE>::One One;
