@@ -803,6 +803,7 @@ __device__ int kahn_lifo_shared(unsigned optr, unsigned adj, unsigned deg, unsig
             const int v0 = lds_u16(optr + 2 * v), v1 = lds_u16(optr + 2 * v + 2);
             const unsigned msk = __ballot_sync(0xffffffffu, has && dv == 0);
             if (has) sts_u8(deg + v, dv);
+            __syncwarp();  // before another lane reads the count (a vote or a shuffle orders no memory)
             if (!msk) continue;
             if (u >= 0) {  // ready in the chunk before (more than 32 out-edges)
                 top--;
@@ -813,7 +814,7 @@ __device__ int kahn_lifo_shared(unsigned optr, unsigned adj, unsigned deg, unsig
             if (rest) {
                 top -= __popc(rest);
                 if ((rest >> lane) & 1u) sts_u16(ord + 2 * (top + __popc(rest & above)), v);
-                __syncwarp();
+                __syncwarp();  // before the entries are taken from the stack
             }
             u = __shfl_sync(0xffffffffu, v, last);
             n0 = __shfl_sync(0xffffffffu, v0, last);
