@@ -714,6 +714,7 @@ __device__ void team_fill_static(const TeamJob& a, char* smem) {
     bar_sync<1, S::THREADS>();
     const int n = a.n;
     int4 h = lds128(stg);
+    bool unpublished = false;  // the row before stored its cells after its barrier
     for (int i = 0; i < n; i++) {
         const int x = i & (STG - 1);
         const unsigned cur = stg + ((i / STG) & 1) * (unsigned)sizeof(TeamStage);
@@ -721,9 +722,13 @@ __device__ void team_fill_static(const TeamJob& a, char* smem) {
         if (x == STG - 1) cp_async_wait_all();  // the next stage, published by this row's barrier
         const unsigned nxt = x == STG - 1 ? stg + (((i / STG) & 1) ^ 1) * (unsigned)sizeof(TeamStage) : cur + (x + 1) * 16;
         if (h.w & FR_GENERAL) {
+            // reads every predecessor from the row store, the row before's among them
+            if (unpublished) t.sync_row();
             t.general(i, h, a.ed + a.in_ptr[i]);
+            unpublished = false;
             h = lds128(nxt);
         } else {
+            unpublished = true;
             const int4 hc = h;
             const unsigned ed = cur + STG * 16 + (hc.w >> FR_EOFF) * 16;
             t.row(i, hc, [&](int e) { return hc.w & FR_UNSTAGED ? a.fe[a.in_ptr[i] + e] : lds128(ed + e * 16); },
