@@ -283,7 +283,10 @@ __device__ int dg_consensus(DevGraph& g, int nn, char* out, int cap) {
 // heaviest edge everywhere, sum the scores along the chosen edges by pointer
 // jumping, let the tied nodes choose again with those scores, and repeat until
 // no choice changes. Choices that agree with the scores they give are the serial
-// ones (by induction along the topological order). Serial after 12 rounds.
+// ones (by induction along the topological order). That holds where the walk,
+// which starts at the source, reaches every node: where the source is the only
+// node without in-edges. Other graphs (a negative match score makes them) and
+// those that do not settle in 12 rounds take the serial walk.
 //  pre: chosen edge per node; W: {ancestor, score up to it} words, 8 bytes a node.
 __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap, unsigned char* sm, int sm_bytes, int lane) {
     constexpr int CU = 4;
@@ -297,7 +300,13 @@ __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap
     int32_t* pre = g.pre;
     unsigned long long* key = reinterpret_cast<unsigned long long*>(g.scratch8b);
     int32_t* ties = g.csr_adj;
-    for (int u = lane; u < nn; u += 32) pre[u] = g.hin[u];
+    bool unreached = false;
+    for (int u = lane; u < nn; u += 32) {
+        const int e = g.hin[u];
+        pre[u] = e;
+        unreached |= e < 0 && u != 0;
+    }
+    const int rounds = __any_sync(0xffffffffu, unreached) ? 0 : 12;
     // edges that tie with their end node's heaviest (list order is edge order: hin is the first)
     int nt = 0;
     for (int e0 = 0; e0 < ne; e0 += 32 * CU) {
@@ -321,7 +330,7 @@ __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap
     }
     __syncwarp();
     bool settled = false;
-    for (int round = 0; round < 12 && !settled; round++) {
+    for (int round = 0; round < rounds && !settled; round++) {
         for (int u0 = lane; u0 < nn; u0 += 32 * CU) {
             int e[CU], f[CU], w[CU];
 #pragma unroll
