@@ -733,62 +733,13 @@ __device__ bool scan_degrees(const DevGraph& g, int nn, P* optr, CUR* cur, uint8
 // order, successors pushed in list order. The order itself is a serial chain;
 // the warp takes a node's out-edges at once (they end at distinct nodes) and
 // reads the lists' ends of every successor before it is known which one comes
-// next. The node on top of the stack stays in a register; ord takes the order
-// from its start and the rest of the stack from its end (never more than n
-// entries together). Returns the number of ranks.
-template <typename P, typename A>
-__device__ int kahn_lifo(const P* optr, const A* adj, uint8_t* deg, uint16_t* ord, int nn, int sp, int lane) {
-    int nr = 0, top = nn - sp;  // ord[top]: the stack's top entry
-    int u = -1, k = 0, k1 = 0;
-    while (true) {
-        if (u < 0) {
-            if (top == nn) break;
-            u = ord[top++];
-            k = (int)optr[u];
-            k1 = (int)optr[u + 1];
-        }
-        __syncwarp();
-        if (lane == 0) ord[nr] = (uint16_t)u;
-        nr++;
-        u = -1;
-        int n0 = 0, n1 = 0;
-        for (; k < k1; k += 32) {
-            bool ready = false;
-            int v = 0, v0 = 0, v1 = 0;
-            if (k + lane < k1) {
-                v = (int)adj[k + lane];
-                const int dv = deg[v] - 1;
-                v0 = (int)optr[v];
-                v1 = (int)optr[v + 1];
-                ready = dv == 0;
-                deg[v] = (uint8_t)dv;
-            }
-            const unsigned msk = __ballot_sync(0xffffffffu, ready);
-            if (!msk) continue;
-            if (u >= 0) {  // ready in the chunk before (more than 32 out-edges)
-                top--;
-                if (lane == 0) ord[top] = (uint16_t)u;
-            }
-            const int last = 31 - __clz(msk);
-            const unsigned rest = msk & ~(1u << last);
-            if (rest) {
-                top -= __popc(rest);
-                if ((rest >> lane) & 1u) ord[top + __popc(rest >> 1 >> lane)] = (uint16_t)v;
-            }
-            u = __shfl_sync(0xffffffffu, v, last);
-            n0 = __shfl_sync(0xffffffffu, v0, last);
-            n1 = __shfl_sync(0xffffffffu, v1, last);
-        }
-        k = n0;
-        k1 = n1;
-        __syncwarp();
-    }
-    return nr;
-}
-
-// kahn_lifo over 16-bit lists in shared memory, by their shared-memory
-// addresses: the loop is a serial chain, so every instruction of it counts
-// (with generic pointers 425 cycles a node).
+// next. The node on top of the stack stays in a register. Both forms return the
+// number of ranks.
+//
+// Over 16-bit lists in shared memory, by their shared-memory addresses: every
+// instruction of the chain counts (with generic pointers 425 cycles a node, now
+// 315). ord takes the order from its start and the rest of the stack from its
+// end (never more than nn entries together).
 __device__ int kahn_lifo_shared(unsigned optr, unsigned adj, unsigned deg, unsigned ord, int nn, int sp, int lane) {
     int nr = 0, top = nn - sp, u = -1, k = 0, k1 = 0;
     const unsigned above = 0xfffffffeu << lane;  // the lanes above this one
@@ -835,55 +786,167 @@ __device__ int kahn_lifo_shared(unsigned optr, unsigned adj, unsigned deg, unsig
     return nr;
 }
 
-// Topological sort with the whole warp: out-lists as CSR (16 bits in shared
-// memory; 32 bits in the slot's view arrays for graphs that do not fit), the
-// Kahn loop on lane 0, ranks written in parallel, then hlen/tlen
+// Graphs whose lists outgrow the warp's shared memory. The chain is then the reads
+// from the slot, so a node's record holds what the next step needs, {first
+// successor | second << 16, list start | out-degree << 18}, and the records of all
+// successors are read with their in-degrees: one such read a node instead of the
+// list's ends and then the list. The in-degrees are in shared memory when a byte a
+// node fits (else in the slot, too); the first `cap` entries of the stack are,
+// the others in `far`. Ranks are stored as they come.
+//
+// 400 windows of 20 to 100 reads of 2,000 bp at 15 % error, 10,240 B a warp (graphs
+// of 3,000 to 8,000 nodes): sorts 291 M cycles a window, the kernel 3.85 s. Keeping
+// the order in shared memory too (3 bytes a node) and walking the linked lists
+// serially where that did not fit took 1,272 M and 5.02 s; the record fill's kernel
+// 622 M.
+__device__ __noinline__ int kahn_lifo_slot(const int2* rec, const int32_t* adj, uint8_t* deg, uint16_t* stk, int cap,
+                                           uint16_t* far, int sp, int32_t* rank_to_id, int32_t* rank, int lane) {
+    const unsigned below = (1u << lane) - 1u;
+    auto entry = [&](int p) { return p < cap ? stk + p : far + (p - cap); };
+    int nr = 0, u = -1;
+    int2 r = make_int2(0, 0);
+    while (true) {
+        if (u < 0) {
+            if (sp == 0) break;
+            sp--;
+            u = *entry(sp);
+            r = rec[u];
+        }
+        if (lane == 0) {
+            rank_to_id[nr] = u;
+            rank[u] = nr;
+        }
+        nr++;
+        const int d = (int)((unsigned)r.y >> 18), k0 = r.y & 0x3ffff;
+        int2 rn = r;
+        u = -1;
+        for (int c = 0; c < d; c += 32) {
+            const int k = c + lane;
+            const bool has = k < d;
+            int v = k == 0 ? r.x & 0xffff : (int)((unsigned)r.x >> 16), dv = 0;
+            int2 rv = make_int2(0, 0);
+            if (has) {
+                if (k > 1) v = adj[k0 + k];
+                rv = rec[v];
+                dv = deg[v] - 1;
+            }
+            const unsigned msk = __ballot_sync(0xffffffffu, has && dv == 0);
+            if (has) deg[v] = (uint8_t)dv;
+            if (msk) {
+                if (u >= 0) {  // ready in the chunk before (more than 32 out-edges)
+                    if (lane == 0) *entry(sp) = (uint16_t)u;
+                    sp++;
+                }
+                const int last = 31 - __clz(msk);
+                const unsigned rest = msk ^ (1u << last);
+                if ((rest >> lane) & 1u) *entry(sp + __popc(rest & below)) = (uint16_t)v;
+                sp += __popc(rest);
+                u = __shfl_sync(0xffffffffu, v, last);
+                rn.x = __shfl_sync(0xffffffffu, rv.x, last);
+                rn.y = __shfl_sync(0xffffffffu, rv.y, last);
+            }
+            __syncwarp();  // the counts and the stack, before another lane reads them
+        }
+        r = rn;
+    }
+    return nr;
+}
+
+// kahn_lifo_slot's inputs from the edge array, then its loop; -1 when a degree is beyond
+// its fields. Not inlined, and so the graph's pointers lie in local memory: with them in
+// registers the other phases spilled (240 ragged adaptive windows 57.1 ms, so 51.0;
+// 8,000 polishing windows 234 and 228).
+__device__ __noinline__ int topsort_slot(const DevGraph& g, int nn, int ne, uint16_t* sm, int sm_bytes, int lane) {
+    const int n_deg = (nn + 3) & ~3;
+    const bool near = n_deg + 512 <= sm_bytes;
+    uint8_t* deg = near ? (uint8_t*)sm : (uint8_t*)g.score;
+    uint16_t* stk = near ? (uint16_t*)((uint8_t*)sm + n_deg) : sm;
+    const int cap = (sm_bytes - (near ? n_deg : 0)) / 2;
+    uint16_t* far = (uint16_t*)g.stk;
+    int2* rec = (int2*)g.scratch8;
+    if (!scan_degrees(g, nn, g.csr_ptr, g.deg, deg, lane)) return -1;
+    __syncwarp();
+    fill_out_csr(g, ne, g.csr_adj, g.deg, lane);
+    int seeds = 0;
+    bool big = false;
+    for (int c0 = 0; c0 < nn; c0 += 32 * GU) {
+        int p[GU], d[GU], x[GU], y[GU];
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int u = c0 + 32 * q + lane;
+            p[q] = u < nn ? g.csr_ptr[u] : 0;
+            d[q] = u < nn ? g.csr_ptr[u + 1] - p[q] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            x[q] = d[q] > 0 ? g.csr_adj[p[q]] : 0;
+            y[q] = d[q] > 1 ? g.csr_adj[p[q] + 1] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < GU; q++) {
+            const int u = c0 + 32 * q + lane;
+            if (u < nn) rec[u] = make_int2(x[q] | (y[q] << 16), (int)((unsigned)p[q] | ((unsigned)d[q] << 18)));
+            big |= d[q] >= 1 << 14;
+            // zero in-degree seeds in id order, the last on top
+            const bool z = u < nn && deg[u] == 0;
+            const unsigned msk = __ballot_sync(0xffffffffu, z);
+            const int at = seeds + __popc(msk & ((1u << lane) - 1u));
+            if (z) *(at < cap ? stk + at : far + (at - cap)) = (uint16_t)u;
+            seeds += __popc(msk);
+        }
+    }
+    if (__any_sync(0xffffffffu, big)) return -1;
+    __syncwarp();
+    return kahn_lifo_slot(rec, g.csr_adj, deg, stk, cap, far, seeds, g.rank_to_id, g.rank, lane);
+}
+
+// Topological sort with the whole warp: out-lists as CSR from the edge array,
+// the Kahn loop over 16-bit lists in shared memory, or over records in the slot
+// for graphs that do not fit (about 9 bytes a node); then hlen/tlen
 // (src/graph.cpp:86-123) as depths in the heaviest-in-edge and
 // heaviest-out-edge forests by pointer jumping (shared memory when it fits).
-// Graphs beyond the shared-memory budget, or with an in-degree above 255, use
-// the sequential global-memory version.
+// Only graphs with an in-degree above 255 take the serial walk of the lists.
 __device__ void dg_topsort_warp(DevGraph& g, int nn, int ne, bool with_lens, uint16_t* sm, int sm_bytes, int lane) {
     auto up4 = [](size_t x) { return (x + 3) & ~(size_t)3; };
     const size_t n_ord = up4(2 * (size_t)nn), n_deg = up4((size_t)nn), n_ptr = up4(2 * ((size_t)nn + 1));
-    uint16_t* ord = sm;
-    uint8_t* deg = (uint8_t*)sm + n_ord;
-    uint16_t* optr = (uint16_t*)(deg + n_deg);
-    uint16_t* adj = (uint16_t*)((uint8_t*)optr + n_ptr);
-    const bool small = nn < 65535 && ne < 65535 && n_ord + n_deg + n_ptr + 2 * (size_t)ne <= (size_t)sm_bytes;
-    const bool large = !small && nn < 65535 && n_ord + n_deg <= (size_t)sm_bytes;
-    bool ok = small || large;
-    if (ok) {
-        if (small) ok = scan_degrees(g, nn, optr, ord, deg, lane);
-        else ok = scan_degrees(g, nn, g.csr_ptr, g.deg, deg, lane);
+    int nr;
+    if (nn < 65535 && ne < 65535 && n_ord + n_deg + n_ptr + 2 * (size_t)ne <= (size_t)sm_bytes) {
+        uint16_t* ord = sm;
+        uint8_t* deg = (uint8_t*)sm + n_ord;
+        uint16_t* optr = (uint16_t*)(deg + n_deg);
+        uint16_t* adj = (uint16_t*)((uint8_t*)optr + n_ptr);
+        nr = -1;
+        if (scan_degrees(g, nn, optr, ord, deg, lane)) {
+            __syncwarp();
+            fill_out_csr(g, ne, adj, ord, lane);
+            // zero in-degree seeds: the last in id order on top
+            int seeds = 0;
+            for (int c0 = 0; c0 < nn; c0 += 32) {
+                const int u = c0 + lane;
+                const bool z = u < nn && deg[u] == 0;
+                const unsigned msk = __ballot_sync(0xffffffffu, z);
+                if (z) ord[nn - 1 - seeds - __popc(msk & ((1u << lane) - 1u))] = (uint16_t)u;
+                seeds += __popc(msk);
+            }
+            __syncwarp();
+            auto sa = [](const void* p) { return (unsigned)__cvta_generic_to_shared(p); };
+            nr = kahn_lifo_shared(sa(optr), sa(adj), sa(deg), sa(ord), nn, seeds, lane);
+            __syncwarp();
+            for (int i = lane; i < nr; i += 32) {
+                const int u = ord[i];
+                g.rank_to_id[i] = u;
+                g.rank[u] = i;
+            }
+        }
+    } else {
+        nr = topsort_slot(g, nn, ne, sm, sm_bytes, lane);
     }
-    if (!ok) {
+    if (nr < 0) {
         if (lane == 0) g.hdr[3] = dg_topsort(g, nn, with_lens);
         __syncwarp();
         return;
     }
-    __syncwarp();
-    if (small) fill_out_csr(g, ne, adj, ord, lane);
-    else fill_out_csr(g, ne, g.csr_adj, g.deg, lane);
-    // zero in-degree seeds: the last in id order on top
-    int seeds = 0;
-    for (int c0 = 0; c0 < nn; c0 += 32) {
-        const int u = c0 + lane;
-        const bool z = u < nn && deg[u] == 0;
-        const unsigned msk = __ballot_sync(0xffffffffu, z);
-        if (z) ord[nn - 1 - seeds - __popc(msk & ((1u << lane) - 1u))] = (uint16_t)u;
-        seeds += __popc(msk);
-    }
-    __syncwarp();
-    auto sa = [](const void* p) { return (unsigned)__cvta_generic_to_shared(p); };
-    const int nr = small ? kahn_lifo_shared(sa(optr), sa(adj), sa(deg), sa(ord), nn, seeds, lane)
-                         : kahn_lifo(g.csr_ptr, g.csr_adj, deg, ord, nn, seeds, lane);
     if (lane == 0) g.hdr[3] = nr;
-    __syncwarp();
-    for (int i = lane; i < nr; i += 32) {
-        const int u = ord[i];
-        g.rank_to_id[i] = u;
-        g.rank[u] = i;
-    }
     __syncwarp();
     if (!with_lens) return;
     uint32_t* W = 4 * (size_t)nn <= (size_t)sm_bytes ? reinterpret_cast<uint32_t*>(sm) : reinterpret_cast<uint32_t*>(g.deg);
