@@ -1582,8 +1582,10 @@ void BatchEngine::run() {
     // cost order; its windows that outgrow their slot fall back to the sizing
     // below. Without one, a first pass with capacities estimated from the read
     // lengths. Windows that outgrow their slot (ST_CAPACITY / ST_OOM) are re-run
-    // with doubled capacities, up to three times.
+    // with doubled capacities, up to three times (default_caps), as long as the
+    // device's memory holds such slots.
     int first = 1;
+    bool fits = true;
     if (!plan_nodes_.empty()) {
         Caps c;
         c.NC = 64;
@@ -1593,11 +1595,12 @@ void BatchEngine::run() {
             c.cells = std::max(c.cells, plan_cells_[w]);
         }
         c.NC = std::min<int64_t>(c.NC, 60000);
-        launch(plan_order_.data(), n_windows_, c, PLAN_HEADROOM);
+        fits = launch(plan_order_.data(), n_windows_, c, PLAN_HEADROOM);
         first = 0;
     } else {
-        launch(order_.data(), n_windows_, default_caps(1));
+        fits = launch(order_.data(), n_windows_, default_caps(1));
     }
+    if (!fits) throw std::runtime_error("not enough device memory for one batch slot");
     for (int attempt = first ? 2 : 1; attempt <= 8; attempt *= 2) {
         cudaStream_t s = (cudaStream_t)stream_;
         char* h = (char*)h_out_;
@@ -1609,9 +1612,9 @@ void BatchEngine::run() {
         for (int w = 0; w < n_windows_; w++)
             if (st[w] == ST_CAPACITY || st[w] == ST_OOM) redo.push_back(w);
         if (redo.empty()) break;
+        if (!launch(redo.data(), (int32_t)redo.size(), default_caps(attempt))) break;  // they keep their status
         if (attempt == 1) stats.fallback = (int32_t)redo.size();
         else stats.retried += (int32_t)redo.size();
-        launch(redo.data(), (int32_t)redo.size(), default_caps(attempt));
     }
     cuda_check(cudaEventRecord((cudaEvent_t)evr1_, rs), "event");
     cuda_check(cudaEventSynchronize((cudaEvent_t)evr1_), "batch run");
@@ -1642,11 +1645,14 @@ BatchEngine::Caps BatchEngine::default_caps(int scale) const {
     Caps c;
     c.NC = (int32_t)std::max<int64_t>(NC64, 64);
     const int rb = ring_blocks();
-    const int tb_blocks = adaptive ? std::min(m / BLK + 2, (std::min(m / BLK + 2, (4 * wb) / BLK + 4)) * scale) : rb;
-    // static rows can be wider than tb_blocks where hlen and tlen disagree; adaptive rows of
-    // noisy reads widen past twice the initial band
-    c.cells = (int64_t)c.NC * tb_blocks * BLK;
-    c.cells = (adaptive ? c.cells * 3 / 2 : c.cells * std::min(scale, 2)) + 4096;
+    // rows of the band's width, more on retries: adaptive rows of noisy reads widen past twice
+    // the initial band; a static row spans the difference of hlen's and tlen's columns as well,
+    // the whole query at most (reads of 5 and 10 kb: 3.8 times the band)
+    const int full = m / BLK + 2;
+    const int64_t row = adaptive ? std::min(full, std::min(full, (4 * wb) / BLK + 4) * scale)
+                                 : scale >= 8 ? full : std::min(full, rb * scale);
+    c.cells = c.NC * row * BLK;
+    c.cells = (adaptive ? c.cells * 3 / 2 : c.cells) + 4096;
     return c;
 }
 
@@ -1683,7 +1689,7 @@ int BatchEngine::shared_per_warp(int32_t count, int warps, int sms) const {
     return std::max(smem_per_warp, std::min(share, 48 * 1024));
 }
 
-void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps, double headroom) {
+bool BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps, double headroom) {
     cudaStream_t s = (cudaStream_t)stream_;
     int sms = 0;
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "attr");
@@ -1777,7 +1783,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
             L = h > 1.0 ? planned(h) : L_planned;
         }
         const int64_t max_by_mem = (int64_t)(budget / (size_t)L.bytes) / warps;
-        if (max_by_mem < 1) throw std::runtime_error("not enough device memory for one batch slot");
+        if (max_by_mem < 1) return false;
         blocks = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, max_by_mem));
     }
     const int64_t slots = (int64_t)blocks * warps;
@@ -1866,6 +1872,7 @@ void BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     cuda_check(cudaEventElapsedTime(&ms, (cudaEvent_t)ev0_, (cudaEvent_t)ev1_), "elapsed");
     stats.kernel_ms += ms;
     stats.launches++;
+    return true;
 }
 
 void BatchEngine::sync_stats() {

@@ -110,8 +110,9 @@ class BatchEngine {
     int shared_per_warp(int32_t count, int warps, int sms) const;
     int ring_blocks() const;
     // one persistent launch over `count` windows (ids) with slots of the given
-    // capacities, grown by up to `headroom` when memory allows every resident warp one
-    void launch(const int32_t* windows, int32_t count, const Caps& caps, double headroom = 1.0);
+    // capacities, grown by up to `headroom` when memory allows every resident warp one;
+    // false, and nothing launched, when the device's memory does not hold one block's slots
+    bool launch(const int32_t* windows, int32_t count, const Caps& caps, double headroom = 1.0);
     static constexpr double PLAN_HEADROOM = 1.5;
     Proposer* proposer_ = nullptr;
     void* kgraph_exec_ = nullptr;      // the launch as a CUDA graph, and the launch it was recorded for
