@@ -1748,9 +1748,10 @@ bool BatchEngine::launch(const int32_t* windows, int32_t count, const Caps& caps
     while (state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) + qn_bytes > smem_w) state_rows /= 2;
     if (WED * 16 + warp_state_bytes(state_rows) + qn_bytes > smem_w)
         for (state_rows = 128; state_rows > 32 && WED * 16 + warp_state_bytes(state_rows) > smem_w;) state_rows /= 2;
-    // read statistics count spilled rows against a ring of 32 full-width rows (dynamic bands) or
-    // of up to 8 rows of 64 bytes a block in the warp's shared memory (static band)
-    int stat_rows = stat ? std::min(8, (smem_w - qsm_bytes - kStageBytes) / std::max(1, ring_blocks * 64)) : 32;
+    // read statistics count the rows that would leave a ring of recent rows: 32 full-width ones
+    // (dynamic bands), or up to 8 of 64 bytes a block in the configured shared memory (static
+    // band) whatever this launch uses, so that a window's numbers do not depend on its batch
+    int stat_rows = stat ? std::min(8, (smem_per_warp - qsm_bytes - kStageBytes) / std::max(1, ring_blocks * 64)) : 32;
     if (stat_rows < 2) stat_rows = 0;
     int occ = 0;
     // windows that leave two blocks to an SM run the build with twice the registers
