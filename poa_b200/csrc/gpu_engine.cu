@@ -81,12 +81,20 @@ void launch_team(int njobs, const TeamJob* d_jobs, cudaStream_t s) {
 }
 
 // One warp per 128 columns of the widest row, up to 16 (rows beyond that take
-// laps).
+// laps, with every predecessor from the row store). Measured against the record
+// fill, which took 4,096 columns at a time: three static reads of 45 kb 298 -> 210
+// ms, of 60 kb 552 -> 294; full band, reads of 2.5 kb 46 -> 32, of 5 kb 110 -> 60;
+// wide cells, full band, 1.2 kb 12.7 -> 6.2, 2.5 kb 36.1 -> 33.2 (39.5 with 8 warps at
+// most), 5 kb 109 -> 77; static wide, 30 kb 164 -> 80.
 void launch_teams(bool adaptive, bool wide, int cols, int njobs, const TeamJob* d, cudaStream_t s) {
     const int strips = (cols + STRIP - 1) / STRIP;
-    if (wide) {
-        if (adaptive) launch_team<8, true, true>(njobs, d, s);
-        else launch_team<8, false, true>(njobs, d, s);
+    if (wide && adaptive) {
+        launch_team<8, true, true>(njobs, d, s);
+    } else if (wide) {
+        // (8 bytes a cell: 16 warps keep 8 rows in shared memory, 8 or 12 warps 16)
+        if (strips <= 8) launch_team<8, false, true>(njobs, d, s);
+        else if (strips <= 12) launch_team<12, false, true>(njobs, d, s);
+        else launch_team<16, false, true>(njobs, d, s);
     } else if (adaptive) {
         if (strips <= 2) launch_team<2, true, false>(njobs, d, s);
         else if (strips <= 4) launch_team<4, true, false>(njobs, d, s);

@@ -288,7 +288,7 @@ struct TeamSmem {
     static constexpr int ROWB = 32 * W * CELLB;
     // rows of the ring (a power of two): noisy graphs have predecessors tens of rows back, and
     // one read from the row store costs as much as a row
-    static constexpr int TR = ROWB * 64 <= RING_MAX ? 64 : ROWB * 32 <= RING_MAX ? 32 : 16;
+    static constexpr int TR = ROWB * 64 <= RING_MAX ? 64 : ROWB * 32 <= RING_MAX ? 32 : ROWB * 16 <= RING_MAX ? 16 : 8;
     static constexpr int RING = TR * ROWB;
     static constexpr int PUB = RING;                               // int4 [2][W]
     static constexpr int BEST = PUB + 2 * W * 16;                  // int4 [2][W]

@@ -41,3 +41,34 @@ def test_rows_around_the_teams_columns(scores, warps, b, oracle_bin, tmp_path):
     with poa_b200.Context(poa_b200.Params.from_cli(opts)) as ctx:
         got, _ = ctx.run(reads, fasta.headers(str(fa)))
     assert got == want
+
+
+def _check(reads, opts, oracle_bin, tmp_path):
+    fa = tmp_path / "in.fa"
+    synth.write_fasta(str(fa), reads)
+    want = subprocess.run([oracle_bin, str(fa)] + opts, capture_output=True, check=True, timeout=600).stdout
+    with poa_b200.Context(poa_b200.Params.from_cli(opts)) as ctx:
+        got, _ = ctx.run(reads, fasta.headers(str(fa)))
+    assert got == want
+
+
+# wide cells: teams of 8, 12 and 16 warps, and rows of two laps
+@pytest.mark.parametrize("band", [["-f", "0"], ["-b", "2000"], ["-B", "-b", "60"], ["-B", "-b", "400"]],
+                         ids=["full", "whole", "adaptive", "adaptive_b400"])
+@pytest.mark.parametrize("length", [1016, 1030, 1528, 1540, 2040, 2056, 2600])
+def test_wide_team_widths(length, band, oracle_bin, tmp_path):
+    rng = np.random.default_rng(length)
+    t = synth.random_root(rng, length)
+    reads = [synth.to_ascii(r) for r in synth.mutate(rng, t, 3, 0.04, 0.02, 0.02)]
+    # predecessors up to 40 rows back, beyond the rows kept in shared memory
+    reads += [reads[0][:400] + reads[0][400 + k:] for k in (6, 7, 8, 9, 15, 16, 17, 40)]
+    _check(reads, band + ["-r", "1"] + BIG, oracle_bin, tmp_path)
+
+
+def test_wide_rows_around_sixteen_strips(oracle_bin, tmp_path):
+    rng = np.random.default_rng(16)
+    t = synth.random_root(rng, 3000)
+    reads = [synth.to_ascii(r) for r in synth.mutate(rng, t, 4, 0.03, 0.01, 0.01)]
+    s = _strips(3000, 925)
+    assert sum(x <= 16 < y for x, y in zip(s, s[1:])) >= 5
+    _check(reads, ["-b", "925", "-r", "1"] + BIG, oracle_bin, tmp_path)
