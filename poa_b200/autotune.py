@@ -5,7 +5,7 @@
 
 Needs a GPU. For one workload it times the persistent batch kernel under each
 candidate launch shape (the knobs of ``poa_batch_config``: blocks per SM,
-i.e. the 168-, 128- or 96-register build, and shared memory per warp, which
+i.e. the 168- or 128-register build, and shared memory per warp, which
 trades the static-band row ring and staging against L1 capacity) on a seeded
 sample of the workload's windows, and records the fastest shape, with every
 measurement, in a JSON file that ``bench.py`` and ``Context.batch_autotuned``

@@ -1454,8 +1454,9 @@ TeamKernel team_kernel(int cols) {
 }
 BatchKernel batch_kernel(bool stat, bool wide, int blocks_per_sm) {
     if (wide) return stat ? (BatchKernel)k_batch<4, true, true, 3> : (BatchKernel)k_batch<4, false, true, 3>;
-    if (blocks_per_sm >= 5) return stat ? (BatchKernel)k_batch<4, true, false, 5> : (BatchKernel)k_batch<4, false, false, 5>;
     if (blocks_per_sm <= 2 && !stat) return (BatchKernel)k_batch<4, false, false, 2>;  // two chunks of a row at a time
+    // 128 registers also where more blocks were asked for: a build of 96 for 5 spilled (6 KB a
+    // warp, 5 blocks against 4: 8,000 static windows 107 and 97 ms, 3,000 adaptive 140 and 104)
     if (blocks_per_sm >= 4) return stat ? (BatchKernel)k_batch<4, true, false, 4> : (BatchKernel)k_batch<4, false, false, 4>;
     return stat ? (BatchKernel)k_batch<4, true, false, 3> : (BatchKernel)k_batch<4, false, false, 3>;
 }

@@ -93,7 +93,7 @@ class BatchEngine {
     void read_stats(std::vector<int32_t>& out);
     BatchStats stats;
     int32_t warps_per_block = 4;
-    int32_t blocks_per_sm = 3;  // 3: 168-register build; 4: 128; >= 5: 96 (occupancy still caps it)
+    int32_t blocks_per_sm = 3;  // up to 3: 168-register build (adaptive up to 2: 255); from 4: 128 (occupancy still caps it)
     int32_t smem_per_warp = 18432;  // shared-memory row ring + staging / topsort workspace per warp
     bool blocks_set = false;        // blocks_per_sm was configured: used as it is
     bool smem_set = false;          // smem_per_warp was configured: used as it is
