@@ -287,7 +287,8 @@ __device__ int dg_consensus(DevGraph& g, int nn, char* out, int cap) {
 // which starts at the source, reaches every node: where the source is the only
 // node without in-edges. Other graphs (a negative match score makes them) and
 // those that do not settle in 12 rounds take the serial walk.
-//  pre: chosen edge per node; W: {ancestor, score up to it} words, 8 bytes a node.
+//  pre: chosen edge per node; W: ancestor (low half) and score up to it, one 64-bit word a
+//  node, so that a word read while its lane changes it is one pair or the other.
 __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap, unsigned char* sm, int sm_bytes, int lane) {
     constexpr int CU = 4;
     if (nn <= 2) {
@@ -295,10 +296,14 @@ __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap
         if (lane == 0) len = dg_consensus(g, nn, out, cap);
         return __shfl_sync(0xffffffffu, len, 0);
     }
-    // int2 per node; a slot's deg and stk arrays are not contiguous, so large graphs use the row arrays
-    int2* W = 8 * (size_t)nn <= (size_t)sm_bytes ? reinterpret_cast<int2*>(sm) : reinterpret_cast<int2*>(g.scratch8);
+    // (a slot's deg and stk arrays are not contiguous, so large graphs use the row arrays)
+    typedef unsigned long long u64;
+    u64* W = 8 * (size_t)nn <= (size_t)sm_bytes ? reinterpret_cast<u64*>(sm) : reinterpret_cast<u64*>(g.scratch8);
+    auto word = [](int anc, int score) { return (u64)(uint32_t)score << 32 | (uint32_t)anc; };
+    auto anc_of = [](u64 w) { return (int)(uint32_t)w; };
+    auto score_of = [](u64 w) { return (uint32_t)(w >> 32); };
     int32_t* pre = g.pre;
-    unsigned long long* key = reinterpret_cast<unsigned long long*>(g.scratch8b);
+    u64* key = reinterpret_cast<u64*>(g.scratch8b);
     int32_t* ties = g.csr_adj;
     bool unreached = false;
     for (int u = lane; u < nn; u += 32) {
@@ -342,21 +347,21 @@ __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap
             }
 #pragma unroll
             for (int q = 0; q < CU; q++)
-                if (u0 + 32 * q < nn) W[u0 + 32 * q] = make_int2(f[q], w[q]);
+                if (u0 + 32 * q < nn) W[u0 + 32 * q] = word(f[q], w[q]);
         }
         __syncwarp();
         for (int it = 0; it < 40; it++) {
             bool moved = false;
             for (int u0 = lane; u0 < nn; u0 += 32 * CU) {
-                int2 x[CU], a[CU];
+                u64 x[CU], a[CU];
 #pragma unroll
-                for (int q = 0; q < CU; q++) x[q] = u0 + 32 * q < nn ? W[u0 + 32 * q] : make_int2(-1, 0);
+                for (int q = 0; q < CU; q++) x[q] = u0 + 32 * q < nn ? W[u0 + 32 * q] : word(-1, 0);
 #pragma unroll
-                for (int q = 0; q < CU; q++) a[q] = x[q].x >= 0 ? W[x[q].x] : make_int2(-1, 0);
+                for (int q = 0; q < CU; q++) a[q] = anc_of(x[q]) >= 0 ? W[anc_of(x[q])] : word(-1, 0);
 #pragma unroll
                 for (int q = 0; q < CU; q++)
-                    if (x[q].x >= 0) {
-                        W[u0 + 32 * q] = make_int2(a[q].x, a[q].y + x[q].y);
+                    if (anc_of(x[q]) >= 0) {
+                        W[u0 + 32 * q] = word(anc_of(a[q]), (int)(score_of(a[q]) + score_of(x[q])));
                         moved = true;
                     }
             }
@@ -367,12 +372,12 @@ __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap
         bool changed = false;
         for (int t = lane; t < nt; t += 32) {
             const int v = g.e_to[ties[t]], h = g.hin[v];
-            key[v] = ((unsigned long long)(uint32_t)W[g.e_from[h]].y << 32) | (uint32_t)(0x7fffffff - h);
+            key[v] = (u64)score_of(W[g.e_from[h]]) << 32 | (uint32_t)(0x7fffffff - h);
         }
         __syncwarp();
         for (int t = lane; t < nt; t += 32) {
             const int e = ties[t];
-            atomicMax(&key[g.e_to[e]], ((unsigned long long)(uint32_t)W[g.e_from[e]].y << 32) | (uint32_t)(0x7fffffff - e));
+            atomicMax(&key[g.e_to[e]], (u64)score_of(W[g.e_from[e]]) << 32 | (uint32_t)(0x7fffffff - e));
         }
         __syncwarp();
         for (int t = lane; t < nt; t += 32) {
@@ -399,12 +404,12 @@ __device__ int dg_consensus_warp(DevGraph& g, int nn, int ne, char* out, int cap
         for (int q = 0; q < CU; q++) e[q] = u0 + 32 * q < nn ? pre[u0 + 32 * q] : -1;
 #pragma unroll
         for (int q = 0; q < CU; q++)
-            if (u0 + 32 * q < nn) W[u0 + 32 * q].x = e[q] >= 0 ? g.e_from[e[q]] : 0;
+            if (u0 + 32 * q < nn) W[u0 + 32 * q] = word(e[q] >= 0 ? g.e_from[e[q]] : 0, 0);
     }
     __syncwarp();
     int32_t* path = g.stk;
     if (lane == 0)
-        for (int id = W[1].x; id != 0; id = W[id].x) path[len++] = id;
+        for (int id = anc_of(W[1]); id != 0; id = anc_of(W[id])) path[len++] = id;
     len = __shfl_sync(0xffffffffu, len, 0);
     __syncwarp();
     if (len > cap) return -1;
