@@ -165,14 +165,7 @@ void GpuEngine::align_many(const std::vector<const HostWindow*>& wins, const std
     // one launch runs one kind of band
     bool any_adaptive = false, any_static = false;
     for (int t = 0; t < J; t++) (p.f > 0 && abs[t] ? any_adaptive : any_static) = true;
-    if (any_adaptive && any_static) {
-        for (int t = 0; t < J; t++) {
-            std::vector<AlignOut> one;
-            align_many({wins[t]}, {qs[t]}, {qlens[t]}, {abs[t]}, p, one);
-            outs[t] = one[0];
-        }
-        return;
-    }
+    if (any_adaptive && any_static) throw std::invalid_argument("align_many: one kind of band a call");
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     cudaStream_t s = (cudaStream_t)stream_;
     const Scoring sc = scoring_of(p);

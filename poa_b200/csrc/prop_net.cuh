@@ -62,7 +62,7 @@ struct Smem {
     bf16 w4[CH * SW4], w5[OUT * SW4];
     float b[4 * CH + OUT];
     float h[RT * CH], z[RT * CH], dz[RT * CH];
-    float o[RT * OUT], d[RT * OUT];
+    float d[RT * OUT];
     float red[THREADS];
 };
 

@@ -106,7 +106,7 @@ class Proposer {
     std::vector<float> host_w_;
     // device parameters
     float* d_w_ = nullptr;        // FP32 master
-    uint16_t* d_wb_ = nullptr;    // BF16 copy (GEMM operands)
+    uint16_t* d_wb_ = nullptr;    // BF16 copy (the network's weights)
     float* d_g_ = nullptr;        // gradients, then the loss
     float* d_m_ = nullptr;        // Adam first moment
     float* d_v_ = nullptr;        // Adam second moment
