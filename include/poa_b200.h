@@ -166,7 +166,8 @@ int poa_batch_stats(poa_ctx* ctx, int64_t* out19);
  * traceback record bytes and spilled row-store entries (int32) of its
  * largest alignment, and a relative cost; typically a band proposer's
  * prediction from poa_batch_read_stats-style targets. The plan sizes the
- * device slots and orders the windows (largest cost first); it never changes
+ * device slots (by the nodes, and the record bytes as a bound of the band
+ * cells) and orders the windows (largest cost first); it never changes
  * a band, so results are the same with or without it. A window that
  * outgrows its slot is re-run with the default sizing. nodes == NULL clears
  * the plan; poa_batch_upload clears it too. */
@@ -181,8 +182,9 @@ int poa_batch_plan_get(poa_ctx* ctx, int32_t* nodes, int64_t* tb_bytes, int64_t*
 /* Per read of the last run, 8 values each (n_reads * 8 entries): widest DP
  * row in 8-column blocks, band cells, DP rows, graph nodes after fusing the
  * read, traceback record bytes, spilled row-store entries (int32), graph
- * edges after fusing the read, 0. A window's first read has no DP: its DP
- * values are zero. These are the band statistics the band proposer learns. */
+ * edges after fusing the read, mean band centre in thousandths of the query
+ * length. A window's first read has no DP: its DP values are zero. These are
+ * the band statistics the band proposer learns. */
 int poa_batch_read_stats(poa_ctx* ctx, int32_t* out, int64_t cap);
 
 /* One poa() alignment on inputs already in device memory, without

@@ -302,7 +302,8 @@ class Context:
 
     def batch_read_stats(self):
         """int32 array [n_reads, 8] of the last run: widest row (blocks), cells, rows,
-        nodes after fusion, record bytes, spilled row-store entries, edges after fusion, 0."""
+        nodes after fusion, record bytes, spilled row-store entries, edges after fusion,
+        mean band centre in thousandths of the query length."""
         import numpy as np
         n = int(self._keep[2].shape[0]) if getattr(self, "_keep", None) is not None else 0
         out = np.zeros((max(n, 1), 8), dtype=np.int32)

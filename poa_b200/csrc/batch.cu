@@ -7,11 +7,12 @@
 // its endpoints, weight and the next links of both lists. One warp runs a
 // window: fusion (src/graph.cpp:170-235) is warp-parallel with stamp-based
 // conflict detection and a sequential fallback (dg_fuse_warp / dg_fuse_seq);
-// the LIFO topological sort (src/graph.cpp:21-128) runs its Kahn loop over a
-// shared-memory CSR copy, with hlen/tlen as depths by pointer jumping over the
-// warp; the DP rows (build_rows), the fill (warp.cuh) and the backtrack
-// (team.cuh) use the whole warp; the consensus (src/graph.cpp:294-351) is the
-// reference's sequential walk, run by lane 0.
+// the LIFO topological sort (src/graph.cpp:21-128) runs its Kahn loop with the
+// whole warp over a CSR copy, in shared memory when it fits, with hlen/tlen as
+// depths by pointer jumping; the DP rows (build_rows), the fill (warp.cuh) and
+// the backtrack (team.cuh) use the whole warp; so does the consensus
+// (src/graph.cpp:294-351), except on graphs where it takes the reference's
+// sequential walk on lane 0 (dg_consensus_warp).
 //
 // The graph steps are bound by the latency of dependent reads from a slot, so
 // they go over the edge array, not over the nodes' lists (coalesced, and a
@@ -613,7 +614,10 @@ constexpr int GU = 4;  // chunks of 32 taken together
 // array already holds at their rank (the reference resizes the vector and
 // never writes there), except the sink, whose tlen is 1. Written back by rank.
 // Pointer jumping in place: a word holds (ancestor, distance to it), 16 bits
-// each, so a word read while others change is a valid pair all the same.
+// each, so a word read while others change is a valid pair all the same. A root's
+// value cannot carry into the ancestor: hlen at rank r never exceeds r and tlen
+// never N - r, whatever an earlier sort left there (a child's rank lies beyond its
+// parent's, and N only grows), and N is at most 60,000.
 __device__ void depth_jump(DevGraph& g, int nn, int pass, int32_t* arr, uint32_t* W, int lane) {
     constexpr uint32_t NONE = 0xffffu;
     const int32_t* heavy = pass == 0 ? g.hin : g.hout;

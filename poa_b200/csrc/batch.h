@@ -1,8 +1,8 @@
 // batch.h - the batched window engine: thousands of independent POA windows
-// (one read set -> one consensus each) in one persistent launch. Each warp
-// owns a slot of device memory holding one window's graph and DP buffers
-// and runs minipoa's whole per-window loop on the device: align the read
-// (the same DP fill as the plain kernel, on a warp), fuse the path into the
+// (one read set -> one consensus each) in one persistent launch. Each warp (or
+// team of warps) owns a slot of device memory holding one window's graph and DP
+// buffers and runs minipoa's whole per-window loop on the device: align the read
+// (the value fill of team.cuh, on a warp or a team), fuse the path into the
 // graph, re-sort it, next read; then the heaviest-path consensus.
 #pragma once
 #include <stdint.h>
@@ -71,12 +71,13 @@ class BatchEngine {
     // Resource plan of the uploaded windows (a band proposer's prediction), one
     // value per window: graph nodes, traceback record bytes and spilled
     // row-store entries of its largest alignment, and a relative cost (the
-    // windows run largest first). The plan sizes the slots only; every DP
-    // still runs the reference's band, and a window that outgrows its slot is
-    // re-run with the default sizing (counted in stats.fallback). nullptr
-    // clears the plan. Cleared by upload().
-    // cells: band cells of the largest alignment, nullptr when the plan has
-    // none (its record bytes bound them).
+    // windows run largest first). Nodes and cells size the slots, nothing else;
+    // every DP still runs the reference's band, and a window that outgrows its
+    // slot is re-run with the default sizing (counted in stats.fallback).
+    // nullptr clears the plan. Cleared by upload().
+    // cells: band cells of the largest alignment; nullptr when the plan has none:
+    // its record bytes, at least one a cell, bound them. tb_bytes has no other
+    // use, and spill is kept for plan_spill() alone.
     void set_plan(const int32_t* nodes, const int64_t* tb_bytes, const int64_t* spill, const float* cost,
                   const int64_t* cells = nullptr);
     DeviceWindows device_windows() const;
@@ -86,7 +87,9 @@ class BatchEngine {
     void sync_stats();
     // Per read of the last run(), NRSTAT values: [0] widest DP row in blocks,
     // [1] band cells, [2] DP rows, [3] graph nodes after fusing the read,
-    // [4] traceback record bytes, [5] spilled row-store entries (int32),
+    // [4] traceback record bytes (1 a cell, 4 in rows with several predecessors),
+    // [5] row-store entries (int32) of rows beyond a ring of recent rows whose size
+    // does not depend on the launch (both are what the band proposer learns),
     // [6] graph edges after fusing the read, [7] mean band centre (midpoint
     // column over the DP rows) in thousandths of the query length. A window's
     // first read has no DP ([0..2], [4], [5], [7] zero).

@@ -14,8 +14,8 @@
 //             another read of the window, and the mean anchor multiplicity,
 //             plus read length, first-read length, read index and read count.
 //   network   3 x Conv1d(k=3, 64 channels, ReLU) over 32 bins -> mean pool ->
-//             Linear(64,64)+ReLU -> Linear(64,4). BF16 weights and activations
-//             as GEMM operands, FP32 accumulation, FP32 master weights (Adam).
+//             Linear(64,64)+ReLU -> Linear(64,4). BF16 weights and activations,
+//             FP32 accumulation, FP32 master weights (Adam).
 //   outputs   per read: new graph nodes per query base, mean band width as a
 //             fraction of the query (band cells / (rows * m)), traceback bytes
 //             per cell, mean band centre as a fraction of the query.

@@ -23,8 +23,8 @@
 // Team. Columns are cut into strips of 128; strip s belongs to warp s % W, one
 // thread per 4 cells (half a block). A thread meets the same columns in every
 // row, so predecessor cells come back from the thread's own words in a
-// shared-memory ring of the last TR rows (16 or 32; 16 bytes per thread, no bank
-// conflicts) or, for rows further back, from the row store, and only the cell
+// shared-memory ring of the last TR rows (8 to 64, as many as fit; 16 bytes per
+// thread, no bank conflicts) or, for rows further back, from the row store, and only the cell
 // left of a strip crosses warps. Per row: predecessor pass, warp prefix
 // maximum of the horizontal-gap keys, ONE barrier to exchange the warps'
 // maxima, finalise, store. The left neighbour's last cell is derived from its
@@ -41,10 +41,10 @@
 // so a row with no other predecessor reads no cells at all.
 //
 // Measured on a B200, DP kernels of one run, record fill -> this one: 10 reads
-// of 16,569 bp, static band, 346 -> 132 ms (fill ~1,350 cycles per row of ~1,050
-// cells, backtrack 325 cycles per move); 24 reads of 443 bp 31 -> 11.6 ms; 10
-// reads of 5 kb at 10 % error, adaptive band, 308 -> 107 ms; 840 seeded
-// sub-windows 94 -> 33 ms. What is left is latency: ~215 mostly dependent
+// of 16,569 bp, static band, 346 -> 125 ms (fill ~1,350 cycles per row of ~1,050
+// cells, backtrack 325 cycles per move); 24 reads of 443 bp 31 -> 11 ms; 10
+// reads of 5 kb at 10 % error, adaptive band, 308 -> 92 ms; 840 seeded
+// sub-windows 94 -> 27 ms. What is left is latency: ~215 mostly dependent
 // instructions per warp and row.
 #pragma once
 #include <type_traits>

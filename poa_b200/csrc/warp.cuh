@@ -11,10 +11,12 @@
 // bank conflicts). With the dynamic bands the ring is a circular buffer of blocks
 // that holds as many of the last rows as fit, whatever their width.
 //
-// Measured on a B200 against the record fill it replaced (kernel time):
-// 8,000 polishing windows 651 -> 339 ms, 1,024 windows of 2,000 bp at 15 %
-// error with the adaptive band 1,118 -> 507 ms, one window of 64 reads 282 ->
-// 131 ms. The fill's share of the polishing kernel fell from 62 % to 34 %.
+// Measured on a B200 against the record fill it replaced (kernel time, with the
+// graph steps of batch.cu): 8,000 polishing windows 651 -> 207 ms, 1,024 windows of
+// 2,000 bp at 15 % error with the adaptive band 1,118 -> 349 ms, one window of 64
+// reads 282 -> 94 ms. What is left is latency: of 3.9 cycles an instruction of a
+// lone warp (adaptive band) 1.5 wait for an earlier instruction, 0.65 for global and
+// 0.36 for shared memory; static band 4.9, 1.8, 1.05 and 0.63.
 #pragma once
 #include "team.cuh"
 
